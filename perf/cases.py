@@ -50,14 +50,14 @@ def listed():
         # an in-situ run: one timestep at a time, tracks so far at the end
         dict(name="stream3d", kind="stream", dims="96,101,88", nt=8, f64=False, separate=False, scalar=False,
              classify=False, refined=False, host=False, blobs=32, lo=4.0, hi=12.0, scale=1.0, noise=0.0),
-        # the served unstructured stream: 100 x 100 plane x 40 layers of tets
-        dict(name="extruded_stream", kind="extruded", nx=100, ny=100, layers=40, nt=6, f64=False, stream=True,
+        # the served unstructured stream: 100 x 100 plane x 40 layers of tets, 16 timesteps
+        dict(name="extruded_stream", kind="extruded", nx=100, ny=100, layers=40, nt=16, f64=False, stream=True,
              blobs=48, lo=3.0, hi=9.0),
         # a one-shot extraction on a smaller unstructured tet mesh, double
         dict(name="extruded_once", kind="extruded", nx=61, ny=47, layers=23, nt=5, f64=True, stream=False,
              blobs=24, lo=3.0, hi=9.0),
         # a moving iso-surface of a 3D scalar
-        dict(name="contour3d", kind="contour", dims="96,96,96", nt=12, f64=True, threshold=0.125, blobs=32,
+        dict(name="contour3d", kind="contour", dims="96,96,96", nt=6, f64=True, threshold=0.125, blobs=32,
              lo=4.0, hi=12.0),
         # points where two 2D scalars meet their thresholds, float, odd sizes
         dict(name="fiber2d", kind="fiber", dims="401,323", nt=16, f64=False, threshold=0.0625, blobs=32, lo=8.0,
@@ -100,10 +100,10 @@ def draw(rng):
         return dict(kind=kind, n=_log(rng, 4, 128), spec=rng.randint(1, 9999), f64=f64)
     if kind == "extruded":
         return dict(kind=kind, nx=_log(rng, 16, 100), ny=_log(rng, 16, 100), layers=_log(rng, 4, 40),
-                    nt=rng.randint(2, 6), f64=f64, stream=rng.random() < 0.5, blobs=blobs, lo=3.0, hi=9.0)
+                    nt=rng.randint(2, 12), f64=f64, stream=rng.random() < 0.5, blobs=blobs, lo=3.0, hi=9.0)
     nt = rng.randint(2, 16)
     threshold = rng.choice([0.0, 0.0625, 0.125, 0.25])
-    most = 1_000_000 if threshold == 0.0 and kind == "contour" else 8_000_000 if kind == "contour" else 6_000_000
+    most = 5_000_000 if kind == "contour" else 6_000_000
     return dict(kind=kind, dims=_sides(rng, d, 24 if d == 2 else 12, 512 if d == 2 else 128, nt, most), nt=nt, f64=f64,
                 threshold=threshold, blobs=blobs, lo=4.0, hi=16.0)
 
@@ -236,7 +236,7 @@ def _rows(case):
         return 1 << 16
     nv = math.prod(_dims(case)) * case["nt"]
     if case["kind"] in ("contour", "fiber"):
-        return max(1 << 14, nv * 3 // 4 if case["threshold"] == 0.0 else nv // 4)
+        return max(1 << 14, nv if case["kind"] == "contour" else nv // 4)
     return max(1 << 14, min(nv // 8, 1 << 18))
 
 
@@ -267,7 +267,7 @@ class Out(dict):
         n = _rows(self.case)
         if self.case["kind"] == "batch":  # raveled rows of up to four values
             n *= 4
-        return _pad(a, n * {"cells": 8, "edges": 2}.get(name, 1))
+        return _pad(a, n * {"cells": 7, "edges": 2}.get(name, 1))
 
 
 def _out(case, r):
@@ -308,9 +308,9 @@ def work(case):
     nv = math.prod(d) * case["nt"]
     if case["kind"] == "contour":
         # a crossing edge is 52 bytes (ids, barycentrics, track, value), a cell
-        # 4 bytes a vertex; the zero level runs through the flat far field too
-        feat = 0.27 if case["threshold"] == 0.0 else 0.05
-        cells = feat * (6 if len(d) == 3 else 2)
+        # 4 bytes a vertex
+        feat = 0.25
+        cells = feat * (5.7 if len(d) == 3 else 2)
         return {"bytes": int(nv * (es + feat * 52 + cells * 4 * (len(d) + 1))), "flops": 0}
     if case["kind"] == "fiber":
         return {"bytes": nv * 2 * es, "flops": 0}
