@@ -51,6 +51,35 @@ cudaError_t DevBuf::ensure(size_t want) {
   return cudaSuccess;
 }
 
+cudaError_t PinBuf::alloc(size_t want) {
+  constexpr size_t kPage = 4096;
+  const size_t n = (want + kPage - 1) / kPage * kPage;
+  void* p = nullptr;
+  if (posix_memalign(&p, kPage, n) != 0) return cudaErrorMemoryAllocation;
+  cudaError_t e = cudaHostRegister(p, n, cudaHostRegisterMapped);
+  if (!e) {
+    e = cudaHostGetDevicePointer(&d, p, 0);
+    if (e) cudaHostUnregister(p);
+  }
+  if (e) {
+    free(p);
+    d = nullptr;
+    cudaGetLastError();
+    return e;
+  }
+  h = p;
+  bytes = n;
+  return cudaSuccess;
+}
+
+void PinBuf::release() {
+  if (!h) return;
+  cudaHostUnregister(h);
+  free(h);
+  h = d = nullptr;
+  bytes = 0;
+}
+
 void DevBuf::release() {
   if (p) {
     if (st) cudaFreeAsync(p, st);
@@ -122,10 +151,11 @@ extern "C" ftk2b_status ftk2b_ctx_create(int device, ftk2b_ctx** out) {
     delete ctx;
     return FTK2B_CUDA_ERROR;
   }
-  if (cudaMallocHost((void**)&ctx->h_counters, sizeof(unsigned) * kNumCounters) != cudaSuccess) {
+  if (ctx->pin.alloc((size_t(1) << 20) + 256) != cudaSuccess) {
     delete ctx;
     return FTK2B_OOM;
   }
+  ctx->h_counters = (unsigned*)ctx->pin.h;
   for (DevBuf* b : ctx->all_bufs()) b->st = ctx->stream;
   cudaDeviceProp prop;
   cudaGetDeviceProperties(&prop, device);
@@ -160,7 +190,8 @@ extern "C" void ftk2b_ctx_destroy(ftk2b_ctx* ctx) {
   ctx->release_all();
   cudaStreamSynchronize(ctx->stream);
   ctx->drop_graphs();
-  if (ctx->h_counters) cudaFreeHost(ctx->h_counters);
+  ctx->pin.release();
+  ctx->pin_big.release();
   for (int i = 0; i < 2; ++i) {
     if (ctx->d2h_pin[i]) cudaFreeHost(ctx->d2h_pin[i]);
     if (ctx->d2h_ev[i]) cudaEventDestroy(ctx->d2h_ev[i]);
@@ -247,6 +278,40 @@ extern "C" ftk2b_status ftk2b_ctx_get_option(ftk2b_ctx* ctx, int option, int64_t
     case FTK2B_OPT_TEST_STALL_POLLS: *value = ctx->stall_polls; return FTK2B_OK;
     default: return fail(ctx, FTK2B_INVALID_ARG, "unknown option %d", option);
   }
+}
+
+// Blocks above the context's own grow by replacement (no kernel in flight
+// writes to the old one: every call waits for its own).
+cudaError_t ftk2b_ctx::ensure_pack_pin(size_t want) {
+  if (pack_bytes() >= want) return cudaSuccess;
+  size_t n = size_t(2) << 20;
+  while (n < want) n *= 2;
+  pin_big.release();
+  return pin_big.alloc(n);
+}
+
+// The canonical-order buffers of a run as the pack kernel reads them.
+PackArgs ftk2b_ctx::pack_args(const LastRun& r) {
+  PackArgs a;
+  memset(&a, 0, sizeof(a));
+  unsigned* c = (unsigned*)counters.p;
+  a.counters = c;
+  a.n_counters = kNumCounters;
+  a.count = c + kCountFeatures;
+  a.n_edges = r.want_edges ? c + kCountEdges : nullptr;
+  a.k = r.m + 1;
+  a.classify = r.classify;
+  a.want_edges = r.want_edges;
+  a.lam4 = (const double*)lam_s.p;
+  a.simplices = (const unsigned long long*)simplices.p;
+  a.bary = (const float*)bary.p;
+  a.scalar = (const float*)scalar_s.p;
+  a.track = (const unsigned long long*)track.p;
+  a.cls = (const unsigned*)cls.p;
+  a.edges = (const unsigned*)edges.p;
+  a.dst = pack_dev();
+  a.dst_bytes = pack_bytes();
+  return a;
 }
 
 void ftk2b_ctx::release_all() {
@@ -625,10 +690,12 @@ cudaError_t resolve_cull_mode(ftk2b_ctx* ctx, const RegularMesh& rm, const Field
 }  // namespace ftk2b
 
 // fiber_thr: null for CriticalPointPredicate; the two thresholds for
-// FiberPredicate (2D+t meshes)
+// FiberPredicate (2D+t meshes).  pack: the caller fetches the results next, so
+// the pipeline ends with the kernel that writes them to the pinned block (one
+// launch and one wait fewer than packing on the fetch).
 static ftk2b_status run_regular(ftk2b_ctx* ctx, const ftk2b_mesh_desc* mesh,
                                 const ftk2b_field_desc* field, const ftk2b_cp_params* prm,
-                                const double* fiber_thr = nullptr) {
+                                const double* fiber_thr = nullptr, bool pack = false) {
   using Clk = std::chrono::steady_clock;
   auto msd = [](Clk::time_point a, Clk::time_point b) {
     return std::chrono::duration<double, std::milli>(b - a).count();
@@ -721,6 +788,7 @@ static ftk2b_status run_regular(ftk2b_ctx* ctx, const ftk2b_mesh_desc* mesh,
     rs.big_count = (unsigned*)ctx->counters.p + kCountBig;
     rs.acc_count = (unsigned*)ctx->counters.p + kCountAcc;
     const int f64 = field->dtype == FTK2B_F64;
+    const int classify = prm->classify && !cfg.fiber;
     // the device pipeline after the counters' reset in two parts, so that the
     // fused cull kernel can be timed on its own: [cull] and [exact tests,
     // canonical order, star edges, trajectories, counters readback]
@@ -744,12 +812,28 @@ static ftk2b_status run_regular(ftk2b_ctx* ctx, const ftk2b_mesh_desc* mesh,
       if ((e = launch_refine_staged(f64, rm, fa, cfg, cq, rs, sink, ctx->num_sms, ctx->stream))) return e;
       *nl += 2;
       if ((e = launch_post_regular(rm, nch, B, prm->want_edges, ctx->stream, nl))) return e;
-      if (prm->classify && !cfg.fiber) {
+      if (classify) {
         if ((e = launch_classify_regular(f64, rm, fa, nch, B, ctx->stream))) return e;
         *nl += 1;
       }
+      if (pack) return cudaSuccess;
       return cudaMemcpyAsync(ctx->h_counters, ctx->counters.p, sizeof(unsigned) * kNumCounters,
                              cudaMemcpyDeviceToHost, ctx->stream);
+    };
+    // after the pipeline's last timing event: the results (when they fit) and
+    // the counters to the host
+    auto enqueue3 = [&](unsigned long long* nl) -> cudaError_t {
+      if (!pack) return cudaSuccess;
+      LastRun r;
+      r.m = m;
+      r.classify = classify;
+      r.want_edges = prm->want_edges;
+      PackArgs a = ctx->pack_args(r);
+      a.h_counters = (unsigned*)ctx->pin.d;
+      a.cap = cap;
+      a.edge_cap = edge_cap;
+      *nl += 1;
+      return launch_pack(a, ctx->num_sms, ctx->stream);
     };
     if (cfg.cull_mode == 2) {
       int mode = 0;
@@ -789,6 +873,8 @@ static ftk2b_status run_regular(ftk2b_ctx* ctx, const ftk2b_mesh_desc* mesh,
       key.allow_tma = !ctx->disable_tma;
       key.key_bits = key_bits;
       key.nch = nch;
+      key.pack_dst = pack ? ctx->pack_dev() : nullptr;
+      key.pack_bytes = pack ? ctx->pack_bytes() : 0;
       const unsigned long long gen = ctx->buffer_generation();
       GraphEntry* ent = nullptr;
       for (auto it = ctx->graphs.begin(); it != ctx->graphs.end();) {
@@ -827,6 +913,7 @@ static ftk2b_status run_regular(ftk2b_ctx* ctx, const ftk2b_mesh_desc* mesh,
           if (!ce) ce = cudaEventRecordWithFlags(ctx->ev_x, ctx->stream, cudaEventRecordExternal);
           if (!ce) ce = enqueue2(&nl);
           if (!ce) ce = cudaEventRecordWithFlags(ctx->ev1, ctx->stream, cudaEventRecordExternal);
+          if (!ce) ce = enqueue3(&nl);
           const cudaError_t ee = cudaStreamEndCapture(ctx->stream, &graph);
           if (!ce && !ee && cudaGraphInstantiate(&e.g1, graph, 0) == cudaSuccess) {
             cudaGraphDestroy(graph);
@@ -873,6 +960,9 @@ static ftk2b_status run_regular(ftk2b_ctx* ctx, const ftk2b_mesh_desc* mesh,
         CUDA_TRY(ctx, cudaEventRecord(ctx->ev_x, ctx->stream));
         CUDA_TRY(ctx, cudaGraphLaunch(ent->g2, ctx->stream));
         CUDA_TRY(ctx, cudaEventRecord(ctx->ev1, ctx->stream));
+        unsigned long long nl = 0;
+        CUDA_TRY(ctx, enqueue3(&nl));
+        ctx->launches += nl;
       } else {
         CUDA_TRY(ctx, cudaGraphLaunch(ent->g1, ctx->stream));  // the event records are nodes of the graph
       }
@@ -885,6 +975,7 @@ static ftk2b_status run_regular(ftk2b_ctx* ctx, const ftk2b_mesh_desc* mesh,
       CUDA_TRY(ctx, cudaEventRecord(ctx->ev_x, ctx->stream));
       CUDA_TRY(ctx, enqueue2(&nl));
       CUDA_TRY(ctx, cudaEventRecord(ctx->ev1, ctx->stream));
+      CUDA_TRY(ctx, enqueue3(&nl));
       ctx->launches += nl;
     }
     {
@@ -928,8 +1019,10 @@ static ftk2b_status run_regular(ftk2b_ctx* ctx, const ftk2b_mesh_desc* mesh,
     ctx->last.n_roots = h[kCountRoots];
     ctx->last.n_simplices = nsimp;
     ctx->last.device_ms = ms;
-    ctx->last.classify = prm->classify && !cfg.fiber;
+    ctx->last.classify = classify;
     ctx->last.want_edges = prm->want_edges;
+    ctx->pack_ready =
+        pack && pack_layout(ctx->last.n, ctx->last.ne, m + 1, classify).packed <= ctx->pack_bytes();
     return FTK2B_OK;
   }
   return fail(ctx, FTK2B_OVERFLOW_RETRY, "feature buffer overflow persisted after retries");
@@ -937,17 +1030,16 @@ static ftk2b_status run_regular(ftk2b_ctx* ctx, const ftk2b_mesh_desc* mesh,
 
 // ---------------------------------------------------------------------------
 
-extern "C" ftk2b_status ftk2b_cp_run(ftk2b_ctx* ctx, const ftk2b_mesh_desc* mesh,
-                                     const ftk2b_field_desc* field, const ftk2b_cp_params* params,
-                                     uint64_t* n_features, uint64_t* n_edges) {
-  ftk2b::NvtxRange nvtx_range("ftk2b_cp_run");
+static ftk2b_status run_any(ftk2b_ctx* ctx, const ftk2b_mesh_desc* mesh, const ftk2b_field_desc* field,
+                            const ftk2b_cp_params* params, uint64_t* n_features, uint64_t* n_edges, bool pack) {
   if (!ctx) return FTK2B_INVALID_ARG;
   if (!mesh || !field) return fail(ctx, FTK2B_INVALID_ARG, "null descriptor");
   ftk2b_cp_params prm = params ? *params : ftk2b_cp_params_default();
   if (!(prm.sos_q > 0)) return fail(ctx, FTK2B_INVALID_ARG, "sos_q must be positive");
   if (cudaSetDevice(ctx->device) != cudaSuccess) return fail(ctx, FTK2B_CUDA_ERROR, "cudaSetDevice failed");
   ftk2b_status st;
-  if (mesh->kind == FTK2B_MESH_REGULAR) st = run_regular(ctx, mesh, field, &prm);
+  ctx->pack_ready = false;
+  if (mesh->kind == FTK2B_MESH_REGULAR) st = run_regular(ctx, mesh, field, &prm, nullptr, pack);
   else if (mesh->kind == FTK2B_MESH_EXTRUDED) st = run_extruded(ctx, mesh, field, &prm);
   else st = fail(ctx, FTK2B_INVALID_ARG, "unknown mesh kind %d", mesh->kind);
   if (st == FTK2B_OK) {
@@ -956,6 +1048,18 @@ extern "C" ftk2b_status ftk2b_cp_run(ftk2b_ctx* ctx, const ftk2b_mesh_desc* mesh
   }
   return st;
 }
+
+extern "C" ftk2b_status ftk2b_cp_run(ftk2b_ctx* ctx, const ftk2b_mesh_desc* mesh,
+                                     const ftk2b_field_desc* field, const ftk2b_cp_params* params,
+                                     uint64_t* n_features, uint64_t* n_edges) {
+  ftk2b::NvtxRange nvtx_range("ftk2b_cp_run");
+  return run_any(ctx, mesh, field, params, n_features, n_edges, false);
+}
+
+// Results up to this size are packed into pinned memory by one kernel; larger
+// ones (above 300,000 features) are copied array by array into the result's
+// own memory, so that a context never pins more than this.
+constexpr size_t kPackMax = size_t(32) << 20;
 
 extern "C" ftk2b_status ftk2b_cp_fetch(ftk2b_ctx* ctx, ftk2b_cp_result** out) {
   ftk2b::NvtxRange nvtx_range("ftk2b_cp_fetch");
@@ -971,51 +1075,55 @@ extern "C" ftk2b_status ftk2b_cp_fetch(ftk2b_ctx* ctx, ftk2b_cp_result** out) {
   *out = nullptr;
   const uint64_t n = ctx->last.n, ne = ctx->last.ne;
   const int m = ctx->last.m;
-  ftk2b_cp_result* r = (ftk2b_cp_result*)calloc(1, sizeof(ftk2b_cp_result));
+  const size_t k = (size_t)(m + 1);
+  PackLayout L;
+  ftk2b_cp_result* r = new_result(n, ne, m, ctx->last.classify, &L);
   if (!r) return fail(ctx, FTK2B_OOM, "host allocation failed");
-  r->m = m;
-  r->n_features = n;
-  r->n_edges = ne;
   r->n_tracks = ctx->last.want_edges ? ctx->last.n_roots : 0;
   r->n_simplices = ctx->last.n_simplices;
   r->device_ms = ctx->last.device_ms;
-  const size_t k = (size_t)(m + 1);
-  r->simplices = (uint64_t*)malloc(sizeof(uint64_t) * (n * k + 1));
-  r->lambda = (double*)malloc(sizeof(double) * (n * k + 1));
-  r->barycentric = (float*)malloc(sizeof(float) * (n * k + 1));
-  r->track_id = (uint64_t*)malloc(sizeof(uint64_t) * (n + 1));
-  r->type = (uint32_t*)calloc(n + 1, sizeof(uint32_t));
-  r->cp_class = (uint32_t*)calloc(n + 1, sizeof(uint32_t));
-  r->scalar = (float*)malloc(sizeof(float) * (n + 1));
-  r->edges = (uint32_t*)malloc(sizeof(uint32_t) * (2 * ne + 2));
-  std::vector<double> lam4((size_t)n * 4 + 4);
-  if (!r->simplices || !r->lambda || !r->barycentric || !r->track_id || !r->type || !r->cp_class ||
-      !r->scalar || !r->edges) {
-    ftk2b_cp_result_free(r);
-    return fail(ctx, FTK2B_OOM, "host allocation failed");
-  }
+  unsigned char* data = reinterpret_cast<unsigned char*>(r) + kResultHeader;
   cudaStream_t s = ctx->stream;
-  auto d2h = [&](void* dst, const void* src, size_t bytes) -> cudaError_t {
-    if (!bytes) return cudaSuccess;
-    return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s);
-  };
   cudaError_t e = cudaSuccess;
-  if (!e) e = d2h(r->simplices, ctx->simplices.p, sizeof(uint64_t) * n * k);
-  if (!e) e = d2h(r->barycentric, ctx->bary.p, sizeof(float) * n * k);
-  if (!e) e = d2h(lam4.data(), ctx->lam_s.p, sizeof(double) * n * 4);
-  if (!e) e = d2h(r->scalar, ctx->scalar_s.p, sizeof(float) * n);
-  if (!e && ctx->last.want_edges) e = d2h(r->track_id, ctx->track.p, sizeof(uint64_t) * n);
-  if (!e && ctx->last.classify) e = d2h(r->cp_class, ctx->cls.p, sizeof(uint32_t) * n);
-  if (!e) e = d2h(r->edges, ctx->edges.p, sizeof(uint32_t) * 2 * ne);
-  if (!e) e = ctx->sync();
+  if (ctx->pack_ready) {
+    memcpy(data, ctx->pack_host(), L.packed);
+  } else if (n && L.packed <= kPackMax && ctx->ensure_pack_pin(L.packed) == cudaSuccess) {
+    PackArgs a = ctx->pack_args(ctx->last);
+    a.cap = (unsigned)n;
+    a.edge_cap = (unsigned)ne;
+    a.n = (unsigned)n;
+    a.ne = (unsigned)ne;
+    a.count = nullptr;
+    e = launch_pack(a, ctx->num_sms, s);
+    if (!e) e = ctx->sync();
+    if (!e) memcpy(data, ctx->pack_host(), L.packed);
+    ctx->launches += 1;
+  } else if (n) {
+    auto d2h = [&](void* dst, const void* src, size_t bytes) -> cudaError_t {
+      if (!bytes) return cudaSuccess;
+      return cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, s);
+    };
+    std::vector<double> lam4(k == 4 ? 0 : (size_t)n * 4);
+    if (!e) e = d2h(r->simplices, ctx->simplices.p, sizeof(uint64_t) * n * k);
+    if (!e) e = d2h(r->barycentric, ctx->bary.p, sizeof(float) * n * k);
+    if (!e) e = d2h(k == 4 ? r->lambda : lam4.data(), ctx->lam_s.p, sizeof(double) * n * 4);
+    if (!e) e = d2h(r->scalar, ctx->scalar_s.p, sizeof(float) * n);
+    if (!e && ctx->last.want_edges) e = d2h(r->track_id, ctx->track.p, sizeof(uint64_t) * n);
+    if (!e && ctx->last.classify) e = d2h(r->cp_class, ctx->cls.p, sizeof(uint32_t) * n);
+    if (!e) e = d2h(r->edges, ctx->edges.p, sizeof(uint32_t) * 2 * ne);
+    if (!e) e = ctx->sync();
+    if (!e) {
+      if (k != 4)
+        for (uint64_t i = 0; i < n; ++i)
+          for (size_t v = 0; v < k; ++v) r->lambda[i * k + v] = lam4[i * 4 + v];
+      if (!ctx->last.want_edges)
+        for (uint64_t i = 0; i < n; ++i) r->track_id[i] = i;
+    }
+  }
   if (e) {
     ftk2b_cp_result_free(r);
     return fail(ctx, FTK2B_CUDA_ERROR, "result copy failed: %s", cudaGetErrorString(e));
   }
-  for (uint64_t i = 0; i < n; ++i)
-    for (size_t v = 0; v < k; ++v) r->lambda[i * k + v] = lam4[i * 4 + v];
-  if (!ctx->last.want_edges)
-    for (uint64_t i = 0; i < n; ++i) r->track_id[i] = i;
   *out = r;
   return FTK2B_OK;
 }
@@ -1038,7 +1146,8 @@ extern "C" ftk2b_status ftk2b_fiber_extract(ftk2b_ctx* ctx, const ftk2b_mesh_des
   prm.precision = FTK2B_PRECISION_EXACT;
   prm.classify = 0;
   prm.want_edges = 1;
-  const ftk2b_status st = mesh->kind == FTK2B_MESH_REGULAR ? run_regular(ctx, mesh, field, &prm, thresholds)
+  ctx->pack_ready = false;
+  const ftk2b_status st = mesh->kind == FTK2B_MESH_REGULAR ? run_regular(ctx, mesh, field, &prm, thresholds, true)
                                                           : run_extruded(ctx, mesh, field, &prm, thresholds);
   if (st) return st;
   return ftk2b_cp_fetch(ctx, out);
@@ -1050,20 +1159,8 @@ extern "C" ftk2b_status ftk2b_cp_extract(ftk2b_ctx* ctx, const ftk2b_mesh_desc* 
   ftk2b::NvtxRange nvtx_range("ftk2b_cp_extract");
   if (!out) return ctx ? fail(ctx, FTK2B_INVALID_ARG, "null output") : FTK2B_INVALID_ARG;
   *out = nullptr;
-  ftk2b_status st = ftk2b_cp_run(ctx, mesh, field, params, nullptr, nullptr);
+  ftk2b_status st = run_any(ctx, mesh, field, params, nullptr, nullptr, true);
   if (st) return st;
   return ftk2b_cp_fetch(ctx, out);
 }
 
-extern "C" void ftk2b_cp_result_free(ftk2b_cp_result* r) {
-  if (!r) return;
-  free(r->simplices);
-  free(r->lambda);
-  free(r->barycentric);
-  free(r->track_id);
-  free(r->type);
-  free(r->cp_class);
-  free(r->scalar);
-  free(r->edges);
-  free(r);
-}

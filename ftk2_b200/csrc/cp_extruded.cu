@@ -1143,6 +1143,7 @@ ftk2b_status result_extruded_t(ftk2b_stream* s, ftk2b_cp_result** out) {
   ctx->last.kind = FTK2B_MESH_EXTRUDED;
   ctx->last.m = M;
   ctx->last.f64 = s->dtype == FTK2B_F64;
+  ctx->pack_ready = false;
   ctx->last.n = n;
   ctx->last.ne = s->prm.want_edges ? ne : 0;
   ctx->last.n_roots = ctx->h_counters[kCountRoots];
