@@ -759,13 +759,19 @@ static ftk2b_status run_regular(ftk2b_ctx* ctx, const ftk2b_mesh_desc* mesh,
     if (nloc > 0xFFFFFFF0ull) return fail(ctx, FTK2B_UNSUPPORTED, "mesh too large for fiber extraction");
     ccap = std::max<unsigned>(ccap, (unsigned)nloc);
   }
-  for (int attempt = 0; attempt < 4; ++attempt) {
+  // the inside list's own capacity (1 MB of entries to start with): where the
+  // field is flat, ties let far more simplices past the inside test than the
+  // solve accepts, and a capacity shared with the features would grow these
+  // past kSmallPostCap, onto the long chain (128^3 x 16 f64: post-processing
+  // 138 against 97 us for the same 5,700 features)
+  unsigned acc_cap = ctx->acc_cap_hint ? ctx->acc_cap_hint : 131072u;
+  for (int attempt = 0; attempt < 6; ++attempt) {
     const unsigned edge_cap = cap * 2;
     st = ensure_feature_buffers(ctx, cap, edge_cap, m);
     if (st) return st;
     CUDA_TRY(ctx, ctx->cand_corner.ensure(sizeof(unsigned long long) * (size_t)ccap));
     CUDA_TRY(ctx, ctx->cand_chains.ensure(sizeof(unsigned long long) * (size_t)ccap));
-    CUDA_TRY(ctx, ctx->refine_pairs.ensure(refine_mask_bytes(ccap, cap)));
+    CUDA_TRY(ctx, ctx->refine_pairs.ensure(refine_mask_bytes(ccap, acc_cap)));
     PostBuffers B = ctx->post_buffers(cap, edge_cap, key_bits);
     FeatureSink sink;
     sink.key = B.key;
@@ -782,7 +788,7 @@ static ftk2b_status run_regular(ftk2b_ctx* ctx, const ftk2b_mesh_desc* mesh,
     RefineStage rs;
     // the single-field test keeps values and quantised values in shared
     // memory and reads the field again for the solve: no staging block
-    refine_stage_bind(rs, ctx->refine_pairs.p, ccap, cap);
+    refine_stage_bind(rs, ctx->refine_pairs.p, ccap, acc_cap);
     rs.count = (unsigned*)ctx->counters.p + kCountPairs;
     rs.err = (unsigned*)ctx->counters.p + kCountErr;
     rs.big_count = (unsigned*)ctx->counters.p + kCountBig;
@@ -867,6 +873,7 @@ static ftk2b_status run_regular(ftk2b_ctx* ctx, const ftk2b_mesh_desc* mesh,
       key.cap = cap;
       key.ccap = ccap;
       key.edge_cap = edge_cap;
+      key.acc_cap = acc_cap;
       key.f64 = f64;
       key.want_edges = prm->want_edges;
       key.classify = prm->classify;
@@ -1000,6 +1007,13 @@ static ftk2b_status run_regular(ftk2b_ctx* ctx, const ftk2b_mesh_desc* mesh,
       if (want > 0xFFFFFFF0ull) return fail(ctx, FTK2B_OVERFLOW_RETRY, "candidate count exceeds 2^32");
       ccap = (unsigned)want;
       ctx->cand_cap_hint = ccap;
+      continue;
+    }
+    if (h[kCountAcc] > acc_cap) {
+      const uint64_t want = (uint64_t)h[kCountAcc] + h[kCountAcc] / 4 + 1024;
+      if (want > 0xFFFFFFF0ull) return fail(ctx, FTK2B_OVERFLOW_RETRY, "inside list exceeds 2^32");
+      acc_cap = (unsigned)want;
+      ctx->acc_cap_hint = acc_cap;
       continue;
     }
     if (h[kCountFeatures] > cap || h[kCountEdges] > edge_cap) {

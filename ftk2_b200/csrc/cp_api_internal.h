@@ -68,7 +68,7 @@ struct RegularGraphKey {
   RegularMesh rm;
   FieldAccess fa;
   ExtractConfig cfg;
-  unsigned cap, ccap, edge_cap;
+  unsigned cap, ccap, edge_cap, acc_cap;
   int f64, want_edges, classify, allow_tma, key_bits, nch;
   const void* pack_dst;            // null: the results stay on the device
   unsigned long long pack_bytes;
@@ -174,6 +174,7 @@ struct ftk2b_ctx {
   std::string err;
   unsigned cap_hint = 0;
   unsigned cand_cap_hint = 0;
+  unsigned acc_cap_hint = 0;
   int tune_tchunk = 0;
   int cull_mode = 2;  // FTK2B_OPT_CULL_MODE (2: chosen per workload shape)
   int last_cull_mode = 0;  // the mode the last regular-mesh extraction ran

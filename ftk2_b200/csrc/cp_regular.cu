@@ -1915,11 +1915,10 @@ __global__ void __launch_bounds__(kRefineWarps * 32, 4) refine_test_kernel(Regul
 }
 
 // The single-field exact test, part 2: blocks below solve_blocks solve the
-// simplices on the inside list (one thread each; a list longer than its
-// capacity raises the sink count past the sink's capacity, so that the call
-// reports overflow and runs again with larger buffers); the others run the
-// whole test on the candidates listed for the 128-bit path.  Values are read
-// from the field.
+// simplices on the inside list (one thread each; the host sees a list longer
+// than its capacity by its count, and runs the call again with a larger one);
+// the others run the whole test on the candidates listed for the 128-bit path.
+// Values are read from the field.
 template <typename T, int D>
 __global__ void __launch_bounds__(kRefineWarps * 32, 2) refine_accept_kernel(RegularMesh mesh, FieldAccess fa,
                                                                             ExtractConfig cfg, CandidateQueue cq,
@@ -1935,7 +1934,6 @@ __global__ void __launch_bounds__(kRefineWarps * 32, 2) refine_accept_kernel(Reg
   const int lane = threadIdx.x & 31;
   if ((int)blockIdx.x < solve_blocks) {
     const unsigned na = *rs.acc_count;
-    if (blockIdx.x == 0 && threadIdx.x == 0 && na > rs.acc_cap) atomicMax(sink.count, na);
     const unsigned n = min(na, rs.acc_cap);
     const unsigned stride = solve_blocks * blockDim.x;
     for (unsigned base = blockIdx.x * blockDim.x; base < n; base += stride) {

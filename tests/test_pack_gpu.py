@@ -49,3 +49,17 @@ def test_classes_and_no_edges(dims):
     assert np.array_equal(bare.simplices, typed.simplices) and np.array_equal(bare.lam, typed.lam)
     assert np.array_equal(bare.track_id, np.arange(len(bare.track_id))) and len(bare.edges) == 0
     assert not bare.cp_class.any() and bare.n_tracks == 0
+
+
+def test_inside_list_longer_than_its_first_capacity():
+    """Values that all quantise to 0: every simplex passes the inside test by
+    its ties and only the solve rejects (more than 131,072 listed simplices)."""
+    dims = [17, 15, 13, 3]
+    case = cases.Case("flat", "regular", 3, cases.MULTI, 1e-8 * _noise(dims, 5), 2.0 ** 20, dims)
+    want = oracle_run(case)
+    keep: list = []
+    mesh, fld = cases.gpu_inputs(case, keep)
+    with api.Context(0) as ctx:
+        for _ in range(2):
+            assert_identical(ctx.extract(mesh, fld, api.params(case.sos_q)), want)
+        assert ctx.get_option(api.INFO_LAST_TESTED) > 131072
