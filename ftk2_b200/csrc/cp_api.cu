@@ -753,11 +753,10 @@ static ftk2b_status run_regular(ftk2b_ctx* ctx, const ftk2b_mesh_desc* mesh,
   // overflow; the context remembers the grown value
   unsigned cap = ctx->cap_hint ? ctx->cap_hint : kSmallPostCap;
   unsigned ccap = ctx->cand_cap_hint ? ctx->cand_cap_hint : 65536u;
-  if (fiber_thr) {  // every local vertex is a candidate corner
+  if (fiber_thr) {
     uint64_t nloc = 1;
     for (int k = 0; k < d; ++k) nloc *= rm.ld[k];
     if (nloc > 0xFFFFFFF0ull) return fail(ctx, FTK2B_UNSUPPORTED, "mesh too large for fiber extraction");
-    ccap = std::max<unsigned>(ccap, (unsigned)nloc);
   }
   // the inside list's own capacity (1 MB of entries to start with): where the
   // field is flat, ties let far more simplices past the inside test than the
@@ -805,7 +804,7 @@ static ftk2b_status run_regular(ftk2b_ctx* ctx, const ftk2b_mesh_desc* mesh,
       cudaError_t e;
       int nk = 1;
       if (cfg.fiber) {
-        if ((e = launch_fiber_candidates(rm, cq, ctx->num_sms, ctx->stream))) return e;
+        if ((e = launch_fiber_candidates(f64, rm, fa, cfg, cq, ctx->stream))) return e;
       } else if ((e = launch_extract_regular(f64, rm, fa, cfg, cq, B.err, ctx->stream, !ctx->disable_tma,
                                              &ctx->last_used_tma, &nk))) {
         return e;

@@ -92,9 +92,9 @@ struct ExtractConfig {
   // block waits, at most this many polls, on an mbarrier nothing completes,
   // and leaves through the timeout path (the call reports FTK2B_TIMEOUT)
   int stall_polls;
-  // FiberPredicate<T> (predicate.hpp:341-362): every hypercube is a candidate
-  // (the cull words assume the solve must succeed), values are taken minus
-  // fthr[j], and a simplex whose solve fails is kept at the centroid
+  // FiberPredicate<T> (predicate.hpp:341-362): no cull words (they assume the
+  // solve must succeed), values are taken minus fthr[j], and a simplex whose
+  // solve fails is kept at the centroid
   int fiber;
   double fthr[2];
   // scratch of cull mode 1 (device): 8 ints per (slice, tile), and the runs
@@ -128,10 +128,10 @@ cudaError_t launch_extract_regular(int f64, const RegularMesh& mesh, const Field
 // Scratch of cull mode 1 for a mesh: tile-slice statistics and run list sizes.
 void tile_scratch_size(const RegularMesh& mesh, size_t* stats_bytes, unsigned* runs_cap);
 // Exact SoS + solve of the queued candidates, compacted into the sink.
-// FiberPredicate: queue every local vertex as a corner with all its in-mesh
-// chains (no cull)
-cudaError_t launch_fiber_candidates(const RegularMesh& mesh, const CandidateQueue& cq, int num_sms,
-                                    cudaStream_t st);
+// FiberPredicate (2D+t): queue the hypercubes with a chain whose vertices share
+// no strict sign of a quantised component
+cudaError_t launch_fiber_candidates(int f64, const RegularMesh& mesh, const FieldAccess& fa, const ExtractConfig& cfg,
+                                    const CandidateQueue& cq, cudaStream_t st);
 // The exact test of the queued candidates: the fast-path inside test of
 // every surviving simplex of the candidates whose quantised values all stay
 // below 2^31, listing the simplices it accepts; the solve of the listed
