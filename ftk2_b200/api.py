@@ -325,7 +325,9 @@ def params(sos_q: float = 1e6, precision: int = PRECISION_EXACT, want_edges: boo
 
 @dataclass
 class CPResult:
-    """Flattened FeatureComplex (complex.hpp:14-58) of one extraction."""
+    """Flattened FeatureComplex (complex.hpp:14-58) of one extraction.  The
+    arrays are views of the library's result memory, freed with the last of
+    them."""
     simplices: np.ndarray      # (n, m+1) uint64 sorted vertex ids, canonical order
     lam: np.ndarray            # (n, m+1) float64 barycentrics
     bary: np.ndarray           # (n, m+1) float32 as FeatureElement stores them
@@ -339,24 +341,44 @@ class CPResult:
     device_ms: float = 0.0
 
 
-def _result_from_c(r: CPResultC) -> CPResult:
-    n, k, e = int(r.n_features), int(r.m) + 1, int(r.n_edges)
+class _CPAddresses(C.Structure):
+    """CPResultC with its array pointers as plain addresses."""
+    _fields_ = [(n, C.c_void_p if hasattr(t, "contents") else t) for n, t in CPResultC._fields_]
 
-    def arr(ptr, count, dt):
-        if count == 0:
-            return np.zeros(0, dtype=dt)
-        return np.ctypeslib.as_array(ptr, shape=(count,)).astype(dt, copy=True)
 
+class _CPOwner:
+    """Owns one critical-point result, a single allocation of the library that
+    does not depend on its context, shows its arrays' memory to numpy, and
+    frees it once the last array made of it is gone."""
+
+    __slots__ = ("_free", "_ptr", "__array_interface__")
+
+    def __init__(self, free, ptr, lo: int, hi: int):
+        self._free, self._ptr = free, ptr
+        self.__array_interface__ = {"data": (lo, False), "shape": (hi - lo,), "typestr": "|u1", "version": 3}
+
+    def __del__(self):
+        self._free(self._ptr)
+
+
+def _result_from_c(free, ptr) -> CPResult:
+    """The result at the non-null CPResultC pointer ptr, as views of its
+    memory: the arrays lie in one block from the barycentrics (first) to the
+    types (last)."""
+    r = _CPAddresses.from_address(C.cast(ptr, C.c_void_p).value)
+    n, k, e, lo = r.n_features, r.m + 1, r.n_edges, r.lambda_
+    block = np.asarray(_CPOwner(free, ptr, lo, r.type + 4 * n))
+    nd = np.ndarray
     return CPResult(
-        simplices=arr(r.simplices, n * k, np.uint64).reshape(n, k),
-        lam=arr(r.lambda_, n * k, np.float64).reshape(n, k),
-        bary=arr(r.barycentric, n * k, np.float32).reshape(n, k),
-        track_id=arr(r.track_id, n, np.uint64),
-        type=arr(r.type, n, np.uint32),
-        cp_class=arr(r.cp_class, n, np.uint32),
-        scalar=arr(r.scalar, n, np.float32),
-        edges=arr(r.edges, 2 * e, np.uint32).reshape(e, 2),
-        n_tracks=int(r.n_tracks), n_simplices=int(r.n_simplices), device_ms=float(r.device_ms))
+        simplices=nd((n, k), np.uint64, block, r.simplices - lo),
+        lam=nd((n, k), np.float64, block, 0),
+        bary=nd((n, k), np.float32, block, r.barycentric - lo),
+        track_id=nd((n,), np.uint64, block, r.track_id - lo),
+        type=nd((n,), np.uint32, block, r.type - lo),
+        cp_class=nd((n,), np.uint32, block, r.cp_class - lo),
+        scalar=nd((n,), np.float32, block, r.scalar - lo),
+        edges=nd((e, 2), np.uint32, block, r.edges - lo),
+        n_tracks=r.n_tracks, n_simplices=r.n_simplices, device_ms=r.device_ms)
 
 
 @dataclass
@@ -478,11 +500,9 @@ class Context:
         out = C.POINTER(CPResultC)()
         self._check(self.lib.ftk2b_cp_extract(self.h, C.byref(mesh), C.byref(field), C.byref(prm),
                                               C.byref(out)))
-        try:
-            self._last_n = int(out.contents.n_features)
-            return _result_from_c(out.contents)
-        finally:
-            self.lib.ftk2b_cp_result_free(out)
+        res = _result_from_c(self.lib.ftk2b_cp_result_free, out)
+        self._last_n = len(res.track_id)
+        return res
 
     def contour(self, mesh: MeshDesc, field, threshold: float = 0.0, sos_q: float = 1e6) -> ContourResult:
         """Level sets (ContourPredicate<T>) on a regular mesh.  field: a
@@ -503,11 +523,9 @@ class Context:
         out = C.POINTER(CPResultC)()
         self._check(self.lib.ftk2b_fiber_extract(self.h, C.byref(mesh), C.byref(field), thr, float(sos_q),
                                                  C.byref(out)))
-        try:
-            self._last_n = int(out.contents.n_features)
-            return _result_from_c(out.contents)
-        finally:
-            self.lib.ftk2b_cp_result_free(out)
+        res = _result_from_c(self.lib.ftk2b_cp_result_free, out)
+        self._last_n = len(res.track_id)
+        return res
 
     def fiber_surface(self, mesh: MeshDesc, field: FieldDesc, thresholds=(0.0, 0.0),
                       sos_q: float = 1e6) -> ContourResult:
@@ -539,10 +557,7 @@ class Context:
     def fetch(self) -> CPResult:
         out = C.POINTER(CPResultC)()
         self._check(self.lib.ftk2b_cp_fetch(self.h, C.byref(out)))
-        try:
-            return _result_from_c(out.contents)
-        finally:
-            self.lib.ftk2b_cp_result_free(out)
+        return _result_from_c(self.lib.ftk2b_cp_result_free, out)
 
 
     def attributes(self, mesh: MeshDesc, attrs, base_grid_dims=None) -> np.ndarray:
@@ -599,22 +614,14 @@ class Context:
         n = getattr(self, "_batch_n", 0)
         outs = (C.POINTER(CPResultC) * max(n, 1))()
         self._check(self.lib.ftk2b_cp_fetch_batch(self.h, outs))
-        try:
-            return [_result_from_c(outs[i].contents) for i in range(n)]
-        finally:
-            for i in range(n):
-                self.lib.ftk2b_cp_result_free(outs[i])
+        return [_result_from_c(self.lib.ftk2b_cp_result_free, outs[i]) for i in range(n)]
 
     def extract_batch(self, meshes, fields, prms=None) -> list:
         """One result per field, each identical to extract() on that field."""
         n, ma, fa, pa = self._batch_arrays(meshes, fields, prms)
         outs = (C.POINTER(CPResultC) * n)()
         self._check(self.lib.ftk2b_cp_extract_batch(self.h, n, ma, fa, pa, outs))
-        try:
-            return [_result_from_c(outs[i].contents) for i in range(n)]
-        finally:
-            for i in range(n):
-                self.lib.ftk2b_cp_result_free(outs[i])
+        return [_result_from_c(self.lib.ftk2b_cp_result_free, outs[i]) for i in range(n)]
 
 
 class Stream:
@@ -638,10 +645,7 @@ class Stream:
     def result(self) -> CPResult:
         out = C.POINTER(CPResultC)()
         self.ctx._check(self.lib.ftk2b_stream_result(self.h, C.byref(out)))
-        try:
-            return _result_from_c(out.contents)
-        finally:
-            self.lib.ftk2b_cp_result_free(out)
+        return _result_from_c(self.lib.ftk2b_cp_result_free, out)
 
     def info(self):
         """(timesteps pushed, features so far, device ms of the last push)."""
@@ -749,10 +753,7 @@ class Server:
         self._check(st)
         res = None
         if want_result and out:
-            try:
-                res = _result_from_c(out.contents)
-            finally:
-                self.lib.ftk2b_cp_result_free(out)
+            res = _result_from_c(self.lib.ftk2b_cp_result_free, out)
         stats = {k: getattr(stc, k) for k, _ in RequestStatsC._fields_}
         stats["phase_ms"] = list(stc.phase_ms)
         return res, stats
@@ -760,10 +761,7 @@ class Server:
     def stream_result(self, stream_id: int) -> CPResult:
         out = C.POINTER(CPResultC)()
         self._check(self.lib.ftk2b_server_stream_result(self.h, int(stream_id), C.byref(out)))
-        try:
-            return _result_from_c(out.contents)
-        finally:
-            self.lib.ftk2b_cp_result_free(out)
+        return _result_from_c(self.lib.ftk2b_cp_result_free, out)
 
     def close_stream(self, stream_id: int):
         self._check(self.lib.ftk2b_server_stream_close(self.h, int(stream_id)))

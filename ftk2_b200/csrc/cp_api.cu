@@ -13,6 +13,7 @@
 #include "cp_internal.h"
 #include "cp_post.h"
 #include "cp_api_internal.h"
+#include "cp_host.h"
 
 using namespace ftk2b;
 
@@ -55,7 +56,9 @@ cudaError_t PinBuf::alloc(size_t want) {
   constexpr size_t kPage = 4096;
   const size_t n = (want + kPage - 1) / kPage * kPage;
   void* p = nullptr;
-  if (posix_memalign(&p, kPage, n) != 0) return cudaErrorMemoryAllocation;
+  if (n >= (size_t(4) << 20)) p = host_alloc(n);
+  else if (posix_memalign(&p, kPage, n) != 0) p = nullptr;
+  if (!p) return cudaErrorMemoryAllocation;
   cudaError_t e = cudaHostRegister(p, n, cudaHostRegisterMapped);
   if (!e) {
     e = cudaHostGetDevicePointer(&d, p, 0);
@@ -192,10 +195,9 @@ extern "C" void ftk2b_ctx_destroy(ftk2b_ctx* ctx) {
   ctx->drop_graphs();
   ctx->pin.release();
   ctx->pin_big.release();
-  for (int i = 0; i < 2; ++i) {
-    if (ctx->d2h_pin[i]) cudaFreeHost(ctx->d2h_pin[i]);
-    if (ctx->d2h_ev[i]) cudaEventDestroy(ctx->d2h_ev[i]);
-  }
+  ctx->d2h_ring.release();
+  for (cudaEvent_t ev : ctx->d2h_ev)
+    if (ev) cudaEventDestroy(ev);
   if (ctx->batch.h_tab) cudaFreeHost(ctx->batch.h_tab);
   if (ctx->batch.h_fbase) cudaFreeHost(ctx->batch.h_fbase);
   cudaEventDestroy(ctx->ev0);

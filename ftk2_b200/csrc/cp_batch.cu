@@ -457,16 +457,6 @@ extern "C" ftk2b_status ftk2b_cp_fetch_batch(ftk2b_ctx* ctx, ftk2b_cp_result** o
     const uint64_t cnt = e - b;
     const BatchFieldInfo& inf = bc.info[f];
     const size_t k = (size_t)inf.m + 1;
-    ftk2b_cp_result* r = (ftk2b_cp_result*)calloc(1, sizeof(ftk2b_cp_result));
-    if (r) {
-      r->simplices = (uint64_t*)malloc(sizeof(uint64_t) * (cnt * k + 1));
-      r->lambda = (double*)malloc(sizeof(double) * (cnt * k + 1));
-      r->barycentric = (float*)malloc(sizeof(float) * (cnt * k + 1));
-      r->track_id = (uint64_t*)malloc(sizeof(uint64_t) * (cnt + 1));
-      r->type = (uint32_t*)calloc(cnt + 1, sizeof(uint32_t));
-      r->cp_class = (uint32_t*)calloc(cnt + 1, sizeof(uint32_t));
-      r->scalar = (float*)malloc(sizeof(float) * (cnt + 1));
-    }
     // this field's star edges: their centres lie in [b, e) and the global
     // list is sorted by centre
     auto centre_lb = [&](unsigned v) {
@@ -479,18 +469,14 @@ extern "C" ftk2b_status ftk2b_cp_fetch_batch(ftk2b_ctx* ctx, ftk2b_cp_result** o
       return lo;
     };
     const uint64_t eb = inf.want_edges ? centre_lb(b) : 0, ee = inf.want_edges ? centre_lb(e) : 0;
-    if (r) r->edges = (uint32_t*)malloc(sizeof(uint32_t) * (2 * (ee - eb) + 2));
-    if (!r || !r->simplices || !r->lambda || !r->barycentric || !r->track_id || !r->type || !r->cp_class ||
-        !r->scalar || !r->edges) {
-      ftk2b_cp_result_free(r);
+    ftk2b_cp_result* r = new_result(cnt, ee - eb, inf.m, 0, nullptr);
+    if (!r) {
       for (int g = 0; g < f; ++g) {
         ftk2b_cp_result_free(out[g]);
         out[g] = nullptr;
       }
       return bfail(ctx, FTK2B_OOM, "host allocation failed");
     }
-    r->m = inf.m;
-    r->n_features = cnt;
     r->n_simplices = inf.nsimp;
     r->device_ms = bc.device_ms;
     uint64_t roots = 0;
@@ -510,7 +496,6 @@ extern "C" ftk2b_status ftk2b_cp_fetch_batch(ftk2b_ctx* ctx, ftk2b_cp_result** o
       }
     }
     r->n_tracks = inf.want_edges ? roots : 0;
-    r->n_edges = ee - eb;
     for (uint64_t j = eb; j < ee; ++j) {
       r->edges[2 * (j - eb)] = edges[2 * j] - b;
       r->edges[2 * (j - eb) + 1] = edges[2 * j + 1] - b;

@@ -25,8 +25,6 @@
 //              their leading node, each bucket's few rows sorted, duplicates
 //              flagged
 //   label      track id = the component's smallest feature index
-#include <sys/mman.h>
-
 #include <algorithm>
 #include <array>
 #include <vector>
@@ -39,6 +37,7 @@
 #include "../../include/ftk2b.h"
 #include "cp_api_internal.h"
 #include "cp_device.cuh"
+#include "cp_host.h"
 #include "cp_post.h"
 #include "cp_uf.cuh"
 
@@ -617,67 +616,6 @@ ftk2b_status cfail(ftk2b_ctx* ctx, ftk2b_status st, const char* fmt, ...) {
                    "%s failed: %s (%s:%d)", #call, cudaGetErrorString(e_), __FILE__, __LINE__); \
   } while (0)
 
-// Device -> pageable host memory through two pinned chunks: the device copy
-// of one chunk overlaps the host copy of the previous one (a pageable
-// cudaMemcpy of a large result runs at a few GB/s).
-cudaError_t ct_d2h(ftk2b_ctx* ctx, void* dst, const void* src, size_t bytes) {
-  constexpr size_t kChunk = size_t(32) << 20;
-  if (!bytes) return cudaSuccess;
-  for (int i = 0; i < 2; ++i) {
-    if (!ctx->d2h_pin[i]) {
-      cudaError_t e = cudaHostAlloc(&ctx->d2h_pin[i], kChunk, cudaHostAllocDefault);
-      if (e) {
-        ctx->d2h_pin[i] = nullptr;
-        return e;
-      }
-    }
-    if (!ctx->d2h_ev[i]) {
-      cudaError_t e = cudaEventCreateWithFlags(&ctx->d2h_ev[i], cudaEventDisableTiming);
-      if (e) return e;
-    }
-  }
-  auto* out = static_cast<unsigned char*>(dst);
-  const auto* in = static_cast<const unsigned char*>(src);
-  size_t off = 0, prev_off = 0, prev_n = 0;
-  int cur = 0, prev = -1;
-  while (off < bytes || prev >= 0) {
-    size_t n = 0;
-    if (off < bytes) {
-      n = std::min(kChunk, bytes - off);
-      cudaError_t e = cudaMemcpyAsync(ctx->d2h_pin[cur], in + off, n, cudaMemcpyDeviceToHost, ctx->stream);
-      if (!e) e = cudaEventRecord(ctx->d2h_ev[cur], ctx->stream);
-      if (e) return e;
-    }
-    if (prev >= 0) {
-      cudaError_t e = cudaEventSynchronize(ctx->d2h_ev[prev]);
-      if (e) return e;
-      std::memcpy(out + prev_off, ctx->d2h_pin[prev], prev_n);
-    }
-    if (off < bytes) {
-      prev = cur;
-      prev_off = off;
-      prev_n = n;
-      off += n;
-      cur ^= 1;
-    } else {
-      prev = -1;
-    }
-  }
-  return cudaSuccess;
-}
-
-// Host memory for large results (released with free()): 2 MB-aligned and
-// advised for huge pages, so the first touch while copying in faults once per
-// 2 MB instead of once per 4 KB (about half the copy time for a 1 GB result).
-void* ct_host_alloc(size_t bytes) {
-  constexpr size_t kHuge = size_t(2) << 20;
-  if (bytes < (size_t(64) << 20)) return std::malloc(bytes ? bytes : 1);
-  void* p = nullptr;
-  if (posix_memalign(&p, kHuge, (bytes + kHuge - 1) / kHuge * kHuge) != 0) return nullptr;
-  madvise(p, (bytes + kHuge - 1) / kHuge * kHuge, MADV_HUGEPAGE);
-  return p;
-}
-
 enum {
   kBufField = 0, kBufPos, kBufMask, kBufBlk, kBufVoff, kBufSimp, kBufLam, kBufBary, kBufFirst, kBufParent,
   kBufCells, kBufKey0, kBufKey1, kBufVal0, kBufVal1, kBufHist, kBufCellsOut, kBufTrack, kBufCount, kBufList,
@@ -812,24 +750,24 @@ ftk2b_status run_contour(ftk2b_ctx* ctx, const CtGeom& g, const void* field, T t
   res->n_features = n;
   res->cell_dim = d - 1;
   res->n_cells = ncell;
-  res->simplices = static_cast<uint64_t*>(ct_host_alloc(16 * ncap));
-  res->lambda = static_cast<double*>(ct_host_alloc(16 * ncap));
-  res->barycentric = static_cast<float*>(ct_host_alloc(8 * ncap));
-  res->track_id = static_cast<uint64_t*>(ct_host_alloc(8 * ncap));
-  res->scalar = static_cast<float*>(ct_host_alloc(4 * ncap));
-  res->cells = static_cast<uint32_t*>(ct_host_alloc(4ull * kc * ccap));
+  res->simplices = static_cast<uint64_t*>(host_alloc(16 * ncap));
+  res->lambda = static_cast<double*>(host_alloc(16 * ncap));
+  res->barycentric = static_cast<float*>(host_alloc(8 * ncap));
+  res->track_id = static_cast<uint64_t*>(host_alloc(8 * ncap));
+  res->scalar = static_cast<float*>(host_alloc(4 * ncap));
+  res->cells = static_cast<uint32_t*>(host_alloc(4ull * kc * ccap));
   if (!res->simplices || !res->lambda || !res->barycentric || !res->track_id || !res->scalar || !res->cells)
     return cfail(ctx, FTK2B_OOM, "host result allocation failed");
   C_TRY(ctx->sync());
-  C_TRY(ct_d2h(ctx, res->simplices, simp, 16ull * n));
-  C_TRY(ct_d2h(ctx, res->lambda, lam, 16ull * n));
-  C_TRY(ct_d2h(ctx, res->barycentric, bary, 8ull * n));
-  C_TRY(ct_d2h(ctx, res->track_id, track, 8ull * n));
-  C_TRY(ct_d2h(ctx, res->cells, cells_out, 4ull * kc * ncell));
+  C_TRY(copy_to_host(ctx, {{res->simplices, simp, 16ull * n},
+                           {res->lambda, lam, 16ull * n},
+                           {res->barycentric, bary, 8ull * n},
+                           {res->track_id, track, 8ull * n},
+                           {res->cells, cells_out, 4ull * kc * ncell}}));
   if (hc[3] & 1u) return cfail(ctx, FTK2B_CUDA_ERROR, "union-find did not settle");
   if (hc[3] & 2u) return cfail(ctx, FTK2B_CUDA_ERROR, "duplicate manifold cell");
   const float sc = (float)thr;
-  for (unsigned i = 0; i < n; ++i) res->scalar[i] = sc;
+  host_parallel(n, 4ull * n, [&](size_t b, size_t e) { std::fill(res->scalar + b, res->scalar + e, sc); });
   res->n_tracks = hc[2];
   float ms = 0.f;
   cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
@@ -1198,19 +1136,19 @@ ftk2b_status run_fiber_surface(ftk2b_ctx* ctx, const CtGeom& g, const FsTables& 
   C_TRY(ctx->sync());
   res->n_features = n;
   res->n_cells = nuniq;
-  res->simplices = static_cast<uint64_t*>(ct_host_alloc(24 * ncap));
-  res->lambda = static_cast<double*>(ct_host_alloc(24 * ncap));
-  res->barycentric = static_cast<float*>(ct_host_alloc(12 * ncap));
-  res->track_id = static_cast<uint64_t*>(ct_host_alloc(8 * ncap));
+  res->simplices = static_cast<uint64_t*>(host_alloc(24 * ncap));
+  res->lambda = static_cast<double*>(host_alloc(24 * ncap));
+  res->barycentric = static_cast<float*>(host_alloc(12 * ncap));
+  res->track_id = static_cast<uint64_t*>(host_alloc(8 * ncap));
   res->scalar = static_cast<float*>(std::calloc(ncap, 4));
-  res->cells = static_cast<uint32_t*>(ct_host_alloc(12ull * (nuniq ? nuniq : 1)));
+  res->cells = static_cast<uint32_t*>(host_alloc(12ull * (nuniq ? nuniq : 1)));
   if (!res->simplices || !res->lambda || !res->barycentric || !res->track_id || !res->scalar || !res->cells)
     return cfail(ctx, FTK2B_OOM, "host result allocation failed");
-  C_TRY(ct_d2h(ctx, res->simplices, simp, 24ull * n));
-  C_TRY(ct_d2h(ctx, res->lambda, lam, 24ull * n));
-  C_TRY(ct_d2h(ctx, res->barycentric, bary, 12ull * n));
-  C_TRY(ct_d2h(ctx, res->track_id, track, 8ull * n));
-  C_TRY(ct_d2h(ctx, res->cells, cells_out, 12ull * nuniq));
+  C_TRY(copy_to_host(ctx, {{res->simplices, simp, 24ull * n},
+                           {res->lambda, lam, 24ull * n},
+                           {res->barycentric, bary, 12ull * n},
+                           {res->track_id, track, 8ull * n},
+                           {res->cells, cells_out, 12ull * nuniq}}));
   if (hc[3] & 1u) return cfail(ctx, FTK2B_CUDA_ERROR, "union-find did not settle");
   res->n_tracks = hc[2];
   float ms = 0.f;
@@ -1593,23 +1531,23 @@ ftk2b_status run_contour_extruded(ftk2b_ctx* ctx, CeGeom g, const void* field, T
   res->n_features = n;
   res->cell_dim = d - 1;
   res->n_cells = ncell;
-  res->simplices = static_cast<uint64_t*>(ct_host_alloc(16 * ncap));
-  res->lambda = static_cast<double*>(ct_host_alloc(16 * ncap));
-  res->barycentric = static_cast<float*>(ct_host_alloc(8 * ncap));
-  res->track_id = static_cast<uint64_t*>(ct_host_alloc(8 * ncap));
-  res->scalar = static_cast<float*>(ct_host_alloc(4 * ncap));
-  res->cells = static_cast<uint32_t*>(ct_host_alloc(4ull * kc * ccap));
+  res->simplices = static_cast<uint64_t*>(host_alloc(16 * ncap));
+  res->lambda = static_cast<double*>(host_alloc(16 * ncap));
+  res->barycentric = static_cast<float*>(host_alloc(8 * ncap));
+  res->track_id = static_cast<uint64_t*>(host_alloc(8 * ncap));
+  res->scalar = static_cast<float*>(host_alloc(4 * ncap));
+  res->cells = static_cast<uint32_t*>(host_alloc(4ull * kc * ccap));
   if (!res->simplices || !res->lambda || !res->barycentric || !res->track_id || !res->scalar || !res->cells)
     return cfail(ctx, FTK2B_OOM, "host result allocation failed");
-  C_TRY(ct_d2h(ctx, res->simplices, simp, 16ull * n));
-  C_TRY(ct_d2h(ctx, res->lambda, lam, 16ull * n));
-  C_TRY(ct_d2h(ctx, res->barycentric, bary, 8ull * n));
-  C_TRY(ct_d2h(ctx, res->track_id, track, 8ull * n));
-  C_TRY(ct_d2h(ctx, res->cells, cells_out, 4ull * kc * ncell));
+  C_TRY(copy_to_host(ctx, {{res->simplices, simp, 16ull * n},
+                           {res->lambda, lam, 16ull * n},
+                           {res->barycentric, bary, 8ull * n},
+                           {res->track_id, track, 8ull * n},
+                           {res->cells, cells_out, 4ull * kc * ncell}}));
   if (hc[3] & 1u) return cfail(ctx, FTK2B_CUDA_ERROR, "union-find did not settle");
   if (hc[3] & 2u) return cfail(ctx, FTK2B_CUDA_ERROR, "duplicate manifold cell");
   const float sc = (float)thr;
-  for (unsigned i = 0; i < n; ++i) res->scalar[i] = sc;
+  host_parallel(n, 4ull * n, [&](size_t b, size_t e) { std::fill(res->scalar + b, res->scalar + e, sc); });
   res->n_tracks = hc[2];
   float ms = 0.f;
   cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1);
@@ -2144,19 +2082,19 @@ ftk2b_status run_fiber_surface_extruded(ftk2b_ctx* ctx, const FeGeom& g, const v
   C_TRY(ctx->sync());
   res->n_features = n;
   res->n_cells = nuniq;
-  res->simplices = static_cast<uint64_t*>(ct_host_alloc(24 * ncap));
-  res->lambda = static_cast<double*>(ct_host_alloc(24 * ncap));
-  res->barycentric = static_cast<float*>(ct_host_alloc(12 * ncap));
-  res->track_id = static_cast<uint64_t*>(ct_host_alloc(8 * ncap));
+  res->simplices = static_cast<uint64_t*>(host_alloc(24 * ncap));
+  res->lambda = static_cast<double*>(host_alloc(24 * ncap));
+  res->barycentric = static_cast<float*>(host_alloc(12 * ncap));
+  res->track_id = static_cast<uint64_t*>(host_alloc(8 * ncap));
   res->scalar = static_cast<float*>(std::calloc(ncap, 4));
-  res->cells = static_cast<uint32_t*>(ct_host_alloc(12ull * (nuniq ? nuniq : 1)));
+  res->cells = static_cast<uint32_t*>(host_alloc(12ull * (nuniq ? nuniq : 1)));
   if (!res->simplices || !res->lambda || !res->barycentric || !res->track_id || !res->scalar || !res->cells)
     return cfail(ctx, FTK2B_OOM, "host result allocation failed");
-  C_TRY(ct_d2h(ctx, res->simplices, simp, 24ull * n));
-  C_TRY(ct_d2h(ctx, res->lambda, lam, 24ull * n));
-  C_TRY(ct_d2h(ctx, res->barycentric, bary, 12ull * n));
-  C_TRY(ct_d2h(ctx, res->track_id, track, 8ull * n));
-  C_TRY(ct_d2h(ctx, res->cells, cells_out, 12ull * nuniq));
+  C_TRY(copy_to_host(ctx, {{res->simplices, simp, 24ull * n},
+                           {res->lambda, lam, 24ull * n},
+                           {res->barycentric, bary, 12ull * n},
+                           {res->track_id, track, 8ull * n},
+                           {res->cells, cells_out, 12ull * nuniq}}));
   if (hc[3] & 1u) return cfail(ctx, FTK2B_TIMEOUT, "union-find retry bound reached");
   res->n_tracks = hc[2];
   float ms = 0.f;

@@ -33,6 +33,7 @@
 #include <vector>
 
 #include "cp_api_internal.h"
+#include "cp_host.h"
 #include "cp_stream.h"
 #include "cp_stream_kernels.cuh"
 #include "cp_cull.cuh"
@@ -636,15 +637,6 @@ int grid_of(unsigned long long n, int threads, int max_blocks) {
   return (int)b;
 }
 
-uint64_t hash_cells(const uint64_t* p, uint64_t n) {
-  uint64_t h = 0x9E3779B97F4A7C15ull ^ n;
-  for (uint64_t i = 0; i < n; ++i) {
-    h ^= p[i] + 0x9E3779B97F4A7C15ull + (h << 6) + (h >> 2);
-    h *= 0xBF58476D1CE4E5B9ull;
-  }
-  return h;
-}
-
 ftk2b_status ext_fail(ftk2b_ctx* ctx, ftk2b_status st, const std::string& msg) {
   ctx->err = msg;
   return st;
@@ -682,7 +674,7 @@ ftk2b_status prepare_base(ftk2b_ctx* ctx, const ftk2b_mesh_desc* mesh, int fbits
   ExtCache& C = ctx->ext;
   const int cd = mesh->base_cell_dim;
   const uint64_t nent64 = mesh->n_base_cells * (uint64_t)(cd + 1);
-  const uint64_t h = known_hash ? *known_hash : hash_cells(mesh->base_cells, nent64);
+  const uint64_t h = known_hash ? *known_hash : hash_words(mesh->base_cells, nent64);
   if (C.valid && C.hash == h && C.ncell == mesh->n_base_cells && C.ns == mesh->n_base_verts && C.cd == cd)
     return FTK2B_OK;
   C.valid = false;
@@ -1158,8 +1150,6 @@ ftk2b_status result_extruded_t(ftk2b_stream* s, ftk2b_cp_result** out) {
 }
 
 }  // namespace
-
-uint64_t hash_base_cells(const uint64_t* p, uint64_t n) { return hash_cells(p, n); }
 
 }  // namespace ftk2b
 

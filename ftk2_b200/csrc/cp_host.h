@@ -1,0 +1,69 @@
+// Host memory traffic of the calls that move many megabytes: allocation,
+// copies and content hashes by several threads.
+//
+// One core touches new memory at a few GB/s (a page fault per 4 KB) and copies
+// at about 10, far below the 50 GB/s the device delivers over PCIe, so from
+// kHostThreadBytes on the work is shared by up to kHostThreads threads that
+// live for the call.  Below that, starting them (about 20 us each) costs more
+// than it saves.
+#pragma once
+
+#include <cstddef>
+#include <cstdint>
+#include <functional>
+#include <vector>
+
+#include <cuda_runtime.h>
+
+struct ftk2b_ctx;
+
+namespace ftk2b {
+
+constexpr size_t kHostThreads = 8;
+constexpr size_t kHostThreadBytes = size_t(2) << 20;  // per thread, at least
+
+// f(begin, end) over [0, n) in contiguous shares, one per thread; `bytes` is
+// the memory the whole range touches.  A thread that cannot be started leaves
+// its share to the caller.
+void host_parallel(size_t n, size_t bytes, const std::function<void(size_t, size_t)>& f);
+
+// Memory for a large array, released with free(); from 4 MB on aligned and
+// advised for 2 MB pages, which fault once per 2 MB instead of once per 4 KB.
+void* host_alloc(size_t bytes);
+
+// 64-bit content hash of n words (any change to how it is formed is a change
+// of the checkpoint format: a blob holds it).
+uint64_t hash_words(const uint64_t* p, size_t n);
+
+// Uninitialised array of 64-bit words of host_alloc memory.
+class HostWords {
+ public:
+  HostWords() = default;
+  HostWords(const HostWords&) = delete;
+  HostWords& operator=(const HostWords&) = delete;
+  ~HostWords();
+  bool alloc(size_t n);
+  uint64_t* data() const { return p_; }
+  size_t size() const { return n_; }
+  bool empty() const { return n_ == 0; }
+
+ private:
+  uint64_t* p_ = nullptr;
+  size_t n_ = 0;
+};
+
+// Copies src (any alignment) to dst and returns the words' hash.
+uint64_t copy_hash_words(uint64_t* dst, const void* src, size_t n);
+
+struct HostCopy {
+  void* dst;
+  const void* src;  // device
+  size_t bytes;
+};
+
+// Device arrays to pageable host memory through a ring of pinned chunks of the
+// context: the host threads empty chunks while the next ones arrive.  Waits
+// for the copies (and all work queued on the stream before).
+cudaError_t copy_to_host(ftk2b_ctx* ctx, const std::vector<HostCopy>& copies);
+
+}  // namespace ftk2b

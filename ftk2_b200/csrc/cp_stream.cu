@@ -540,9 +540,12 @@ extern "C" ftk2b_status ftk2b_stream_open(ftk2b_ctx* ctx, const ftk2b_mesh_desc*
     s->d = cd + 1;
     s->m = cd;
     s->emesh = *mesh;
-    s->ecells.assign(mesh->base_cells, mesh->base_cells + mesh->n_base_cells * (cd + 1));
+    if (!s->ecells.alloc(mesh->n_base_cells * (cd + 1))) {
+      delete s;
+      return sfail(ctx, FTK2B_OOM, "host allocation failed");
+    }
     s->emesh.base_cells = s->ecells.data();
-    s->ebase_hash = ftk2b::hash_base_cells(s->ecells.data(), (uint64_t)s->ecells.size());
+    s->ebase_hash = copy_hash_words(s->ecells.data(), mesh->base_cells, s->ecells.size());
     s->slice_elems = mesh->n_base_verts;
   } else {
     delete s;
@@ -660,6 +663,16 @@ struct StreamCkpt {
   uint64_t T, slice_elems;
   uint32_t n, n_edges, n_prev, n_first;
 };
+
+// the content hash that earlier blobs of this version hold: one chain over all words
+uint64_t serial_hash(const uint64_t* p, uint64_t n) {
+  uint64_t h = 0x9E3779B97F4A7C15ull ^ n;
+  for (uint64_t i = 0; i < n; ++i) {
+    h ^= p[i] + 0x9E3779B97F4A7C15ull + (h << 6) + (h >> 2);
+    h *= 0xBF58476D1CE4E5B9ull;
+  }
+  return h;
+}
 
 // the device sections of a stream's state, in blob order
 std::vector<std::pair<ftk2b::DevBuf*, size_t>> ckpt_sections(ftk2b_stream* s) {
@@ -813,11 +826,13 @@ extern "C" ftk2b_status ftk2b_stream_restore(ftk2b_ctx* ctx, const void* buf, ui
   }
   if (!regular) {
     s->emesh = h.emesh;
-    s->ecells.resize(h.n_ecells);  // the caller's blob need not be 8-byte aligned
-    memcpy(s->ecells.data(), p, 8 * h.n_ecells);
+    if (!s->ecells.alloc(h.n_ecells)) {
+      delete s;
+      return sfail(ctx, FTK2B_OOM, "host allocation failed");
+    }
     s->emesh.base_cells = s->ecells.data();
-    s->ebase_hash = ftk2b::hash_base_cells(s->ecells.data(), (uint64_t)s->ecells.size());
-    if (s->ebase_hash != h.ebase_hash) {
+    s->ebase_hash = copy_hash_words(s->ecells.data(), p, s->ecells.size());  // the caller's blob need not be aligned
+    if (s->ebase_hash != h.ebase_hash && serial_hash(s->ecells.data(), s->ecells.size()) != h.ebase_hash) {
       delete s;
       return sfail(ctx, FTK2B_INVALID_ARG, "stream checkpoint's base cells are damaged");
     }

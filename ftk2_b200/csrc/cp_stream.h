@@ -1,9 +1,8 @@
 // Time streams: a spatial mesh whose timesteps arrive one at a time.
 #pragma once
 
-#include <vector>
-
 #include "cp_api_internal.h"
+#include "cp_host.h"
 
 struct ftk2b_stream {
   ftk2b_ctx* ctx = nullptr;
@@ -17,7 +16,7 @@ struct ftk2b_stream {
   uint64_t ld[3] = {0, 0, 0}, off[3] = {0, 0, 0}, gd[3] = {0, 0, 0}, adims[3] = {0, 0, 0};
   // extruded: the base mesh (cells copied at open)
   ftk2b_mesh_desc emesh;
-  std::vector<uint64_t> ecells;
+  ftk2b::HostWords ecells;
   uint64_t ebase_hash = 0;     // content hash of ecells (computed once)
 
   uint64_t T = 0;              // timesteps pushed
@@ -48,8 +47,6 @@ namespace ftk2b {
 cudaError_t grow_keep(DevBuf& b, size_t used, size_t want, cudaStream_t st);
 // grows the feature store (and union-find / boundary lists) to hold `want`
 ftk2b_status ensure_stream_store(ftk2b_stream* s, unsigned want);
-// content hash of an extruded mesh's base cells (the prepared-mesh cache key)
-uint64_t hash_base_cells(const uint64_t* p, uint64_t n);
 
 }  // namespace ftk2b
 
