@@ -860,6 +860,52 @@ __global__ void ext_window_fill_kernel(const unsigned* __restrict__ ids, const u
   }
 }
 
+// The window in Simplex order by one rank sort of its tuples (cp_ranksort.cuh):
+// the spatial features of the previous layer, then the new ones, which also
+// become components of their own and, when they lie in the newest layer, go
+// to its list.
+struct LoadTuple {
+  const unsigned long long *hi, *lo;
+  const unsigned* prev;  // null: ids 0, 1, ..
+  unsigned n_prev, first_new;
+  __device__ __forceinline__ unsigned id(unsigned i) const {
+    return i < n_prev ? prev[i] : first_new + (i - n_prev);
+  }
+  __device__ __forceinline__ void operator()(unsigned i, unsigned long long (&k)[2]) const {
+    const unsigned j = id(i);
+    k[0] = hi[j];
+    k[1] = lo[j];
+  }
+};
+template <int M>
+struct StoreTuple {
+  LoadTuple in;
+  unsigned long long *hi_s, *lo_s;
+  const unsigned* phase;
+  unsigned *phase_s, *ids;
+  unsigned* parent;
+  unsigned *newest, *n_newest;
+  unsigned long long ns, t;
+  __device__ __forceinline__ void operator()(unsigned pos, unsigned i, const unsigned long long (&k)[2]) const {
+    const unsigned id = in.id(i);
+    hi_s[pos] = k[0];
+    lo_s[pos] = k[1];
+    phase_s[pos] = phase[id];
+    ids[pos] = id;
+    if (i < in.n_prev) return;
+    parent[id] = id;
+    unsigned long long v[4];
+    unpack_tuple<M>(k[0], k[1], kStreamVb, v);
+    if (v[0] / ns == t && v[M] / ns == t) newest[atomicAdd(n_newest, 1u)] = id;
+  }
+};
+struct StoreTupleOrder {
+  StoreOrder order;
+  __device__ __forceinline__ void operator()(unsigned pos, unsigned i, const unsigned long long (&)[2]) const {
+    order.put(pos, i);
+  }
+};
+
 // window star edges (packed window indices) -> stream ids, united and stored
 __global__ void ext_append_edges_kernel(const unsigned long long* __restrict__ ek, const unsigned* n_ptr,
                                         unsigned cap, const unsigned* __restrict__ ids, unsigned* parent,
@@ -1025,16 +1071,28 @@ ftk2b_status push_extruded_t(ftk2b_stream* s) {
     s->edge_cap = nc;
   }
   const int g = grid_of(wcap, 256, 4096);
-  set_u32_kernel<<<1, 1, 0, st>>>(counters + kSWin, nS);
-  ext_window_build_kernel<<<g, 256, 0, st>>>((const unsigned long long*)s->lo.p, (const unsigned*)s->prev_ids.p,
-                                             s->n_prev, first_new, n_new, (unsigned long long*)s->s_key.p,
-                                             (unsigned*)s->s_id.p);
-  const int bits = kStreamVb + bits_of(ns * (tnow + 1));
-  const unsigned* ids = sort_by_tuple(ctx, s, counters + kSWin, wcap, bits, &nl);
-  ext_window_fill_kernel<<<g, 256, 0, st>>>(ids, counters + kSWin, wcap, (const unsigned long long*)s->hi.p,
-                                            (const unsigned long long*)s->lo.p, (const unsigned*)s->phase.p,
-                                            (unsigned long long*)s->s_hi.p, (unsigned long long*)s->s_lo.p,
-                                            (unsigned*)s->s_phase.p);
+  const bool ranked = wcap <= kRankCap2;
+  const unsigned* ids;
+  if (ranked) {
+    const LoadTuple ld{(const unsigned long long*)s->hi.p, (const unsigned long long*)s->lo.p,
+                       (const unsigned*)s->prev_ids.p, s->n_prev, first_new};
+    const StoreTuple<M> sw{ld, (unsigned long long*)s->s_hi.p, (unsigned long long*)s->s_lo.p,
+                           (const unsigned*)s->phase.p, (unsigned*)s->s_phase.p, (unsigned*)s->s_id.p,
+                           (unsigned*)s->parent.p, (unsigned*)s->prev_ids2.p, counters + kSPrev, ns, tnow};
+    EXT_TRY(launch_rank_sort<2>(ld, sw, nullptr, nS, counters + kSWin, ctx->num_sms, st));
+    ids = sw.ids;
+  } else {
+    set_u32_kernel<<<1, 1, 0, st>>>(counters + kSWin, nS);
+    ext_window_build_kernel<<<g, 256, 0, st>>>((const unsigned long long*)s->lo.p, (const unsigned*)s->prev_ids.p,
+                                               s->n_prev, first_new, n_new, (unsigned long long*)s->s_key.p,
+                                               (unsigned*)s->s_id.p);
+    const int bits = kStreamVb + bits_of(ns * (tnow + 1));
+    ids = sort_by_tuple(ctx, s, counters + kSWin, wcap, bits, &nl);
+    ext_window_fill_kernel<<<g, 256, 0, st>>>(ids, counters + kSWin, wcap, (const unsigned long long*)s->hi.p,
+                                              (const unsigned long long*)s->lo.p, (const unsigned*)s->phase.p,
+                                              (unsigned long long*)s->s_hi.p, (unsigned long long*)s->s_lo.p,
+                                              (unsigned*)s->s_phase.p);
+  }
   ExtFeatures Fs;
   Fs.hi = (const unsigned long long*)s->s_hi.p;
   Fs.lo = (const unsigned long long*)s->s_lo.p;
@@ -1048,18 +1106,20 @@ ftk2b_status push_extruded_t(ftk2b_stream* s) {
   ext_edges_kernel<M, 0><<<g, 256, 0, st>>>(X, Fs, ecnt, nullptr, ek, wecap, err);
   EXT_TRY(launch_scan(ecnt, wcap, counters + kSWinEdges, counters + kSWin, st));
   ext_edges_kernel<M, 1><<<g, 256, 0, st>>>(X, Fs, nullptr, ecnt, ek, wecap, err);
-  if (n_new) uf_init_range_kernel<<<grid_of(n_new, 256, 4096), 256, 0, st>>>((unsigned*)s->parent.p, first_new, n_new);
+  if (n_new && !ranked)
+    uf_init_range_kernel<<<grid_of(n_new, 256, 4096), 256, 0, st>>>((unsigned*)s->parent.p, first_new, n_new);
   ext_append_edges_kernel<<<grid_of(wecap, 256, 4096), 256, 0, st>>>(ek, counters + kSWinEdges, wecap, ids,
                                                                     (unsigned*)s->parent.p, (unsigned*)s->edges.p,
                                                                     s->n_edges, s->edge_cap, err);
   if (M == 3) ext_coface_union_kernel<<<g, 256, 0, st>>>(X, Fs, ids, (unsigned*)s->parent.p, err);
-  if (n_new)
+  if (n_new && !ranked)
     ext_collect_spatial_kernel<M><<<grid_of(n_new, 256, 4096), 256, 0, st>>>(
         (const unsigned long long*)s->hi.p, (const unsigned long long*)s->lo.p, first_new, n_new, ns, tnow,
         (unsigned*)s->prev_ids2.p, counters + kSPrev);
   nl += 9;
   EXT_TRY(cudaGetLastError());
   EXT_TRY(cudaMemcpyAsync(ctx->h_counters, counters, sizeof(unsigned) * kNumCounters, cudaMemcpyDeviceToHost, st));
+  EXT_TRY(cudaEventRecord(ctx->ev1, st));
   EXT_TRY(ctx->sync());
   ctx->launches += nl;
   const unsigned* h = ctx->h_counters;
@@ -1101,17 +1161,24 @@ ftk2b_status result_extruded_t(ftk2b_stream* s, ftk2b_cp_result** out) {
   EXT_TRY(ctx->hist.ensure(sizeof(unsigned) * 256 * (size_t)ctx->sort_grid(mc)));
   const int g = grid_of(mc, 256, 4096);
   EXT_TRY(cudaMemsetAsync(counters, 0, sizeof(unsigned) * kNumCounters, st));
-  set_u32_kernel<<<1, 1, 0, st>>>(counters + kSWin, n);
-  set_u32_kernel<<<1, 1, 0, st>>>(counters + kSWinEdges, ne);
-  if (n) EXT_TRY(cudaMemcpyAsync(s->s_key.p, s->lo.p, 8 * (size_t)n, cudaMemcpyDeviceToDevice, st));
-  iota_u32_kernel<<<g, 256, 0, st>>>((unsigned*)s->s_id.p, n);
-  const unsigned long long ns = s->emesh.n_base_verts;
-  const unsigned* perm = sort_by_tuple(ctx, s, counters + kSWin, nc, kStreamVb + bits_of(ns * (s->T + 1)), &nl);
   unsigned* inv = (unsigned*)ctx->perm0.p;
   unsigned* root = (unsigned*)ctx->perm1.p;
   unsigned* cmin = (unsigned*)ctx->parent.p;
-  invert_kernel<<<g, 256, 0, st>>>(perm, n, inv);
-  fill_u32_kernel<<<g, 256, 0, st>>>(cmin, n, 0xFFFFFFFFu);
+  const unsigned* perm;
+  if (nc <= kRankCap2) {
+    const LoadTuple ld{(const unsigned long long*)s->hi.p, (const unsigned long long*)s->lo.p, nullptr, 0u, 0u};
+    const StoreTupleOrder so{{(unsigned*)s->s_id.p, inv, cmin}};
+    EXT_TRY(launch_rank_sort<2>(ld, so, nullptr, n, counters + kSWin, ctx->num_sms, st));
+    perm = so.order.perm;
+  } else {
+    set_u32_kernel<<<1, 1, 0, st>>>(counters + kSWin, n);
+    EXT_TRY(cudaMemcpyAsync(s->s_key.p, s->lo.p, 8 * (size_t)n, cudaMemcpyDeviceToDevice, st));
+    iota_u32_kernel<<<g, 256, 0, st>>>((unsigned*)s->s_id.p, n);
+    const unsigned long long ns = s->emesh.n_base_verts;
+    perm = sort_by_tuple(ctx, s, counters + kSWin, nc, kStreamVb + bits_of(ns * (s->T + 1)), &nl);
+    invert_kernel<<<g, 256, 0, st>>>(perm, n, inv);
+    fill_u32_kernel<<<g, 256, 0, st>>>(cmin, n, 0xFFFFFFFFu);
+  }
   comp_min_kernel<<<g, 256, 0, st>>>((unsigned*)s->parent.p, inv, n, root, cmin, counters + kCountRoots);
   gather_result_kernel<<<g, 256, 0, st>>>(perm, n, root, cmin, (const double*)s->lam.p, (const float*)s->bary4.p,
                                           (const float*)s->scalar.p, (const unsigned*)s->cls.p, (double*)ctx->lam_s.p,
@@ -1120,25 +1187,18 @@ ftk2b_status result_extruded_t(ftk2b_stream* s, ftk2b_cp_result** out) {
   ext_stream_expand_kernel<M><<<g, 256, 0, st>>>(perm, n, (const unsigned long long*)s->hi.p,
                                                  (const unsigned long long*)s->lo.p, (const float*)ctx->bary4_s.p,
                                                  (unsigned long long*)ctx->simplices.p, (float*)ctx->bary.p);
-  // edges in canonical ids, sorted; the id buffers are free after the gathers
-  unsigned long long* ek = (unsigned long long*)(perm == (const unsigned*)s->s_id.p ? s->s_key2.p : s->s_key.p);
-  unsigned long long* ek2 = (unsigned long long*)(perm == (const unsigned*)s->s_id.p ? s->s_key.p : s->s_key2.p);
-  canon_edges_kernel<<<g, 256, 0, st>>>((const unsigned*)s->edges.p, ne, inv, ek);
-  const bool ealt = radix_sort(ek, (unsigned*)s->s_id.p, ek2, (unsigned*)s->s_id2.p, counters + kSWinEdges, ec, 64,
-                               (unsigned*)ctx->hist.p, ctx->sort_grid(mc), st, &nl);
-  unpack_edges_kernel<<<g, 256, 0, st>>>(ealt ? ek2 : ek, ne, (unsigned*)ctx->edges.p);
-  nl += 8;
+  nl += 4;
   EXT_TRY(cudaGetLastError());
-  EXT_TRY(cudaMemcpyAsync(ctx->h_counters, counters, sizeof(unsigned) * kNumCounters, cudaMemcpyDeviceToHost, st));
-  EXT_TRY(ctx->sync());
   ctx->launches += nl;
+  // edges in canonical ids, sorted; the id and key buffers are free after the gathers
+  const ftk2b_status rc = canonical_edges(s, inv, (unsigned long long*)s->s_key.p, (unsigned long long*)s->s_key2.p);
+  if (rc) return rc;
   ctx->last.kind = FTK2B_MESH_EXTRUDED;
   ctx->last.m = M;
   ctx->last.f64 = s->dtype == FTK2B_F64;
   ctx->pack_ready = false;
   ctx->last.n = n;
   ctx->last.ne = s->prm.want_edges ? ne : 0;
-  ctx->last.n_roots = ctx->h_counters[kCountRoots];
   // m-simplices of the T-timestep mesh, from the prepared base mesh's counts
   const uint64_t L = s->T ? s->T - 1 : 0;
   ctx->last.n_simplices =
@@ -1146,7 +1206,7 @@ ftk2b_status result_extruded_t(ftk2b_stream* s, ftk2b_cp_result** out) {
   ctx->last.device_ms = 0;
   ctx->last.classify = 0;
   ctx->last.want_edges = s->prm.want_edges;
-  return ftk2b_cp_fetch(ctx, out);
+  return stream_fetch(s, out);
 }
 
 }  // namespace

@@ -1082,14 +1082,23 @@ cudaError_t launch_uf_label(unsigned* parent, const unsigned* n_ptr, unsigned ca
   return cudaGetLastError();
 }
 
+cudaError_t launch_window_star_slots(const RegularMesh& mesh, int nch, const unsigned long long* skeys,
+                                     const unsigned* n_ptr, unsigned cap, unsigned* edge_cnt, unsigned* edge_slots,
+                                     unsigned* n_edges, cudaStream_t st) {
+  edges_regular_warp_kernel<<<grid_for(cap, 8, 8192), 256, 0, st>>>(mesh, nch, skeys, n_ptr, cap, edge_cnt,
+                                                                   edge_slots);
+  scan_inplace_kernel<<<1, 1024, 0, st>>>(edge_cnt, cap, n_edges, n_ptr, nullptr);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_window_edges_regular(const RegularMesh& mesh, int nch, const unsigned long long* skeys,
                                         const unsigned* n_ptr, unsigned cap, unsigned* edge_cnt,
                                         unsigned* edge_slots, unsigned* edges, unsigned* n_edges,
                                         unsigned edge_cap, cudaStream_t st) {
   const int g = grid_for(cap, 256, 4096);
-  edges_regular_warp_kernel<<<grid_for(cap, 8, 8192), 256, 0, st>>>(mesh, nch, skeys, n_ptr, cap, edge_cnt,
-                                                                   edge_slots);
-  scan_inplace_kernel<<<1, 1024, 0, st>>>(edge_cnt, cap, n_edges, n_ptr, nullptr);
+  const cudaError_t e =
+      launch_window_star_slots(mesh, nch, skeys, n_ptr, cap, edge_cnt, edge_slots, n_edges, st);
+  if (e) return e;
   edges_compact_kernel<<<g, 256, 0, st>>>(n_ptr, cap, edge_cnt, n_edges, edge_slots, edges, edge_cap);
   return cudaGetLastError();
 }

@@ -1,0 +1,91 @@
+// Sorting a few thousand keys in one launch: every block copies all keys into
+// shared memory and each warp counts, for four keys at a time, the keys below
+// them; a key's rank is its place.
+//
+// n^2 / 32 warp steps in all, each a shared-memory read and four compares, so
+// a few thousand keys are bound by the launch.  An LSD radix sort of the same
+// keys is three launches per 8 bits, and a 55-bit tuple takes two such sorts.  A
+// stream's push, whose window of some 500 features was sorted that way, went
+// from 165 to 110 us (96 x 101 x 88 float) and from 880 to 720 us (100 x 100 x 40
+// tets); its result from 270 to 102 us (2,200 features).  Sets beyond what
+// shared memory holds take the radix passes.
+#pragma once
+
+#include <cuda_runtime.h>
+
+#include "cp_pdl.cuh"
+
+namespace ftk2b {
+
+constexpr int kRankThreads = 512;
+constexpr unsigned kRankCap1 = 24576;  // keys of one word: 192 KB
+constexpr unsigned kRankCap2 = 12288;  // keys of two words
+
+// Keys of W 64-bit words, compared word by word, equal keys by index.
+//   load(i, k)          writes the W words of key i
+//   store(pos, i, k)    called once per key: key i is the pos-th smallest
+// for i < n = min(*n_ptr, cap) (n_ptr null: cap); n is also written to *n_out
+// when that is not null.  Shared memory: W * cap words.
+template <int W, typename Load, typename Store>
+__global__ void __launch_bounds__(kRankThreads, 1)
+    rank_sort_kernel(Load load, Store store, const unsigned* n_ptr, unsigned cap, unsigned* n_out) {
+  extern __shared__ unsigned long long rank_keys[];
+  pdl_enter();
+  const unsigned n = n_ptr ? min(*n_ptr, cap) : cap;
+  if (n_out && blockIdx.x == 0 && threadIdx.x == 0) *n_out = n;
+  if (blockIdx.x * (kRankThreads / 8) >= n) return;  // no key of this block's
+  for (unsigned i = threadIdx.x; i < n; i += kRankThreads) {
+    unsigned long long k[W];
+    load(i, k);
+#pragma unroll
+    for (int w = 0; w < W; ++w) rank_keys[w * (size_t)cap + i] = k[w];
+  }
+  __syncthreads();
+  constexpr int U = 4;
+  const unsigned lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (unsigned e0 = (blockIdx.x * (kRankThreads / 32) + warp) * U; e0 < n;
+       e0 += gridDim.x * (kRankThreads / 32) * U) {
+    unsigned long long k[U][W];
+    unsigned below[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      below[u] = 0;
+#pragma unroll
+      for (int w = 0; w < W; ++w) k[u][w] = rank_keys[w * (size_t)cap + min(e0 + u, n - 1)];
+    }
+    for (unsigned j = lane; j < n; j += 32) {
+      unsigned long long x[W];
+#pragma unroll
+      for (int w = 0; w < W; ++w) x[w] = rank_keys[w * (size_t)cap + j];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        bool less = j < e0 + u;
+#pragma unroll
+        for (int w = W - 1; w >= 0; --w) less = x[w] < k[u][w] || (x[w] == k[u][w] && less);
+        below[u] += less ? 1u : 0u;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const unsigned pos = __reduce_add_sync(0xFFFFFFFFu, below[u]);
+      if (lane == (unsigned)u && e0 + u < n) store(pos, e0 + u, k[u]);
+    }
+  }
+}
+
+template <int W, typename Load, typename Store>
+inline cudaError_t launch_rank_sort(const Load& load, const Store& store, const unsigned* n_ptr, unsigned cap,
+                                    unsigned* n_out, int num_sms, cudaStream_t st) {
+  auto k = rank_sort_kernel<W, Load, Store>;
+  const size_t smem = 8 * (size_t)W * (cap ? cap : 1);
+  // always the most any call needs: another thread may be launching the same kernel
+  constexpr int kMost = 8 * (W == 1 ? kRankCap1 : W * kRankCap2);
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost);
+  if (e) return e;
+  unsigned grid = (cap + kRankThreads / 8 - 1) / (kRankThreads / 8);
+  if (grid > (unsigned)num_sms) grid = (unsigned)num_sms;
+  k<<<grid ? grid : 1, kRankThreads, smem, st>>>(load, store, n_ptr, cap, n_out);
+  return cudaGetLastError();
+}
+
+}  // namespace ftk2b

@@ -76,6 +76,68 @@ __global__ void window_build_kernel(const unsigned long long* __restrict__ key, 
   }
 }
 
+// The window in key order by one rank sort (cp_ranksort.cuh): the spatial
+// features of the previous layer, then the new ones, which also become
+// components of their own and, when they lie in the newest layer, go to its list.
+struct LoadWindow {
+  const unsigned long long* key;
+  const unsigned* prev;
+  unsigned n_prev, first_new;
+  __device__ __forceinline__ unsigned id(unsigned i) const {
+    return i < n_prev ? prev[i] : first_new + (i - n_prev);
+  }
+  __device__ __forceinline__ void operator()(unsigned i, unsigned long long (&k)[1]) const { k[0] = key[id(i)]; }
+};
+struct StoreWindow {
+  LoadWindow in;
+  unsigned long long* skey;
+  unsigned* sid;
+  unsigned* parent;
+  unsigned *newest, *n_newest;
+  int nch;
+  unsigned long long time_chains;
+  __device__ __forceinline__ void operator()(unsigned pos, unsigned i, const unsigned long long (&k)[1]) const {
+    const unsigned id = in.id(i);
+    skey[pos] = k[0];
+    sid[pos] = id;
+    if (i < in.n_prev) return;
+    parent[id] = id;
+    if (!((time_chains >> (unsigned)(k[0] % (unsigned long long)nch)) & 1ull)) newest[atomicAdd(n_newest, 1u)] = id;
+  }
+};
+struct LoadKey {
+  const unsigned long long* key;
+  __device__ __forceinline__ void operator()(unsigned i, unsigned long long (&k)[1]) const { k[0] = key[i]; }
+};
+struct StoreCanon {
+  StoreOrder order;
+  unsigned long long* skey;
+  __device__ __forceinline__ void operator()(unsigned pos, unsigned i, const unsigned long long (&k)[1]) const {
+    skey[pos] = k[0];
+    order.put(pos, i);
+  }
+};
+
+// The window's star edges, from their padded slots (off: scanned counts), as
+// stream ids: united and appended to the store's edges.
+__global__ void append_star_edges_kernel(const unsigned* n_ptr, unsigned cap, const unsigned* __restrict__ off,
+                                         const unsigned* n_edges, const unsigned* __restrict__ slots,
+                                         const unsigned* __restrict__ s_id, unsigned* parent,
+                                         unsigned* __restrict__ out, unsigned base, unsigned out_cap, unsigned* err) {
+  const unsigned n = min(*n_ptr, cap), ne = *n_edges;
+  // a thread per slot: the lanes of a feature unite side by side
+  for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < 8 * n; t += gridDim.x * blockDim.x) {
+    const unsigned i = t >> 3, k = t & 7, o = off[i];
+    if (k >= (i + 1 < n ? off[i + 1] : ne) - o) continue;
+    const unsigned a = s_id[i], b = s_id[slots[t]];
+    if (o + k < out_cap - base) {
+      out[2 * (size_t)(base + o + k)] = a;
+      out[2 * (size_t)(base + o + k) + 1] = b;
+    }
+    uf_unite(parent, a, b, err);
+  }
+}
+
 __global__ void append_edges_kernel(const unsigned* __restrict__ wedges, const unsigned* wn_ptr, unsigned wcap,
                                     const unsigned* __restrict__ s_id, unsigned* parent, unsigned* __restrict__ out,
                                     unsigned base, unsigned out_cap, unsigned* err) {
@@ -272,30 +334,44 @@ ftk2b_status push_regular(ftk2b_stream* s) {
     S_TRY(ctx, grow_keep(s->edges, 8 * (size_t)s->n_edges, 8 * (size_t)nc, st));
     s->edge_cap = nc;
   }
-  const int g = grid_of(wcap, 256, 4096);
-  set_u32_kernel<<<1, 1, 0, st>>>(counters + kSWin, nS);
-  window_build_kernel<<<g, 256, 0, st>>>((const unsigned long long*)s->key.p, (const unsigned*)s->prev_ids.p,
-                                         s->n_prev, first_new, n_new, (unsigned long long*)s->s_key.p,
-                                         (unsigned*)s->s_id.p);
-  const unsigned long long nv_hi = (unsigned long long)rm.gstride[d - 1] * (T + 1);
-  const int key_bits = bits_for(nv_hi * (unsigned long long)nch);
-  const bool alt = radix_sort((unsigned long long*)s->s_key.p, (unsigned*)s->s_id.p,
-                              (unsigned long long*)s->s_key2.p, (unsigned*)s->s_id2.p, counters + kSWin, wcap,
-                              key_bits, (unsigned*)ctx->hist.p, sgrid, st, &ctx->launches);
-  const unsigned long long* skeys = (const unsigned long long*)(alt ? s->s_key2.p : s->s_key.p);
-  const unsigned* sids = (const unsigned*)(alt ? s->s_id2.p : s->s_id.p);
-  S_TRY(ctx, launch_window_edges_regular(rm, nch, skeys, counters + kSWin, wcap, (unsigned*)ctx->edge_cnt.p,
-                                         (unsigned*)ctx->edge_slots.p, (unsigned*)s->wedges.p,
-                                         counters + kSWinEdges, 8 * wcap, st));
-  if (n_new) uf_init_range_kernel<<<grid_of(n_new, 256, 4096), 256, 0, st>>>((unsigned*)s->parent.p, first_new, n_new);
-  append_edges_kernel<<<grid_of(8ull * wcap, 256, 4096), 256, 0, st>>>(
-      (const unsigned*)s->wedges.p, counters + kSWinEdges, 8 * wcap, sids, (unsigned*)s->parent.p,
-      (unsigned*)s->edges.p, s->n_edges, s->edge_cap, counters + kCountErr);
-  if (n_new)
-    collect_spatial_kernel<<<grid_of(n_new, 256, 4096), 256, 0, st>>>(
-        (const unsigned long long*)s->key.p, first_new, n_new, nch, time_chain_mask(d), (unsigned*)s->prev_ids2.p,
-        counters + kSPrev);
-  ctx->launches += 8;
+  if (wcap <= kRankCap1) {
+    LoadWindow ld{(const unsigned long long*)s->key.p, (const unsigned*)s->prev_ids.p, s->n_prev, first_new};
+    StoreWindow sw{ld, (unsigned long long*)s->s_key2.p, (unsigned*)s->s_id2.p, (unsigned*)s->parent.p,
+                   (unsigned*)s->prev_ids2.p, counters + kSPrev, nch, time_chain_mask(d)};
+    S_TRY(ctx, launch_rank_sort<1>(ld, sw, nullptr, nS, counters + kSWin, ctx->num_sms, st));
+    S_TRY(ctx, launch_window_star_slots(rm, nch, sw.skey, counters + kSWin, wcap, (unsigned*)ctx->edge_cnt.p,
+                                        (unsigned*)ctx->edge_slots.p, counters + kSWinEdges, st));
+    append_star_edges_kernel<<<grid_of(8ull * wcap, 256, 4096), 256, 0, st>>>(
+        counters + kSWin, wcap, (const unsigned*)ctx->edge_cnt.p, counters + kSWinEdges,
+        (const unsigned*)ctx->edge_slots.p, sw.sid, (unsigned*)s->parent.p, (unsigned*)s->edges.p, s->n_edges,
+        s->edge_cap, counters + kCountErr);
+    ctx->launches += 4;
+  } else {
+    const int g = grid_of(wcap, 256, 4096);
+    set_u32_kernel<<<1, 1, 0, st>>>(counters + kSWin, nS);
+    window_build_kernel<<<g, 256, 0, st>>>((const unsigned long long*)s->key.p, (const unsigned*)s->prev_ids.p,
+                                           s->n_prev, first_new, n_new, (unsigned long long*)s->s_key.p,
+                                           (unsigned*)s->s_id.p);
+    const unsigned long long nv_hi = (unsigned long long)rm.gstride[d - 1] * (T + 1);
+    const int key_bits = bits_for(nv_hi * (unsigned long long)nch);
+    const bool alt = radix_sort((unsigned long long*)s->s_key.p, (unsigned*)s->s_id.p,
+                                (unsigned long long*)s->s_key2.p, (unsigned*)s->s_id2.p, counters + kSWin, wcap,
+                                key_bits, (unsigned*)ctx->hist.p, sgrid, st, &ctx->launches);
+    const unsigned long long* skeys = (const unsigned long long*)(alt ? s->s_key2.p : s->s_key.p);
+    const unsigned* sids = (const unsigned*)(alt ? s->s_id2.p : s->s_id.p);
+    S_TRY(ctx, launch_window_edges_regular(rm, nch, skeys, counters + kSWin, wcap, (unsigned*)ctx->edge_cnt.p,
+                                           (unsigned*)ctx->edge_slots.p, (unsigned*)s->wedges.p,
+                                           counters + kSWinEdges, 8 * wcap, st));
+    if (n_new) uf_init_range_kernel<<<grid_of(n_new, 256, 4096), 256, 0, st>>>((unsigned*)s->parent.p, first_new, n_new);
+    append_edges_kernel<<<grid_of(8ull * wcap, 256, 4096), 256, 0, st>>>(
+        (const unsigned*)s->wedges.p, counters + kSWinEdges, 8 * wcap, sids, (unsigned*)s->parent.p,
+        (unsigned*)s->edges.p, s->n_edges, s->edge_cap, counters + kCountErr);
+    if (n_new)
+      collect_spatial_kernel<<<grid_of(n_new, 256, 4096), 256, 0, st>>>(
+          (const unsigned long long*)s->key.p, first_new, n_new, nch, time_chain_mask(d), (unsigned*)s->prev_ids2.p,
+          counters + kSPrev);
+    ctx->launches += 8;
+  }
 
   // classification while the window's values are resident: the new features,
   // and at the second push the first layer's (their coface lies in slab [0, 1])
@@ -320,6 +396,7 @@ ftk2b_status push_regular(ftk2b_stream* s) {
     if (T == 1) S_TRY(ctx, classify(0, s->n_first, counters + kCountRoots));
   }
   S_TRY(ctx, cudaMemcpyAsync(ctx->h_counters, counters, sizeof(unsigned) * kNumCounters, cudaMemcpyDeviceToHost, st));
+  S_TRY(ctx, cudaEventRecord(ctx->ev1, st));
   S_TRY(ctx, ctx->sync());
   const unsigned* h = ctx->h_counters;
   if (h[kCountErr] & 1u) return sfail(ctx, FTK2B_TIMEOUT, "union-find retry bound reached");
@@ -338,6 +415,7 @@ ftk2b_status result_regular(ftk2b_stream* s, ftk2b_cp_result** out) {
   const int d = s->d, M = s->m, nch = d == 3 ? 12 : 60;
   const unsigned n = s->n, ne = s->n_edges;
   const unsigned nc = n ? n : 1, ec = ne ? ne : 1;
+  ftk2b_status rc = FTK2B_OK;
   S_TRY(ctx, ctx->counters.ensure(sizeof(unsigned) * kNumCounters));
   unsigned* counters = (unsigned*)ctx->counters.p;
   // canonical order of the whole store
@@ -360,22 +438,32 @@ ftk2b_status result_regular(ftk2b_stream* s, ftk2b_cp_result** out) {
   S_TRY(ctx, ctx->hist.ensure(sizeof(unsigned) * 256 * (size_t)sgrid));
   const int g = grid_of(nc > ec ? nc : ec, 256, 4096);
   S_TRY(ctx, cudaMemsetAsync(counters, 0, sizeof(unsigned) * kNumCounters, st));
-  set_u32_kernel<<<1, 1, 0, st>>>(counters + kSWin, n);
-  set_u32_kernel<<<1, 1, 0, st>>>(counters + kSWinEdges, ne);
-  if (n) S_TRY(ctx, cudaMemcpyAsync(s->s_key.p, s->key.p, 8 * (size_t)n, cudaMemcpyDeviceToDevice, st));
-  iota_u32_kernel<<<g, 256, 0, st>>>((unsigned*)s->s_id.p, n);
   const RegularMesh full = window_mesh(s, 0, s->T);
-  const unsigned long long nv_hi = (unsigned long long)full.gstride[d - 1] * (s->T + 1);
-  const bool alt = radix_sort((unsigned long long*)s->s_key.p, (unsigned*)s->s_id.p, (unsigned long long*)s->s_key2.p,
-                              (unsigned*)s->s_id2.p, counters + kSWin, nc, bits_for(nv_hi * (unsigned long long)nch),
-                              (unsigned*)ctx->hist.p, sgrid, st, &ctx->launches);
-  const unsigned long long* skeys = (const unsigned long long*)(alt ? s->s_key2.p : s->s_key.p);
-  const unsigned* perm = (const unsigned*)(alt ? s->s_id2.p : s->s_id.p);
   unsigned* inv = (unsigned*)ctx->perm0.p;
   unsigned* root = (unsigned*)ctx->perm1.p;
   unsigned* cmin = (unsigned*)ctx->parent.p;
-  invert_kernel<<<g, 256, 0, st>>>(perm, n, inv);
-  fill_u32_kernel<<<g, 256, 0, st>>>(cmin, n, 0xFFFFFFFFu);
+  const unsigned long long* skeys;
+  const unsigned* perm;
+  if (nc <= kRankCap1) {
+    const StoreCanon sc{{(unsigned*)s->s_id.p, inv, cmin}, (unsigned long long*)s->s_key.p};
+    S_TRY(ctx, launch_rank_sort<1>(LoadKey{(const unsigned long long*)s->key.p}, sc, nullptr, n, counters + kSWin,
+                                   ctx->num_sms, st));
+    skeys = sc.skey;
+    perm = sc.order.perm;
+  } else {
+    set_u32_kernel<<<1, 1, 0, st>>>(counters + kSWin, n);
+    S_TRY(ctx, cudaMemcpyAsync(s->s_key.p, s->key.p, 8 * (size_t)n, cudaMemcpyDeviceToDevice, st));
+    iota_u32_kernel<<<g, 256, 0, st>>>((unsigned*)s->s_id.p, n);
+    const unsigned long long nv_hi = (unsigned long long)full.gstride[d - 1] * (s->T + 1);
+    const bool alt = radix_sort((unsigned long long*)s->s_key.p, (unsigned*)s->s_id.p,
+                                (unsigned long long*)s->s_key2.p, (unsigned*)s->s_id2.p, counters + kSWin, nc,
+                                bits_for(nv_hi * (unsigned long long)nch), (unsigned*)ctx->hist.p, sgrid, st,
+                                &ctx->launches);
+    skeys = (const unsigned long long*)(alt ? s->s_key2.p : s->s_key.p);
+    perm = (const unsigned*)(alt ? s->s_id2.p : s->s_id.p);
+    invert_kernel<<<g, 256, 0, st>>>(perm, n, inv);
+    fill_u32_kernel<<<g, 256, 0, st>>>(cmin, n, 0xFFFFFFFFu);
+  }
   comp_min_kernel<<<g, 256, 0, st>>>((unsigned*)s->parent.p, inv, n, root, cmin, counters + kCountRoots);
   gather_result_kernel<<<g, 256, 0, st>>>(perm, n, root, cmin, (const double*)s->lam.p, (const float*)s->bary4.p,
                                           (const float*)s->scalar.p, (const unsigned*)s->cls.p,
@@ -383,16 +471,10 @@ ftk2b_status result_regular(ftk2b_stream* s, ftk2b_cp_result** out) {
                                           (unsigned*)ctx->cls.p, (unsigned long long*)ctx->track.p);
   S_TRY(ctx, launch_expand_regular(full, nch, skeys, counters + kSWin, nc, (const float*)ctx->bary4_s.p,
                                    (unsigned long long*)ctx->simplices.p, (float*)ctx->bary.p, st));
+  ctx->launches += 4;
   // edges in canonical ids, sorted (each pair spans one top cell: no duplicates)
-  unsigned long long* ek = (unsigned long long*)s->s_key.p;  // free again after the gathers
-  canon_edges_kernel<<<g, 256, 0, st>>>((const unsigned*)s->edges.p, ne, inv, ek);
-  const bool ealt = radix_sort(ek, (unsigned*)s->s_id.p, (unsigned long long*)s->s_key2.p, (unsigned*)s->s_id2.p,
-                               counters + kSWinEdges, ec, 2 * 32, (unsigned*)ctx->hist.p, sgrid, st, &ctx->launches);
-  unpack_edges_kernel<<<g, 256, 0, st>>>(ealt ? (const unsigned long long*)s->s_key2.p : ek, ne,
-                                         (unsigned*)ctx->edges.p);
-  ctx->launches += 7;
-  S_TRY(ctx, cudaMemcpyAsync(ctx->h_counters, counters, sizeof(unsigned) * kNumCounters, cudaMemcpyDeviceToHost, st));
-  S_TRY(ctx, ctx->sync());
+  rc = canonical_edges(s, inv, (unsigned long long*)s->s_key.p, (unsigned long long*)s->s_key2.p);
+  if (rc) return rc;
   // hand the canonical buffers to the context's fetch
   ctx->last.kind = FTK2B_MESH_REGULAR;
   ctx->last.m = M;
@@ -400,7 +482,6 @@ ftk2b_status result_regular(ftk2b_stream* s, ftk2b_cp_result** out) {
   ctx->pack_ready = false;
   ctx->last.n = n;
   ctx->last.ne = s->prm.want_edges ? ne : 0;
-  ctx->last.n_roots = ctx->h_counters[kCountRoots];
   ftk2b_mesh_desc md;
   memset(&md, 0, sizeof(md));
   md.kind = FTK2B_MESH_REGULAR;
@@ -411,12 +492,55 @@ ftk2b_status result_regular(ftk2b_stream* s, ftk2b_cp_result** out) {
   ctx->last.device_ms = 0;
   ctx->last.classify = s->prm.classify;
   ctx->last.want_edges = s->prm.want_edges;
-  return ftk2b_cp_fetch(ctx, out);
+  return stream_fetch(s, out);
 }
 
 }  // namespace
 
 namespace ftk2b {
+
+ftk2b_status canonical_edges(ftk2b_stream* s, const unsigned* inv, unsigned long long* k0, unsigned long long* k1) {
+  ftk2b_ctx* ctx = s->ctx;
+  cudaStream_t st = ctx->stream;
+  unsigned* counters = (unsigned*)ctx->counters.p;
+  const unsigned ne = s->n_edges, ec = ne ? ne : 1;
+  if (ec <= kRankCap1) {
+    S_TRY(ctx, launch_rank_sort<1>(LoadCanonEdge{(const unsigned*)s->edges.p, inv}, StoreEdge{(unsigned*)ctx->edges.p},
+                                   nullptr, ne, counters + kSWinEdges, ctx->num_sms, st));
+    ctx->launches += 1;
+    return FTK2B_OK;
+  }
+  const int g = grid_of(ec, 256, 4096);
+  set_u32_kernel<<<1, 1, 0, st>>>(counters + kSWinEdges, ne);
+  canon_edges_kernel<<<g, 256, 0, st>>>((const unsigned*)s->edges.p, ne, inv, k0);
+  const bool alt = radix_sort(k0, (unsigned*)s->s_id.p, k1, (unsigned*)s->s_id2.p, counters + kSWinEdges, ec, 2 * 32,
+                              (unsigned*)ctx->hist.p, ctx->sort_grid(s->n > ne ? s->n : ec), st, &ctx->launches);
+  unpack_edges_kernel<<<g, 256, 0, st>>>(alt ? k1 : k0, ne, (unsigned*)ctx->edges.p);
+  ctx->launches += 3;
+  S_TRY(ctx, cudaGetLastError());
+  return FTK2B_OK;
+}
+
+ftk2b_status stream_fetch(ftk2b_stream* s, ftk2b_cp_result** out) {
+  ftk2b_ctx* ctx = s->ctx;
+  const PackLayout L = pack_layout(ctx->last.n, ctx->last.ne, ctx->last.m + 1, ctx->last.classify);
+  ctx->pack_ready = L.packed <= ctx->pack_bytes();
+  if (ctx->pack_ready) {  // the results and the counters in one launch and one wait
+    PackArgs a = ctx->pack_args(ctx->last);
+    a.h_counters = (unsigned*)ctx->pin.d;
+    a.count = nullptr;
+    a.n = a.cap = (unsigned)ctx->last.n;
+    a.ne = a.edge_cap = (unsigned)ctx->last.ne;
+    S_TRY(ctx, launch_pack(a, ctx->num_sms, ctx->stream));
+    ctx->launches += 1;
+  } else {
+    S_TRY(ctx, cudaMemcpyAsync(ctx->h_counters, ctx->counters.p, sizeof(unsigned) * kNumCounters,
+                               cudaMemcpyDeviceToHost, ctx->stream));
+  }
+  S_TRY(ctx, ctx->sync());
+  ctx->last.n_roots = ctx->h_counters[kCountRoots];
+  return ftk2b_cp_fetch(ctx, out);
+}
 
 cudaError_t grow_keep(DevBuf& b, size_t used, size_t want, cudaStream_t st) {
   if (b.p && b.bytes >= want) return cudaSuccess;
@@ -600,9 +724,7 @@ extern "C" ftk2b_status ftk2b_stream_push(ftk2b_stream* s, const ftk2b_field_des
                                st));
   }
   ftk2b_status rc = s->kind == FTK2B_MESH_REGULAR ? push_regular(s) : stream_push_extruded(s);
-  if (rc) return rc;
-  S_TRY(ctx, cudaEventRecord(ctx->ev1, st));
-  S_TRY(ctx, ctx->sync());
+  if (rc) return rc;  // a push that succeeds has waited for its ev1
   float ms = 0.f;
   if (cudaEventElapsedTime(&ms, ctx->ev0, ctx->ev1) != cudaSuccess) ms = 0.f;
   cudaGetLastError();

@@ -47,6 +47,12 @@ namespace ftk2b {
 cudaError_t grow_keep(DevBuf& b, size_t used, size_t want, cudaStream_t st);
 // grows the feature store (and union-find / boundary lists) to hold `want`
 ftk2b_status ensure_stream_store(ftk2b_stream* s, unsigned want);
+// the store's star edges in canonical ids (inv: canonical id of a stream id),
+// sorted, to the context's edges; k0, k1: scratch of one key per edge
+ftk2b_status canonical_edges(ftk2b_stream* s, const unsigned* inv, unsigned long long* k0, unsigned long long* k1);
+// the result whose arrays and description (all but the track count) the
+// context holds
+ftk2b_status stream_fetch(ftk2b_stream* s, ftk2b_cp_result** out);
 
 }  // namespace ftk2b
 

@@ -3,9 +3,39 @@
 // copies.
 #pragma once
 
+#include "cp_ranksort.cuh"
 #include "cp_uf.cuh"
 
 namespace ftk2b {
+
+// Rank-sort callbacks of a stream's result (cp_ranksort.cuh).
+
+// a sorted store: its permutation, the inverse, and the components' minima
+// reset
+struct StoreOrder {
+  unsigned *perm, *inv, *cmin;
+  __device__ __forceinline__ void put(unsigned pos, unsigned id) const {
+    perm[pos] = id;
+    inv[id] = pos;
+    cmin[id] = 0xFFFFFFFFu;
+  }
+};
+
+// star edges of the store in canonical ids, (min, max) pairs in order
+struct LoadCanonEdge {
+  const unsigned *edges, *inv;
+  __device__ __forceinline__ void operator()(unsigned e, unsigned long long (&k)[1]) const {
+    const unsigned a = inv[edges[2 * (size_t)e]], b = inv[edges[2 * (size_t)e + 1]];
+    k[0] = ((unsigned long long)min(a, b) << 32) | max(a, b);
+  }
+};
+struct StoreEdge {
+  unsigned* out;
+  __device__ __forceinline__ void operator()(unsigned pos, unsigned, const unsigned long long (&k)[1]) const {
+    out[2 * (size_t)pos] = (unsigned)(k[0] >> 32);
+    out[2 * (size_t)pos + 1] = (unsigned)k[0];
+  }
+};
 
 static __global__ void set_u32_kernel(unsigned* p, unsigned v) { *p = v; }
 
