@@ -83,10 +83,10 @@ struct ExtCache {
   int cd = 0;
   unsigned nface = 0;
   int fbits = 0;
-  DevBuf cells, fkeys, cof_start, cof;
+  DevBuf cells, fkeys, cof_start, cof, own;
   DevBuf words, hi, lo, phase, hi_s, lo_s, phase_s, sort_k, sort_v, sort_k2, sort_v2, ekeys;
   std::vector<DevBuf*> bufs() {
-    return {&cells, &fkeys, &cof_start, &cof, &words, &hi, &lo, &phase, &hi_s, &lo_s, &phase_s,
+    return {&cells, &fkeys, &cof_start, &cof, &own, &words, &hi, &lo, &phase, &hi_s, &lo_s, &phase_s,
             &sort_k, &sort_v, &sort_k2, &sort_v2, &ekeys};
   }
 };

@@ -19,9 +19,10 @@
 //      32 bits, every (m-1)-face keyed, radix-sorted, de-duplicated, and the
 //      coface cells of each unique face gathered (unstructured_mesh.hpp:44-53)
 //   1. cull words of every spacetime vertex: one coalesced pass over the field
-//   2. one thread per (spatial cell | base face | base cell, layer): the AND of
-//      each simplex's vertex words culls it or it runs the exact integer SoS
-//      and the bit-exact solve; accepted simplices are compacted by ballot
+//   2. one thread per (base cell, layer): the AND of the prism's vertex words
+//      culls all its simplices at once; those of the prisms left are culled by
+//      their own words or run the exact integer SoS and the bit-exact solve;
+//      accepted simplices are compacted by ballot
 //   3. canonical order: two stable radix sorts on the packed vertex tuple
 //   4. star edges per top cell, centre = smallest node id (phase, then
 //      canonical position: engine.hpp:1375-1387 for non-regular meshes)
@@ -63,6 +64,7 @@ struct ExtMeshDev {
   const unsigned long long* fkeys;   // [nface], ascending packed faces
   const unsigned* cof_start;         // [nface+1]
   const unsigned* cof;               // coface cells, grouped by face
+  const unsigned* own;               // [ncell], byte r: 1 when the face without vertex r is this cell's to extract
 };
 
 struct ExtSink {
@@ -174,7 +176,8 @@ __global__ void ext_face_flags_kernel(const unsigned long long* __restrict__ k, 
 __global__ void ext_face_build_kernel(const unsigned long long* __restrict__ k,
                                       const unsigned* __restrict__ v, const unsigned* __restrict__ pos,
                                       unsigned n, int cd, unsigned long long* __restrict__ fkeys,
-                                      unsigned* __restrict__ cof_start, unsigned* __restrict__ cof) {
+                                      unsigned* __restrict__ cof_start, unsigned* __restrict__ cof,
+                                      unsigned char* __restrict__ own) {
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const bool head = i == 0 || k[i] != k[i - 1];
     const unsigned f = head ? pos[i] : pos[i] - 1;
@@ -183,7 +186,9 @@ __global__ void ext_face_build_kernel(const unsigned long long* __restrict__ k,
       cof_start[f] = i;
     }
     if (i == n - 1) cof_start[f + 1] = n;
-    cof[i] = v[i] / (unsigned)(cd + 1);
+    const unsigned c = v[i] / (unsigned)(cd + 1);
+    cof[i] = c;
+    own[4 * (size_t)c + (v[i] - c * (unsigned)(cd + 1))] = head;  // a face is its first coface cell's
   }
 }
 
@@ -257,129 +262,204 @@ __device__ __forceinline__ bool ext_test(const FieldAccess& fa, const ExtractCon
   return true;
 }
 
-// grid: x over the items of one layer, y = local layer t.  Items of layer t:
-// [0, ncell) spatial cells, then (t < L only) [ncell, ncell + nface) base
-// faces (m lateral pieces each) and [ncell + nface, 2 ncell + nface) base
-// cells (m interior simplices each).  Values and words of local layer l sit
-// at storage layer l xor tflip; vertex ids use the global layer t0 + l.
+// The simplices a prism gives: its lower spatial cell, the M interior ones, M
+// pieces over each of its M + 1 faces, and its upper spatial cell.
+template <int M>
+constexpr int kPrismSlots = 2 + M + M * (M + 1);
+
+// Slot s of a prism: output vertex k is base vertex src(k) of the cell, at the
+// upper layer when k > split.  face: the base vertex a lateral piece leaves
+// out (M + 1: not lateral).  live: the bit of a cell that asks for the slot.
+template <int M>
+struct PrismSlot {
+  int split, face, live;
+  __device__ __forceinline__ explicit PrismSlot(int s) {
+    face = M + 1;
+    if (s == 0 || s == kPrismSlots<M> - 1) {
+      split = s ? -1 : M;
+      live = s ? M + 3 : 0;
+    } else if (s <= M) {
+      split = s - 1;  // u[0..split]@t, u[split+1..M]@t+1
+      live = 1;
+    } else {
+      face = (s - M - 1) / M;
+      split = (s - M - 1) % M;  // f[0..split]@t, f[split..M-1]@t+1
+      live = 2 + face;
+    }
+  }
+  __device__ __forceinline__ bool interior() const { return live == 1; }
+  __device__ __forceinline__ int upper(int k) const { return k > split ? 1 : 0; }
+  __device__ __forceinline__ int src(int k) const {
+    if (face > M) return k;
+    const int f = k - upper(k);
+    return f + (f >= face ? 1 : 0);
+  }
+};
+
+// grid: x over the base cells, y = slab between local layers t and t + 1 (the
+// last one also has the upper layer's spatial cells; one layer alone is slab 0
+// without a prism).  Values and words of local layer l sit at storage layer
+// l xor tflip; vertex ids use the global layer t0 + l.
+//
+// A thread ANDs the words of its cells' prisms.  What is culled on a superset
+// is culled on every simplex of it, so a prism whose AND is culled has no
+// simplex to test: a cell costs one 16-byte load and eight gathers instead of
+// one pass for the cell, one for its interior and one for each of its faces.
+// The few prisms left are listed in shared memory, a thread per simplex of them
+// ANDs that simplex's words, and the simplices left after that run the exact
+// test in full warps.  A face belongs to its first coface cell (X.own).  Bound
+// by the latency of the gathers, so a thread has kCellsPer cells in flight and
+// the exact test, rare here, gives up registers (164 unbounded) for three
+// blocks an SM.  2.3M tets, one slab, float: 525 us with a thread per cell,
+// face and interior, 110 with one 256-cell block an SM, 48 with three, 35 with
+// two cells a thread; 364,000 tets, four slabs, double: 253 -> 21 us.
+constexpr int kCellsPer = 2;
+
 template <typename T, int M>
-__global__ void __launch_bounds__(kThreadsX) ext_extract_kernel(ExtMeshDev X, FieldAccess fa,
-                                                                const unsigned* __restrict__ words,
-                                                                ExtractConfig cfg, ExtSink sink, int vb) {
+__global__ void __launch_bounds__(kThreadsX, 3) ext_extract_kernel(ExtMeshDev X, FieldAccess fa,
+                                                                   const unsigned* __restrict__ words,
+                                                                   ExtractConfig cfg, ExtSink sink, int vb) {
+  constexpr int NS = kPrismSlots<M>, NC = kCellsPer * kThreadsX;
+  __shared__ unsigned s_u[M + 1][NC], s_w[2][M + 1][NC];  // listed cells: vertices, words per layer
+  __shared__ unsigned short s_live[NC];                   // PrismSlot::live bits
+  __shared__ unsigned short s_list[NC * NS];
+  __shared__ unsigned s_n[2];  // cells, simplices listed
   const unsigned t = blockIdx.y;
-  const unsigned nitems = (t < X.L) ? 2u * X.ncell + X.nface : X.ncell;
-  const unsigned first = (X.skip_first_spatial && t == 0) ? X.ncell : 0u;
+  const bool slab = t < X.L, spatial = !(X.skip_first_spatial && t == 0), top = t + 1 == X.L;
   const unsigned long long bt = (unsigned long long)(X.t0 + t) * X.ns, bt1 = bt + X.ns;
   const unsigned long long st = (unsigned long long)(t ^ X.tflip) * X.ns;
   const unsigned long long st1 = (unsigned long long)((t + 1) ^ X.tflip) * X.ns;
-  const int lane = threadIdx.x & 31;
-  const unsigned fmask = (X.fbits >= 32) ? 0xFFFFFFFFu : ((1u << X.fbits) - 1u);
-  for (unsigned base = blockIdx.x * kThreadsX; base < nitems; base += gridDim.x * kThreadsX) {
-    const unsigned i = base + threadIdx.x;
-    const bool valid = i < nitems && i >= first;
-    int kind = 0;
-    unsigned u[M + 1];
-    unsigned wa[M + 1], wb[M + 1];
+  const unsigned tid = threadIdx.x, lane = tid & 31, below = (1u << lane) - 1;
+  for (unsigned long long base = blockIdx.x * (unsigned long long)NC; base < X.ncell;
+       base += gridDim.x * (unsigned long long)NC) {
+    if (tid < 2) s_n[tid] = 0;
+    __syncthreads();
+    unsigned u[kCellsPer][M + 1], w[2][kCellsPer][M + 1], live[kCellsPer];
 #pragma unroll
-    for (int k = 0; k <= M; ++k) {
-      u[k] = 0;
-      wa[k] = kAbsent;
-      wb[k] = kAbsent;
-    }
-    if (valid) {
-      if (i < X.ncell) {
-        kind = 0;
-#pragma unroll
-        for (int k = 0; k <= M; ++k) u[k] = X.cells[(size_t)i * (M + 1) + k];
-      } else if (i < X.ncell + X.nface) {
-        kind = 1;
-        const unsigned long long key = X.fkeys[i - X.ncell];
-#pragma unroll
-        for (int k = 0; k < M; ++k) u[k] = (unsigned)(key >> (X.fbits * (M - 1 - k))) & fmask;
+    for (int q = 0; q < kCellsPer; ++q) {
+      const unsigned long long c = min(base + q * kThreadsX + tid, (unsigned long long)X.ncell - 1);
+      if constexpr (M == 3) {
+        const uint4 v = *reinterpret_cast<const uint4*>(X.cells + 4 * c);
+        u[q][0] = v.x;
+        u[q][1] = v.y;
+        u[q][2] = v.z;
+        u[q][M] = v.w;
       } else {
-        kind = 2;
-        const unsigned c = i - X.ncell - X.nface;
 #pragma unroll
-        for (int k = 0; k <= M; ++k) u[k] = X.cells[(size_t)c * (M + 1) + k];
+        for (int k = 0; k <= M; ++k) u[q][k] = X.cells[c * (M + 1) + k];
       }
-      const int nu = (kind == 1) ? M : M + 1;
-#pragma unroll
-      for (int k = 0; k <= M; ++k)
-        if (k < nu) {
-          wa[k] = words[st + u[k]];
-          if (kind != 0) wb[k] = words[st1 + u[k]];
-        }
     }
 #pragma unroll
-    for (int p = 0; p < M; ++p) {
-      const bool live = valid && (kind != 0 || p == 0);
+    for (int q = 0; q < kCellsPer; ++q)
+#pragma unroll
+      for (int k = 0; k <= M; ++k) {
+        w[0][q][k] = words[st + u[q][k]];
+        w[1][q][k] = slab ? words[st1 + u[q][k]] : kAbsent;
+      }
+#pragma unroll
+    for (int q = 0; q < kCellsPer; ++q) {
+      const unsigned long long c = base + q * kThreadsX + tid;
+      unsigned lo = kAbsent, hi = kAbsent;
+#pragma unroll
+      for (int k = 0; k <= M; ++k) {
+        lo &= w[0][q][k];
+        hi &= w[1][q][k];
+      }
+      live[q] = 0;
+      if (c < X.ncell) {
+        // the cull words assume an accepted simplex has a successful solve,
+        // which fibers do not require
+        if (spatial && (cfg.fiber || !word_culled(lo))) live[q] = 1;
+        if (slab && (cfg.fiber || !word_culled(lo & hi))) {
+          const unsigned own = X.own[c];
+          live[q] |= 2;
+#pragma unroll
+          for (int r = 0; r <= M; ++r) live[q] |= ((own >> (8 * r)) & 1u) << (2 + r);
+        }
+        if (top && (cfg.fiber || !word_culled(hi))) live[q] |= 1u << (M + 3);
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < kCellsPer; ++q) {
+      const unsigned ball = __ballot_sync(0xFFFFFFFFu, live[q] != 0);
+      if (!ball) continue;
+      unsigned at = 0;
+      if (lane == 0) at = atomicAdd(&s_n[0], (unsigned)__popc(ball));
+      at = __shfl_sync(0xFFFFFFFFu, at, 0) + __popc(ball & below);
+      if (live[q]) {
+        s_live[at] = (unsigned short)live[q];
+#pragma unroll
+        for (int k = 0; k <= M; ++k) {
+          s_u[k][at] = u[q][k];
+          s_w[0][k][at] = w[0][q][k];
+          s_w[1][k][at] = w[1][q][k];
+        }
+      }
+    }
+    __syncthreads();
+    const unsigned n_slots = s_n[0] * NS;
+    for (unsigned i0 = 0; i0 < n_slots; i0 += kThreadsX) {
+      const unsigned i = i0 + tid;
+      bool keep = false;
+      if (i < n_slots) {
+        const unsigned cell = i / NS;
+        const PrismSlot<M> p((int)(i % NS));
+        if ((s_live[cell] >> p.live) & 1u) {
+          unsigned acc = kAbsent;
+#pragma unroll
+          for (int k = 0; k <= M; ++k) acc &= s_w[p.upper(k)][p.src(k)][cell];
+          keep = cfg.fiber || !word_culled(acc);
+        }
+      }
+      const unsigned kb = __ballot_sync(0xFFFFFFFFu, keep);
+      if (!kb) continue;
+      unsigned at = 0;
+      if (lane == 0) at = atomicAdd(&s_n[1], (unsigned)__popc(kb));
+      at = __shfl_sync(0xFFFFFFFFu, at, 0) + __popc(kb & below);
+      if (keep) s_list[at] = (unsigned short)i;
+    }
+    __syncthreads();
+    const unsigned n_list = s_n[1];
+    for (unsigned i0 = 0; i0 < n_list; i0 += kThreadsX) {
+      const unsigned i = i0 + tid;
+      bool acc = false, interior = false;
       unsigned long long vid[M + 1], sidx[M + 1];
-      unsigned wacc = kAbsent;
-      if (kind == 0) {
-#pragma unroll
-        for (int k = 0; k <= M; ++k) {
-          vid[k] = bt + u[k];
-          sidx[k] = st + u[k];
-          wacc &= wa[k];
-        }
-      } else if (kind == 1) {
-        // lateral piece j = p: f[0..j]@t, f[j..m-1]@t+1
-        int w = 0;
-#pragma unroll
-        for (int k = 0; k < M; ++k)
-          if (k <= p) {
-            sidx[w] = st + u[k];
-            vid[w++] = bt + u[k];
-            wacc &= wa[k];
-          }
-#pragma unroll
-        for (int k = 0; k < M; ++k)
-          if (k >= p) {
-            sidx[w] = st1 + u[k];
-            vid[w++] = bt1 + u[k];
-            wacc &= wb[k];
-          }
-      } else {
-        // interior s = p + 1: u[0..s-1]@t, u[s..m]@t+1
-#pragma unroll
-        for (int k = 0; k <= M; ++k) {
-          const bool lo = k <= p;
-          vid[k] = (lo ? bt : bt1) + u[k];
-          sidx[k] = (lo ? st : st1) + u[k];
-          wacc &= lo ? wa[k] : wb[k];
-        }
-      }
-      bool acc = false;
       double lam_out[4] = {0, 0, 0, 0};
       float bary_out[4] = {0.f, 0.f, 0.f, 0.f};
       float sc_out = 0.f;
-      // the cull words assume an accepted simplex has a successful solve,
-      // which fibers do not require
-      if (live && (cfg.fiber || !word_culled(wacc))) acc = ext_test<T, M>(fa, cfg, sidx, lam_out, bary_out, sc_out);
-      const unsigned ball = __ballot_sync(0xFFFFFFFFu, acc);
-      if (ball) {
-        unsigned basei = 0;
-        const int leader = __ffs(ball) - 1;
-        if (lane == leader) basei = atomicAdd(sink.count, (unsigned)__popc(ball));
-        basei = __shfl_sync(0xFFFFFFFFu, basei, leader);
-        if (acc) {
-          const unsigned idx = basei + __popc(ball & ((1u << lane) - 1));
-          if (idx < sink.cap) {
-            unsigned long long hi, lo;
-            pack_tuple<M>(vid, vb, hi, lo);
-            sink.hi[idx] = hi;
-            sink.lo[idx] = lo;
-            sink.phase[idx] = kind == 2 ? 1u : 0u;
+      if (i < n_list) {
+        const unsigned e = s_list[i], cell = e / NS;
+        const PrismSlot<M> p((int)(e % NS));
+        interior = p.interior();
 #pragma unroll
-            for (int k = 0; k < 4; ++k) {
-              sink.lam[4 * (size_t)idx + k] = lam_out[k];
-              sink.bary4[4 * (size_t)idx + k] = bary_out[k];
-            }
-            sink.scalar[idx] = sc_out;
-          }
+        for (int k = 0; k <= M; ++k) {
+          const unsigned x = s_u[p.src(k)][cell];
+          vid[k] = (p.upper(k) ? bt1 : bt) + x;
+          sidx[k] = (p.upper(k) ? st1 : st) + x;
         }
+        acc = ext_test<T, M>(fa, cfg, sidx, lam_out, bary_out, sc_out);
+      }
+      const unsigned ab = __ballot_sync(0xFFFFFFFFu, acc);
+      if (!ab) continue;
+      unsigned basei = 0;
+      if (lane == 0) basei = atomicAdd(sink.count, (unsigned)__popc(ab));
+      basei = __shfl_sync(0xFFFFFFFFu, basei, 0);
+      const unsigned idx = basei + __popc(ab & below);
+      if (acc && idx < sink.cap) {
+        unsigned long long hi, lo;
+        pack_tuple<M>(vid, vb, hi, lo);
+        sink.hi[idx] = hi;
+        sink.lo[idx] = lo;
+        sink.phase[idx] = interior ? 1u : 0u;
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          sink.lam[4 * (size_t)idx + k] = lam_out[k];
+          sink.bary4[4 * (size_t)idx + k] = bary_out[k];
+        }
+        sink.scalar[idx] = sc_out;
       }
     }
+    __syncthreads();
   }
 }
 
@@ -685,6 +765,7 @@ ftk2b_status prepare_base(ftk2b_ctx* ctx, const ftk2b_mesh_desc* mesh, int fbits
   EXT_TRY(C.fkeys.ensure(sizeof(unsigned long long) * ne));
   EXT_TRY(C.cof_start.ensure(sizeof(unsigned) * (ne + 1)));
   EXT_TRY(C.cof.ensure(sizeof(unsigned) * ne));
+  EXT_TRY(C.own.ensure(sizeof(unsigned) * (ncell ? ncell : 1)));
   EXT_TRY(C.ekeys.ensure(sizeof(unsigned long long) * ne));
   EXT_TRY(C.sort_k.ensure(sizeof(unsigned long long) * ne));
   EXT_TRY(C.sort_k2.ensure(sizeof(unsigned long long) * ne));
@@ -715,7 +796,8 @@ ftk2b_status prepare_base(ftk2b_ctx* ctx, const ftk2b_mesh_desc* mesh, int fbits
     ext_face_flags_kernel<<<g, 256, 0, st>>>(k, nent, flags);
     EXT_TRY(launch_scan(flags, nent, counters + kCountFaces, nullptr, st));
     ext_face_build_kernel<<<g, 256, 0, st>>>(k, v, flags, nent, cd, (unsigned long long*)C.fkeys.p,
-                                             (unsigned*)C.cof_start.p, (unsigned*)C.cof.p);
+                                             (unsigned*)C.cof_start.p, (unsigned*)C.cof.p,
+                                             (unsigned char*)C.own.p);
     *nl += 3;
     EXT_TRY(cudaGetLastError());
     EXT_TRY(cudaMemcpyAsync(ctx->h_counters, counters, sizeof(unsigned) * kNumCounters,
@@ -742,8 +824,7 @@ cudaError_t enqueue_extract(ftk2b_ctx* ctx, const ExtMeshDev& X, const FieldAcce
   cudaStream_t st = ctx->stream;
   ext_words_kernel<T, M><<<grid_of(nv, 256, 32 * ctx->num_sms), 256, 0, st>>>(fa, nv,
                                                                               (unsigned*)ctx->ext.words.p);
-  const unsigned long long items = 2ull * X.ncell + X.nface;
-  dim3 grid((unsigned)grid_of(items, kThreadsX, 1 << 20), X.L + 1);
+  const dim3 grid((unsigned)grid_of(X.ncell, kCellsPer * kThreadsX, 1 << 20), std::max(X.L, 1u));
   ext_extract_kernel<T, M><<<grid, kThreadsX, 0, st>>>(X, fa, (const unsigned*)ctx->ext.words.p, cfg, sink, vb);
   *nl += 2;
   return cudaGetLastError();
@@ -966,6 +1047,7 @@ ExtMeshDev stream_mesh(ftk2b_ctx* ctx, const ftk2b_stream* s, unsigned t0, unsig
   X.fkeys = (const unsigned long long*)C.fkeys.p;
   X.cof_start = (const unsigned*)C.cof_start.p;
   X.cof = (const unsigned*)C.cof.p;
+  X.own = (const unsigned*)C.own.p;
   return X;
 }
 
@@ -1294,6 +1376,7 @@ ftk2b_status run_extruded(ftk2b_ctx* ctx, const ftk2b_mesh_desc* mesh, const ftk
   X.fkeys = (const unsigned long long*)C.fkeys.p;
   X.cof_start = (const unsigned*)C.cof_start.p;
   X.cof = (const unsigned*)C.cof.p;
+  X.own = (const unsigned*)C.own.p;
   X.t0 = 0;
   X.tflip = 0;
   X.skip_first_spatial = 0;
