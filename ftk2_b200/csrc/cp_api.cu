@@ -1055,7 +1055,7 @@ static ftk2b_status run_any(ftk2b_ctx* ctx, const ftk2b_mesh_desc* mesh, const f
   ftk2b_status st;
   ctx->pack_ready = false;
   if (mesh->kind == FTK2B_MESH_REGULAR) st = run_regular(ctx, mesh, field, &prm, nullptr, pack);
-  else if (mesh->kind == FTK2B_MESH_EXTRUDED) st = run_extruded(ctx, mesh, field, &prm);
+  else if (mesh->kind == FTK2B_MESH_EXTRUDED) st = run_extruded(ctx, mesh, field, &prm, nullptr, pack);
   else st = fail(ctx, FTK2B_INVALID_ARG, "unknown mesh kind %d", mesh->kind);
   if (st == FTK2B_OK) {
     if (n_features) *n_features = ctx->last.n;
@@ -1163,7 +1163,7 @@ extern "C" ftk2b_status ftk2b_fiber_extract(ftk2b_ctx* ctx, const ftk2b_mesh_des
   prm.want_edges = 1;
   ctx->pack_ready = false;
   const ftk2b_status st = mesh->kind == FTK2B_MESH_REGULAR ? run_regular(ctx, mesh, field, &prm, thresholds, true)
-                                                          : run_extruded(ctx, mesh, field, &prm, thresholds);
+                                                          : run_extruded(ctx, mesh, field, &prm, thresholds, true);
   if (st) return st;
   return ftk2b_cp_fetch(ctx, out);
 }

@@ -291,7 +291,8 @@ cudaError_t resolve_cull_mode(ftk2b_ctx* ctx, const RegularMesh& rm, const Field
 
 // extruded meshes (cp_extruded.cu)
 // fiber_thr: null for CriticalPointPredicate; the two thresholds for
-// FiberPredicate (triangle bases)
+// FiberPredicate (triangle bases); pack: the caller fetches the results next,
+// so they are packed before the run's last wait
 ftk2b_status run_extruded(ftk2b_ctx* ctx, const ftk2b_mesh_desc* mesh, const ftk2b_field_desc* field,
-                          const ftk2b_cp_params* prm, const double* fiber_thr = nullptr);
+                          const ftk2b_cp_params* prm, const double* fiber_thr = nullptr, bool pack = false);
 uint64_t extruded_simplex_count(const ftk2b_mesh_desc* mesh, int m);

@@ -23,7 +23,8 @@
 //      culls all its simplices at once; those of the prisms left are culled by
 //      their own words or run the exact integer SoS and the bit-exact solve;
 //      accepted simplices are compacted by ballot
-//   3. canonical order: two stable radix sorts on the packed vertex tuple
+//   3. canonical order: one rank sort of the packed vertex tuples, or two stable
+//      radix sorts where they are too many for it
 //   4. star edges per top cell, centre = smallest node id (phase, then
 //      canonical position: engine.hpp:1375-1387 for non-regular meshes)
 //   5. union-find over the edges, plus for 4-D meshes the extra coface unions
@@ -114,18 +115,6 @@ __device__ __forceinline__ long long find_tuple(const unsigned long long* __rest
     const unsigned long long hm = H[mid], lm = Lo[mid];
     if (hm == h && lm == l) return mid;
     if (hm < h || (hm == h && lm < l)) a = mid + 1;
-    else b = mid;
-  }
-  return -1;
-}
-
-__device__ __forceinline__ long long find_face(const ExtMeshDev& X, unsigned long long k) {
-  unsigned a = 0, b = X.nface;
-  while (a < b) {
-    const unsigned mid = (a + b) >> 1;
-    const unsigned long long v = X.fkeys[mid];
-    if (v == k) return mid;
-    if (v < k) a = mid + 1;
     else b = mid;
   }
   return -1;
@@ -474,30 +463,43 @@ __global__ void ext_gather_by_perm_kernel(const unsigned long long* __restrict__
     dst[i] = src[perm[i]];
 }
 
+// Features in canonical order.
+struct ExtSorted {
+  unsigned long long *hi, *lo;
+  unsigned* phase;
+  double* lam;
+  float* scalar;
+  unsigned long long* simplices;
+  float* bary;
+  unsigned* parent;
+};
+
+// feature p of the extraction is the i-th of the canonical order
 template <int M>
-__global__ void ext_finalize_kernel(const unsigned* __restrict__ perm, const unsigned* n_ptr, unsigned cap,
-                                    int vb, ExtSink in, unsigned long long* __restrict__ hi_s,
-                                    unsigned long long* __restrict__ lo_s, unsigned* __restrict__ phase_s,
-                                    double* __restrict__ lam_s, float* __restrict__ sc_s,
-                                    unsigned long long* __restrict__ simplices, float* __restrict__ bary) {
-  const unsigned n = min(*n_ptr, cap);
-  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const unsigned p = perm[i];
-    const unsigned long long h = in.hi[p], l = in.lo[p];
-    hi_s[i] = h;
-    lo_s[i] = l;
-    phase_s[i] = in.phase[p];
+__device__ __forceinline__ void ext_finalize(const ExtSink& in, unsigned p, int vb, const ExtSorted& out, unsigned i) {
+  const unsigned long long h = in.hi[p], l = in.lo[p];
+  out.hi[i] = h;
+  out.lo[i] = l;
+  out.phase[i] = in.phase[p];
+  out.parent[i] = i;
 #pragma unroll
-    for (int k = 0; k < 4; ++k) lam_s[4 * (size_t)i + k] = in.lam[4 * (size_t)p + k];
-    sc_s[i] = in.scalar[p];
-    unsigned long long v[4];
-    unpack_tuple<M>(h, l, vb, v);
+  for (int k = 0; k < 4; ++k) out.lam[4 * (size_t)i + k] = in.lam[4 * (size_t)p + k];
+  out.scalar[i] = in.scalar[p];
+  unsigned long long v[4];
+  unpack_tuple<M>(h, l, vb, v);
 #pragma unroll
-    for (int k = 0; k <= M; ++k) {
-      simplices[(size_t)i * (M + 1) + k] = v[k];
-      bary[(size_t)i * (M + 1) + k] = in.bary4[4 * (size_t)p + k];
-    }
+  for (int k = 0; k <= M; ++k) {
+    out.simplices[(size_t)i * (M + 1) + k] = v[k];
+    out.bary[(size_t)i * (M + 1) + k] = in.bary4[4 * (size_t)p + k];
   }
+}
+
+template <int M>
+__global__ void ext_finalize_kernel(const unsigned* __restrict__ perm, const unsigned* n_ptr, unsigned cap, int vb,
+                                    ExtSink in, ExtSorted out) {
+  const unsigned n = min(*n_ptr, cap);
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
+    ext_finalize<M>(in, perm[i], vb, out, i);
 }
 
 // ---------------------------------------------------------------------------
@@ -512,133 +514,6 @@ struct ExtFeatures {
   int vb;
 };
 
-// Calls visit(cell) for every top cell (m+2 ascending vertex ids) that has
-// the feature's simplex v[0..m] as a face.
-template <int M, typename F>
-__device__ __forceinline__ void for_each_coface(const ExtMeshDev& X, const unsigned long long* v, F visit) {
-  const unsigned long long ns = X.ns;
-  const unsigned long long t = v[0] / ns;
-  unsigned long long tl[M + 1];
-  unsigned sp[M + 1];
-  int n_at_t = 0;
-#pragma unroll
-  for (int k = 0; k <= M; ++k) {
-    tl[k] = v[k] / ns;
-    sp[k] = (unsigned)(v[k] - tl[k] * ns);
-    n_at_t += tl[k] == t;
-  }
-  unsigned long long cell[M + 2];
-  auto piece = [&](const unsigned* u, unsigned long long tt, int p) {
-    int w = 0;
-    for (int k = 0; k <= p; ++k) cell[w++] = tt * ns + u[k];
-    for (int k = p; k <= M; ++k) cell[w++] = (tt + 1) * ns + u[k];
-  };
-  if (n_at_t == M + 1) {
-    // spatial simplex (a base cell at layer t): piece m of slab t, piece 0 of slab t-1
-    if (t < (unsigned long long)X.t0 + X.L) {
-      piece(sp, t, M);
-      visit(cell);
-    }
-    if (t > X.t0) {
-      piece(sp, t - 1, 0);
-      visit(cell);
-    }
-    return;
-  }
-  const int j = n_at_t - 1;
-  if (sp[j] == sp[j + 1]) {
-    // lateral piece j over base face f: piece j + (e <= j) of every cell u
-    // containing f, e = position of u's vertex outside f
-    unsigned f[M];
-    int w = 0;
-    for (int k = 0; k <= M; ++k)
-      if (k != j + 1) f[w++] = sp[k];
-    const long long fi = find_face(X, face_key(f, M, X.fbits));
-    if (fi < 0) return;
-    for (unsigned q = X.cof_start[fi]; q < X.cof_start[fi + 1]; ++q) {
-      const unsigned* u = X.cells + (size_t)X.cof[q] * (M + 1);
-      int e = -1, wi = 0;
-      for (int k = 0; k <= M; ++k) {
-        if (wi < M && u[k] == f[wi]) ++wi;
-        else e = k;
-      }
-      if (e < 0) continue;
-      piece(u, t, j + (e <= j ? 1 : 0));
-      visit(cell);
-    }
-  } else {
-    // interior s = j + 1 of the prism over base cell sp: pieces s-1 and s
-    piece(sp, t, j);
-    visit(cell);
-    piece(sp, t, j + 1);
-    visit(cell);
-  }
-}
-
-// Indices of the features among the m+2 faces of a top cell.
-template <int M>
-__device__ __forceinline__ int cell_features(const ExtFeatures& Fs, unsigned n, const unsigned long long* cell,
-                                             long long* out) {
-  int na = 0;
-#pragma unroll
-  for (int r = 0; r <= M + 1; ++r) {
-    unsigned long long face[M + 1];
-    int w = 0;
-#pragma unroll
-    for (int k = 0; k <= M + 1; ++k)
-      if (k != r) face[w++] = cell[k];
-    unsigned long long h, l;
-    pack_tuple<M>(face, Fs.vb, h, l);
-    const long long idx = find_tuple(Fs.hi, Fs.lo, n, h, l);
-    if (idx >= 0) out[na++] = idx;
-  }
-  return na;
-}
-
-// pass 0: number of star edges each feature emits as a centre; pass 1: the
-// edges themselves, packed (min << 32 | max), at the scanned offsets
-template <int M, int PASS>
-__global__ void ext_edges_kernel(ExtMeshDev X, ExtFeatures Fs, unsigned* __restrict__ cnt,
-                                 const unsigned* __restrict__ off, unsigned long long* __restrict__ ekeys,
-                                 unsigned edge_cap, unsigned* err) {
-  const unsigned n = min(*Fs.n_ptr, Fs.cap);
-  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    unsigned long long v[4];
-    unpack_tuple<M>(Fs.hi[i], Fs.lo[i], Fs.vb, v);
-    unsigned others[kMaxOthers];
-    int no = 0;
-    bool over = false;
-    for_each_coface<M>(X, v, [&](const unsigned long long* cell) {
-      long long act[M + 2];
-      const int na = cell_features<M>(Fs, n, cell, act);
-      if (na < 2) return;
-      int c = 0;
-      for (int a = 1; a < na; ++a) {
-        const unsigned pa = Fs.phase[act[a]], pc = Fs.phase[act[c]];
-        if (pa < pc || (pa == pc && act[a] < act[c])) c = a;
-      }
-      if (act[c] != (long long)i) return;
-      for (int a = 0; a < na; ++a)
-        if (a != c) {
-          if (no < kMaxOthers) others[no++] = (unsigned)act[a];
-          else over = true;
-        }
-    });
-    if (over) atomicOr(err, kErrCofaces);
-    if (PASS == 0) {
-      cnt[i] = (unsigned)no;
-    } else {
-      const unsigned o = off[i];
-      for (int a = 0; a < no; ++a)
-        if (o + a < edge_cap) {
-          const unsigned x = others[a];
-          const unsigned lo = min(x, i), hi = max(x, i);
-          ekeys[o + a] = ((unsigned long long)lo << 32) | hi;
-        }
-    }
-  }
-}
-
 __global__ void ext_unpack_edges_kernel(const unsigned long long* __restrict__ ekeys, const unsigned* ne_ptr,
                                         unsigned edge_cap, unsigned* __restrict__ edges) {
   const unsigned ne = min(*ne_ptr, edge_cap);
@@ -649,55 +524,181 @@ __global__ void ext_unpack_edges_kernel(const unsigned long long* __restrict__ e
   }
 }
 
-// 4-D meshes: every non-spatial feature is united with the features among the
-// faces of the top cells that ExtrudedSimplicialMesh::cofaces lists for it.
+// Where a set of features' star edges and unions go.
+struct ExtStars {
+  const unsigned* ids;        // union-find index of each feature (null: the feature's own)
+  unsigned* parent;           // initialised
+  unsigned long long* ekeys;  // packed (min << 32 | max) feature indices, or
+  unsigned* pairs;            // (null: ekeys) pairs of ids, from row `base` on
+  unsigned base, cap;         // rows of ekeys or pairs
+  unsigned* n_edges;
+  unsigned* err;
+};
+
+constexpr int kStarLanes = 16;
+
+// The face with key k, searched by a group's 16 lanes (gm): each round keeps a
+// sixteenth of the range, so 4.6 million faces take six dependent loads.
+__device__ __forceinline__ long long find_face_group(const ExtMeshDev& X, unsigned long long k, unsigned gm,
+                                                     unsigned hl, unsigned shift) {
+  unsigned lo = 0, len = X.nface;
+  while (len > kStarLanes) {
+    const unsigned step = (len + kStarLanes - 1) / kStarLanes;
+    const bool le = hl * step < len && X.fkeys[lo + hl * step] <= k;
+    const unsigned c = __popc(__ballot_sync(gm, le) >> shift & 0xFFFFu);
+    if (c == 0) return -1;
+    lo += (c - 1) * step;
+    len = min(step, len - (c - 1) * step);
+  }
+  const bool hit = hl < len && X.fkeys[lo + hl] == k;
+  const unsigned ball = __ballot_sync(gm, hit) >> shift & 0xFFFFu;
+  return ball ? (long long)(lo + __ffs(ball) - 1) : -1;
+}
+
+// Star edges and unions of the features: 16 lanes a feature, a lane per face
+// of its top cells (three cells of five faces, four of four, at a time).
+//
+// A feature's top cells: of a spatial simplex (a base cell at layer t) piece m
+// of slab t and piece 0 of slab t - 1; of an interior simplex s of the prism
+// over a base cell, pieces s - 1 and s; of a lateral piece j over base face f,
+// piece j + (e <= j) of the prism over every cell that contains f, e the
+// position of the cell's vertex outside f.  The features among a cell's faces
+// form a star around the one with the smallest node id (phase, then canonical
+// position), which emits the edges.
+//
+// 4-D meshes: every non-spatial feature is also united with the features among
+// the faces of the top cells that ExtrudedSimplicialMesh::cofaces lists for it.
 // That routine lifts the base face obtained by dropping the vertex after the
 // last layer-t vertex: for a lateral piece that is its own base face (the true
 // cofaces); for an interior simplex it is a face of its cell, and the pieces
 // of the neighbouring cell across that face join the component as well.
-// ids: union-find index of each feature (null: the feature index itself)
-__global__ void ext_coface_union_kernel(ExtMeshDev X, ExtFeatures Fs, const unsigned* __restrict__ ids,
-                                        unsigned* parent, unsigned* err) {
-  constexpr int M = 3;
+//
+// Bound by chains of dependent loads (the face, its cells, the features'
+// binary searches).  A thread a feature walked them one after the other, twice
+// for the edges and once more for the cofaces: 57 + 54 + 37 us for the 570
+// features of a 100 x 100 x 40 tet slab, now 19 for all three.
+template <int M>
+__global__ void __launch_bounds__(256) ext_stars_kernel(ExtMeshDev X, ExtFeatures Fs, ExtStars out) {
+  constexpr int kFaces = M + 2, kCells = kStarLanes / kFaces;
   const unsigned n = min(*Fs.n_ptr, Fs.cap);
+  const unsigned lane = threadIdx.x & 31, hl = lane & (kStarLanes - 1), shift = lane & kStarLanes;
+  const unsigned gm = 0xFFFFu << shift;
+  const unsigned q_lane = hl / kFaces, r = hl % kFaces;  // this lane's cell of the round and the vertex its face leaves out
+  const bool used = q_lane < kCells;
+  const unsigned first = shift + (used ? q_lane * kFaces : 0u);  // lane of the cell's first face
   const unsigned long long ns = X.ns;
-  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+  for (unsigned i = (blockIdx.x * blockDim.x + threadIdx.x) / kStarLanes; i < n;
+       i += gridDim.x * blockDim.x / kStarLanes) {
     unsigned long long v[4];
     unpack_tuple<M>(Fs.hi[i], Fs.lo[i], Fs.vb, v);
     const unsigned long long t = v[0] / ns;
-    unsigned sp[4];
+    unsigned sp[M + 1];
     int n_at_t = 0;
+#pragma unroll
     for (int k = 0; k <= M; ++k) {
       const unsigned long long tk = v[k] / ns;
       sp[k] = (unsigned)(v[k] - tk * ns);
       n_at_t += tk == t;
     }
-    if (n_at_t == M + 1) continue;  // spatial: its cofaces are its star cells
-    const int j0 = n_at_t - 1;
-    unsigned bs[3];
-    int bi = 0;
-    for (int k = 0; k <= j0; ++k) bs[bi++] = sp[k];
-    for (int k = j0 + 2; k <= M; ++k) bs[bi++] = sp[k];
-    const long long fi = find_face(X, face_key(bs, M, X.fbits));
-    if (fi < 0) continue;
-    for (unsigned q = X.cof_start[fi]; q < X.cof_start[fi + 1]; ++q) {
-      const unsigned* u = X.cells + (size_t)X.cof[q] * (M + 1);
-      int e = -1, wi = 0;
-      for (int k = 0; k <= M; ++k) {
-        if (wi < M && u[k] == bs[wi]) ++wi;
-        else e = k;
-      }
-      if (e < 0) continue;
-      const int jp = j0 + (e <= j0 ? 1 : 0);
-      unsigned long long cell[5];
-      int w = 0;
-      for (int k = 0; k <= jp; ++k) cell[w++] = t * ns + u[k];
-      for (int k = jp; k <= M; ++k) cell[w++] = (t + 1) * ns + u[k];
-      long long act[5];
-      const int na = cell_features<M>(Fs, n, cell, act);
-      for (int a = 0; a < na; ++a)
-        uf_unite(parent, ids ? ids[i] : i, ids ? ids[act[a]] : (unsigned)act[a], err);
+    const unsigned id = out.ids ? out.ids[i] : i;
+    const bool spatial = n_at_t == M + 1;
+    const int j = n_at_t - 1;
+    bool lateral = false;
+#pragma unroll
+    for (int k = 0; k < M; ++k) lateral |= !spatial && k == j && sp[k] == sp[k + 1];
+    // base face without the vertex after the last layer-t one
+    unsigned f[M];
+    long long fi = -1;
+    if (!spatial && (lateral || M == 3)) {
+#pragma unroll
+      for (int k = 0; k < M; ++k) f[k] = k <= j ? sp[k] : sp[k + 1];
+      fi = find_face_group(X, face_key(f, M, X.fbits), gm, hl, shift);
     }
+    unsigned others = 0;
+    // star: the feature's own top cells; the second pass (interior simplices
+    // of 4-D meshes): the lifted face's
+    for (int pass = 0; pass < 2; ++pass) {
+      const bool over_face = pass ? M == 3 && !spatial && !lateral : lateral;
+      if (pass && !over_face) break;
+      const bool star = pass == 0;
+      const bool unite_all = M == 3 && (pass || lateral);
+      const unsigned q0 = over_face ? (fi < 0 ? 0u : X.cof_start[fi]) : 0u;
+      const unsigned nq = over_face ? (fi < 0 ? 0u : X.cof_start[fi + 1] - q0) : 2u;
+      for (unsigned qb = 0; qb < nq; qb += kCells) {
+        const unsigned q = qb + q_lane;
+        bool valid = used && q < nq;
+        unsigned u[M + 1];
+        unsigned long long tt = t;
+        int p = 0;
+#pragma unroll
+        for (int k = 0; k <= M; ++k) u[k] = sp[k];
+        if (valid && over_face) {
+          const unsigned* cell = X.cells + (size_t)X.cof[q0 + q] * (M + 1);
+          int e = -1, wi = 0;
+#pragma unroll
+          for (int k = 0; k <= M; ++k) {
+            u[k] = cell[k];
+            const unsigned fw = wi == 0 ? f[0] : wi == 1 ? f[1] : f[M - 1];
+            if (wi < M && u[k] == fw) ++wi;
+            else e = k;
+          }
+          valid = e >= 0;
+          p = j + (e <= j ? 1 : 0);
+        } else if (spatial) {
+          p = q ? 0 : M;
+          tt = q ? t - 1 : t;
+          valid = valid && (q ? t > X.t0 : t < (unsigned long long)X.t0 + X.L);
+        } else {
+          p = j + (int)q;
+        }
+        // the cell u[0..p]@tt, u[p..M]@tt+1 without its vertex r
+        long long idx = -1;
+        if (valid) {
+          unsigned long long face[M + 1];
+#pragma unroll
+          for (int k = 0; k <= M; ++k) {
+            const unsigned long long a = k <= p ? tt * ns + u[k] : (tt + 1) * ns + u[k ? k - 1 : 0];
+            const unsigned long long b = k + 1 <= p ? tt * ns + u[k < M ? k + 1 : M] : (tt + 1) * ns + u[k];
+            face[k] = k < (int)r ? a : b;
+          }
+          unsigned long long h, l;
+          pack_tuple<M>(face, Fs.vb, h, l);
+          idx = find_tuple(Fs.hi, Fs.lo, n, h, l);
+        }
+        bool emit = false;
+        if (star) {
+          const unsigned long long node =
+              idx >= 0 ? ((unsigned long long)Fs.phase[idx] << 32) | (unsigned long long)idx : ~0ull;
+          unsigned long long centre = ~0ull;
+#pragma unroll
+          for (int k = 0; k < kFaces; ++k) {
+            const unsigned long long o = __shfl_sync(gm, node, first + k);
+            if (o < centre) centre = o;
+          }
+          emit = idx >= 0 && (unsigned)centre == i && idx != (long long)i;
+        }
+        const unsigned ball = __ballot_sync(gm, emit) >> shift & 0xFFFFu;
+        if (ball) {
+          others += __popc(ball);
+          unsigned at = 0;
+          if (hl == 0) at = atomicAdd(out.n_edges, (unsigned)__popc(ball));
+          at = __shfl_sync(gm, at, shift) + __popc(ball & ((1u << hl) - 1));
+          if (emit) {
+            const unsigned x = (unsigned)idx, lo = min(x, i), hi = max(x, i);
+            if (!out.pairs) {
+              if (at < out.cap) out.ekeys[at] = ((unsigned long long)lo << 32) | hi;
+            } else if (at < out.cap - out.base) {
+              out.pairs[2 * (size_t)(out.base + at)] = out.ids ? out.ids[lo] : lo;
+              out.pairs[2 * (size_t)(out.base + at) + 1] = out.ids ? out.ids[hi] : hi;
+            }
+          }
+        }
+        if (idx >= 0 && (emit || unite_all))
+          uf_unite(out.parent, id, out.ids ? out.ids[idx] : (unsigned)idx, out.err);
+        __syncwarp(gm);
+      }
+    }
+    if (others > kMaxOthers && hl == 0) atomicOr(out.err, kErrCofaces);
   }
 }
 
@@ -830,68 +831,106 @@ cudaError_t enqueue_extract(ftk2b_ctx* ctx, const ExtMeshDev& X, const FieldAcce
   return cudaGetLastError();
 }
 
+// The packed edges of C.ekeys in order to the context's edges, any number of them.
+cudaError_t sort_edges(ftk2b_ctx* ctx, unsigned edge_cap, unsigned long long* nl) {
+  ExtCache& C = ctx->ext;
+  const unsigned* n_edges = (const unsigned*)ctx->counters.p + kCountEdges;
+  const bool alt = radix_sort((unsigned long long*)C.ekeys.p, (unsigned*)C.sort_v.p, (unsigned long long*)C.sort_k2.p,
+                              (unsigned*)C.sort_v2.p, n_edges, edge_cap, 64, (unsigned*)ctx->hist.p,
+                              ctx->sort_grid(edge_cap), ctx->stream, nl);
+  ext_unpack_edges_kernel<<<grid_of(edge_cap, 256, 4096), 256, 0, ctx->stream>>>(
+      (const unsigned long long*)(alt ? C.sort_k2.p : C.ekeys.p), n_edges, edge_cap, (unsigned*)ctx->edges.p);
+  *nl += 1;
+  return cudaGetLastError();
+}
+
+// The features of one extraction in canonical order by one rank sort of their
+// tuples (cp_ranksort.cuh); each also becomes a component of its own.
+struct LoadFound {
+  const unsigned long long *hi, *lo;
+  __device__ __forceinline__ void operator()(unsigned i, unsigned long long (&k)[2]) const {
+    k[0] = hi[i];
+    k[1] = lo[i];
+  }
+};
 template <int M>
-cudaError_t enqueue_post(ftk2b_ctx* ctx, const ExtMeshDev& X, const ExtSink& sink, unsigned cap,
-                         unsigned edge_cap, int vb, int want_edges, unsigned long long* nl) {
+struct StoreFound {
+  ExtSink in;
+  ExtSorted out;
+  int vb;
+  __device__ __forceinline__ void operator()(unsigned pos, unsigned i, const unsigned long long (&)[2]) const {
+    ext_finalize<M>(in, i, vb, out, pos);
+  }
+};
+// their star edges in order
+struct LoadEdgeKey {
+  const unsigned long long* key;
+  __device__ __forceinline__ void operator()(unsigned e, unsigned long long (&k)[1]) const { k[0] = key[e]; }
+};
+
+// Canonical order, star edges, trajectories.  n: the features found (at most
+// cap).  Sets kCountEdges and kCountRoots; *edges_ranked says whether the edges
+// were sorted by one launch that holds for up to kRankCap1 of them.
+template <int M>
+cudaError_t enqueue_post(ftk2b_ctx* ctx, const ExtMeshDev& X, const ExtSink& sink, unsigned n, unsigned cap,
+                         unsigned edge_cap, int vb, int want_edges, bool* edges_ranked, unsigned long long* nl) {
   cudaStream_t st = ctx->stream;
   ExtCache& C = ctx->ext;
   unsigned* counters = (unsigned*)ctx->counters.p;
   unsigned* count = counters + kCountFeatures;
-  const int sgrid = ctx->sort_grid(cap);
-  unsigned* hist = (unsigned*)ctx->hist.p;
-  const int g = grid_of(cap, 256, 4096);
   cudaError_t e;
-  // canonical order: stable sort by the low word, then by the high word
-  if ((e = cudaMemcpyAsync(C.sort_k.p, sink.lo, sizeof(unsigned long long) * cap, cudaMemcpyDeviceToDevice, st)))
-    return e;
-  if ((e = launch_iota((unsigned*)ctx->perm0.p, count, cap, st))) return e;
-  const int lo_bits = (M == 3) ? 2 * vb : vb;
-  bool alt = radix_sort((unsigned long long*)C.sort_k.p, (unsigned*)ctx->perm0.p,
-                        (unsigned long long*)C.sort_k2.p, (unsigned*)ctx->perm1.p, count, cap, lo_bits,
-                        hist, sgrid, st, nl);
-  unsigned* p1 = (unsigned*)(alt ? ctx->perm1.p : ctx->perm0.p);
-  unsigned* p1_other = (unsigned*)(alt ? ctx->perm0.p : ctx->perm1.p);
-  ext_gather_by_perm_kernel<<<g, 256, 0, st>>>(sink.hi, p1, count, cap, (unsigned long long*)C.sort_k.p);
-  alt = radix_sort((unsigned long long*)C.sort_k.p, p1, (unsigned long long*)C.sort_k2.p, p1_other, count, cap,
-                   2 * vb, hist, sgrid, st, nl);
-  const unsigned* perm = alt ? p1_other : p1;
-  ext_finalize_kernel<M><<<g, 256, 0, st>>>(perm, count, cap, vb, sink, (unsigned long long*)C.hi_s.p,
-                                            (unsigned long long*)C.lo_s.p, (unsigned*)C.phase_s.p,
-                                            (double*)ctx->lam_s.p, (float*)ctx->scalar_s.p,
-                                            (unsigned long long*)ctx->simplices.p, (float*)ctx->bary.p);
-  *nl += 3;  // iota, gather, finalize
+  const ExtSorted out{(unsigned long long*)C.hi_s.p, (unsigned long long*)C.lo_s.p, (unsigned*)C.phase_s.p,
+                      (double*)ctx->lam_s.p, (float*)ctx->scalar_s.p, (unsigned long long*)ctx->simplices.p,
+                      (float*)ctx->bary.p, (unsigned*)ctx->parent.p};
+  const bool ranked = n <= kRankCap2;
+  *edges_ranked = ranked;
+  if (ranked) {
+    const LoadFound ld{sink.hi, sink.lo};
+    const StoreFound<M> sw{sink, out, vb};
+    if ((e = launch_rank_sort<2>(ld, sw, nullptr, n, nullptr, ctx->num_sms, st))) return e;
+    *nl += 1;
+  } else {
+    const int sgrid = ctx->sort_grid(cap);
+    unsigned* hist = (unsigned*)ctx->hist.p;
+    const int g = grid_of(n, 256, 4096);
+    // stable sort by the low word, then by the high word
+    if ((e = cudaMemcpyAsync(C.sort_k.p, sink.lo, sizeof(unsigned long long) * n, cudaMemcpyDeviceToDevice, st)))
+      return e;
+    if ((e = launch_iota((unsigned*)ctx->perm0.p, count, n, st))) return e;
+    const int lo_bits = (M == 3) ? 2 * vb : vb;
+    bool alt = radix_sort((unsigned long long*)C.sort_k.p, (unsigned*)ctx->perm0.p,
+                          (unsigned long long*)C.sort_k2.p, (unsigned*)ctx->perm1.p, count, cap, lo_bits,
+                          hist, sgrid, st, nl);
+    unsigned* p1 = (unsigned*)(alt ? ctx->perm1.p : ctx->perm0.p);
+    unsigned* p1_other = (unsigned*)(alt ? ctx->perm0.p : ctx->perm1.p);
+    ext_gather_by_perm_kernel<<<g, 256, 0, st>>>(sink.hi, p1, count, cap, (unsigned long long*)C.sort_k.p);
+    alt = radix_sort((unsigned long long*)C.sort_k.p, p1, (unsigned long long*)C.sort_k2.p, p1_other, count, cap,
+                     2 * vb, hist, sgrid, st, nl);
+    const unsigned* perm = alt ? p1_other : p1;
+    ext_finalize_kernel<M><<<g, 256, 0, st>>>(perm, count, cap, vb, sink, out);
+    *nl += 3;  // iota, gather, finalize
+  }
   if (!want_edges) return cudaGetLastError();
-  ExtFeatures Fs;
-  Fs.hi = (const unsigned long long*)C.hi_s.p;
-  Fs.lo = (const unsigned long long*)C.lo_s.p;
-  Fs.phase = (const unsigned*)C.phase_s.p;
-  Fs.n_ptr = count;
-  Fs.cap = cap;
-  Fs.vb = vb;
-  unsigned* err = counters + kCountErr;
-  unsigned* n_edges = counters + kCountEdges;
-  unsigned* ecnt = (unsigned*)ctx->edge_cnt.p;
-  unsigned long long* ekeys = (unsigned long long*)C.ekeys.p;
-  ext_edges_kernel<M, 0><<<g, 256, 0, st>>>(X, Fs, ecnt, nullptr, ekeys, edge_cap, err);
-  if ((e = launch_scan(ecnt, cap, n_edges, count, st))) return e;
-  ext_edges_kernel<M, 1><<<g, 256, 0, st>>>(X, Fs, nullptr, ecnt, ekeys, edge_cap, err);
+  const ExtFeatures Fs{out.hi, out.lo, out.phase, count, cap, vb};
+  const ExtStars stars{nullptr, out.parent, (unsigned long long*)C.ekeys.p, nullptr, 0u, edge_cap,
+                       counters + kCountEdges, counters + kCountErr};
+  ext_stars_kernel<M><<<grid_of(kStarLanes * (unsigned long long)n, 256, 4096), 256, 0, st>>>(X, Fs, stars);
   // (min, max) pairs sorted lexicographically; a pair spans exactly one top
   // cell, so there are no duplicates
-  const int eb = 2 * 32;
-  const bool ealt = radix_sort(ekeys, (unsigned*)C.sort_v.p, (unsigned long long*)C.sort_k2.p,
-                               (unsigned*)C.sort_v2.p, n_edges, edge_cap, eb, hist, ctx->sort_grid(edge_cap), st,
-                               nl);
-  const unsigned long long* es = ealt ? (const unsigned long long*)C.sort_k2.p : ekeys;
-  ext_unpack_edges_kernel<<<grid_of(edge_cap, 256, 4096), 256, 0, st>>>(es, n_edges, edge_cap,
-                                                                       (unsigned*)ctx->edges.p);
-  if ((e = launch_uf((unsigned*)ctx->parent.p, count, cap, (const unsigned*)ctx->edges.p, n_edges, edge_cap, err,
-                     st)))
+  if (ranked) {
+    const LoadEdgeKey ld{(const unsigned long long*)C.ekeys.p};
+    const StoreEdge so{(unsigned*)ctx->edges.p};
+    if ((e = launch_rank_sort<1>(ld, so, counters + kCountEdges, std::min(edge_cap, kRankCap1), nullptr,
+                                 ctx->num_sms, st)))
+      return e;
+    *nl += 1;
+  } else if ((e = sort_edges(ctx, edge_cap, nl))) {
     return e;
-  if (M == 3) ext_coface_union_kernel<<<g, 256, 0, st>>>(X, Fs, nullptr, (unsigned*)ctx->parent.p, err);
-  if ((e = launch_uf_label((unsigned*)ctx->parent.p, count, cap, (unsigned long long*)ctx->track.p,
-                           counters + kCountRoots, st)))
+  }
+  if ((e = launch_uf_label(out.parent, count, n ? n : 1, (unsigned long long*)ctx->track.p, counters + kCountRoots,
+                           st)))
     return e;
-  *nl += 8 + (M == 3 ? 1 : 0);
+  *nl += 2;
   return cudaGetLastError();
 }
 
@@ -986,21 +1025,6 @@ struct StoreTupleOrder {
     order.put(pos, i);
   }
 };
-
-// window star edges (packed window indices) -> stream ids, united and stored
-__global__ void ext_append_edges_kernel(const unsigned long long* __restrict__ ek, const unsigned* n_ptr,
-                                        unsigned cap, const unsigned* __restrict__ ids, unsigned* parent,
-                                        unsigned* __restrict__ out, unsigned base, unsigned out_cap, unsigned* err) {
-  const unsigned n = min(*n_ptr, cap);
-  for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x) {
-    const unsigned a = ids[(unsigned)(ek[e] >> 32)], b = ids[(unsigned)ek[e]];
-    uf_unite(parent, a, b, err);
-    if (base + e < out_cap) {
-      out[2 * (size_t)(base + e)] = a;
-      out[2 * (size_t)(base + e) + 1] = b;
-    }
-  }
-}
 
 template <int M>
 __global__ void ext_collect_spatial_kernel(const unsigned long long* __restrict__ hi,
@@ -1142,9 +1166,7 @@ ftk2b_status push_extruded_t(ftk2b_stream* s) {
   EXT_TRY(s->s_hi.ensure(8 * (size_t)wcap));
   EXT_TRY(s->s_lo.ensure(8 * (size_t)wcap));
   EXT_TRY(s->s_phase.ensure(4 * (size_t)wcap));
-  EXT_TRY(s->wedges.ensure(8 * (size_t)wecap));
-  EXT_TRY(ctx->edge_cnt.ensure(4 * (size_t)wcap));
-  EXT_TRY(ctx->hist.ensure(sizeof(unsigned) * 256 * (size_t)ctx->sort_grid(wcap > wecap ? wcap : wecap)));
+  EXT_TRY(ctx->hist.ensure(sizeof(unsigned) * 256 * (size_t)ctx->sort_grid(wcap)));
   const unsigned edge_room = s->n_edges + wecap;
   if (edge_room > s->edge_cap) {
     unsigned nc = s->edge_cap ? s->edge_cap : 262144u;
@@ -1183,22 +1205,16 @@ ftk2b_status push_extruded_t(ftk2b_stream* s) {
   Fs.cap = wcap;
   Fs.vb = kStreamVb;
   unsigned* err = counters + kCountErr;
-  unsigned* ecnt = (unsigned*)ctx->edge_cnt.p;
-  unsigned long long* ek = (unsigned long long*)s->wedges.p;
-  ext_edges_kernel<M, 0><<<g, 256, 0, st>>>(X, Fs, ecnt, nullptr, ek, wecap, err);
-  EXT_TRY(launch_scan(ecnt, wcap, counters + kSWinEdges, counters + kSWin, st));
-  ext_edges_kernel<M, 1><<<g, 256, 0, st>>>(X, Fs, nullptr, ecnt, ek, wecap, err);
   if (n_new && !ranked)
     uf_init_range_kernel<<<grid_of(n_new, 256, 4096), 256, 0, st>>>((unsigned*)s->parent.p, first_new, n_new);
-  ext_append_edges_kernel<<<grid_of(wecap, 256, 4096), 256, 0, st>>>(ek, counters + kSWinEdges, wecap, ids,
-                                                                    (unsigned*)s->parent.p, (unsigned*)s->edges.p,
-                                                                    s->n_edges, s->edge_cap, err);
-  if (M == 3) ext_coface_union_kernel<<<g, 256, 0, st>>>(X, Fs, ids, (unsigned*)s->parent.p, err);
+  const ExtStars stars{ids, (unsigned*)s->parent.p, nullptr, (unsigned*)s->edges.p, s->n_edges, s->edge_cap,
+                       counters + kSWinEdges, err};
+  ext_stars_kernel<M><<<grid_of(kStarLanes * (unsigned long long)wcap, 256, 4096), 256, 0, st>>>(X, Fs, stars);
   if (n_new && !ranked)
     ext_collect_spatial_kernel<M><<<grid_of(n_new, 256, 4096), 256, 0, st>>>(
         (const unsigned long long*)s->hi.p, (const unsigned long long*)s->lo.p, first_new, n_new, ns, tnow,
         (unsigned*)s->prev_ids2.p, counters + kSPrev);
-  nl += 9;
+  nl += ranked ? 2 : 6;
   EXT_TRY(cudaGetLastError());
   EXT_TRY(cudaMemcpyAsync(ctx->h_counters, counters, sizeof(unsigned) * kNumCounters, cudaMemcpyDeviceToHost, st));
   EXT_TRY(cudaEventRecord(ctx->ev1, st));
@@ -1337,7 +1353,7 @@ uint64_t extruded_simplex_count(const ftk2b_mesh_desc* mesh, int m) {
 }
 
 ftk2b_status run_extruded(ftk2b_ctx* ctx, const ftk2b_mesh_desc* mesh, const ftk2b_field_desc* field,
-                          const ftk2b_cp_params* prm, const double* fiber_thr) {
+                          const ftk2b_cp_params* prm, const double* fiber_thr, bool pack) {
   int fbits = 0;
   ftk2b_status st = validate_mesh(ctx, mesh, &fbits);
   if (st) return st;
@@ -1435,11 +1451,37 @@ ftk2b_status run_extruded(ftk2b_ctx* ctx, const ftk2b_mesh_desc* mesh, const ftk
               : enqueue_extract<float, 2>(ctx, X, fa, cfg, sink, vb, nv, &nl);
     EXT_TRY(e);
     EXT_TRY(cudaEventRecord(ctx->ev_x, s));
-    e = (M == 3) ? enqueue_post<3>(ctx, X, sink, cap, edge_cap, vb, prm->want_edges, &nl)
-                 : enqueue_post<2>(ctx, X, sink, cap, edge_cap, vb, prm->want_edges, &nl);
-    EXT_TRY(e);
+    // the number of features decides how they are sorted: reading it costs a
+    // wait (about 12 us), the radix passes for a capacity unread some 150 us
     EXT_TRY(cudaMemcpyAsync(ctx->h_counters, ctx->counters.p, sizeof(unsigned) * kNumCounters,
                             cudaMemcpyDeviceToHost, s));
+    EXT_TRY(ctx->sync());
+    const unsigned n = ctx->h_counters[kCountFeatures];
+    if (n > cap) {
+      const uint64_t want = (uint64_t)n + n / 4 + 1024;
+      if (want > 0x7FFFFFF0ull) return ext_fail(ctx, FTK2B_OVERFLOW_RETRY, "feature count exceeds 2^31");
+      cap = (unsigned)want;
+      ctx->cap_hint = cap;
+      continue;
+    }
+    bool edges_ranked = false;
+    e = (M == 3) ? enqueue_post<3>(ctx, X, sink, n, cap, edge_cap, vb, prm->want_edges, &edges_ranked, &nl)
+                 : enqueue_post<2>(ctx, X, sink, n, cap, edge_cap, vb, prm->want_edges, &edges_ranked, &nl);
+    EXT_TRY(e);
+    LastRun r;
+    r.m = M;
+    r.want_edges = prm->want_edges;
+    if (pack) {
+      PackArgs a = ctx->pack_args(r);
+      a.h_counters = (unsigned*)ctx->pin.d;
+      a.cap = cap;
+      a.edge_cap = edges_ranked ? std::min(edge_cap, kRankCap1) : edge_cap;
+      EXT_TRY(launch_pack(a, ctx->num_sms, s));
+      nl += 1;
+    } else {
+      EXT_TRY(cudaMemcpyAsync(ctx->h_counters, ctx->counters.p, sizeof(unsigned) * kNumCounters,
+                              cudaMemcpyDeviceToHost, s));
+    }
     EXT_TRY(cudaEventRecord(ctx->ev1, s));
     EXT_TRY(ctx->sync());
     ctx->launches += nl;
@@ -1454,14 +1496,18 @@ ftk2b_status run_extruded(ftk2b_ctx* ctx, const ftk2b_mesh_desc* mesh, const ftk
     if (h[kCountErr] & kErrCofaces)
       return ext_fail(ctx, FTK2B_UNSUPPORTED, "a base face has more than 8 coface cells");
     if (h[kCountErr] & 1u) return ext_fail(ctx, FTK2B_TIMEOUT, "union-find retry bound reached");
-    if (h[kCountFeatures] > cap || h[kCountEdges] > edge_cap) {
-      uint64_t want = (uint64_t)h[kCountFeatures] + h[kCountFeatures] / 4 + 1024;
-      const uint64_t want_e = ((uint64_t)h[kCountEdges] + 1) / 2 + 1024;
-      if (want_e > want) want = want_e;
+    if (h[kCountEdges] > edge_cap) {
+      const uint64_t want = ((uint64_t)h[kCountEdges] + 1) / 2 + 1024;
       if (want > 0x7FFFFFF0ull) return ext_fail(ctx, FTK2B_OVERFLOW_RETRY, "feature count exceeds 2^31");
       cap = (unsigned)want;
       ctx->cap_hint = cap;
       continue;
+    }
+    const bool edges_left = edges_ranked && h[kCountEdges] > kRankCap1;  // few features, very many edges
+    if (edges_left) {
+      EXT_TRY(sort_edges(ctx, edge_cap, &nl));
+      EXT_TRY(ctx->sync());
+      ctx->launches += nl;
     }
     ctx->last.kind = FTK2B_MESH_EXTRUDED;
     ctx->last.m = M;
@@ -1473,6 +1519,8 @@ ftk2b_status run_extruded(ftk2b_ctx* ctx, const ftk2b_mesh_desc* mesh, const ftk
     ctx->last.device_ms = ms;
     ctx->last.classify = 0;
     ctx->last.want_edges = prm->want_edges;
+    ctx->pack_ready =
+        pack && !edges_left && pack_layout(ctx->last.n, ctx->last.ne, M + 1, 0).packed <= ctx->pack_bytes();
     return FTK2B_OK;
   }
   return ext_fail(ctx, FTK2B_OVERFLOW_RETRY, "feature buffer overflow persisted after retries");
