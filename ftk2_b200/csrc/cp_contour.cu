@@ -61,9 +61,26 @@ struct CtGeom {
   unsigned long long aoff[16];  // array step to corner e
   unsigned long long lstr[4];   // local linear strides
   unsigned char perm[24][4];    // axis order of the p-th Kuhn simplex (CPU mesh order)
+  int linear;                   // array index = local linear index
+  int small;                    // nv < 2^31: i / L[k] = (i * mul[k]) >> shf[k]
+  unsigned mul[4];
+  int shf[4];
 };
 
+// Local coordinates of local vertex i.  Meshes below 2^31 vertices divide by
+// multiplying with rounded-up reciprocals (exact for such i): three or four
+// 64-bit divisions a vertex bounded every kernel that walks the vertices.
 __device__ __forceinline__ void ct_coords(const CtGeom& g, unsigned long long i, unsigned long long* c) {
+  if (g.small) {
+    unsigned r = (unsigned)i;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      const unsigned q = k + 1 < g.d ? (unsigned)(((unsigned long long)r * g.mul[k]) >> g.shf[k]) : 0u;
+      c[k] = k < g.d ? r - q * (unsigned)g.L[k] : 0u;
+      r = q;
+    }
+    return;
+  }
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     if (k < g.d) {
@@ -77,13 +94,15 @@ __device__ __forceinline__ void ct_coords(const CtGeom& g, unsigned long long i,
 
 __device__ __forceinline__ unsigned long long ct_gid(const CtGeom& g, const unsigned long long* c) {
   unsigned long long v = g.g0;
-  for (int k = 0; k < g.d; ++k) v += c[k] * g.gs[k];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) v += c[k] * g.gs[k];  // strides of axes the mesh has not are 0
   return v;
 }
 
 __device__ __forceinline__ unsigned long long ct_aidx(const CtGeom& g, const unsigned long long* c) {
   unsigned long long v = 0;
-  for (int k = 0; k < g.d; ++k) v += c[k] * g.as[k];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) v += c[k] * g.as[k];
   return v;
 }
 
@@ -105,16 +124,71 @@ __device__ __forceinline__ bool ct_positive(T adj, unsigned long long gid, doubl
   return (gid & 1ull) == 0;
 }
 
-template <typename T>
-__global__ void ct_sign_kernel(CtGeom g, const T* __restrict__ a, T thr, double q,
-                               unsigned char* __restrict__ pos) {
-  for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < g.nv;
-       i += (unsigned long long)gridDim.x * blockDim.x) {
-    unsigned long long c[4];
-    ct_coords(g, i, c);
-    const unsigned long long gid = ct_gid(g, c);
-    pos[i] = ct_positive(ct_adj(g, a, ct_aidx(g, c), gid, thr), gid, q) ? 1 : 0;
+// Bit planes: bit i & 31 of word i >> 5 belongs to local vertex i.  The 32
+// neighbours of 32 consecutive vertices in one corner direction are then one
+// shifted word, and a warp settles its vertices with a word per corner and lane
+// instead of a load per corner and vertex.
+__host__ __device__ inline unsigned long long ct_words(const CtGeom& g) {
+  return (g.nv + g.loff[(1 << g.d) - 1]) / 32 + 2;  // the corners of out-of-mesh cubes included
+}
+
+// Each warp takes 128 consecutive vertices, four per lane in flight:
+// load(i, j) by every lane (the last vertex again beyond the end; it must not
+// use the value), then words(w, j) by the whole warp for the 32 of word w.
+template <typename Load, typename Words>
+__device__ __forceinline__ void ct_each_word(unsigned long long n, Load load, Words words) {
+  const unsigned lane = threadIdx.x & 31;
+  const unsigned long long step = (unsigned long long)gridDim.x * blockDim.x * 4;
+  for (unsigned long long i0 = (blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x - lane) * 4; i0 < n;
+       i0 += step) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) load(min(i0 + 32 * j + lane, n - 1), j);
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (i0 + 32 * j < n) words(i0 / 32 + j, j);
   }
+}
+
+// step from a vertex to its corner e (lane-varying, so not from the table)
+__device__ __forceinline__ unsigned long long ct_corner_step(const CtGeom& g, unsigned e) {
+  unsigned long long v = 0;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) v += (e >> k) & 1u ? g.lstr[k] : 0ull;
+  return v;
+}
+
+// array index of local vertex i
+__device__ __forceinline__ unsigned long long ct_index(const CtGeom& g, unsigned long long i) {
+  if (g.linear) return i;
+  unsigned long long c[4];
+  ct_coords(g, i, c);
+  return g.per_vertex ? ct_gid(g, c) : ct_aidx(g, c);
+}
+
+// Bound by the field's bytes (96^3 x 6 double: 56 us with 64-bit divisions for
+// each vertex's coordinates, which only ties need, now 14).
+template <typename T>
+__global__ void ct_sign_kernel(CtGeom g, const T* __restrict__ a, T thr, double q, unsigned* __restrict__ pos) {
+  const unsigned lane = threadIdx.x & 31;
+  T v[4];
+  ct_each_word(
+      g.nv, [&](unsigned long long i, int j) { v[j] = __ldg(a + ct_index(g, i)); },
+      [&](unsigned long long w, int j) {
+        const unsigned long long i = 32 * w + lane;
+        bool p = false;
+        if (i < g.nv) {
+          const T y = fp<T>::sub(v[j], thr);
+          const double x = __dadd_rn(__dmul_rn((double)y, q), y > T(0) ? 0.5 : -0.5);
+          p = x >= 1.0;
+          if (!p && !(x <= -1.0)) {
+            unsigned long long c[4];
+            ct_coords(g, i, c);
+            p = ct_positive(y, ct_gid(g, c), q);
+          }
+        }
+        const unsigned word = __ballot_sync(0xffffffffu, p);
+        if (lane == 0) pos[w] = word;
+      });
 }
 
 // block-wide exclusive scan of one count per thread; returns the thread's
@@ -145,32 +219,128 @@ __device__ __forceinline__ unsigned ct_block_scan(unsigned v, unsigned* total) {
   return wsum[warp] + incl - v;
 }
 
+// Kernels over the vertices of a regular mesh give a block kCtPer shares of
+// kCtThreads consecutive vertices: vertex share * kCtThreads + thread.  One
+// atomic per block then reserves list rows or adds to a total; one per warp on
+// the same address took longer than everything else these kernels do.
+constexpr int kCtPer = 4;
+constexpr int kCtBlock = kCtPer * kCtThreads;
+
+// Exclusive prefix in vertex order over the block of kCtPer counts per thread;
+// returns the block's sum.
+__device__ __forceinline__ unsigned ct_block_ranks(unsigned (&v)[kCtPer]) {
+  constexpr int kWarps = kCtThreads / 32;
+  static_assert(kCtPer * kWarps == 32, "one warp scans the words' sums");
+  __shared__ unsigned sum[32], total;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int j = 0; j < kCtPer; ++j) {
+    unsigned incl = v[j];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    if (lane == 31) sum[j * kWarps + warp] = incl;
+    v[j] = incl - v[j];
+  }
+  __syncthreads();
+  if (warp == 0) {
+    const unsigned w = sum[lane];
+    unsigned wi = w;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned y = __shfl_up_sync(0xffffffffu, wi, o);
+      if (lane >= o) wi += y;
+    }
+    sum[lane] = wi - w;
+    if (lane == 31) total = wi;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < kCtPer; ++j) v[j] += sum[j * kWarps + warp];
+  return total;
+}
+
 __device__ __forceinline__ unsigned ct_inbounds(const CtGeom& g, const unsigned long long* c) {
   unsigned inb = 0;
-  for (int k = 0; k < g.d; ++k)
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
     if (c[k] + 1 < g.L[k]) inb |= 1u << k;
   return inb;
 }
 
-__global__ void ct_mask_kernel(CtGeom g, const unsigned char* __restrict__ pos, unsigned short* __restrict__ mask,
-                               unsigned* __restrict__ blk, unsigned long long* __restrict__ total64) {
-  __shared__ unsigned tot;
-  const unsigned long long i = blockIdx.x * (unsigned long long)kCtThreads + threadIdx.x;
-  unsigned m = 0;
-  if (i < g.nv) {
-    unsigned long long c[4];
-    ct_coords(g, i, c);
-    const unsigned inb = ct_inbounds(g, c);
-    const unsigned char p = pos[i];
-    const int ne = 1 << g.d;
-    for (int e = 1; e < ne; ++e)
-      if ((e & ~inb) == 0 && pos[i + g.loff[e]] != p) m |= 1u << (e - 1);
-    mask[i] = (unsigned short)m;
+// Crossing mask of every vertex (bit e - 1: the edge to corner e), the counts
+// of each block, and the list of mixed hypercubes (corner signs not all equal),
+// each one word: base vertex (local linear index) << 20 | upper-face axes << 16
+// | corner signs (bit e: corner e positive).  An upper-face axis k is one where
+// the cube's corners with bit k set lie on the mesh's last layer (c_k = L_k - 2).
+// A cube's signs are its lowest vertex's and mask, so the cubes need no pass of
+// their own (96^3 x 6: 90 + 57 us for both, now 38).
+constexpr int kCtBaseShift = 20;
+
+__global__ void __launch_bounds__(kCtThreads) ct_mask_kernel(
+    CtGeom g, const unsigned* __restrict__ pos, unsigned short* __restrict__ mask, unsigned* __restrict__ blk,
+    unsigned long long* __restrict__ total64, unsigned long long* __restrict__ list,
+    unsigned* __restrict__ list_cnt) {
+  __shared__ unsigned s_at;
+  const unsigned long long i0 = blockIdx.x * (unsigned long long)kCtBlock + threadIdx.x;
+  const int ne = 1 << g.d;
+  const unsigned lane = threadIdx.x & 31;
+  // lane e: the signs of the warp's vertices, and those at their corners e
+  unsigned here[kCtPer], cross[kCtPer];
+#pragma unroll
+  for (int j = 0; j < kCtPer; ++j) {
+    const unsigned long long w0 = i0 - lane + j * kCtThreads;
+    here[j] = cross[j] = 0;
+    if (w0 < g.nv) {
+      here[j] = pos[w0 / 32];
+      if ((int)lane < ne) {
+        const unsigned long long o = w0 + ct_corner_step(g, lane);
+        cross[j] = here[j] ^ __funnelshift_r(pos[o / 32], pos[o / 32 + 1], (unsigned)o & 31u);
+      }
+    }
   }
-  ct_block_scan(__popc(m), &tot);
+  unsigned rank[kCtPer];  // crossing edges, mixed cubes << 16
+  unsigned upper[kCtPer], m[kCtPer];
+#pragma unroll
+  for (int j = 0; j < kCtPer; ++j) {
+    const unsigned long long i = i0 + j * kCtThreads;
+    m[j] = upper[j] = rank[j] = 0;
+    if (__any_sync(0xffffffffu, cross[j] != 0)) {
+      unsigned long long c[4];
+      ct_coords(g, i, c);
+      const unsigned inb = i < g.nv ? ct_inbounds(g, c) : 0u;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const unsigned in = __ballot_sync(0xffffffffu, (inb >> k) & 1u);
+        if ((lane >> k) & 1u) cross[j] &= in;
+        if (c[k] + 2 == g.L[k]) upper[j] |= 1u << k;
+      }
+#pragma unroll
+      for (int e = 1; e < 16; ++e) m[j] |= ((__shfl_sync(0xffffffffu, cross[j], e) >> lane) & 1u) << (e - 1);
+      rank[j] = __popc(m[j]);
+      if (m[j] != 0 && inb == (1u << g.d) - 1u) rank[j] |= 1u << 16;
+    }
+    if (i < g.nv) mask[i] = (unsigned short)m[j];
+  }
+  bool mixed[kCtPer];
+#pragma unroll
+  for (int j = 0; j < kCtPer; ++j) mixed[j] = rank[j] >> 16;
+  const unsigned n = ct_block_ranks(rank);
   if (threadIdx.x == 0) {
-    blk[blockIdx.x] = tot;
-    atomicAdd(total64, (unsigned long long)tot);  // exact count: the offsets are 32-bit
+    blk[blockIdx.x] = n & 0xFFFFu;
+    if (n & 0xFFFFu) atomicAdd(total64, (unsigned long long)(n & 0xFFFFu));  // exact: the offsets are 32-bit
+    if (n >> 16) s_at = atomicAdd(list_cnt, n >> 16);
+  }
+  if (n >> 16 == 0) return;
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < kCtPer; ++j) {
+    if (!mixed[j]) continue;
+    const unsigned all = (1u << ne) - 1u, sgn = (here[j] >> lane) & 1u ? ~(m[j] << 1) & all : m[j] << 1;
+    list[s_at + (rank[j] >> 16)] =
+        ((i0 + j * kCtThreads) << kCtBaseShift) | ((unsigned long long)upper[j] << 16) | sgn;
   }
 }
 
@@ -193,180 +363,295 @@ __device__ __forceinline__ void ct_solve(T a0, T a1, T* l0, T* l1) {
   *l1 = ok ? x1 : T(0.5);
 }
 
+// The crossing edges of a block's vertices in rank order: entry k is vertex of
+// the block << 4 | corner.  Returns their number; n edges start at rank
+// blk_off[block].  s_mask: the vertices' masks.
+struct CtEdges {
+  unsigned short edge[kCtBlock * 15];
+  unsigned short mask[kCtBlock];
+};
+__device__ __forceinline__ unsigned ct_list_edges(const CtGeom& g, const unsigned short* __restrict__ mask,
+                                                  unsigned base, unsigned* __restrict__ voff, CtEdges& s) {
+  const unsigned long long i0 = blockIdx.x * (unsigned long long)kCtBlock;
+  unsigned m[kCtPer], rank[kCtPer];
+#pragma unroll
+  for (int j = 0; j < kCtPer; ++j) {
+    const unsigned long long i = i0 + j * kCtThreads + threadIdx.x;
+    m[j] = i < g.nv ? mask[i] : 0u;
+    rank[j] = __popc(m[j]);
+  }
+  const unsigned n = ct_block_ranks(rank);
+  if (n == 0) return 0;
+#pragma unroll
+  for (int j = 0; j < kCtPer; ++j) {
+    const unsigned v = j * kCtThreads + threadIdx.x;
+    unsigned w = rank[j];
+    s.mask[v] = (unsigned short)m[j];
+    if (m[j] && voff) voff[i0 + v] = base + w;
+    for (unsigned x = m[j]; x; x &= x - 1) s.edge[w++] = (unsigned short)(v << 4 | __ffs(x));
+  }
+  __syncthreads();
+  return n;
+}
+
+// number of crossing edges of mask m below corner e
+__device__ __forceinline__ unsigned ct_below(unsigned m, unsigned e) { return __popc(m & ((1u << (e - 1)) - 1u)); }
+// The crossing edges at one vertex that certainly belong together: all of them
+// when the main diagonal is one (every corner is a subset of it), else those
+// whose corner contains the first one's (a triangle holds both edges).  The
+// others stand alone until a triangle joins them.
+__device__ __forceinline__ bool ct_with_first(unsigned m, unsigned e, unsigned diag) {
+  const unsigned f = __ffs(m);
+  return ((m >> (diag - 1)) & 1u) || (e & f) == f;
+}
+
+// A thread per crossing edge; listed in shared memory first, so the rows leave
+// in whole lines (96^3 x 6 double: 106 us with a thread per vertex, now 28).
+// voff (first rank) is written where a vertex has edges; parent starts at the
+// vertex's first edge where the two belong together (a mesh of single layers
+// has triangles but no cells, which are what joins).
 template <typename T>
-__global__ void ct_emit_kernel(CtGeom g, const T* __restrict__ a, T thr, const unsigned short* __restrict__ mask,
-                               const unsigned* __restrict__ blk_off, unsigned* __restrict__ voff,
-                               unsigned long long* __restrict__ simp, double* __restrict__ lam,
-                               float* __restrict__ bary) {
-  __shared__ unsigned tot;
-  const unsigned long long i = blockIdx.x * (unsigned long long)kCtThreads + threadIdx.x;
-  const unsigned m = i < g.nv ? mask[i] : 0u;
-  const unsigned base = blk_off[blockIdx.x] + ct_block_scan(__popc(m), &tot);
-  if (i >= g.nv) return;
-  voff[i] = base;
-  if (!m) return;
-  unsigned long long c[4];
-  ct_coords(g, i, c);
-  const unsigned long long gid = ct_gid(g, c), ai = ct_aidx(g, c);
-  const T a0 = ct_adj(g, a, ai, gid, thr);
-  unsigned r = base;
-  const int ne = 1 << g.d;
-  for (int e = 1; e < ne; ++e) {
-    if (!((m >> (e - 1)) & 1u)) continue;
-    const T a1 = ct_adj(g, a, ai + g.aoff[e], gid + g.goff[e], thr);
+__global__ void __launch_bounds__(kCtThreads) ct_emit_kernel(
+    CtGeom g, const T* __restrict__ a, T thr, const unsigned short* __restrict__ mask,
+    const unsigned* __restrict__ blk_off, unsigned* __restrict__ voff, unsigned long long* __restrict__ simp,
+    double* __restrict__ lam, float* __restrict__ bary, unsigned* __restrict__ parent) {
+  __shared__ CtEdges s;
+  const unsigned base = blk_off[blockIdx.x];
+  const unsigned n = ct_list_edges(g, mask, base, voff, s);
+  const unsigned long long i0 = blockIdx.x * (unsigned long long)kCtBlock;
+  for (unsigned k = threadIdx.x; k < n; k += kCtThreads) {
+    const unsigned x = s.edge[k] >> 4, e = s.edge[k] & 15u;
+    unsigned long long c[4];
+    ct_coords(g, i0 + x, c);
+    const unsigned long long gid = ct_gid(g, c), ai = ct_aidx(g, c);
+    const T a0 = ct_adj(g, a, ai, gid, thr), a1 = ct_adj(g, a, ai + g.aoff[e], gid + g.goff[e], thr);
     T l0, l1;
     ct_solve(a0, a1, &l0, &l1);
-    simp[2 * (size_t)r] = gid;
-    simp[2 * (size_t)r + 1] = gid + g.goff[e];
-    lam[2 * (size_t)r] = (double)l0;
-    lam[2 * (size_t)r + 1] = (double)l1;
-    bary[2 * (size_t)r] = (float)l0;
-    bary[2 * (size_t)r + 1] = (float)l1;
-    ++r;
+    const unsigned r = base + k, m = s.mask[x];
+    reinterpret_cast<ulonglong2*>(simp)[r] = make_ulonglong2(gid, gid + g.goff[e]);
+    reinterpret_cast<double2*>(lam)[r] = make_double2((double)l0, (double)l1);
+    reinterpret_cast<float2*>(bary)[r] = make_float2((float)l0, (float)l1);
+    parent[r] = g.ncube && ct_with_first(m, e, (1u << g.d) - 1u) ? r - ct_below(m, e) : r;
   }
 }
 
-// Mixed hypercubes (corner signs not all equal) are listed once, each as one
-// word: base vertex (local linear index) << 20 | upper-face axes << 16 |
-// corner signs (bit e: corner e positive).  An upper-face axis k is one where
-// the cube's corners with bit k set lie on the mesh's last layer (c_k = L_k - 2).
-constexpr int kCtBaseShift = 20;
-
-__global__ void ct_mixed_kernel(CtGeom g, const unsigned char* __restrict__ pos,
-                                unsigned long long* __restrict__ list, unsigned* __restrict__ cnt) {
-  const int lane = threadIdx.x & 31;
-  const int ne = 1 << g.d;
-  for (unsigned long long q0 = blockIdx.x * (unsigned long long)blockDim.x; q0 < g.ncube;
-       q0 += (unsigned long long)gridDim.x * blockDim.x) {
-    const unsigned long long q = q0 + threadIdx.x;
-    unsigned long long word = 0;
-    bool mixed = false;
-    if (q < g.ncube) {
-      unsigned long long base = 0, r = q;
-      unsigned upper = 0;
-      for (int k = 0; k < g.d; ++k) {
-        const unsigned long long n = g.L[k] - 1, c = r % n;
-        r /= n;
-        base += c * g.lstr[k];
-        if (c + 2 == g.L[k]) upper |= 1u << k;
-      }
-      unsigned sgn = 0;
-      for (int e = 0; e < ne; ++e) sgn |= (unsigned)pos[base + g.loff[e]] << e;
-      mixed = sgn != 0 && sgn != (1u << ne) - 1u;
-      word = (base << kCtBaseShift) | ((unsigned long long)upper << 16) | sgn;
+// The first crossing edge (v, v + e) of every vertex starts at an edge of a lower
+// vertex w = v - a, a an axis outside e: in the triangle (w, w + a, w + a + e)
+// exactly one of (w, a) and (w, a + e) crosses too.  Most edges then hang in
+// one long tree before the joins, which otherwise meet everywhere at once.
+__global__ void __launch_bounds__(kCtThreads) ct_hook_kernel(CtGeom g, const unsigned short* __restrict__ mask,
+                                                             const unsigned* __restrict__ voff,
+                                                             unsigned* __restrict__ parent) {
+  const unsigned long long i0 = blockIdx.x * (unsigned long long)kCtBlock + threadIdx.x;
+#pragma unroll
+  for (int j = 0; j < kCtPer; ++j) {
+    const unsigned long long i = i0 + j * kCtThreads;
+    const unsigned m = i < g.nv ? mask[i] : 0u;
+    if (!m) continue;
+    unsigned long long c[4];
+    ct_coords(g, i, c);
+    const unsigned e = __ffs(m);
+    for (int k = g.d - 1; k >= 0; --k) {
+      if (((e >> k) & 1u) || c[k] == 0) continue;
+      const unsigned long long w = i - g.lstr[k];
+      const unsigned mw = mask[w], a = 1u << k;
+      parent[voff[i]] = voff[w] + ct_below(mw, (mw >> (a - 1)) & 1u ? a : a | e);
+      break;
     }
-    const unsigned bal = __ballot_sync(0xffffffffu, mixed);
-    unsigned wbase = 0;
-    if (lane == 0 && bal) wbase = atomicAdd(cnt, (unsigned)__popc(bal));
-    wbase = __shfl_sync(0xffffffffu, wbase, 0);
-    if (mixed) list[wbase + __popc(bal & ((1u << lane) - 1u))] = word;
   }
 }
 
-// One Kuhn simplex of a listed cube, for the lane that owns it: path corners
-// (corner bit masks along the CPU mesh's permutation order) and signs.
-struct CtSimplex {
-  int pe[5];      // corner of path vertex i
-  unsigned ps;    // bit i: path vertex i positive
-  int npos;
+// Joins the crossing edges of every mesh triangle that has two.  The crossing
+// edges of a simplex hang together through its triangles, so this gives the
+// components of the cells; a triangle (v, v + a, v + b), a a subset of b, is met
+// once, at a vertex with crossing edges (one of the two is at v):
+//   (v, a) and (v, b)            unless the vertex's edges started joined
+//   (v, a) and (v + a, b - a)    all edges at v + a disjoint from a
+//   (v, b) and (v + a, b - a)    v has no edge to a
+// A thread takes one vertex and corner a; of edges that started joined on both
+// sides one pair is enough.  Bound by the dependent loads of ranks and roots.
+// Joining every cell's nodes from the cells kernel took four times as many
+// unions from divergent lanes and most of that kernel's time, a thread per edge
+// here 375 us, of which 75 without any union: threads that join the same two
+// large trees queue on their roots.  So the hooked trees are flattened, one
+// vertex of kCtSample joins along its axes, the trees (few by then) are
+// flattened again, and the rest mostly finds equal parents: 250 us in all
+// (96^3 x 6, 1.3 million edges).
+constexpr unsigned kCtSample = 4;
+
+__global__ void __launch_bounds__(kCtThreads) ct_join_kernel(CtGeom g, const unsigned short* __restrict__ mask,
+                                                             const unsigned* __restrict__ voff, unsigned* parent,
+                                                             unsigned* err, bool sample) {
+  __shared__ unsigned short s_vert[kCtBlock], s_mask[kCtBlock];
+  __shared__ unsigned long long s_off[16];
+  if (threadIdx.x < 16) s_off[threadIdx.x] = ct_corner_step(g, threadIdx.x);
+  const unsigned long long i0 = blockIdx.x * (unsigned long long)kCtBlock;
+  unsigned m[kCtPer], at[kCtPer];
+#pragma unroll
+  for (int j = 0; j < kCtPer; ++j) {
+    const unsigned long long i = i0 + j * kCtThreads + threadIdx.x;
+    m[j] = i < g.nv ? mask[i] : 0u;
+    at[j] = m[j] ? 1u : 0u;
+  }
+  const unsigned n = ct_block_ranks(at);
+  if (n == 0) return;
+#pragma unroll
+  for (int j = 0; j < kCtPer; ++j)
+    if (m[j]) {
+      s_vert[at[j]] = (unsigned short)(j * kCtThreads + threadIdx.x);
+      s_mask[at[j]] = (unsigned short)m[j];
+    }
+  __syncthreads();
+  const unsigned diag = (1u << g.d) - 1u;
+  const unsigned per = sample ? (unsigned)g.d : diag, step = sample ? kCtSample : 1u;
+  for (unsigned k = threadIdx.x; k < (n + step - 1) / step * per; k += kCtThreads) {
+    const unsigned z = k / per * step, mv = s_mask[z], a = sample ? 1u << k % per : k % per + 1;
+    const bool edge = (mv >> (a - 1)) & 1u;
+    unsigned with = 0;  // no edge to a: the corners b above a that have one
+    if (!edge) {
+      for (unsigned y = mv; y; y &= y - 1) {
+        const unsigned b = __ffs(y);
+        if ((b & a) == a) with |= 1u << (b - 1);
+      }
+      if (!with) continue;
+    }
+    const unsigned long long v = i0 + s_vert[z], u = v + s_off[a];
+    const unsigned mu = mask[u], ov = voff[v];
+    const unsigned ou = mu ? voff[u] : 0u;
+    bool met = false;
+    if (edge) {
+      const unsigned r = ov + ct_below(mv, a);
+      for (unsigned y = mu; y; y &= y - 1) {
+        const unsigned f = __ffs(y);
+        if (f & a) continue;
+        if (ct_with_first(mu, f, diag)) {
+          if (met) continue;
+          met = true;
+        }
+        uf_unite_flat(parent, r, ou + ct_below(mu, f), err);
+      }
+      if (!ct_with_first(mv, a, diag))
+        for (unsigned y = mv; y; y &= y - 1) {
+          const unsigned b = __ffs(y);
+          if ((b & a) == a && b != a) uf_unite_flat(parent, r, ov + ct_below(mv, b), err);
+        }
+    } else {
+      for (unsigned y = with; y; y &= y - 1) {
+        const unsigned b = __ffs(y);
+        if (ct_with_first(mv, b, diag) && ct_with_first(mu, b ^ a, diag)) {
+          if (met) continue;
+          met = true;
+        }
+        uf_unite_flat(parent, ov + ct_below(mv, b), ou + ct_below(mu, b ^ a), err);
+      }
+    }
+  }
+}
+
+// A warp takes 32 / (D!) listed cubes, a lane per Kuhn simplex.  A lane's path
+// (corner masks along the CPU mesh's permutation order) is the same for every
+// cube, so its corners and their steps lie in shared memory, a column per lane:
+// lane-varying indexes into the kernel's parameters are served one address at
+// a time, and indexes into arrays of a thread's own go through local memory.
+template <int D>
+struct CtPaths {
+  unsigned corner[D + 1][32];
+  unsigned long long off[D + 1][32];
 };
-
-__device__ __forceinline__ void ct_simplex(const CtGeom& g, unsigned sgn, int p_idx, CtSimplex* x) {
-  x->pe[0] = 0;
-  x->ps = sgn & 1u;
-  x->npos = (int)(sgn & 1u);
-  for (int i = 0; i < g.d; ++i) {
-    x->pe[i + 1] = x->pe[i] | (1 << g.perm[p_idx][i]);
-    const unsigned b = (sgn >> x->pe[i + 1]) & 1u;
-    x->ps |= b << (i + 1);
-    x->npos += (int)b;
-  }
-}
-
-// feature index of the crossing edge from path vertex a to path vertex b of
-// the cube at local vertex base
-__device__ __forceinline__ unsigned ct_node(const CtGeom& g, unsigned long long base, const CtSimplex& x,
-                                            const unsigned short* __restrict__ mask,
-                                            const unsigned* __restrict__ voff, int a, int b) {
-  const int lo = x.pe[min(a, b)], hi = x.pe[max(a, b)];
-  const unsigned long long v = base + g.loff[lo];
-  const int dir = hi ^ lo;
-  return __ldg(voff + v) + __popc((unsigned)__ldg(mask + v) & ((1u << (dir - 1)) - 1u));
-}
-
-// The crossing edges of a 1-vs-rest or 2D+t 2-2 split in the order the
-// reference's marching functions meet them, as path-vertex pairs: the lone
-// vertex with the others in order; positives outer, others inner.
-__device__ __forceinline__ int ct_crossings(const CtSimplex& x, int nvtx, int* ea, int* eb) {
-  int ne = 0;
-  if (x.npos == 1 || x.npos == nvtx - 1) {
-    const bool lone_pos = x.npos == 1;
-    int lone = 0;
-    for (int i = 0; i < nvtx; ++i)
-      if ((((x.ps >> i) & 1u) != 0) == lone_pos) lone = i;
-    for (int o = 0; o < nvtx; ++o)
-      if (o != lone) {
-        ea[ne] = lone;
-        eb[ne] = o;
-        ++ne;
-      }
-  } else {
-    for (int a = 0; a < nvtx; ++a) {
-      if (!((x.ps >> a) & 1u)) continue;
-      for (int b = 0; b < nvtx; ++b) {
-        if ((x.ps >> b) & 1u) continue;
-        ea[ne] = a;
-        eb[ne] = b;
-        ++ne;
-      }
-    }
-  }
-  return ne;
-}
-
-// lanes of a warp: np lanes per listed cube (one per Kuhn simplex), 32 / np
-// cubes per warp
+template <int D>
 struct CtLane {
-  int np, per, sub, p_idx;
+  static constexpr int kSimp = D == 3 ? 6 : 24, kCubes = 32 / kSimp;
+  unsigned lane, sub, simp;
   bool active;
+  const CtPaths<D>* P;
+
+  // by all threads of the block
+  __device__ __forceinline__ CtLane(const CtGeom& g, CtPaths<D>& paths) {
+    lane = threadIdx.x & 31;
+    sub = lane / kSimp;
+    simp = lane % kSimp;
+    active = sub < kCubes;
+    P = &paths;
+    if (threadIdx.x < 32) {
+      unsigned c = 0;
+      for (int i = 0; i <= D; ++i) {
+        paths.corner[i][lane] = c;
+        paths.off[i][lane] = ct_corner_step(g, c);
+        if (i < D) c |= 1u << g.perm[simp][i];
+      }
+    }
+    __syncthreads();
+  }
+  // bit i: path vertex i positive, given the cube's corner signs
+  __device__ __forceinline__ unsigned signs(unsigned sgn) const {
+    unsigned ps = 0;
+#pragma unroll
+    for (int i = 0; i <= D; ++i) ps |= ((sgn >> P->corner[i][lane]) & 1u) << i;
+    return ps;
+  }
+  __device__ __forceinline__ unsigned corner(int i) const { return P->corner[i][lane]; }
+  // feature index of the crossing edge between path vertices a and b of the
+  // cube at local vertex base
+  __device__ __forceinline__ unsigned node(unsigned long long base, const unsigned short* __restrict__ mask,
+                                           const unsigned* __restrict__ voff, int a, int b) const {
+    const int lo = min(a, b), hi = max(a, b);
+    const unsigned long long v = base + P->off[lo][lane];
+    const unsigned dir = P->corner[hi][lane] ^ P->corner[lo][lane];
+    return __ldg(voff + v) + __popc((unsigned)__ldg(mask + v) & ((1u << (dir - 1)) - 1u));
+  }
 };
 
-__device__ __forceinline__ CtLane ct_lane(int d) {
-  CtLane l;
-  const int lane = threadIdx.x & 31;
-  l.np = d == 3 ? 6 : 24;
-  l.per = 32 / l.np;
-  l.sub = lane / l.np;
-  l.p_idx = lane % l.np;
-  l.active = l.sub < l.per;
-  return l;
+// The sides of a simplex's sign split in path order: `few` the vertices of the
+// smaller side (of two positives and two negatives the positives), `rest` the
+// others; n: how many few has (0: not crossed).
+template <int D>
+struct CtSplit {
+  unsigned few, rest;
+  int n;
+  __device__ __forceinline__ explicit CtSplit(unsigned ps) {
+    constexpr unsigned kAll = (1u << (D + 1)) - 1u;
+    const int np = __popc(ps);
+    const bool pos = 2 * np <= D + 1;
+    n = pos ? np : D + 1 - np;
+    few = pos ? ps : ps ^ kAll;
+    rest = few ^ kAll;
+  }
+};
+
+__device__ __forceinline__ int ct_pop(unsigned& bits) {
+  const int i = __ffs(bits) - 1;
+  bits &= bits - 1;
+  return i;
 }
 
 // (2D+t) where the reference's sequential patching first meets each node whose
 // edge starts on an upper boundary face: (cube base, permutation index,
-// position in the marching enumeration), minimised over every meeting
+// position in the marching enumeration), minimised over every meeting.  The
+// marching functions meet the lone vertex with the others in order, or
+// positives outer and others inner.
 __global__ void ct_first_kernel(CtGeom g, const unsigned long long* __restrict__ list, const unsigned* list_cnt,
                                 const unsigned short* __restrict__ mask, const unsigned* __restrict__ voff,
                                 unsigned long long* __restrict__ first) {
-  const CtLane ln = ct_lane(3);
+  __shared__ CtPaths<3> paths;
+  const CtLane<3> ln(g, paths);
   const unsigned nl = *list_cnt;
   const unsigned long long warp = (blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x) >> 5;
   const unsigned long long nwarps = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
-  for (unsigned long long it = warp * ln.per + ln.sub; ln.active && it < nl; it += nwarps * ln.per) {
+  for (unsigned long long it = warp * ln.kCubes + ln.sub; ln.active && it < nl; it += nwarps * ln.kCubes) {
     const unsigned long long w = list[it];
     const unsigned long long base = w >> kCtBaseShift;
-    const unsigned upper = (unsigned)(w >> 16) & 0xFu, sgn = (unsigned)w & 0xFFFFu;
-    CtSimplex x;
-    ct_simplex(g, sgn, ln.p_idx, &x);
-    if (x.npos == 0 || x.npos == 4) continue;
-    int ea[4], eb[4];
-    const int ne = ct_crossings(x, 4, ea, eb);
-    for (int k = 0; k < ne; ++k) {
-      const int lo = x.pe[min(ea[k], eb[k])];
-      if (!(lo & (int)upper)) continue;  // the edge starts at a hypercube base
-      const unsigned nd = ct_node(g, base, x, mask, voff, ea[k], eb[k]);
-      const unsigned long long key = ((base * 6ull) + (unsigned long long)ln.p_idx) * 4ull + (unsigned long long)k;
-      atomicMin(first + nd, key);
+    const unsigned upper = (unsigned)(w >> 16) & 0xFu;
+    const CtSplit<3> x(ln.signs((unsigned)w & 0xFFFFu));
+    int k = 0;
+    for (unsigned f = x.few; f;) {
+      const int a = ct_pop(f);
+      for (unsigned r = x.rest; r; ++k) {
+        const int b = ct_pop(r);
+        if (!(ln.corner(min(a, b)) & upper)) continue;  // the edge starts at a hypercube base
+        const unsigned nd = ln.node(base, mask, voff, a, b);
+        const unsigned long long key = ((base * 6ull) + (unsigned long long)ln.simp) * 4ull + (unsigned long long)k;
+        atomicMin(first + nd, key);
+      }
     }
   }
 }
@@ -380,87 +665,61 @@ __device__ __forceinline__ void ct_sort4(unsigned* v, int k) {
     }
 }
 
+__device__ __forceinline__ void ct_order(unsigned& a, unsigned& b) {
+  const unsigned lo = min(a, b);
+  b = max(a, b);
+  a = lo;
+}
+
+// row `slot` of the cells, its D entries ascending, counted at its leading node
+template <int D>
+__device__ __forceinline__ void ct_put_cell(unsigned* __restrict__ cells, unsigned long long slot, unsigned cap,
+                                            unsigned* __restrict__ bcount, unsigned a, unsigned b, unsigned c,
+                                            unsigned d) {
+  if constexpr (D == 4) {
+    ct_order(a, b), ct_order(c, d), ct_order(a, c), ct_order(b, d), ct_order(b, c);
+    if (slot < cap) {
+      reinterpret_cast<uint4*>(cells)[slot] = make_uint4(a, b, c, d);
+      atomicAdd(bcount + a, 1u);
+    }
+  } else {
+    ct_order(a, b), ct_order(b, c), ct_order(a, b);
+    if (slot < cap) {
+      cells[3 * slot] = a;
+      cells[3 * slot + 1] = b;
+      cells[3 * slot + 2] = c;
+      atomicAdd(bcount + a, 1u);
+    }
+  }
+}
+
 // Marching tetrahedra (2D+t) / pentatopes (3D+t) on the listed cubes, one
-// Kuhn simplex per lane: up to three cells each, slots reserved per warp;
-// the simplex's crossing nodes are joined in the union-find by a star from its
-// first node (the same components as joining every cell's nodes).
-__global__ void ct_cells_kernel(CtGeom g, const unsigned long long* __restrict__ list, const unsigned* list_cnt,
-                                const unsigned short* __restrict__ mask, const unsigned* __restrict__ voff,
-                                const unsigned long long* __restrict__ first, unsigned n,
-                                unsigned* __restrict__ cells, unsigned long long* cnt, unsigned cap,
-                                unsigned* parent,
-                                unsigned* err) {
-  const int d = g.d;
-  const int kc = d;  // entries per cell
-  const CtLane ln = ct_lane(d);
-  const int lane = threadIdx.x & 31;
-  const unsigned nl = *list_cnt;
+// Kuhn simplex per lane: up to three cells each.  A warp reserves the slots of
+// kCtBatch rounds at once: the signs alone give the number of cells, and the
+// counter takes one atomic at a time.  Bound by the gathers of ranks and masks.
+// 96^3 x 6 double, 7.5 million tets: 938 us with the joins, paths indexed in
+// the kernel's parameters and an atomic per warp and round, now 89.
+template <int D>
+__global__ void __launch_bounds__(256) ct_cells_kernel(
+    CtGeom g, const unsigned long long* __restrict__ list, const unsigned* list_cnt,
+    const unsigned short* __restrict__ mask, const unsigned* __restrict__ voff,
+    const unsigned long long* __restrict__ first, unsigned n, unsigned* __restrict__ cells, unsigned long long* cnt,
+    unsigned cap, unsigned* __restrict__ bcount) {
+  constexpr int kCtBatch = 8;
+  __shared__ CtPaths<D> paths;
+  const CtLane<D> ln(g, paths);
+  const unsigned lane = ln.lane, nl = *list_cnt;
   const unsigned long long warp = (blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x) >> 5;
   const unsigned long long nwarps = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
-  for (unsigned long long it0 = warp * ln.per; it0 < nl; it0 += nwarps * ln.per) {
-    const unsigned long long it = it0 + ln.sub;
-    unsigned cell[3][4];
-    unsigned nodes[6];
-    int nn = 0, ncell = 0;
-    if (ln.active && it < nl) {
-      const unsigned long long w = list[it];
-      const unsigned long long base = w >> kCtBaseShift;
-      CtSimplex x;
-      ct_simplex(g, (unsigned)w & 0xFFFFu, ln.p_idx, &x);
-      if (x.npos != 0 && x.npos != d + 1) {
-        if (x.npos == 1 || x.npos == d || d == 3) {
-          int ea[6], eb[6];
-          const int ne = ct_crossings(x, d + 1, ea, eb);
-          for (int k = 0; k < ne; ++k) nodes[k] = ct_node(g, base, x, mask, voff, ea[k], eb[k]);
-          nn = ne;
-          if (ne == d) {  // 1-vs-rest: one cell
-            for (int k = 0; k < d; ++k) cell[0][k] = nodes[k];
-            ncell = 1;
-          } else {  // 2D+t 2-2 split: the quad cut along the diagonal from the
-                    // node the reference numbered first
-            unsigned nd[4];
-            unsigned long long key[4];
-            for (int k = 0; k < 4; ++k) {
-              nd[k] = nodes[k];
-              const unsigned long long f = first[nd[k]];
-              key[k] = f == ~0ull ? (unsigned long long)nd[k] : (unsigned long long)n + f;
-            }
-            for (int i = 1; i < 4; ++i)
-              for (int j = i; j > 0 && key[j - 1] > key[j]; --j) {
-                const unsigned long long kx = key[j - 1];
-                key[j - 1] = key[j];
-                key[j] = kx;
-                const unsigned nx = nd[j - 1];
-                nd[j - 1] = nd[j];
-                nd[j] = nx;
-              }
-            cell[0][0] = nd[0], cell[0][1] = nd[1], cell[0][2] = nd[2];
-            cell[1][0] = nd[0], cell[1][1] = nd[2], cell[1][2] = nd[3];
-            ncell = 2;
-          }
-        } else {  // pentatope 2-3 split
-          const bool two_pos = x.npos == 2;
-          int two[2], three[3], n2 = 0, n3 = 0;
-          for (int i = 0; i < 5; ++i) {
-            if ((((x.ps >> i) & 1u) != 0) == two_pos) two[n2++] = i;
-            else three[n3++] = i;
-          }
-          unsigned T0[3], T1[3];
-          for (int t = 0; t < 3; ++t) {
-            T0[t] = ct_node(g, base, x, mask, voff, two[0], three[t]);
-            T1[t] = ct_node(g, base, x, mask, voff, two[1], three[t]);
-          }
-          cell[0][0] = T0[0], cell[0][1] = T0[1], cell[0][2] = T0[2], cell[0][3] = T1[2];
-          cell[1][0] = T0[0], cell[1][1] = T0[1], cell[1][2] = T1[1], cell[1][3] = T1[2];
-          cell[2][0] = T0[0], cell[2][1] = T1[0], cell[2][2] = T1[1], cell[2][3] = T1[2];
-          for (int t = 0; t < 3; ++t) nodes[t] = T0[t], nodes[3 + t] = T1[t];
-          nn = 6;
-          ncell = 3;
-        }
-      }
+  for (unsigned long long r0 = warp * kCtBatch; r0 * ln.kCubes < nl; r0 += nwarps * kCtBatch) {
+    unsigned mine = 0;
+    for (int r = 0; r < kCtBatch; ++r) {
+      const unsigned long long it = (r0 + r) * ln.kCubes + ln.sub;
+      if (!ln.active || it >= nl) break;
+      const CtSplit<D> x(ln.signs((unsigned)list[it] & 0xFFFFu));
+      mine += x.n == 0 ? 0u : x.n == 1 ? 1u : (unsigned)D - 1u;
     }
-    // slots for the warp's cells
-    unsigned incl = (unsigned)ncell;
+    unsigned incl = mine;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
       const unsigned y = __shfl_up_sync(0xffffffffu, incl, o);
@@ -469,14 +728,60 @@ __global__ void ct_cells_kernel(CtGeom g, const unsigned long long* __restrict__
     const unsigned wtot = __shfl_sync(0xffffffffu, incl, 31);
     unsigned long long wbase = 0;
     if (lane == 31 && wtot) wbase = atomicAdd(cnt, (unsigned long long)wtot);
-    wbase = __shfl_sync(0xffffffffu, wbase, 31);
-    unsigned long long slot = wbase + incl - (unsigned)ncell;
-    for (int c = 0; c < ncell; ++c, ++slot) {
-      ct_sort4(cell[c], kc);
-      if (slot < cap)
-        for (int k = 0; k < kc; ++k) cells[(size_t)slot * kc + k] = cell[c][k];
+    unsigned long long slot = __shfl_sync(0xffffffffu, wbase, 31) + incl - mine;
+    for (int r = 0; r < kCtBatch; ++r) {
+      const unsigned long long it = (r0 + r) * ln.kCubes + ln.sub;
+      if (!ln.active || it >= nl) break;
+      const unsigned long long w = list[it];
+      const unsigned long long base = w >> kCtBaseShift;
+      const CtSplit<D> x(ln.signs((unsigned)w & 0xFFFFu));
+      if (x.n == 0) continue;
+      unsigned few = x.few, rest = x.rest;
+      if (x.n == 1) {  // 1-vs-rest: one cell
+        const int a = ct_pop(few);
+        unsigned nd[4] = {0, 0, 0, 0};
+#pragma unroll
+        for (int k = 0; k < D; ++k) nd[k] = ln.node(base, mask, voff, a, ct_pop(rest));
+        ct_put_cell<D>(cells, slot++, cap, bcount, nd[0], nd[1], nd[2], nd[3]);
+      } else if constexpr (D == 3) {  // 2D+t 2-2 split: the quad cut along the diagonal from the
+                                      // node the reference numbered first
+        const int p0 = ct_pop(few), p1 = ct_pop(few), q0 = ct_pop(rest), q1 = ct_pop(rest);
+        unsigned nd[4] = {ln.node(base, mask, voff, p0, q0), ln.node(base, mask, voff, p0, q1),
+                          ln.node(base, mask, voff, p1, q0), ln.node(base, mask, voff, p1, q1)};
+        unsigned long long key[4];
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const unsigned long long f = first[nd[k]];
+          key[k] = f == ~0ull ? (unsigned long long)nd[k] : (unsigned long long)n + f;
+        }
+#pragma unroll
+        for (int i = 1; i < 4; ++i)
+#pragma unroll
+          for (int j = i; j > 0; --j)
+            if (key[j - 1] > key[j]) {
+              const unsigned long long kx = key[j - 1];
+              key[j - 1] = key[j];
+              key[j] = kx;
+              const unsigned nx = nd[j - 1];
+              nd[j - 1] = nd[j];
+              nd[j] = nx;
+            }
+        ct_put_cell<D>(cells, slot++, cap, bcount, nd[0], nd[1], nd[2], 0);
+        ct_put_cell<D>(cells, slot++, cap, bcount, nd[0], nd[2], nd[3], 0);
+      } else {  // pentatope 2-3 split
+        const int a = ct_pop(few), b = ct_pop(few);
+        unsigned T0[3], T1[3];
+#pragma unroll
+        for (int k = 0; k < 3; ++k) {
+          const int c = ct_pop(rest);
+          T0[k] = ln.node(base, mask, voff, a, c);
+          T1[k] = ln.node(base, mask, voff, b, c);
+        }
+        ct_put_cell<D>(cells, slot++, cap, bcount, T0[0], T0[1], T0[2], T1[2]);
+        ct_put_cell<D>(cells, slot++, cap, bcount, T0[0], T0[1], T1[1], T1[2]);
+        ct_put_cell<D>(cells, slot++, cap, bcount, T0[0], T1[0], T1[1], T1[2]);
+      }
     }
-    for (int k = 1; k < nn; ++k) uf_unite(parent, nodes[0], nodes[k], err);
   }
 }
 
@@ -515,38 +820,103 @@ __device__ __forceinline__ bool ct_row_less(const unsigned* x, const unsigned* y
   return false;
 }
 
-// one thread per leading node: insertion sort of its bucket's rows by their
-// remaining entries.  Without uniq, equal neighbours (duplicate cells) raise
-// bit 1 of *err; with uniq, they are dropped (the unique rows stay at the
-// start of the bucket, their count in uniq[a]).
-__global__ void ct_bucket_sort_kernel(unsigned* __restrict__ rows, const unsigned* __restrict__ boff, unsigned n,
-                                      int k, unsigned* err, unsigned* __restrict__ uniq) {
-  for (unsigned a = blockIdx.x * blockDim.x + threadIdx.x; a < n; a += gridDim.x * blockDim.x) {
-    const unsigned lo = boff[a], hi = boff[a + 1];
-    for (unsigned i = lo + 1; i < hi; ++i) {
-      unsigned cur[4];
-      for (int j = 0; j < k; ++j) cur[j] = rows[(size_t)i * k + j];
-      unsigned p = i;
-      while (p > lo && ct_row_less(cur, rows + (size_t)(p - 1) * k, k)) {
-        for (int j = 0; j < k; ++j) rows[(size_t)p * k + j] = rows[(size_t)(p - 1) * k + j];
-        --p;
+// Sorts each bucket's rows by their remaining entries: a block takes the buckets
+// of kSortNodes leading nodes, copies their rows to shared memory, and a thread
+// per row counts the rows of its bucket below it.  Without uniq, equal rows
+// (duplicate cells) raise bit 1 of *err; with uniq, they are dropped (the unique
+// rows stay at the start of the bucket, their count in uniq[a]).  Blocks whose
+// rows do not fit sort each bucket by insertion where it lies.  96^3 x 6 double,
+// 7.5 million tets: 480 us when every bucket was sorted that way by one thread,
+// now 112.
+constexpr int kSortNodes = 128;
+constexpr unsigned kSortRows = 1536;
+
+template <int K>
+__global__ void __launch_bounds__(kCtThreads) ct_bucket_sort_kernel(unsigned* __restrict__ rows,
+                                                                    const unsigned* __restrict__ boff, unsigned n,
+                                                                    unsigned* err, unsigned* __restrict__ uniq) {
+  __shared__ unsigned s_row[K][kSortRows];
+  __shared__ unsigned s_off[kSortNodes + 1], s_uniq[kSortNodes];
+  __shared__ unsigned char s_first[kSortRows];
+  const unsigned a0 = blockIdx.x * kSortNodes, na = min((unsigned)kSortNodes, n - a0);
+  for (unsigned i = threadIdx.x; i <= na; i += kCtThreads) s_off[i] = boff[a0 + i];
+  if (threadIdx.x < kSortNodes) s_uniq[threadIdx.x] = 0;
+  __syncthreads();
+  const unsigned lo = s_off[0], cnt = s_off[na] - lo;
+  if (cnt > kSortRows) {
+    for (unsigned a = threadIdx.x; a < na; a += kCtThreads) {
+      const unsigned first = s_off[a], last = s_off[a + 1];
+      for (unsigned i = first + 1; i < last; ++i) {
+        unsigned cur[K];
+        for (int j = 0; j < K; ++j) cur[j] = rows[(size_t)i * K + j];
+        unsigned p = i;
+        while (p > first && ct_row_less(cur, rows + (size_t)(p - 1) * K, K)) {
+          for (int j = 0; j < K; ++j) rows[(size_t)p * K + j] = rows[(size_t)(p - 1) * K + j];
+          --p;
+        }
+        for (int j = 0; j < K; ++j) rows[(size_t)p * K + j] = cur[j];
       }
-      for (int j = 0; j < k; ++j) rows[(size_t)p * k + j] = cur[j];
-    }
-    if (!uniq) {
-      for (unsigned i = lo + 1; i < hi; ++i)
-        if (!ct_row_less(rows + (size_t)(i - 1) * k, rows + (size_t)i * k, k)) atomicOr(err, 2u);
-    } else {
-      unsigned w = lo;
-      for (unsigned i = lo; i < hi; ++i) {
-        if (i > lo && !ct_row_less(rows + (size_t)(w - 1) * k, rows + (size_t)i * k, k)) continue;
+      unsigned w = first;
+      for (unsigned i = first; i < last; ++i) {
+        if (i > first && !ct_row_less(rows + (size_t)(w - 1) * K, rows + (size_t)i * K, K)) {
+          if (!uniq) atomicOr(err, 2u);
+          continue;
+        }
         if (w != i)
-          for (int j = 0; j < k; ++j) rows[(size_t)w * k + j] = rows[(size_t)i * k + j];
+          for (int j = 0; j < K; ++j) rows[(size_t)w * K + j] = rows[(size_t)i * K + j];
         ++w;
       }
-      uniq[a] = w - lo;
+      if (uniq) uniq[a0 + a] = w - first;
+    }
+    return;
+  }
+  for (unsigned i = threadIdx.x; i < cnt * K; i += kCtThreads) s_row[i % K][i / K] = rows[(size_t)lo * K + i];
+  __syncthreads();
+  // -1, 0, 1: row x against row y of the same bucket
+  auto order = [&](unsigned x, unsigned y) {
+#pragma unroll
+    for (int j = 1; j < K; ++j)
+      if (s_row[j][x] != s_row[j][y]) return s_row[j][x] < s_row[j][y] ? -1 : 1;
+    return 0;
+  };
+  if (uniq) {
+    for (unsigned i = threadIdx.x; i < cnt; i += kCtThreads) {
+      const unsigned a = s_row[0][i] - a0;
+      bool first = true;
+      for (unsigned y = s_off[a] - lo; y < i && first; ++y) first = order(y, i) != 0;
+      s_first[i] = first;
+      if (first) atomicAdd(&s_uniq[a], 1u);
+    }
+    __syncthreads();
+  }
+  for (unsigned i = threadIdx.x; i < cnt; i += kCtThreads) {
+    if (uniq && !s_first[i]) continue;
+    const unsigned a = s_row[0][i] - a0, first = s_off[a] - lo, last = s_off[a + 1] - lo;
+    unsigned below = 0;
+    for (unsigned y = first; y < last; ++y) {
+      const int o = order(y, i);
+      if (o < 0 && (!uniq || s_first[y])) ++below;
+      if (!uniq && o == 0 && y < i) {  // keeps the rows distinct places
+        atomicOr(err, 2u);
+        ++below;
+      }
+    }
+    const size_t dst = (size_t)lo + first + below;
+    if constexpr (K == 4) {
+      reinterpret_cast<uint4*>(rows)[dst] = make_uint4(s_row[0][i], s_row[1][i], s_row[2][i], s_row[3][i]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < K; ++j) rows[dst * K + j] = s_row[j][i];
     }
   }
+  if (uniq && threadIdx.x < na) uniq[a0 + threadIdx.x] = s_uniq[threadIdx.x];
+}
+
+void launch_bucket_sort(unsigned* rows, const unsigned* boff, unsigned n, int k, unsigned* err, unsigned* uniq,
+                        cudaStream_t st) {
+  if (n == 0) return;
+  auto kernel = k == 4 ? ct_bucket_sort_kernel<4> : ct_bucket_sort_kernel<3>;
+  kernel<<<(n + kSortNodes - 1) / kSortNodes, kCtThreads, 0, st>>>(rows, boff, n, err, uniq);
 }
 
 // unique rows of every bucket to their place in the output (uoff: scanned
@@ -631,13 +1001,13 @@ ftk2b_status run_contour(ftk2b_ctx* ctx, const CtGeom& g, const void* field, T t
   cudaStream_t st = ctx->stream;
   DevBuf* B = ctx->contour;
   const int d = g.d;
-  const unsigned long long nblk = (g.nv + kCtThreads - 1) / kCtThreads;
-  C_TRY(B[kBufPos].ensure(g.nv));
+  const unsigned long long nblk = (g.nv + kCtBlock - 1) / kCtBlock;
+  C_TRY(B[kBufPos].ensure(4 * ct_words(g)));
   C_TRY(B[kBufMask].ensure(2 * g.nv));
   C_TRY(B[kBufVoff].ensure(4 * g.nv));
   C_TRY(B[kBufBlk].ensure(4 * (nblk + 1)));
   C_TRY(B[kBufCount].ensure(64));
-  auto* pos = static_cast<unsigned char*>(B[kBufPos].p);
+  auto* pos = static_cast<unsigned*>(B[kBufPos].p);
   auto* mask = static_cast<unsigned short*>(B[kBufMask].p);
   auto* voff = static_cast<unsigned*>(B[kBufVoff].p);
   auto* blk = static_cast<unsigned*>(B[kBufBlk].p);
@@ -647,10 +1017,15 @@ ftk2b_status run_contour(ftk2b_ctx* ctx, const CtGeom& g, const void* field, T t
   const T* a = static_cast<const T*>(field);
   const unsigned sms = (unsigned)ctx->num_sms;
 
+  // the mixed hypercubes, once: every later stage walks this list
+  C_TRY(B[kBufList].ensure(8 * (g.ncube ? g.ncube : 1)));
+  auto* list = static_cast<unsigned long long*>(B[kBufList].p);
+  unsigned* list_cnt = counts + 4;
+
   C_TRY(cudaMemsetAsync(counts, 0, 64, st));
   C_TRY(cudaEventRecord(ctx->ev0, st));
-  ct_sign_kernel<T><<<grid_of(g.nv, 256, 32ull * sms), 256, 0, st>>>(g, a, thr, q, pos);
-  ct_mask_kernel<<<(unsigned)nblk, kCtThreads, 0, st>>>(g, pos, mask, blk, total64);
+  ct_sign_kernel<T><<<grid_of(g.nv, 4 * 256, 32ull * sms), 256, 0, st>>>(g, a, thr, q, pos);
+  ct_mask_kernel<<<(unsigned)nblk, kCtThreads, 0, st>>>(g, pos, mask, blk, total64, list, list_cnt);
   C_TRY(launch_scan(blk, (unsigned)nblk, counts + 0, nullptr, st));
   ctx->launches += 3;
   unsigned long long n64 = 0;
@@ -672,13 +1047,15 @@ ftk2b_status run_contour(ftk2b_ctx* ctx, const CtGeom& g, const void* field, T t
   auto* parent = static_cast<unsigned*>(B[kBufParent].p);
   auto* track = static_cast<unsigned long long*>(B[kBufTrack].p);
   auto* first = d == 3 ? static_cast<unsigned long long*>(B[kBufFirst].p) : nullptr;
-  ct_emit_kernel<T><<<(unsigned)nblk, kCtThreads, 0, st>>>(g, a, thr, mask, blk, voff, simp, lam, bary);
-  ctx->launches += 1;
-  // the mixed hypercubes, once: every later stage walks this list
-  C_TRY(B[kBufList].ensure(8 * (g.ncube ? g.ncube : 1)));
-  auto* list = static_cast<unsigned long long*>(B[kBufList].p);
-  unsigned* list_cnt = counts + 4;
-  ct_mixed_kernel<<<grid_of(g.ncube, 256, 64ull * sms), 256, 0, st>>>(g, pos, list, list_cnt);
+  ct_emit_kernel<T><<<(unsigned)nblk, kCtThreads, 0, st>>>(g, a, thr, mask, blk, voff, simp, lam, bary, parent);
+  if (n && g.ncube) {
+    ct_hook_kernel<<<(unsigned)nblk, kCtThreads, 0, st>>>(g, mask, voff, parent);
+    uf_flatten_kernel<<<grid_of(n, 256, 8ull * sms), 256, 0, st>>>(parent, n);
+    ct_join_kernel<<<(unsigned)nblk, kCtThreads, 0, st>>>(g, mask, voff, parent, counts + 3, true);
+    uf_flatten_kernel<<<grid_of(n, 256, 8ull * sms), 256, 0, st>>>(parent, n);
+    ct_join_kernel<<<(unsigned)nblk, kCtThreads, 0, st>>>(g, mask, voff, parent, counts + 3, false);
+    ctx->launches += 5;
+  }
   ctx->launches += 1;
   const unsigned wgrid = 16u * sms;  // 8 warps per block
   if (d == 3 && n) {
@@ -693,15 +1070,17 @@ ftk2b_status run_contour(ftk2b_ctx* ctx, const CtGeom& g, const void* field, T t
       0x7FFFFFFFull, std::max<unsigned long long>(1024ull, (d == 4 ? 8ull : 4ull) * n));
   unsigned ncell = 0;
   const int kc = d;  // entries per cell: 3 (triangles) or 4 (tets)
+  const unsigned nb = n + 1;  // bucket offsets, the last one the total
+  C_TRY(B[kBufKey0].ensure(4ull * nb));  // counts of the leading nodes, then offsets
+  auto* boff = static_cast<unsigned*>(B[kBufKey0].p);
   for (int attempt = 0; attempt < 2; ++attempt) {
     C_TRY(B[kBufCells].ensure((size_t)4 * kc * cap));
     auto* cells = static_cast<unsigned*>(B[kBufCells].p);
-    C_TRY(cudaMemsetAsync(counts + 1, 0, 12, st));
     C_TRY(cudaMemsetAsync(cell64, 0, 8, st));
-    if (n) ct_iota_kernel<<<grid_of(n, 256, 8ull * sms), 256, 0, st>>>(parent, n);
-    ct_cells_kernel<<<wgrid, 256, 0, st>>>(g, list, list_cnt, mask, voff, first, n, cells, cell64, cap, parent,
-                                           counts + 3);
-    ctx->launches += 2;
+    C_TRY(cudaMemsetAsync(boff, 0, 4ull * nb, st));
+    auto cells_kernel = d == 3 ? ct_cells_kernel<3> : ct_cells_kernel<4>;
+    cells_kernel<<<wgrid, 256, 0, st>>>(g, list, list_cnt, mask, voff, first, n, cells, cell64, cap, boff);
+    ctx->launches += 1;
     unsigned long long nc64 = 0;
     C_TRY(cudaMemcpyAsync(&nc64, cell64, 8, cudaMemcpyDeviceToHost, st));
     C_TRY(ctx->sync());
@@ -715,28 +1094,22 @@ ftk2b_status run_contour(ftk2b_ctx* ctx, const CtGeom& g, const void* field, T t
   // lexicographic order of the cells: buckets by leading node, then each
   // bucket's rows sorted
   const unsigned ccap = ncell ? ncell : 1;
-  const unsigned nb = n + 1;  // bucket offsets, the last one the total
   const unsigned sblocks = (unsigned)((nb + kCtThreads * kScanPer - 1) / (kCtThreads * kScanPer));
-  C_TRY(B[kBufKey0].ensure(4ull * nb));            // counts, then offsets
   C_TRY(B[kBufKey1].ensure(4ull * nb));            // scatter cursors
   C_TRY(B[kBufVal0].ensure(4ull * (sblocks + 1)));  // scan block totals
   C_TRY(B[kBufCellsOut].ensure(4ull * kc * ccap));
-  auto* boff = static_cast<unsigned*>(B[kBufKey0].p);
   auto* bcur = static_cast<unsigned*>(B[kBufKey1].p);
   auto* btot = static_cast<unsigned*>(B[kBufVal0].p);
   auto* cells_out = static_cast<unsigned*>(B[kBufCellsOut].p);
   const unsigned cg = grid_of(ccap, 256, 16ull * sms);
   if (ncell) {
-    C_TRY(cudaMemsetAsync(boff, 0, 4ull * nb, st));
     C_TRY(cudaMemsetAsync(bcur, 0, 4ull * nb, st));
-    ct_bucket_count_kernel<<<cg, 256, 0, st>>>(cells, ncell, kc, boff);
     ct_scan_blocks_kernel<<<sblocks, kCtThreads, 0, st>>>(boff, nb, btot);
     C_TRY(launch_scan(btot, sblocks, nullptr, nullptr, st));
     ct_scan_add_kernel<<<sblocks, kCtThreads, 0, st>>>(boff, nb, btot);
     ct_bucket_scatter_kernel<<<cg, 256, 0, st>>>(cells, ncell, kc, boff, bcur, cells_out);
-    ct_bucket_sort_kernel<<<grid_of(n, 128, 32ull * sms), 128, 0, st>>>(cells_out, boff, n, kc, counts + 3,
-                                                                         nullptr);
-    ctx->launches += 6;
+    launch_bucket_sort(cells_out, boff, n, kc, counts + 3, nullptr, st);
+    ctx->launches += 5;
   }
   if (n) {
     C_TRY(launch_uf_label(parent, counts + 0, n, track, counts + 2, st));
@@ -792,26 +1165,32 @@ struct FsTables {
   unsigned char idx[16][16];     // type of (a, b), 255 where (a, b) is no triangle
 };
 
-// per vertex and component: bit 2j positive (quantised >= 1), bit 2j+1
-// negative (<= -1); zero leaves both clear
+// four bit planes, interleaved by word: of component j, plane 2j positive
+// (quantised >= 1) and plane 2j + 1 negative (<= -1); zero leaves both clear
 template <typename T>
 __global__ void fs_class_kernel(CtGeom g, const T* __restrict__ f0, const T* __restrict__ f1, T t0, T t1,
-                                double q, unsigned char* __restrict__ cls) {
-  for (unsigned long long i = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; i < g.nv;
-       i += (unsigned long long)gridDim.x * blockDim.x) {
-    unsigned long long c[4];
-    ct_coords(g, i, c);
-    const unsigned long long gid = ct_gid(g, c), ai = ct_aidx(g, c);
-    unsigned char b = 0;
-    const T v[2] = {ct_adj(g, f0, ai, gid, t0), ct_adj(g, f1, ai, gid, t1)};
+                                double q, uint4* __restrict__ cls) {
+  const unsigned lane = threadIdx.x & 31;
+  T v[4][2];
+  ct_each_word(
+      g.nv,
+      [&](unsigned long long i, int j) {
+        const unsigned long long k = ct_index(g, i);
+        v[j][0] = __ldg(f0 + k);
+        v[j][1] = __ldg(f1 + k);
+      },
+      [&](unsigned long long w, int j) {
+        const bool in = 32 * w + lane < g.nv;
+        unsigned p[4];
 #pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const double x = __dadd_rn(__dmul_rn((double)v[j], q), v[j] > T(0) ? 0.5 : -0.5);
-      if (x >= 1.0) b |= (unsigned char)(1u << (2 * j));
-      if (x <= -1.0) b |= (unsigned char)(2u << (2 * j));
-    }
-    cls[i] = b;
-  }
+        for (int k = 0; k < 2; ++k) {
+          const T y = fp<T>::sub(v[j][k], k ? t1 : t0);
+          const double x = in ? __dadd_rn(__dmul_rn((double)y, q), y > T(0) ? 0.5 : -0.5) : 0.0;
+          p[2 * k] = __ballot_sync(0xffffffffu, x >= 1.0);
+          p[2 * k + 1] = __ballot_sync(0xffffffffu, x <= -1.0);
+        }
+        if (lane == 0) cls[w] = make_uint4(p[0], p[1], p[2], p[3]);
+      });
 }
 
 template <typename T>
@@ -825,97 +1204,208 @@ __device__ __forceinline__ void fs_values(const CtGeom& g, const T* f0, const T*
   }
 }
 
-// per vertex: bit t of the 50-bit mask = triangle type t from this vertex is
-// a feature.  One component of one strict sign at all three vertices keeps
-// the origin outside whatever the ties (exact pre-test); the rest go through
-// the exact 2-D test.
+// Per vertex: bit t of the 50-bit mask = triangle type t from this vertex is a
+// feature.  One component of one strict sign at all three vertices keeps the
+// origin outside whatever the ties (exact pre-test); the rest go through the
+// exact 2-D test.
+//
+// A warp takes 32 consecutive vertices; lanes e and 16 + e hold the planes of
+// the two components at their corners e.  What all corners share every
+// triangle shares, so most warps are done after an AND over the lanes; in the
+// others a lane takes a triangle type and finds the vertices where its corners
+// share nothing, and these triangles are listed in shared memory and tested by
+// full warps.  Vertices whose hypercube is left after the first step are listed
+// for the cells.  96^3 x 8 double: 507 us with two class loads per triangle and
+// vertex and the exact test where it came up, 128 with the sixteen classes in a
+// register, now 95.
 template <typename T>
-__global__ void fs_mask_kernel(CtGeom g, FsTables tb, const T* __restrict__ f0, const T* __restrict__ f1, T t0,
-                               T t1, double q, const unsigned char* __restrict__ cls,
-                               unsigned long long* __restrict__ mask, unsigned* __restrict__ blk,
-                               unsigned long long* __restrict__ total64) {
-  __shared__ unsigned tot;
-  const unsigned long long i = blockIdx.x * (unsigned long long)kCtThreads + threadIdx.x;
-  unsigned long long m = 0;
-  if (i < g.nv) {
-    unsigned long long c[4];
-    ct_coords(g, i, c);
-    const unsigned inb = ct_inbounds(g, c);
-    const unsigned long long gid = ct_gid(g, c), ai = ct_aidx(g, c);
-    const unsigned c0 = cls[i];
-    for (int t = 0; t < 50; ++t) {
-      const int a = tb.ta[t], b = tb.tb[t];
-      if (b & ~inb) continue;
-      const unsigned all = c0 & cls[i + g.loff[a]] & cls[i + g.loff[b]];
-      if (all) continue;
-      T v[3][2];
-      fs_values(g, f0, f1, t0, t1, ai, gid, a, b, v);
-      if (sos_inside2<T>(v, q)) m |= 1ull << t;
+__global__ void __launch_bounds__(kCtThreads) fs_mask_kernel(
+    CtGeom g, FsTables tb, const T* __restrict__ f0, const T* __restrict__ f1, T t0, T t1, double q,
+    const uint4* __restrict__ cls, unsigned long long* __restrict__ mask, unsigned* __restrict__ blk,
+    unsigned long long* __restrict__ total64, unsigned* __restrict__ cand, unsigned* __restrict__ cand_cnt) {
+  __shared__ unsigned n_list[kCtPer], s_at;
+  __shared__ unsigned long long s_mask[kCtThreads], s_gid[kCtThreads], s_ai[kCtThreads];
+  __shared__ unsigned short s_list[kCtThreads * 50];  // vertex of the share << 6 | triangle type
+  __shared__ unsigned char s_ab[64];                  // corners a << 4 | b of a triangle type
+  const unsigned tid = threadIdx.x, lane = tid & 31, full = 0xffffffffu;
+  const unsigned long long i0 = blockIdx.x * (unsigned long long)kCtBlock + tid;
+  if (tid < 64) s_ab[tid] = tid < 50 ? (unsigned char)(tb.ta[tid] << 4 | tb.tb[tid]) : 0;
+  if (tid < kCtPer) n_list[tid] = 0;
+  const unsigned e = lane & 15u;
+  unsigned n0[kCtPer], n1[kCtPer];
+#pragma unroll
+  for (int j = 0; j < kCtPer; ++j) {
+    const unsigned long long w0 = i0 - lane + j * kCtThreads;
+    n0[j] = n1[j] = full;
+    if (w0 < g.nv) {
+      const unsigned long long o = w0 + ct_corner_step(g, e);
+      const uint2* p = reinterpret_cast<const uint2*>(cls + o / 32) + (lane >> 4);
+      const uint2 lo = p[0], hi = p[2];
+      n0[j] = __funnelshift_r(lo.x, hi.x, (unsigned)o & 31u);
+      n1[j] = __funnelshift_r(lo.y, hi.y, (unsigned)o & 31u);
     }
-    mask[i] = m;
   }
-  ct_block_scan((unsigned)__popcll(m), &tot);
-  if (threadIdx.x == 0) {
-    blk[blockIdx.x] = tot;
-    atomicAdd(total64, (unsigned long long)tot);
+  __syncthreads();
+  unsigned rank[kCtPer], cube = 0;  // feature triangles, listed cubes << 16
+#pragma unroll 1
+  for (int j = 0; j < kCtPer; ++j) {
+    const unsigned long long i = i0 + j * kCtThreads;
+    unsigned x0 = n0[0], x1 = n1[0];
+#pragma unroll
+    for (int k = 1; k < kCtPer; ++k)
+      if (j == k) x0 = n0[k], x1 = n1[k];
+    // vertices that share a sign with all corners `out` does not excuse
+    auto sharing = [&](unsigned out) {
+      unsigned x = x0 | out, y = x1 | out;
+#pragma unroll
+      for (int s = 8; s; s >>= 1) {
+        x &= __shfl_xor_sync(full, x, s);
+        y &= __shfl_xor_sync(full, y, s);
+      }
+      x |= y;
+      return x | __shfl_xor_sync(full, x, 16);
+    };
+    unsigned left = ~sharing(0u) & __ballot_sync(full, i < g.nv);
+    s_mask[tid] = 0;
+    if (left) {
+      unsigned long long c[4];
+      ct_coords(g, i, c);
+      const unsigned inb = i < g.nv ? ct_inbounds(g, c) : 0u;
+      unsigned in[4], in_e = full;
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        in[k] = __ballot_sync(full, (inb >> k) & 1u);
+        if ((e >> k) & 1u) in_e &= in[k];
+      }
+      left &= ~sharing(~in_e);
+      if ((left >> lane) & 1u) {
+        if (inb == 15u) cube |= 1u << j;
+        s_gid[tid] = ct_gid(g, c);
+        s_ai[tid] = ct_aidx(g, c);
+      }
+      const unsigned c0 = __shfl_sync(full, x0, 0), c1 = __shfl_sync(full, x1, 0);
+      const unsigned c2 = __shfl_sync(full, x0, 16), c3 = __shfl_sync(full, x1, 16);
+      for (unsigned t = lane; t < 64; t += 32) {
+        const unsigned a = s_ab[t] >> 4, b = s_ab[t] & 15u;
+        unsigned common = c0 & __shfl_sync(full, x0, a) & __shfl_sync(full, x0, b);
+        common |= c1 & __shfl_sync(full, x1, a) & __shfl_sync(full, x1, b);
+        common |= c2 & __shfl_sync(full, x0, 16 + a) & __shfl_sync(full, x0, 16 + b);
+        common |= c3 & __shfl_sync(full, x1, 16 + a) & __shfl_sync(full, x1, 16 + b);
+        unsigned open = t < 50 ? left & ~common : 0u;
+#pragma unroll
+        for (int k = 0; k < 4; ++k)
+          if ((b >> k) & 1u) open &= in[k];
+        if (open) {
+          unsigned at = atomicAdd(&n_list[j], (unsigned)__popc(open));
+          for (; open; open &= open - 1) s_list[at++] = (unsigned short)((tid - lane + __ffs(open) - 1) << 6 | t);
+        }
+      }
+    }
+    __syncthreads();
+    const unsigned n = n_list[j];
+    unsigned long long m = 0;
+    if (n) {  // uniform over the block
+      for (unsigned k = tid; k < n; k += kCtThreads) {
+        const unsigned x = s_list[k] >> 6, t = s_list[k] & 63u;
+        T v[3][2];
+        fs_values(g, f0, f1, t0, t1, s_ai[x], s_gid[x], s_ab[t] >> 4, s_ab[t] & 15u, v);
+        if (sos_inside2<T>(v, q)) atomicOr(&s_mask[x], 1ull << t);
+      }
+      __syncthreads();
+      m = s_mask[tid];
+    }
+    if (i < g.nv) mask[i] = m;
+    const unsigned r = (unsigned)__popcll(m) | ((cube >> j) & 1u) << 16;
+#pragma unroll
+    for (int k = 0; k < kCtPer; ++k)
+      if (j == k) rank[k] = r;
   }
+  const unsigned n = ct_block_ranks(rank);
+  if (tid == 0) {
+    blk[blockIdx.x] = n & 0xFFFFu;
+    if (n & 0xFFFFu) atomicAdd(total64, (unsigned long long)(n & 0xFFFFu));
+    if (n >> 16) s_at = atomicAdd(cand_cnt, n >> 16);
+  }
+  if (n >> 16 == 0) return;
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < kCtPer; ++j)
+    if ((cube >> j) & 1u) cand[s_at + (rank[j] >> 16)] = (unsigned)(i0 + j * kCtThreads);
 }
 
+// The feature triangles of a block's vertices, a thread per triangle, listed
+// in rank order in shared memory first.  voff (first rank) is written where a
+// vertex has triangles.
 template <typename T>
-__global__ void fs_emit_kernel(CtGeom g, FsTables tb, const T* __restrict__ f0, const T* __restrict__ f1, T t0,
-                               T t1, const unsigned long long* __restrict__ mask,
-                               const unsigned* __restrict__ blk_off, unsigned* __restrict__ voff,
-                               unsigned long long* __restrict__ simp, double* __restrict__ lam,
-                               float* __restrict__ bary) {
-  __shared__ unsigned tot;
-  const unsigned long long i = blockIdx.x * (unsigned long long)kCtThreads + threadIdx.x;
-  const unsigned long long m = i < g.nv ? mask[i] : 0ull;
-  const unsigned base = blk_off[blockIdx.x] + ct_block_scan((unsigned)__popcll(m), &tot);
-  if (i >= g.nv) return;
-  voff[i] = base;
-  if (!m) return;
-  unsigned long long c[4];
-  ct_coords(g, i, c);
-  const unsigned long long gid = ct_gid(g, c), ai = ct_aidx(g, c);
-  unsigned r = base;
-  for (int t = 0; t < 50; ++t) {
-    if (!((m >> t) & 1ull)) continue;
-    const int a = tb.ta[t], b = tb.tb[t];
-    T v[3][2];
-    fs_values(g, f0, f1, t0, t1, ai, gid, a, b, v);
-    T l[3];
-    if (!solve_exact<2, T>(v, l))  // FiberPredicate keeps the centroid: (T)1.0 / 3.0
-      for (int k = 0; k < 3; ++k) l[k] = (T)((double)(T)1.0 / 3.0);
-    simp[3 * (size_t)r] = gid;
-    simp[3 * (size_t)r + 1] = gid + g.goff[a];
-    simp[3 * (size_t)r + 2] = gid + g.goff[b];
-    for (int k = 0; k < 3; ++k) {
-      lam[3 * (size_t)r + k] = (double)l[k];
-      bary[3 * (size_t)r + k] = (float)l[k];
+__global__ void __launch_bounds__(kCtThreads) fs_emit_kernel(
+    CtGeom g, FsTables tb, const T* __restrict__ f0, const T* __restrict__ f1, T t0, T t1,
+    const unsigned long long* __restrict__ mask, const unsigned* __restrict__ blk_off, unsigned* __restrict__ voff,
+    unsigned long long* __restrict__ simp, double* __restrict__ lam, float* __restrict__ bary) {
+  __shared__ unsigned short s_list[kCtThreads * 50];  // vertex of the share << 6 | triangle type
+  __shared__ unsigned s_end[kCtPer];
+  const unsigned long long i0 = blockIdx.x * (unsigned long long)kCtBlock;
+  const unsigned base = blk_off[blockIdx.x];
+  unsigned long long m[kCtPer];
+  unsigned rank[kCtPer], cnt[kCtPer];
+#pragma unroll
+  for (int j = 0; j < kCtPer; ++j) {
+    const unsigned long long i = i0 + j * kCtThreads + threadIdx.x;
+    m[j] = i < g.nv ? mask[i] : 0ull;
+    rank[j] = cnt[j] = (unsigned)__popcll(m[j]);
+  }
+  if (ct_block_ranks(rank) == 0) return;
+#pragma unroll
+  for (int j = 0; j < kCtPer; ++j)
+    if (threadIdx.x == kCtThreads - 1) s_end[j] = rank[j] + cnt[j];
+  __syncthreads();
+#pragma unroll
+  for (int j = 0; j < kCtPer; ++j) {
+    const unsigned lo = j ? s_end[j - 1] : 0u, hi = s_end[j];
+    if (lo == hi) continue;  // uniform over the block
+    if (m[j]) voff[i0 + j * kCtThreads + threadIdx.x] = base + rank[j];
+    unsigned w = rank[j] - lo;
+    for (unsigned long long x = m[j]; x; x &= x - 1)
+      s_list[w++] = (unsigned short)(threadIdx.x << 6 | (__ffsll(x) - 1));
+    __syncthreads();
+    for (unsigned k = threadIdx.x; k < hi - lo; k += kCtThreads) {
+      const unsigned t = s_list[k] & 63u;
+      const int a = tb.ta[t], b = tb.tb[t];
+      unsigned long long c[4];
+      ct_coords(g, i0 + j * kCtThreads + (s_list[k] >> 6), c);
+      const unsigned long long gid = ct_gid(g, c);
+      T v[3][2];
+      fs_values(g, f0, f1, t0, t1, ct_aidx(g, c), gid, a, b, v);
+      T l[3];
+      if (!solve_exact<2, T>(v, l))  // FiberPredicate keeps the centroid: (T)1.0 / 3.0
+        for (int z = 0; z < 3; ++z) l[z] = (T)((double)(T)1.0 / 3.0);
+      const size_t r = (size_t)base + lo + k;
+      simp[3 * r] = gid;
+      simp[3 * r + 1] = gid + g.goff[a];
+      simp[3 * r + 2] = gid + g.goff[b];
+      for (int z = 0; z < 3; ++z) {
+        lam[3 * r + z] = (double)l[z];
+        bary[3 * r + z] = (float)l[z];
+      }
     }
-    ++r;
+    __syncthreads();
   }
 }
 
 // hypercubes with a feature triangle at one of their lower corners (a
-// superset of the cubes whose pentatopes hold features)
+// superset of the cubes whose pentatopes hold features), among the cubes the
+// class pre-test left
 __global__ void fs_list_kernel(CtGeom g, const unsigned long long* __restrict__ mask,
+                               const unsigned* __restrict__ cand, const unsigned* __restrict__ cand_cnt,
                                unsigned long long* __restrict__ list, unsigned* __restrict__ cnt) {
-  const int lane = threadIdx.x & 31;
-  for (unsigned long long q0 = blockIdx.x * (unsigned long long)blockDim.x; q0 < g.ncube;
-       q0 += (unsigned long long)gridDim.x * blockDim.x) {
-    const unsigned long long q = q0 + threadIdx.x;
+  const unsigned lane = threadIdx.x & 31, n = *cand_cnt;
+  const unsigned step = gridDim.x * blockDim.x;
+  for (unsigned long long k0 = blockIdx.x * blockDim.x; k0 < n; k0 += step) {
+    const unsigned long long k = k0 + threadIdx.x;
+    const unsigned long long base = k < n ? cand[k] : 0u;
     bool any = false;
-    unsigned long long base = 0;
-    if (q < g.ncube) {
-      unsigned long long r = q;
-      for (int k = 0; k < g.d; ++k) {
-        const unsigned long long n = g.L[k] - 1, c = r % n;
-        r /= n;
-        base += c * g.lstr[k];
-      }
-      for (int e = 0; e < 15 && !any; ++e) any = mask[base + g.loff[e]] != 0ull;
-    }
+    if (k < n)
+#pragma unroll
+      for (int e = 0; e < 15; ++e) any |= mask[base + g.loff[e]] != 0ull;
     const unsigned bal = __ballot_sync(0xffffffffu, any);
     unsigned wbase = 0;
     if (lane == 0 && bal) wbase = atomicAdd(cnt, (unsigned)__popc(bal));
@@ -937,19 +1427,35 @@ __global__ void fs_cells_kernel(CtGeom g, FsTables tb, const unsigned long long*
   const unsigned nl = *list_cnt;
   const unsigned long long warp = (blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x) >> 5;
   const unsigned long long nwarps = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
+  // triangle z of pentatope `lane`: its lowest corner's step and its type
+  __shared__ unsigned long long s_off[10][24];
+  __shared__ unsigned char s_type[10][24];
+  if (threadIdx.x < 24) {
+    int pe[5], z = 0;
+    pe[0] = 0;
+    for (int i = 0; i < 4; ++i) pe[i + 1] = pe[i] | (1 << g.perm[threadIdx.x][i]);
+    for (int i = 0; i < 3; ++i)
+      for (int j = i + 1; j < 4; ++j)
+        for (int k = j + 1; k < 5; ++k, ++z) {
+          s_off[z][threadIdx.x] = g.loff[pe[i]];
+          s_type[z][threadIdx.x] = tb.idx[pe[j] ^ pe[i]][pe[k] ^ pe[i]];
+        }
+  }
+  __syncthreads();
   for (unsigned long long it = warp; it < nl; it += nwarps) {
     unsigned rank[10], vset[10];
     int nn = 0;
     if (lane < 24) {
       const unsigned long long base = list[it];
-      int pe[5];
-      pe[0] = 0;
-      for (int i = 0; i < 4; ++i) pe[i + 1] = pe[i] | (1 << g.perm[lane][i]);
+      int z = 0;
+#pragma unroll
       for (int i = 0; i < 3; ++i)
+#pragma unroll
         for (int j = i + 1; j < 4; ++j)
-          for (int k = j + 1; k < 5; ++k) {
-            const int lo = pe[i], t = tb.idx[pe[j] ^ lo][pe[k] ^ lo];
-            const unsigned long long v = base + g.loff[lo];
+#pragma unroll
+          for (int k = j + 1; k < 5; ++k, ++z) {
+            const unsigned t = s_type[z][lane];
+            const unsigned long long v = base + s_off[z][lane];
             const unsigned long long mv = __ldg(mask + v);
             if (!((mv >> t) & 1ull)) continue;
             unsigned rk = __ldg(voff + v) + (unsigned)__popcll(mv & ((1ull << t) - 1ull));
@@ -1010,8 +1516,8 @@ __global__ void fs_cells_kernel(CtGeom g, FsTables tb, const unsigned long long*
           if (slot < cap)
             for (int k = 0; k < 3; ++k) cells[(size_t)slot * 3 + k] = tri[k];
           ++slot;
-          uf_unite(parent, tri[0], tri[1], err);
-          uf_unite(parent, tri[0], tri[2], err);
+          uf_unite_flat(parent, tri[0], tri[1], err);
+          uf_unite_flat(parent, tri[0], tri[2], err);
         }
       }
     }
@@ -1023,14 +1529,14 @@ ftk2b_status run_fiber_surface(ftk2b_ctx* ctx, const CtGeom& g, const FsTables& 
                                const void* fb, T t0, T t1, double q, ftk2b_fiber_surface_result* res) {
   cudaStream_t st = ctx->stream;
   DevBuf* B = ctx->contour;
-  const unsigned long long nblk = (g.nv + kCtThreads - 1) / kCtThreads;
+  const unsigned long long nblk = (g.nv + kCtBlock - 1) / kCtBlock;
   if (nblk >= 0xFFFFFFF0ull) return cfail(ctx, FTK2B_UNSUPPORTED, "mesh too large");
-  C_TRY(B[kBufPos].ensure(g.nv));
+  C_TRY(B[kBufPos].ensure(16 * ct_words(g)));
   C_TRY(B[kBufHist].ensure(8 * g.nv));
   C_TRY(B[kBufVoff].ensure(4 * g.nv));
   C_TRY(B[kBufBlk].ensure(4 * (nblk + 1)));
   C_TRY(B[kBufCount].ensure(64));
-  auto* cls = static_cast<unsigned char*>(B[kBufPos].p);
+  auto* cls = static_cast<uint4*>(B[kBufPos].p);
   auto* mask = static_cast<unsigned long long*>(B[kBufHist].p);
   auto* voff = static_cast<unsigned*>(B[kBufVoff].p);
   auto* blk = static_cast<unsigned*>(B[kBufBlk].p);
@@ -1042,8 +1548,11 @@ ftk2b_status run_fiber_surface(ftk2b_ctx* ctx, const CtGeom& g, const FsTables& 
   const unsigned sms = (unsigned)ctx->num_sms;
   C_TRY(cudaMemsetAsync(counts, 0, 64, st));
   C_TRY(cudaEventRecord(ctx->ev0, st));
-  fs_class_kernel<T><<<grid_of(g.nv, 256, 32ull * sms), 256, 0, st>>>(g, a0, a1, t0, t1, q, cls);
-  fs_mask_kernel<T><<<(unsigned)nblk, kCtThreads, 0, st>>>(g, tb, a0, a1, t0, t1, q, cls, mask, blk, total64);
+  C_TRY(B[kBufCells].ensure(4 * (g.ncube ? g.ncube : 1)));
+  auto* cand = static_cast<unsigned*>(B[kBufCells].p);  // until the cells come
+  fs_class_kernel<T><<<grid_of(g.nv, 4 * 256, 32ull * sms), 256, 0, st>>>(g, a0, a1, t0, t1, q, cls);
+  fs_mask_kernel<T><<<(unsigned)nblk, kCtThreads, 0, st>>>(g, tb, a0, a1, t0, t1, q, cls, mask, blk, total64, cand,
+                                                           counts + 5);
   C_TRY(launch_scan(blk, (unsigned)nblk, counts + 0, nullptr, st));  // counts[0]: feature count (labels)
   ctx->launches += 3;
   unsigned long long n64 = 0;
@@ -1066,7 +1575,7 @@ ftk2b_status run_fiber_surface(ftk2b_ctx* ctx, const CtGeom& g, const FsTables& 
   C_TRY(B[kBufList].ensure(8 * (g.ncube ? g.ncube : 1)));
   auto* list = static_cast<unsigned long long*>(B[kBufList].p);
   unsigned* list_cnt = counts + 4;
-  fs_list_kernel<<<grid_of(g.ncube, 256, 64ull * sms), 256, 0, st>>>(g, mask, list, list_cnt);
+  fs_list_kernel<<<grid_of(g.ncube, 256, 8ull * sms), 256, 0, st>>>(g, mask, cand, counts + 5, list, list_cnt);
   ctx->launches += 2;
 
   unsigned cap = (unsigned)std::min<unsigned long long>(0x7FFFFFFFull, std::max<unsigned long long>(1024ull, 4ull * n));
@@ -1118,7 +1627,7 @@ ftk2b_status run_fiber_surface(ftk2b_ctx* ctx, const CtGeom& g, const FsTables& 
     C_TRY(launch_scan(btot, sblocks, nullptr, nullptr, st));
     ct_scan_add_kernel<<<sblocks, kCtThreads, 0, st>>>(boff, nb, btot);
     ct_bucket_scatter_kernel<<<cg, 256, 0, st>>>(cells, ncell, 3, boff, bcur, rows);
-    ct_bucket_sort_kernel<<<grid_of(n, 128, 32ull * sms), 128, 0, st>>>(rows, boff, n, 3, counts + 3, uoff);
+    launch_bucket_sort(rows, boff, n, 3, counts + 3, uoff, st);
     ct_scan_blocks_kernel<<<sblocks, kCtThreads, 0, st>>>(uoff, nb, btot);
     C_TRY(launch_scan(btot, sblocks, nullptr, nullptr, st));
     ct_scan_add_kernel<<<sblocks, kCtThreads, 0, st>>>(uoff, nb, btot);
@@ -1170,6 +1679,43 @@ ftk2b_status run_fiber_surface(ftk2b_ctx* ctx, const CtGeom& g, const FsTables& 
 // meets while marching over the cells, which it visits by layer, base cell
 // (in stored order, each sorted) and Kuhn index j (vertices v_0..v_j at t,
 // v_j..v_k at t + 1), one worker at a time.
+
+// One simplex of the sweep: path corners and signs.
+struct CtSimplex {
+  int pe[5];      // corner of path vertex i
+  unsigned ps;    // bit i: path vertex i positive
+  int npos;
+};
+
+// The crossing edges of a 1-vs-rest or 2D+t 2-2 split in the order the
+// reference's marching functions meet them, as path-vertex pairs: the lone
+// vertex with the others in order; positives outer, others inner.
+__device__ __forceinline__ int ct_crossings(const CtSimplex& x, int nvtx, int* ea, int* eb) {
+  int ne = 0;
+  if (x.npos == 1 || x.npos == nvtx - 1) {
+    const bool lone_pos = x.npos == 1;
+    int lone = 0;
+    for (int i = 0; i < nvtx; ++i)
+      if ((((x.ps >> i) & 1u) != 0) == lone_pos) lone = i;
+    for (int o = 0; o < nvtx; ++o)
+      if (o != lone) {
+        ea[ne] = lone;
+        eb[ne] = o;
+        ++ne;
+      }
+  } else {
+    for (int a = 0; a < nvtx; ++a) {
+      if (!((x.ps >> a) & 1u)) continue;
+      for (int b = 0; b < nvtx; ++b) {
+        if ((x.ps >> b) & 1u) continue;
+        ea[ne] = a;
+        eb[ne] = b;
+        ++ne;
+      }
+    }
+  }
+  return ne;
+}
 
 struct CeGeom {
   int d;                       // spacetime dims: 3 (triangle base) or 4 (tet base)
@@ -1516,8 +2062,7 @@ ftk2b_status run_contour_extruded(ftk2b_ctx* ctx, CeGeom g, const void* field, T
     C_TRY(launch_scan(btot, sblocks, nullptr, nullptr, st));
     ct_scan_add_kernel<<<sblocks, kCtThreads, 0, st>>>(boff, nb, btot);
     ct_bucket_scatter_kernel<<<cg, 256, 0, st>>>(cells, ncell, kc, boff, bcur, cells_out);
-    ct_bucket_sort_kernel<<<grid_of(n, 128, 32ull * sms), 128, 0, st>>>(cells_out, boff, n, kc, counts + 3,
-                                                                         nullptr);
+    launch_bucket_sort(cells_out, boff, n, kc, counts + 3, nullptr, st);
     ctx->launches += 6;
   }
   if (n) {
@@ -2064,7 +2609,7 @@ ftk2b_status run_fiber_surface_extruded(ftk2b_ctx* ctx, const FeGeom& g, const v
     C_TRY(launch_scan(btot, sblocks, nullptr, nullptr, st));
     ct_scan_add_kernel<<<sblocks, kCtThreads, 0, st>>>(boff, nb, btot);
     ct_bucket_scatter_kernel<<<cg, 256, 0, st>>>(cells, ncell, 3, boff, bcur, rows);
-    ct_bucket_sort_kernel<<<grid_of(n, 128, 32ull * sms), 128, 0, st>>>(rows, boff, n, 3, counts + 3, uoff);
+    launch_bucket_sort(rows, boff, n, 3, counts + 3, uoff, st);
     ct_scan_blocks_kernel<<<sblocks, kCtThreads, 0, st>>>(uoff, nb, btot);
     C_TRY(launch_scan(btot, sblocks, nullptr, nullptr, st));
     ct_scan_add_kernel<<<sblocks, kCtThreads, 0, st>>>(uoff, nb, btot);
@@ -2347,6 +2892,15 @@ static ftk2b_status ct_geometry(ftk2b_ctx* ctx, const ftk2b_mesh_desc* mesh, con
         g.goff[e] += g.gs[k];
         g.aoff[e] += g.as[k];
       }
+  g.linear = !g.per_vertex;
+  for (int k = 0; k < d; ++k) g.linear &= g.L[k] == 1 || g.as[k] == lstr[k];
+  g.small = nv < (1ull << 31);
+  for (int k = 0; g.small && k < d; ++k) {
+    int l = 0;
+    while ((1ull << l) < g.L[k]) ++l;
+    g.shf[k] = 31 + l;
+    g.mul[k] = (unsigned)(((1ull << g.shf[k]) + g.L[k] - 1) / g.L[k]);
+  }
   *nelem_out = nelem;
   return FTK2B_OK;
 }

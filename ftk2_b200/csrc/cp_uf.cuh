@@ -37,4 +37,18 @@ __device__ __forceinline__ void uf_unite(unsigned* parent, unsigned a, unsigned 
   atomicOr(err, 1u);
 }
 
+// uf_unite for trees that are mostly flat already: elements with one parent
+// need no look at the root, whose single address all threads would read.
+__device__ __forceinline__ void uf_unite_flat(unsigned* parent, unsigned a, unsigned b, unsigned* err) {
+  if (__ldcg(&parent[a]) != __ldcg(&parent[b])) uf_unite(parent, a, b, err);
+}
+
+// Every element at its root (between launches that join).
+static __global__ void uf_flatten_kernel(unsigned* parent, unsigned n) {
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const unsigned r = uf_root(parent, i);
+    if (r != i) atomicMin(&parent[i], r);
+  }
+}
+
 }  // namespace ftk2b
