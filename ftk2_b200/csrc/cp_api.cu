@@ -150,6 +150,8 @@ extern "C" ftk2b_status ftk2b_ctx_create(int device, ftk2b_ctx** out) {
   if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess ||
       cudaEventCreate(&ctx->ev0) != cudaSuccess || cudaEventCreate(&ctx->ev1) != cudaSuccess ||
       cudaEventCreate(&ctx->ev_x) != cudaSuccess || cudaEventCreate(&ctx->ev_r) != cudaSuccess ||
+      cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking) != cudaSuccess ||
+      cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
       cudaEventCreateWithFlags(&ctx->ev_sync, cudaEventBlockingSync | cudaEventDisableTiming) != cudaSuccess) {
     delete ctx;
     return FTK2B_CUDA_ERROR;
@@ -204,6 +206,8 @@ extern "C" void ftk2b_ctx_destroy(ftk2b_ctx* ctx) {
   cudaEventDestroy(ctx->ev1);
   cudaEventDestroy(ctx->ev_x);
   cudaEventDestroy(ctx->ev_r);
+  cudaEventDestroy(ctx->ev_fork);
+  cudaStreamDestroy(ctx->side);
   cudaEventDestroy(ctx->ev_sync);
   cudaStreamDestroy(ctx->stream);
   delete ctx;
@@ -578,7 +582,6 @@ PostBuffers ftk2b_ctx::post_buffers(unsigned cap_, unsigned edge_cap_, int key_b
   B.n_edges = c + kCountEdges;
   B.n_roots = c + kCountRoots;
   B.err = c + kCountErr;
-  B.done = c + kCountDone;
   B.key_alt = (unsigned long long*)key_alt.p;
   B.perm0 = (unsigned*)perm0.p;
   B.perm1 = (unsigned*)perm1.p;
@@ -814,6 +817,19 @@ static ftk2b_status run_regular(ftk2b_ctx* ctx, const ftk2b_mesh_desc* mesh,
       *nl += (unsigned long long)nk;
       return cudaSuccess;
     };
+    const bool small = post_small(B);
+    auto pack_args = [&]() {
+      LastRun r;
+      r.m = m;
+      r.classify = classify;
+      r.want_edges = prm->want_edges;
+      PackArgs a = ctx->pack_args(r);
+      a.cap = cap;
+      a.edge_cap = edge_cap;
+      if (pack) a.h_counters = (unsigned*)ctx->pin.d;
+      else a.dst = nullptr;
+      return a;
+    };
     auto enqueue2 = [&](unsigned long long* nl) -> cudaError_t {
       cudaError_t e;
       if ((e = launch_refine_staged(f64, rm, fa, cfg, cq, rs, sink, ctx->num_sms, ctx->stream))) return e;
@@ -823,24 +839,19 @@ static ftk2b_status run_regular(ftk2b_ctx* ctx, const ftk2b_mesh_desc* mesh,
         if ((e = launch_classify_regular(f64, rm, fa, nch, B, ctx->stream))) return e;
         *nl += 1;
       }
+      if (small) {
+        if ((e = launch_post_finish(B, pack_args(), ctx->stream, nl)) || pack) return e;
+      }
       if (pack) return cudaSuccess;
       return cudaMemcpyAsync(ctx->h_counters, ctx->counters.p, sizeof(unsigned) * kNumCounters,
                              cudaMemcpyDeviceToHost, ctx->stream);
     };
-    // after the pipeline's last timing event: the results (when they fit) and
-    // the counters to the host
+    // the long chain, after its last timing event: the results (when they fit)
+    // and the counters to the host
     auto enqueue3 = [&](unsigned long long* nl) -> cudaError_t {
-      if (!pack) return cudaSuccess;
-      LastRun r;
-      r.m = m;
-      r.classify = classify;
-      r.want_edges = prm->want_edges;
-      PackArgs a = ctx->pack_args(r);
-      a.h_counters = (unsigned*)ctx->pin.d;
-      a.cap = cap;
-      a.edge_cap = edge_cap;
+      if (!pack || small) return cudaSuccess;
       *nl += 1;
-      return launch_pack(a, ctx->num_sms, ctx->stream);
+      return launch_pack(pack_args(), ctx->num_sms, ctx->stream);
     };
     if (cfg.cull_mode == 2) {
       int mode = 0;
@@ -918,8 +929,14 @@ static ftk2b_status run_regular(ftk2b_ctx* ctx, const ftk2b_mesh_desc* mesh,
           cudaError_t ce = enqueue0();
           if (!ce) ce = cudaEventRecordWithFlags(ctx->ev0, ctx->stream, cudaEventRecordExternal);
           if (!ce) ce = enqueue1(&nl);
-          if (!ce) ce = cudaEventRecordWithFlags(ctx->ev_x, ctx->stream, cudaEventRecordExternal);
+          // the cull's end is recorded on a branch of its own: between the cull
+          // and the exact test it took 4 us of every call
+          if (!ce) ce = cudaEventRecord(ctx->ev_fork, ctx->stream);
+          if (!ce) ce = cudaStreamWaitEvent(ctx->side, ctx->ev_fork, 0);
+          if (!ce) ce = cudaEventRecordWithFlags(ctx->ev_x, ctx->side, cudaEventRecordExternal);
           if (!ce) ce = enqueue2(&nl);
+          if (!ce) ce = cudaEventRecord(ctx->ev_fork, ctx->side);
+          if (!ce) ce = cudaStreamWaitEvent(ctx->stream, ctx->ev_fork, 0);
           if (!ce) ce = cudaEventRecordWithFlags(ctx->ev1, ctx->stream, cudaEventRecordExternal);
           if (!ce) ce = enqueue3(&nl);
           const cudaError_t ee = cudaStreamEndCapture(ctx->stream, &graph);

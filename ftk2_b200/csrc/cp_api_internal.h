@@ -58,8 +58,7 @@ enum {
   kCountPairs = 6,  // simplices the exact test ran on
   kCountBig = 7,    // candidates listed for the 128-bit inside test
   kCountAcc = 8,    // simplices inside by the fast path (listed for the solve)
-  kCountDone = 9,   // blocks of the short chain's edge kernel that finished
-  kNumCounters = 10
+  kNumCounters = 9
 };
 
 // Everything a regular-mesh run bakes into its kernel launches; a cached CUDA
@@ -167,6 +166,8 @@ struct ftk2b_ctx {
   int num_sms = 148;
   cudaStream_t stream = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev_x = nullptr;
+  cudaStream_t side = nullptr;     // branches of captured graphs (nothing runs on it)
+  cudaEvent_t ev_fork = nullptr;
   unsigned long long launches = 0;
   double last_extract_ms = 0;
   double last_refine_ms = 0;

@@ -13,6 +13,8 @@
 //   3. trajectories: lock-free union-find that always hooks the larger root
 //      under the smaller one, so every component's root is its smallest
 //      canonical id = the reference's track_id (engine.hpp:46-74, 965-983).
+#include <algorithm>
+
 #include "cp_batch.h"
 #include "cp_post.h"
 #include "cp_kuhn.cuh"
@@ -607,21 +609,27 @@ static int grid_for(unsigned cap, int threads, int max_blocks) {
 
 // ---------------------------------------------------------------------------
 // Post-extraction for small feature counts (capacity <= kSmallPostCap, keys
-// below 2^50): the outputs of the general chain above in two launches.
+// below 2^50): the outputs of the general chain above in three launches.
 //   1. sort, one block: a counting sort of the keys (each packed with its
 //      feature index in the low kIdxBits bits) by their top bits in shared
 //      memory, then each key's canonical position = its bucket's start + the
 //      keys of its bucket below it (the keys of one extraction are
-//      distinct); the packed keys land in key_alt in canonical order.
+//      distinct); the packed keys land in key_alt in canonical order.  Ranks
+//      among all keys (cp_ranksort.cuh) cost 2.5 us instead of 3.5 at 530
+//      features, but 21 instead of 11 at 5,700.
 //   2. star edges, one block of 1024 threads per SM: every block copies the
 //      sorted keys into shared memory, its warps find the star edges of the
 //      sorted features (one warp per feature) in the sorted keys and join
 //      each feature with its linked faces in a lock-free union-find (parents
 //      initialised by the sort); then each block writes the outputs of its
-//      contiguous share of positions, and the last block to finish runs the
-//      final step: exclusive scan of the edge counts, edge compaction, and
-//      every feature's root (the union-find's parents copied to shared
-//      memory): track ids and root count.
+//      contiguous share of positions.
+//   3. finish: every block copies the union-find's parents and the edge counts
+//      to shared memory, finds all roots and edge offsets there, and writes a
+//      share of the track ids, edges and, where the caller fetches the results
+//      next, of the packed host block (cp_pack.h).  One block ran this step
+//      alone after all others of the edges' launch had finished, and a pack
+//      launch followed: edges, last step and pack took 35 us for 533 features
+//      (64 x 64 x 10) and 66 for 5,700 (128^3 x 16), now 23 and 49.
 
 constexpr int kSortThreads = 1024;
 constexpr int kBucketBits = 13;
@@ -885,8 +893,6 @@ __device__ __forceinline__ void write_sorted_feature(const RegularMesh& mesh, in
   expand_feature(mesh, nch, key, pos, mesh.d, B.bary4_sorted, B.simplices, B.bary);
 }
 
-__device__ __forceinline__ void finish_block(const PostBuffers& B, unsigned* sh, unsigned* wsum, unsigned& s_roots);
-
 __global__ void __launch_bounds__(kSortThreads, 1)
     small_edges_kernel(RegularMesh mesh, int nch, PostBuffers B, int want_edges) {
   extern __shared__ unsigned long long sk[];  // the n sorted keys
@@ -911,104 +917,150 @@ __global__ void __launch_bounds__(kSortThreads, 1)
     const unsigned long long v = B.key_alt[p];
     write_sorted_feature(mesh, nch, B, (unsigned)(v & ((1ull << kIdxBits) - 1)), p, v >> kIdxBits);
   }
-  if (!want_edges) return;
-  // the last block to finish runs the final step: every block's edge
-  // counts, slots and union-find hooks are visible to it (each block fences
-  // its writes before counting itself done)
-  __shared__ unsigned s_last, s_roots;
-  __shared__ unsigned wsum[33];
-  __threadfence();
-  __syncthreads();
-  if (threadIdx.x == 0) s_last = atomicAdd(B.done, 1u) == G - 1 ? 1u : 0u;
-  __syncthreads();
-  if (!s_last) return;
-  __threadfence();
-  finish_block(B, reinterpret_cast<unsigned*>(sk), wsum, s_roots);
 }
 
-// The short chain's last step, by one block of 1024 threads: exclusive scan
-// of the edge counts, edge compaction, every feature's root from the union-find
-// parents (copied to shared memory), track ids and root count.  sh: n words
-// of shared memory.
-__device__ __forceinline__ void finish_block(const PostBuffers& B, unsigned* sh, unsigned* wsum, unsigned& s_roots) {
-  constexpr int kPer = (int)(kSmallPostCap / 1024);  // features per thread, at most
-  const unsigned n = min(*B.count, B.cap);
-  unsigned* const sp = sh;  // the union-find parents
-  const unsigned t = threadIdx.x;
-  // exclusive scan of the per-feature edge counts: each thread's contiguous
-  // segment, its counts loaded first (independent loads)
-  const unsigned seg = (n + 1023) / 1024;
-  const unsigned s0 = min(t * seg, n);
-  unsigned c[kPer];
-  unsigned sum = 0;
-#pragma unroll
-  for (int k = 0; k < kPer; ++k) {
-    c[k] = (k < (int)seg && s0 + k < n) ? __ldcg(&B.edge_cnt[s0 + k]) : 0u;
-    sum += c[k];
+constexpr int kFinishThreads = 1024;  // what block_exclusive_scan takes
+
+template <typename W, typename F>
+__device__ __forceinline__ void finish_words(unsigned char* dst, unsigned long long n, unsigned long long t,
+                                             unsigned long long nt, F word) {
+  W* out = reinterpret_cast<W*>(dst);
+  for (unsigned long long i = t; i < n; i += nt) out[i] = word(i);
+}
+
+// a.dst null: device results only.  sh: 2 n words.  The first kFinishRoots
+// blocks find roots and offsets; the others send the arrays whose place does
+// not depend on them over PCIe meanwhile.
+constexpr unsigned kFinishRoots = 8;
+__global__ void __launch_bounds__(kFinishThreads) small_finish_kernel(PostBuffers B, PackArgs a) {
+  extern __shared__ unsigned sh[];
+  __shared__ unsigned wsum[33], s_roots;
+  pdl_enter();
+  constexpr int kPer = (int)(kSmallPostCap / kFinishThreads);  // features per thread, at most
+  const unsigned count = *B.count, n = min(count, B.cap), t = threadIdx.x;
+  unsigned* const root = sh;
+  unsigned* const off = sh + n;
+  const unsigned k = (unsigned)a.k;
+  // consecutive lanes store consecutive words, so a warp's stores leave as
+  // whole 128-byte lines
+  if (blockIdx.x >= kFinishRoots) {
+    const PackLayout L = pack_layout(n, 0, a.k, a.classify);
+    if (!a.dst || count > a.cap || L.edges > a.dst_bytes) return;
+    const unsigned w = (blockIdx.x - kFinishRoots) * kFinishThreads + t;
+    const unsigned nw = (gridDim.x - kFinishRoots) * kFinishThreads;
+    finish_words<double>(a.dst + L.lam, (unsigned long long)n * k, w, nw,
+                         [&](unsigned long long i) { return k == 4 ? a.lam4[i] : a.lam4[i / k * 4 + i % k]; });
+    finish_words<unsigned long long>(a.dst + L.simplices, (unsigned long long)n * k, w, nw,
+                                     [&](unsigned long long i) { return a.simplices[i]; });
+    finish_words<float>(a.dst + L.bary, (unsigned long long)n * k, w, nw,
+                        [&](unsigned long long i) { return a.bary[i]; });
+    finish_words<float>(a.dst + L.scalar, n, w, nw, [&](unsigned long long i) { return a.scalar[i]; });
+    return;
   }
-  // the edge kernel's union-find is complete: its parents into shared memory
-  for (unsigned i = t; i < n; i += 1024) sp[i] = __ldcg(&B.parent[i]);
-  if (t == 0) s_roots = 0;
-  unsigned total;
-  unsigned run = block_exclusive_scan(sum, wsum, &total);
-  if (t == 0) *B.n_edges = total;
-  // the edges of each thread's contiguous run of features at their scanned
-  // offsets: the counts are in registers, the slots contiguous in memory
+  const unsigned gt = blockIdx.x * kFinishThreads + t, nt = min(gridDim.x, kFinishRoots) * kFinishThreads;
+  if (blockIdx.x && blockIdx.x * kFinishThreads >= n) return;  // no feature of this block's
+  unsigned ne = 0, roots = 0;
+  if (a.want_edges) {
+    for (unsigned i = t; i < n; i += kFinishThreads) {
+      root[i] = B.parent[i];
+      off[i] = B.edge_cnt[i];
+    }
+    if (t == 0) s_roots = 0;
+    __syncthreads();
+    // exclusive scan of the per-feature edge counts, a contiguous run of
+    // features a thread
+    const unsigned seg = (n + kFinishThreads - 1) / kFinishThreads, s0 = min(t * seg, n);
+    unsigned c[kPer], sum = 0;
 #pragma unroll
-  for (int k = 0; k < kPer; ++k) {
-    const unsigned i = s0 + k;
-    if (k < (int)seg && i < n) {
-      for (unsigned r = 0; r < c[k]; ++r) {
-        const unsigned other = __ldcg(&B.edge_slots[(size_t)i * kEdgeSlots + r]);
-        const unsigned e = run + r;
+    for (int k = 0; k < kPer; ++k) {
+      c[k] = (k < (int)seg && s0 + k < n) ? off[s0 + k] : 0u;
+      sum += c[k];
+    }
+    unsigned run = block_exclusive_scan(sum, wsum, &ne);
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      if (k < (int)seg && s0 + k < n) off[s0 + k] = run;
+      run += c[k];
+    }
+    // every feature's root (the minimum of its component) by pointer jumping:
+    // each round replaces every parent by its parent's parent, halving every
+    // path (reads may see this round's or the last round's values, both
+    // ancestors); a path of length L needs log2(L) rounds, at most 14 here
+    for (int round = 0; round < 16; ++round) {
+      bool changed = false;
+      for (unsigned i = t; i < n; i += kFinishThreads) {
+        const unsigned p = root[i];
+        if (!FTK2B_CHECK(p < n, B.err)) continue;
+        const unsigned pp = root[p];
+        if (pp != p) {
+          root[i] = pp;
+          changed = true;
+        }
+      }
+      if (!__syncthreads_or(changed)) break;
+    }
+    if (blockIdx.x == 0) {
+      for (unsigned i = t; i < n; i += kFinishThreads) roots += root[i] == i ? 1u : 0u;
+      roots = __reduce_add_sync(0xFFFFFFFFu, roots);
+      if ((t & 31) == 0) atomicAdd(&s_roots, roots);
+      __syncthreads();
+      if (t == 0) {
+        *B.n_edges = ne;
+        *B.n_roots = s_roots;
+      }
+    }
+  }
+  if (a.h_counters && gt < (unsigned)a.n_counters) {  // of block 0
+    unsigned v = a.counters[gt];
+    if (a.want_edges && a.counters + gt == B.n_edges) v = ne;
+    if (a.want_edges && a.counters + gt == B.n_roots) v = s_roots;
+    a.h_counters[gt] = v;
+  }
+  const PackLayout L = pack_layout(n, ne, a.k, a.classify);
+  const bool pack = a.dst && count <= a.cap && ne <= a.edge_cap && L.packed <= a.dst_bytes;
+  if (a.want_edges) {
+    unsigned* const out = reinterpret_cast<unsigned*>(a.dst + L.edges);
+    for (unsigned i = gt; i < n; i += nt) {
+      B.track[i] = root[i];
+      const unsigned o = off[i], e1 = i + 1 < n ? off[i + 1] : ne;
+      for (unsigned e = o; e < e1; ++e) {
+        const unsigned other = B.edge_slots[(size_t)i * kEdgeSlots + (e - o)];
         if (e < B.edge_cap) {
           B.edges[2 * (size_t)e] = i;
           B.edges[2 * (size_t)e + 1] = other;
+          if (pack) *reinterpret_cast<uint2*>(out + 2 * (size_t)e) = make_uint2(i, other);
         }
       }
     }
-    run += c[k];
   }
-  // every feature's root (the minimum of its component) by pointer jumping:
-  // each round replaces every parent by its parent's parent, halving every
-  // path (reads may see this round's or the last round's values, both
-  // ancestors); a path of length L needs log2(L) rounds, at most 14 here
-  for (int round = 0; round < 16; ++round) {
-    bool changed = false;
-    for (unsigned i = t; i < n; i += 1024) {
-      const unsigned p = sp[i];
-      if (!FTK2B_CHECK(p < n, B.err)) continue;
-      const unsigned pp = sp[p];
-      if (pp != p) {
-        sp[i] = pp;
-        changed = true;
-      }
-    }
-    if (!__syncthreads_or(changed)) break;
-  }
-  unsigned roots = 0;
-  for (unsigned i = t; i < n; i += 1024) {
-    const unsigned x = sp[i];
-    B.track[i] = x;
-    roots += x == i ? 1u : 0u;
-  }
-  atomicAdd(&s_roots, roots);
-  __syncthreads();
-  if (t == 0) *B.n_roots = s_roots;
+  if (!pack) return;
+  finish_words<unsigned long long>(a.dst + L.track, n, gt, nt,
+                                   [&](unsigned long long i) { return a.want_edges ? root[i] : i; });
+  if (a.classify) finish_words<unsigned>(a.dst + L.cls, n, gt, nt, [&](unsigned long long i) { return a.cls[i]; });
+}
+
+bool post_small(const PostBuffers& B) { return B.cap <= kSmallPostCap && B.key_bits <= 64 - kIdxBits; }
+
+cudaError_t launch_post_finish(const PostBuffers& B, const PackArgs& a, cudaStream_t st,
+                               unsigned long long* launches) {
+  const size_t smem = 8 * (size_t)(B.cap ? B.cap : 1);
+  cudaError_t e = cudaFuncSetAttribute(small_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                       8 * (int)kSmallPostCap);
+  if (!e) e = launch_pdl(small_finish_kernel, std::max(B.num_sms > 0 ? B.num_sms : 148, (int)kFinishRoots + 1), kFinishThreads, smem, st, B, a);
+  if (e) return e;
+  *launches += 1;
+  return cudaGetLastError();
 }
 
 static cudaError_t launch_post_small(const RegularMesh& mesh, int nch, const PostBuffers& B, int want_edges,
                                      cudaStream_t st, unsigned long long* launches) {
   const unsigned cap = B.cap;
   const size_t key_smem = sizeof(unsigned long long) * (size_t)(cap ? cap : 1);
-  // the edge kernel's last block reuses the keys' shared memory for the
-  // final step's 2n + 1 words
-  const size_t edge_smem = key_smem + 16;
   const int g = B.num_sms > 0 ? B.num_sms : 148;
   cudaError_t e = cudaFuncSetAttribute(small_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)key_smem);
   if (!e) e = launch_pdl(small_sort_kernel, 1, kSortThreads, key_smem, st, B);
-  if (!e) e = cudaFuncSetAttribute(small_edges_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)edge_smem);
-  if (!e) e = launch_pdl(small_edges_kernel, g, kSortThreads, edge_smem, st, mesh, nch, B, want_edges);
+  if (!e) e = cudaFuncSetAttribute(small_edges_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)key_smem);
+  if (!e) e = launch_pdl(small_edges_kernel, g, kSortThreads, key_smem, st, mesh, nch, B, want_edges);
   if (e) return e;
   *launches += 2;
   return cudaGetLastError();
@@ -1017,7 +1069,7 @@ static cudaError_t launch_post_small(const RegularMesh& mesh, int nch, const Pos
 cudaError_t launch_post_regular(const RegularMesh& mesh, int nch, const PostBuffers& B,
                                 int want_edges, cudaStream_t st, unsigned long long* launches) {
   const unsigned cap = B.cap;
-  if (cap <= kSmallPostCap && B.key_bits <= 64 - kIdxBits)
+  if (post_small(B))
     return launch_post_small(mesh, nch, B, want_edges, st, launches);
   const int gsort = B.sort_grid;
   const int g = grid_for(cap, 256, 4096);

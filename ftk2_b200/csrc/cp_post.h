@@ -2,6 +2,7 @@
 #pragma once
 
 #include "cp_internal.h"
+#include "cp_pack.h"
 
 namespace ftk2b {
 
@@ -40,13 +41,18 @@ struct PostBuffers {
   unsigned* parent;
   unsigned* n_roots;
   unsigned* err;
-  unsigned* done;                   // short chain: edge-kernel blocks finished (zeroed per call)
   unsigned* cls;                    // per feature classification (FTK2B_CLASS_*)
 };
 
 void upload_post_tables();
 cudaError_t launch_post_regular(const RegularMesh& mesh, int nch, const PostBuffers& B,
                                 int want_edges, cudaStream_t st, unsigned long long* launches);
+// Whether launch_post_regular runs the short chain, which leaves its last step
+// to launch_post_finish: edges, track ids and their counts and, unless a.dst is
+// null, what launch_pack does (after the classes, where a wants them).
+bool post_small(const PostBuffers& B);
+cudaError_t launch_post_finish(const PostBuffers& B, const PackArgs& a, cudaStream_t st,
+                               unsigned long long* launches);
 cudaError_t launch_classify_regular(int f64, const RegularMesh& mesh, const FieldAccess& fa, int nch,
                                     const PostBuffers& B, cudaStream_t st);
 cudaError_t launch_iota(unsigned* v, const unsigned* n_ptr, unsigned cap, cudaStream_t st);
