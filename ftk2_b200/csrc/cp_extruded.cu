@@ -887,7 +887,7 @@ cudaError_t enqueue_post(ftk2b_ctx* ctx, const ExtMeshDev& X, const ExtSink& sin
   if (ranked) {
     const LoadFound ld{sink.hi, sink.lo};
     const StoreFound<M> sw{sink, out, vb};
-    if ((e = launch_rank_sort<2>(ld, sw, nullptr, n, nullptr, ctx->num_sms, st))) return e;
+    if ((e = launch_rank_sort<2>(ld, sw, RankCount{n, nullptr, nullptr, 0}, n ? n : 1, nullptr, ctx->num_sms, st))) return e;
     *nl += 1;
   } else {
     const int sgrid = ctx->sort_grid(cap);
@@ -920,7 +920,7 @@ cudaError_t enqueue_post(ftk2b_ctx* ctx, const ExtMeshDev& X, const ExtSink& sin
   if (ranked) {
     const LoadEdgeKey ld{(const unsigned long long*)C.ekeys.p};
     const StoreEdge so{(unsigned*)ctx->edges.p};
-    if ((e = launch_rank_sort<1>(ld, so, counters + kCountEdges, std::min(edge_cap, kRankCap1), nullptr,
+    if ((e = launch_rank_sort<1>(ld, so, RankCount{0, counters + kCountEdges, nullptr, 0}, std::min(edge_cap, kRankCap1), nullptr,
                                  ctx->num_sms, st)))
       return e;
     *nl += 1;
@@ -1108,6 +1108,7 @@ ftk2b_status push_extruded_t(ftk2b_stream* s) {
   if (ns * (tnow + 1) > 0xFFFFFFFFull) return ext_fail(ctx, FTK2B_UNSUPPORTED, "spacetime vertex ids exceed 32 bits");
   rc = prepare_base(ctx, &s->emesh, fbits, &nl, &s->ebase_hash);
   if (rc) return rc;
+  if (nl) s->counters_clear = false;  // the preparation counts too
   const unsigned t0 = tnow ? (unsigned)(tnow - 1) : 0u, L = tnow ? 1u : 0u;
   ExtMeshDev X = stream_mesh(ctx, s, t0, L);
   X.skip_first_spatial = tnow > 0;
@@ -1125,13 +1126,49 @@ ftk2b_status push_extruded_t(ftk2b_stream* s) {
   EXT_TRY(ctx->counters.ensure(sizeof(unsigned) * kNumCounters));
   unsigned* counters = (unsigned*)ctx->counters.p;
   unsigned n_new = 0;
+  // window: spatial features of layer t-1 plus the new ones, in Simplex order;
+  // it goes ahead of the host's look at the counters as in regular streams
+  const unsigned first_new = s->n;
+  const unsigned* ids = nullptr;
+  auto room = [&](unsigned wcap) -> ftk2b_status {
+    EXT_TRY(s->s_id.ensure(4 * (size_t)wcap));
+    EXT_TRY(s->s_hi.ensure(8 * (size_t)wcap));
+    EXT_TRY(s->s_lo.ensure(8 * (size_t)wcap));
+    EXT_TRY(s->s_phase.ensure(4 * (size_t)wcap));
+    return ensure_stream_edges(s, (unsigned long long)kMaxOthers * wcap);
+  };
+  auto window = [&](const RankCount& count, unsigned wcap) -> cudaError_t {
+    const LoadTuple ld{(const unsigned long long*)s->hi.p, (const unsigned long long*)s->lo.p,
+                       (const unsigned*)s->prev_ids.p, s->n_prev, first_new};
+    const StoreTuple<M> sw{ld, (unsigned long long*)s->s_hi.p, (unsigned long long*)s->s_lo.p,
+                           (const unsigned*)s->phase.p, (unsigned*)s->s_phase.p, (unsigned*)s->s_id.p,
+                           (unsigned*)s->parent.p, (unsigned*)s->prev_ids2.p, counters + kSPrev, ns, tnow};
+    ids = sw.ids;
+    nl += 1;
+    return launch_rank_sort<2>(ld, sw, count, wcap, counters + kSWin, ctx->num_sms, st);
+  };
+  auto stars = [&](unsigned wcap) -> cudaError_t {
+    const ExtFeatures Fs{(const unsigned long long*)s->s_hi.p, (const unsigned long long*)s->s_lo.p,
+                         (const unsigned*)s->s_phase.p, counters + kSWin, wcap, kStreamVb};
+    const ExtStars to{ids, (unsigned*)s->parent.p, nullptr, (unsigned*)s->edges.p, s->n_edges, s->edge_cap,
+                      counters + kSWinEdges, counters + kCountErr};
+    ext_stars_kernel<M><<<grid_of(kStarLanes * (unsigned long long)wcap, 256, 4096), 256, 0, st>>>(X, Fs, to);
+    nl += 1;
+    return cudaGetLastError();
+  };
+  const unsigned guess = window_guess(s, kRankCap2);
+  if (guess) {
+    rc = room(guess);
+    if (rc) return rc;
+  }
   for (int attempt = 0;; ++attempt) {
     if (attempt == 6) return ext_fail(ctx, FTK2B_OVERFLOW_RETRY, "stream buffers kept overflowing");
     if (s->cap < s->n + 1024) {
       rc = ensure_stream_store(s, s->n + 1024);
       if (rc) return rc;
     }
-    EXT_TRY(cudaMemsetAsync(counters, 0, sizeof(unsigned) * kNumCounters, st));
+    if (!s->counters_clear) EXT_TRY(cudaMemsetAsync(counters, 0, sizeof(unsigned) * kNumCounters, st));
+    s->counters_clear = false;
     ExtSink sink;
     sink.hi = (unsigned long long*)s->hi.p + s->n;
     sink.lo = (unsigned long long*)s->lo.p + s->n;
@@ -1142,7 +1179,12 @@ ftk2b_status push_extruded_t(ftk2b_stream* s) {
     sink.count = counters + kCountFeatures;
     sink.cap = s->cap - s->n;
     EXT_TRY((enqueue_extract<T, M>(ctx, X, fa, cfg, sink, kStreamVb, nv, &nl)));
+    if (guess) {
+      EXT_TRY(window({s->n_prev, counters + kCountFeatures, counters + kCountFeatures, sink.cap}, guess));
+      EXT_TRY(stars(guess));
+    }
     EXT_TRY(cudaMemcpyAsync(ctx->h_counters, counters, sizeof(unsigned) * kNumCounters, cudaMemcpyDeviceToHost, st));
+    EXT_TRY(cudaEventRecord(ctx->ev1, st));
     EXT_TRY(ctx->sync());
     const unsigned got = ctx->h_counters[kCountFeatures];
     if (got > s->cap - s->n) {
@@ -1154,38 +1196,23 @@ ftk2b_status push_extruded_t(ftk2b_stream* s) {
     break;
   }
 
-  // window: spatial features of layer t-1 plus the new ones, in Simplex order
-  const unsigned first_new = s->n;
   const unsigned nS = s->n_prev + n_new;
   const unsigned wcap = nS ? nS : 1;
-  const unsigned wecap = kMaxOthers * wcap;
-  EXT_TRY(s->s_key.ensure(8 * (size_t)wcap));
-  EXT_TRY(s->s_key2.ensure(8 * (size_t)wcap));
-  EXT_TRY(s->s_id.ensure(4 * (size_t)wcap));
-  EXT_TRY(s->s_id2.ensure(4 * (size_t)wcap));
-  EXT_TRY(s->s_hi.ensure(8 * (size_t)wcap));
-  EXT_TRY(s->s_lo.ensure(8 * (size_t)wcap));
-  EXT_TRY(s->s_phase.ensure(4 * (size_t)wcap));
-  EXT_TRY(ctx->hist.ensure(sizeof(unsigned) * 256 * (size_t)ctx->sort_grid(wcap)));
-  const unsigned edge_room = s->n_edges + wecap;
-  if (edge_room > s->edge_cap) {
-    unsigned nc = s->edge_cap ? s->edge_cap : 262144u;
-    while (nc < edge_room) nc *= 2;
-    EXT_TRY(grow_keep(s->edges, 8 * (size_t)s->n_edges, 8 * (size_t)nc, st));
-    s->edge_cap = nc;
-  }
-  const int g = grid_of(wcap, 256, 4096);
   const bool ranked = wcap <= kRankCap2;
-  const unsigned* ids;
-  if (ranked) {
-    const LoadTuple ld{(const unsigned long long*)s->hi.p, (const unsigned long long*)s->lo.p,
-                       (const unsigned*)s->prev_ids.p, s->n_prev, first_new};
-    const StoreTuple<M> sw{ld, (unsigned long long*)s->s_hi.p, (unsigned long long*)s->s_lo.p,
-                           (const unsigned*)s->phase.p, (unsigned*)s->s_phase.p, (unsigned*)s->s_id.p,
-                           (unsigned*)s->parent.p, (unsigned*)s->prev_ids2.p, counters + kSPrev, ns, tnow};
-    EXT_TRY(launch_rank_sort<2>(ld, sw, nullptr, nS, counters + kSWin, ctx->num_sms, st));
-    ids = sw.ids;
-  } else {
+  const bool done = guess && nS <= guess;  // the window that went ahead held it
+  if (!done) {
+    rc = room(wcap);
+    if (rc) return rc;
+  }
+  if (!done && ranked) {
+    EXT_TRY(window({nS, nullptr, nullptr, 0}, wcap));
+    EXT_TRY(stars(wcap));
+  } else if (!done) {
+    EXT_TRY(s->s_key.ensure(8 * (size_t)wcap));
+    EXT_TRY(s->s_key2.ensure(8 * (size_t)wcap));
+    EXT_TRY(s->s_id2.ensure(4 * (size_t)wcap));
+    EXT_TRY(ctx->hist.ensure(sizeof(unsigned) * 256 * (size_t)ctx->sort_grid(wcap)));
+    const int g = grid_of(wcap, 256, 4096);
     set_u32_kernel<<<1, 1, 0, st>>>(counters + kSWin, nS);
     ext_window_build_kernel<<<g, 256, 0, st>>>((const unsigned long long*)s->lo.p, (const unsigned*)s->prev_ids.p,
                                                s->n_prev, first_new, n_new, (unsigned long long*)s->s_key.p,
@@ -1196,34 +1223,27 @@ ftk2b_status push_extruded_t(ftk2b_stream* s) {
                                               (const unsigned long long*)s->lo.p, (const unsigned*)s->phase.p,
                                               (unsigned long long*)s->s_hi.p, (unsigned long long*)s->s_lo.p,
                                               (unsigned*)s->s_phase.p);
-  }
-  ExtFeatures Fs;
-  Fs.hi = (const unsigned long long*)s->s_hi.p;
-  Fs.lo = (const unsigned long long*)s->s_lo.p;
-  Fs.phase = (const unsigned*)s->s_phase.p;
-  Fs.n_ptr = counters + kSWin;
-  Fs.cap = wcap;
-  Fs.vb = kStreamVb;
-  unsigned* err = counters + kCountErr;
-  if (n_new && !ranked)
-    uf_init_range_kernel<<<grid_of(n_new, 256, 4096), 256, 0, st>>>((unsigned*)s->parent.p, first_new, n_new);
-  const ExtStars stars{ids, (unsigned*)s->parent.p, nullptr, (unsigned*)s->edges.p, s->n_edges, s->edge_cap,
-                       counters + kSWinEdges, err};
-  ext_stars_kernel<M><<<grid_of(kStarLanes * (unsigned long long)wcap, 256, 4096), 256, 0, st>>>(X, Fs, stars);
-  if (n_new && !ranked)
-    ext_collect_spatial_kernel<M><<<grid_of(n_new, 256, 4096), 256, 0, st>>>(
+    if (n_new)
+      uf_init_range_kernel<<<grid_of(n_new, 256, 4096), 256, 0, st>>>((unsigned*)s->parent.p, first_new, n_new);
+    EXT_TRY(stars(wcap));
+    if (n_new)
+      ext_collect_spatial_kernel<M><<<grid_of(n_new, 256, 4096), 256, 0, st>>>(
         (const unsigned long long*)s->hi.p, (const unsigned long long*)s->lo.p, first_new, n_new, ns, tnow,
         (unsigned*)s->prev_ids2.p, counters + kSPrev);
-  nl += ranked ? 2 : 6;
+    nl += 5;
+  }
   EXT_TRY(cudaGetLastError());
-  EXT_TRY(cudaMemcpyAsync(ctx->h_counters, counters, sizeof(unsigned) * kNumCounters, cudaMemcpyDeviceToHost, st));
-  EXT_TRY(cudaEventRecord(ctx->ev1, st));
-  EXT_TRY(ctx->sync());
+  if (!done) {
+    EXT_TRY(cudaMemcpyAsync(ctx->h_counters, counters, sizeof(unsigned) * kNumCounters, cudaMemcpyDeviceToHost, st));
+    EXT_TRY(cudaEventRecord(ctx->ev1, st));
+    EXT_TRY(ctx->sync());
+  }
   ctx->launches += nl;
   const unsigned* h = ctx->h_counters;
   if (h[kCountErr] & kErrCofaces) return ext_fail(ctx, FTK2B_UNSUPPORTED, "a base face has more than 8 coface cells");
   if (h[kCountErr] & 1u) return ext_fail(ctx, FTK2B_TIMEOUT, "union-find retry bound reached");
   s->n_edges += h[kSWinEdges];
+  s->last_window = nS;
   s->n_prev = h[kSPrev];
   std::swap(s->prev_ids, s->prev_ids2);
   s->n += n_new;
@@ -1266,7 +1286,7 @@ ftk2b_status result_extruded_t(ftk2b_stream* s, ftk2b_cp_result** out) {
   if (nc <= kRankCap2) {
     const LoadTuple ld{(const unsigned long long*)s->hi.p, (const unsigned long long*)s->lo.p, nullptr, 0u, 0u};
     const StoreTupleOrder so{{(unsigned*)s->s_id.p, inv, cmin}};
-    EXT_TRY(launch_rank_sort<2>(ld, so, nullptr, n, counters + kSWin, ctx->num_sms, st));
+    EXT_TRY(launch_rank_sort<2>(ld, so, RankCount{n, nullptr, nullptr, 0}, nc, counters + kSWin, ctx->num_sms, st));
     perm = so.order.perm;
   } else {
     set_u32_kernel<<<1, 1, 0, st>>>(counters + kSWin, n);

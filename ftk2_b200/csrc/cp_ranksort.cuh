@@ -21,17 +21,28 @@ constexpr int kRankThreads = 512;
 constexpr unsigned kRankCap1 = 24576;  // keys of one word: 192 KB
 constexpr unsigned kRankCap2 = 12288;  // keys of two words
 
+// How many keys there are: `add`, plus *n where n is not null; none when that is
+// more than the launch holds, or *gate (not null) is above gate_max, so that a
+// launch may precede the host's look at the counters.
+struct RankCount {
+  unsigned add;
+  const unsigned* n;
+  const unsigned* gate;
+  unsigned gate_max;
+};
+
 // Keys of W 64-bit words, compared word by word, equal keys by index.
 //   load(i, k)          writes the W words of key i
 //   store(pos, i, k)    called once per key: key i is the pos-th smallest
-// for i < n = min(*n_ptr, cap) (n_ptr null: cap); n is also written to *n_out
-// when that is not null.  Shared memory: W * cap words.
+// for i below the count, which is also written to *n_out when that is not null.
+// Shared memory: W * cap words.
 template <int W, typename Load, typename Store>
 __global__ void __launch_bounds__(kRankThreads, 1)
-    rank_sort_kernel(Load load, Store store, const unsigned* n_ptr, unsigned cap, unsigned* n_out) {
+    rank_sort_kernel(Load load, Store store, RankCount count, unsigned cap, unsigned* n_out) {
   extern __shared__ unsigned long long rank_keys[];
   pdl_enter();
-  const unsigned n = n_ptr ? min(*n_ptr, cap) : cap;
+  const unsigned long long all = (unsigned long long)count.add + (count.n ? *count.n : 0u);
+  const unsigned n = all > cap || (count.gate && *count.gate > count.gate_max) ? 0u : (unsigned)all;
   if (n_out && blockIdx.x == 0 && threadIdx.x == 0) *n_out = n;
   if (blockIdx.x * (kRankThreads / 8) >= n) return;  // no key of this block's
   for (unsigned i = threadIdx.x; i < n; i += kRankThreads) {
@@ -74,7 +85,7 @@ __global__ void __launch_bounds__(kRankThreads, 1)
 }
 
 template <int W, typename Load, typename Store>
-inline cudaError_t launch_rank_sort(const Load& load, const Store& store, const unsigned* n_ptr, unsigned cap,
+inline cudaError_t launch_rank_sort(const Load& load, const Store& store, const RankCount& count, unsigned cap,
                                     unsigned* n_out, int num_sms, cudaStream_t st) {
   auto k = rank_sort_kernel<W, Load, Store>;
   const size_t smem = 8 * (size_t)W * (cap ? cap : 1);
@@ -84,8 +95,8 @@ inline cudaError_t launch_rank_sort(const Load& load, const Store& store, const 
   if (e) return e;
   unsigned grid = (cap + kRankThreads / 8 - 1) / (kRankThreads / 8);
   if (grid > (unsigned)num_sms) grid = (unsigned)num_sms;
-  k<<<grid ? grid : 1, kRankThreads, smem, st>>>(load, store, n_ptr, cap, n_out);
-  return cudaGetLastError();
+  e = launch_pdl(k, grid ? grid : 1, kRankThreads, smem, st, load, store, count, cap, n_out);
+  return e ? e : cudaGetLastError();
 }
 
 }  // namespace ftk2b

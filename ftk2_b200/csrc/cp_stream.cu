@@ -19,6 +19,7 @@
 //   4. the resident union-find over stream ids takes the new edges.
 // The result sorts the store (canonical ids = rank in Simplex order) and
 // labels every component with its smallest canonical id (engine.hpp:46-74).
+#include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
@@ -162,6 +163,27 @@ __global__ void collect_spatial_kernel(const unsigned long long* __restrict__ ke
   }
 }
 
+// One timestep's arrays to their ring slots (grid y: the array) and the
+// counters cleared: a copy node per array and a memset cost 25 us of a push of
+// 3 x 1.6 MB, this launch 6.
+struct RingCopy {
+  const void* src[3];
+  void* dst[3];
+  unsigned long long bytes;  // a multiple of 4
+  unsigned* counters;
+};
+__global__ void ring_copy_kernel(RingCopy c) {
+  const unsigned long long t = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x;
+  const unsigned long long nt = (unsigned long long)gridDim.x * blockDim.x;
+  if (blockIdx.y == 0 && t < kNumCounters) c.counters[t] = 0;
+  const char* src = (const char*)c.src[blockIdx.y];
+  char* dst = (char*)c.dst[blockIdx.y];
+  const bool wide = (((uintptr_t)src | (uintptr_t)dst) & 15) == 0;
+  const unsigned long long n16 = wide ? c.bytes / 16 : 0;
+  for (unsigned long long i = t; i < n16; i += nt) ((uint4*)dst)[i] = __ldcs((const uint4*)src + i);
+  for (unsigned long long i = 4 * n16 + t; i < c.bytes / 4; i += nt) ((unsigned*)dst)[i] = ((const unsigned*)src)[i];
+}
+
 unsigned long long time_chain_mask(int d) {
   // chains (canonical order) whose last vertex mask has the time bit
   const int m = d - 1, full = (1 << d) - 1, tbit = 1 << (d - 1);
@@ -254,11 +276,45 @@ ftk2b_status push_regular(ftk2b_stream* s) {
   if (rc) return rc;
   unsigned ccap = ctx->cand_cap_hint ? ctx->cand_cap_hint : 65536u;
   unsigned n_new = 0;
+  // window: spatial features of layer t-1 plus the new ones, in key order
+  const unsigned first_new = s->n;
+  auto room = [&](unsigned wcap) -> ftk2b_status {
+    S_TRY(ctx, s->s_key2.ensure(8 * (size_t)wcap));
+    S_TRY(ctx, s->s_id2.ensure(4 * (size_t)wcap));
+    S_TRY(ctx, ctx->edge_cnt.ensure(4 * (size_t)wcap));
+    S_TRY(ctx, ctx->edge_slots.ensure(4 * 8 * (size_t)wcap));
+    return ensure_stream_edges(s, 8ull * wcap);
+  };
+  auto window = [&](const RankCount& count, unsigned wcap) -> cudaError_t {
+    LoadWindow ld{(const unsigned long long*)s->key.p, (const unsigned*)s->prev_ids.p, s->n_prev, first_new};
+    StoreWindow sw{ld, (unsigned long long*)s->s_key2.p, (unsigned*)s->s_id2.p, (unsigned*)s->parent.p,
+                   (unsigned*)s->prev_ids2.p, counters + kSPrev, nch, time_chain_mask(d)};
+    cudaError_t e = launch_rank_sort<1>(ld, sw, count, wcap, counters + kSWin, ctx->num_sms, st);
+    if (!e) e = launch_window_star_slots(rm, nch, sw.skey, counters + kSWin, wcap, (unsigned*)ctx->edge_cnt.p,
+                                         (unsigned*)ctx->edge_slots.p, counters + kSWinEdges, st);
+    if (e) return e;
+    append_star_edges_kernel<<<grid_of(8ull * wcap, 256, 4096), 256, 0, st>>>(
+        counters + kSWin, wcap, (const unsigned*)ctx->edge_cnt.p, counters + kSWinEdges,
+        (const unsigned*)ctx->edge_slots.p, sw.sid, (unsigned*)s->parent.p, (unsigned*)s->edges.p, s->n_edges,
+        s->edge_cap, counters + kCountErr);
+    ctx->launches += 4;
+    return cudaGetLastError();
+  };
+  // The window goes ahead of the host's look at the counters when it is no
+  // larger than four times the last one: a push of a few hundred features spends
+  // 20 us of 105 on the wait between its two halves.  The kernels find no
+  // window when it is larger, or when lists overflowed, and it is run again.
+  const unsigned guess = window_guess(s, kRankCap1);
+  if (guess) {
+    rc = room(guess);
+    if (rc) return rc;
+  }
   for (int attempt = 0;; ++attempt) {
     if (attempt == 6) return sfail(ctx, FTK2B_OVERFLOW_RETRY, "stream buffers kept overflowing");
     S_TRY(ctx, ctx->cand_corner.ensure(8 * (size_t)ccap));
     S_TRY(ctx, ctx->cand_chains.ensure(8 * (size_t)ccap));
-    S_TRY(ctx, cudaMemsetAsync(counters, 0, sizeof(unsigned) * kNumCounters, st));
+    if (!s->counters_clear) S_TRY(ctx, cudaMemsetAsync(counters, 0, sizeof(unsigned) * kNumCounters, st));
+    s->counters_clear = false;
     FeatureSink sink;
     sink.key = (unsigned long long*)s->key.p + s->n;
     sink.lam = (double*)s->lam.p + 4 * (size_t)s->n;
@@ -273,8 +329,10 @@ ftk2b_status push_regular(ftk2b_stream* s) {
     cq.cap = ccap;
     if (cfg.cull_mode == 2) {
       int mode = 0;
+      bool timed = false;  // a shape not seen before
       S_TRY(ctx, resolve_cull_mode(ctx, rm, fa, f64, s->layout == FTK2B_LAYOUT_MULTICOMPONENT,
                                    [&](int md) -> cudaError_t {
+                                     timed = true;
                                      ExtractConfig c = cfg;
                                      c.cull_mode = md;
                                      cudaError_t e = cudaMemsetAsync(counters, 0, sizeof(unsigned) * kNumCounters, st);
@@ -287,7 +345,7 @@ ftk2b_status push_regular(ftk2b_stream* s) {
                                    },
                                    &mode));
       cfg.cull_mode = mode;
-      S_TRY(ctx, cudaMemsetAsync(counters, 0, sizeof(unsigned) * kNumCounters, st));
+      if (timed) S_TRY(ctx, cudaMemsetAsync(counters, 0, sizeof(unsigned) * kNumCounters, st));
     }
     ctx->last_cull_mode = cfg.cull_mode;
     int nk = 1;
@@ -295,8 +353,13 @@ ftk2b_status push_regular(ftk2b_stream* s) {
                                       &ctx->last_used_tma, &nk));
     S_TRY(ctx, launch_refine_regular(f64, rm, fa, cfg, cq, sink, ctx->num_sms, st));
     ctx->launches += 1 + nk;
+    if (guess) {
+      const unsigned fits = (unsigned)std::min<unsigned long long>(guess, (unsigned long long)s->n_prev + sink.cap);
+      S_TRY(ctx, window({s->n_prev, counters + kCountFeatures, counters + kCountCand, ccap}, fits));
+    }
     S_TRY(ctx, cudaMemcpyAsync(ctx->h_counters, counters, sizeof(unsigned) * kNumCounters, cudaMemcpyDeviceToHost,
                                st));
+    S_TRY(ctx, cudaEventRecord(ctx->ev1, st));
     S_TRY(ctx, ctx->sync());
     const unsigned* h = ctx->h_counters;
     if (h[kCountErr] & 2u) return sfail(ctx, FTK2B_TIMEOUT, "a TMA slice copy did not complete in time");
@@ -314,39 +377,21 @@ ftk2b_status push_regular(ftk2b_stream* s) {
     break;
   }
 
-  // window: spatial features of layer t-1 plus the new ones, in key order
-  const unsigned first_new = s->n;
   const unsigned nS = s->n_prev + n_new;
   const unsigned wcap = nS ? nS : 1;
-  S_TRY(ctx, s->s_key.ensure(8 * (size_t)wcap));
-  S_TRY(ctx, s->s_key2.ensure(8 * (size_t)wcap));
-  S_TRY(ctx, s->s_id.ensure(4 * (size_t)wcap));
-  S_TRY(ctx, s->s_id2.ensure(4 * (size_t)wcap));
-  S_TRY(ctx, s->wedges.ensure(8 * 8 * (size_t)wcap));
-  S_TRY(ctx, ctx->edge_cnt.ensure(4 * (size_t)wcap));
-  S_TRY(ctx, ctx->edge_slots.ensure(4 * 8 * (size_t)wcap));
-  const int sgrid = ctx->sort_grid(wcap);
-  S_TRY(ctx, ctx->hist.ensure(sizeof(unsigned) * 256 * (size_t)sgrid));
-  const unsigned edge_room = s->n_edges + 8 * nS;
-  if (edge_room > s->edge_cap) {
-    unsigned nc = s->edge_cap ? s->edge_cap : 262144u;
-    while (nc < edge_room) nc *= 2;
-    S_TRY(ctx, grow_keep(s->edges, 8 * (size_t)s->n_edges, 8 * (size_t)nc, st));
-    s->edge_cap = nc;
-  }
-  if (wcap <= kRankCap1) {
-    LoadWindow ld{(const unsigned long long*)s->key.p, (const unsigned*)s->prev_ids.p, s->n_prev, first_new};
-    StoreWindow sw{ld, (unsigned long long*)s->s_key2.p, (unsigned*)s->s_id2.p, (unsigned*)s->parent.p,
-                   (unsigned*)s->prev_ids2.p, counters + kSPrev, nch, time_chain_mask(d)};
-    S_TRY(ctx, launch_rank_sort<1>(ld, sw, nullptr, nS, counters + kSWin, ctx->num_sms, st));
-    S_TRY(ctx, launch_window_star_slots(rm, nch, sw.skey, counters + kSWin, wcap, (unsigned*)ctx->edge_cnt.p,
-                                        (unsigned*)ctx->edge_slots.p, counters + kSWinEdges, st));
-    append_star_edges_kernel<<<grid_of(8ull * wcap, 256, 4096), 256, 0, st>>>(
-        counters + kSWin, wcap, (const unsigned*)ctx->edge_cnt.p, counters + kSWinEdges,
-        (const unsigned*)ctx->edge_slots.p, sw.sid, (unsigned*)s->parent.p, (unsigned*)s->edges.p, s->n_edges,
-        s->edge_cap, counters + kCountErr);
-    ctx->launches += 4;
-  } else {
+  const bool done = guess && nS <= guess;  // the window that went ahead held it
+  if (!done && wcap <= kRankCap1) {
+    rc = room(wcap);
+    if (rc) return rc;
+    S_TRY(ctx, window({nS, nullptr, nullptr, 0}, wcap));
+  } else if (!done) {
+    rc = room(wcap);
+    if (rc) return rc;
+    S_TRY(ctx, s->s_key.ensure(8 * (size_t)wcap));
+    S_TRY(ctx, s->s_id.ensure(4 * (size_t)wcap));
+    S_TRY(ctx, s->wedges.ensure(8 * 8 * (size_t)wcap));
+    const int sgrid = ctx->sort_grid(wcap);
+    S_TRY(ctx, ctx->hist.ensure(sizeof(unsigned) * 256 * (size_t)sgrid));
     const int g = grid_of(wcap, 256, 4096);
     set_u32_kernel<<<1, 1, 0, st>>>(counters + kSWin, nS);
     window_build_kernel<<<g, 256, 0, st>>>((const unsigned long long*)s->key.p, (const unsigned*)s->prev_ids.p,
@@ -395,12 +440,16 @@ ftk2b_status push_regular(ftk2b_stream* s) {
     S_TRY(ctx, classify(first_new, n_new, counters + kCountRoots));
     if (T == 1) S_TRY(ctx, classify(0, s->n_first, counters + kCountRoots));
   }
-  S_TRY(ctx, cudaMemcpyAsync(ctx->h_counters, counters, sizeof(unsigned) * kNumCounters, cudaMemcpyDeviceToHost, st));
-  S_TRY(ctx, cudaEventRecord(ctx->ev1, st));
-  S_TRY(ctx, ctx->sync());
+  if (!done || s->prm.classify) {
+    S_TRY(ctx, cudaMemcpyAsync(ctx->h_counters, counters, sizeof(unsigned) * kNumCounters, cudaMemcpyDeviceToHost,
+                               st));
+    S_TRY(ctx, cudaEventRecord(ctx->ev1, st));
+    S_TRY(ctx, ctx->sync());
+  }
   const unsigned* h = ctx->h_counters;
   if (h[kCountErr] & 1u) return sfail(ctx, FTK2B_TIMEOUT, "union-find retry bound reached");
   s->n_edges += h[kSWinEdges];
+  s->last_window = nS;
   s->n_prev = h[kSPrev];
   std::swap(s->prev_ids, s->prev_ids2);
   s->n += n_new;
@@ -446,7 +495,7 @@ ftk2b_status result_regular(ftk2b_stream* s, ftk2b_cp_result** out) {
   const unsigned* perm;
   if (nc <= kRankCap1) {
     const StoreCanon sc{{(unsigned*)s->s_id.p, inv, cmin}, (unsigned long long*)s->s_key.p};
-    S_TRY(ctx, launch_rank_sort<1>(LoadKey{(const unsigned long long*)s->key.p}, sc, nullptr, n, counters + kSWin,
+    S_TRY(ctx, launch_rank_sort<1>(LoadKey{(const unsigned long long*)s->key.p}, sc, RankCount{n, nullptr, nullptr, 0}, nc, counters + kSWin,
                                    ctx->num_sms, st));
     skeys = sc.skey;
     perm = sc.order.perm;
@@ -506,7 +555,7 @@ ftk2b_status canonical_edges(ftk2b_stream* s, const unsigned* inv, unsigned long
   const unsigned ne = s->n_edges, ec = ne ? ne : 1;
   if (ec <= kRankCap1) {
     S_TRY(ctx, launch_rank_sort<1>(LoadCanonEdge{(const unsigned*)s->edges.p, inv}, StoreEdge{(unsigned*)ctx->edges.p},
-                                   nullptr, ne, counters + kSWinEdges, ctx->num_sms, st));
+                                   RankCount{ne, nullptr, nullptr, 0}, ec, counters + kSWinEdges, ctx->num_sms, st));
     ctx->launches += 1;
     return FTK2B_OK;
   }
@@ -566,6 +615,23 @@ cudaError_t grow_keep(DevBuf& b, size_t used, size_t want, cudaStream_t st) {
   b.st = st;
   ++b.generation;
   return cudaSuccess;
+}
+
+ftk2b_status ensure_stream_edges(ftk2b_stream* s, unsigned long long more) {
+  const unsigned long long want = s->n_edges + more;
+  if (want <= s->edge_cap) return FTK2B_OK;
+  if (want > 0x7FFFFFFFull) return sfail(s->ctx, FTK2B_UNSUPPORTED, "more than 2^31 - 1 stream edges");
+  unsigned nc = s->edge_cap ? s->edge_cap : 262144u;
+  while (nc < want) nc *= 2;
+  S_TRY(s->ctx, grow_keep(s->edges, 8 * (size_t)s->n_edges, 8 * (size_t)nc, s->ctx->stream));
+  s->edge_cap = nc;
+  return FTK2B_OK;
+}
+
+unsigned window_guess(const ftk2b_stream* s, unsigned most) {
+  if (!s->T) return 0;
+  const unsigned long long g = 4ull * s->last_window + 1024;
+  return g < most ? (unsigned)g : most;
 }
 
 ftk2b_status ensure_stream_store(ftk2b_stream* s, unsigned want) {
@@ -717,8 +783,31 @@ extern "C" ftk2b_status ftk2b_stream_push(ftk2b_stream* s, const ftk2b_field_des
   const int narr = s->layout == FTK2B_LAYOUT_MULTICOMPONENT ? 1 : s->m;
   const size_t bytes = s->slice_elems * s->es;
   const size_t slot = (size_t)(s->T & 1);
-  for (int j = 0; j < narr; ++j) {
+  for (int j = 0; j < narr; ++j)
     if (!step->comp[j]) return sfail(ctx, FTK2B_INVALID_ARG, "component array %d is null", j);
+  // arrays in this device's memory: one launch for all and for the counters
+  s->counters_clear = false;
+  bool here = step->location == FTK2B_DEVICE && ctx->counters.ensure(sizeof(unsigned) * kNumCounters) == cudaSuccess;
+  RingCopy rc_args;
+  memset(&rc_args, 0, sizeof(rc_args));
+  for (int j = 0; j < narr && here; ++j) {
+    cudaPointerAttributes at;
+    here = cudaPointerGetAttributes(&at, step->comp[j]) == cudaSuccess && at.type == cudaMemoryTypeDevice &&
+           at.device == ctx->device && (uintptr_t)step->comp[j] % s->es == 0;
+    rc_args.src[j] = step->comp[j];
+    rc_args.dst[j] = (char*)s->ring[j].p + slot * bytes;
+  }
+  if (here) {
+    rc_args.bytes = bytes;
+    rc_args.counters = (unsigned*)ctx->counters.p;
+    ring_copy_kernel<<<dim3(grid_of(bytes / 16 + 1, 256, 4 * ctx->num_sms), narr), 256, 0, st>>>(rc_args);
+    S_TRY(ctx, cudaGetLastError());
+    ctx->launches += 1;
+    s->counters_clear = true;
+  } else {
+    cudaGetLastError();  // a pointer the driver does not know
+  }
+  for (int j = 0; j < narr && !here; ++j) {
     S_TRY(ctx, cudaMemcpyAsync((char*)s->ring[j].p + slot * bytes, step->comp[j], bytes,
                                step->location == FTK2B_DEVICE ? cudaMemcpyDeviceToDevice : cudaMemcpyHostToDevice,
                                st));

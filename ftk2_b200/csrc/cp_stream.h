@@ -39,6 +39,8 @@ struct ftk2b_stream {
 
   double last_ms = 0;
   unsigned last_new = 0;
+  unsigned last_window = 0;    // features of the last push's window
+  bool counters_clear = false; // the step's copy cleared the context's counters
 };
 
 namespace ftk2b {
@@ -47,6 +49,11 @@ namespace ftk2b {
 cudaError_t grow_keep(DevBuf& b, size_t used, size_t want, cudaStream_t st);
 // grows the feature store (and union-find / boundary lists) to hold `want`
 ftk2b_status ensure_stream_store(ftk2b_stream* s, unsigned want);
+// room for `more` edges after the stored ones
+ftk2b_status ensure_stream_edges(ftk2b_stream* s, unsigned long long more);
+// the largest window (at most `most`) that goes ahead of the host's look at the
+// counters; 0: none
+unsigned window_guess(const ftk2b_stream* s, unsigned most);
 // the store's star edges in canonical ids (inv: canonical id of a stream id),
 // sorted, to the context's edges; k0, k1: scratch of one key per edge
 ftk2b_status canonical_edges(ftk2b_stream* s, const unsigned* inv, unsigned long long* k0, unsigned long long* k1);

@@ -45,3 +45,31 @@ def test_extruded_triangles(ctx, nt):
                       cells=tri.astype(np.uint64), n_layers=nt - 1)
     r = ts.ext_stream_case(ctx, case, check_every=True)
     ts.assert_identical(r, oracle_run(case))
+
+
+@pytest.mark.parametrize("kind", ["regular", "extruded"])
+@pytest.mark.parametrize("loud", [(3, 7), (2, 3, 9)])
+def test_windows_of_sudden_size(ctx, kind, loud):
+    """Steps without features between noisy ones: windows far larger than four
+    times the last, which are run again, and empty ones."""
+    nt = 11
+    rng = np.random.default_rng(10)
+    if kind == "regular":
+        dims = [19, 17, nt]
+        v = rng.standard_normal((nt, 17, 19, 2))
+    else:
+        coords, tets = S.extruded_tet_mesh(9, 8, 5, seed=2)
+        v = rng.standard_normal((nt, coords.shape[0], 3))
+    quiet = [t for t in range(nt) if t not in loud]
+    v[quiet] = np.abs(v[quiet]) + 0.1
+    if kind == "regular":
+        case = cases.Case("sudden", "regular", 2, cases.MULTI, v, 2.0 ** 20, dims)
+        r = ts.stream_case(ctx, case, classify=True, check_every=True)
+    else:
+        arrays = [np.ascontiguousarray(v[..., j].ravel()) for j in range(3)]
+        case = cases.Case("sudden", "extruded", 3, cases.PER_VERTEX, arrays, 2.0 ** 20, coords=coords, cells=tets,
+                          n_layers=nt - 1)
+        r = ts.ext_stream_case(ctx, case, check_every=True)
+    o = oracle_run(case)
+    assert len(o.track_id) > 1200
+    ts.assert_identical(r, o)
