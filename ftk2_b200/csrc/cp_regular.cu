@@ -215,12 +215,42 @@ __device__ __forceinline__ void flush_candidates(const unsigned long long* cbuf,
   __syncthreads();
   if (threadIdx.x == 0) ccount[0] = 0;
   const unsigned cbase = ccount[1];
-  for (unsigned i = threadIdx.x; i < nc; i += kThreads) {
+  for (unsigned i = threadIdx.x; i < nc; i += blockDim.x) {
     const unsigned gi = cbase + i;
     if (gi < cq.cap) {
       cq.corner[gi] = cbuf[2 * i];
       cq.chains[gi] = cbuf[2 * i + 1];
       if (cq.field) cq.field[gi] = field_id;
+    }
+  }
+}
+
+// A surviving hypercube with every chain that fits in the mesh (the exact-test
+// kernel applies the per-simplex word test): entry idx of the block's buffer,
+// or straight to the queue.
+template <int D>
+__device__ __forceinline__ void keep_corner(const RegularMesh& mesh, const ExtractConfig& cfg, const CandidateQueue& cq,
+                                            unsigned long long* cbuf, unsigned idx, int l0, int l1, int l2, int ct) {
+  constexpr int TBIT = 1 << (D - 1);  // mask bit of the time axis
+  int vmask = 0;                      // axes along which the corner can step by +1
+  if (l0 + 1 < (int)mesh.ld[0]) vmask |= 1;
+  if (l1 + 1 < (int)mesh.ld[1]) vmask |= 2;
+  if (D == 4 && l2 + 1 < (int)mesh.ld[2]) vmask |= 4;
+  if (ct + 1 < (int)mesh.ld[D - 1]) vmask |= TBIT;
+  const unsigned long long corner = pack_corner(l0, l1, (D == 4) ? l2 : 0, ct);
+  unsigned long long ch = c_chains_by_vmask[D - 3][vmask];
+  // a stream's window starts one slice before the new timestep: the
+  // purely spatial simplices of that slice were counted already
+  if (cfg.skip_first_spatial && ct == 0) ch &= c_time_chains[D - 3];
+  if (idx < kCandBuf) {
+    cbuf[2 * idx] = corner;
+    cbuf[2 * idx + 1] = ch;
+  } else {
+    const unsigned gi = atomicAdd(cq.count, 1u);
+    if (gi < cq.cap) {
+      cq.corner[gi] = corner;
+      cq.chains[gi] = ch;
+      if (cq.field) cq.field[gi] = cq.field_id;
     }
   }
 }
@@ -253,7 +283,6 @@ __device__ __forceinline__ bool cull_tile(const CUtensorMap* map0, const CUtenso
   constexpr int M = D - 1;
   constexpr int TX = G::TX, TY = G::TY, TZ = G::TZ;
   constexpr int VX = G::VX, VY = G::VY, VZ = G::VZ, VS = G::VS, VPT = G::VPT, VSP = G::VSP;
-  constexpr int TBIT = 1 << (D - 1);  // mask bit of the time axis
   constexpr int HW = sizeof(T) / 4;   // the high 32-bit word of an element is its last
   static_assert(D == 3 ? kWarps * kRows >= TY : kWarps == TY * (TZ / kRows),
                 "every corner row of the tile belongs to exactly one warp");
@@ -610,36 +639,13 @@ __device__ __forceinline__ bool cull_tile(const CUtensorMap* map0, const CUtenso
       const bool keep = ((row_valid >> q) & 1u) && !word_culled(R[q] & R[q + 1]);
       const unsigned ball = __ballot_sync(0xFFFFFFFFu, keep);
       if (ball) {
-        // surviving hypercubes are queued with every chain that fits in the
-        // mesh (the exact-test kernel applies the per-simplex word test),
         // first into the block's buffer
         unsigned basei = 0;
         if (lane == 0) basei = atomicAdd(ccount, (unsigned)__popc(ball));
         basei = __shfl_sync(0xFFFFFFFFu, basei, 0);
         if (keep) {
           const unsigned idx = basei + __popc(ball & ((1u << lane) - 1));
-          const int l0 = x0 + lane, l1 = y0 + cy, l2 = (D == 4) ? z0 + cz : ct;
-          int vmask = 0;  // axes along which the corner can step by +1
-          if (l0 + 1 < ldx) vmask |= 1;
-          if (l1 + 1 < ldy) vmask |= 2;
-          if (D == 4 && l2 + 1 < ldz) vmask |= 4;
-          if (ct + 1 < lt) vmask |= TBIT;
-          const unsigned long long corner = pack_corner(l0, l1, (D == 4) ? l2 : 0, ct);
-          unsigned long long ch = c_chains_by_vmask[D - 3][vmask];
-          // a stream's window starts one slice before the new timestep: the
-          // purely spatial simplices of that slice were counted already
-          if (cfg.skip_first_spatial && ct == 0) ch &= c_time_chains[D - 3];
-          if (idx < kCandBuf) {
-            cbuf[2 * idx] = corner;
-            cbuf[2 * idx + 1] = ch;
-          } else {
-            const unsigned gi = atomicAdd(cq.count, 1u);
-            if (gi < cq.cap) {
-              cq.corner[gi] = corner;
-              cq.chains[gi] = ch;
-              if (cq.field) cq.field[gi] = cq.field_id;
-            }
-          }
+          keep_corner<D>(mesh, cfg, cq, cbuf, idx, x0 + lane, y0 + cy, (D == 4) ? z0 + cz : ct, ct);
         }
       }
     }
@@ -683,6 +689,114 @@ __global__ void __launch_bounds__(kThreads, 2)
   cull_tile<T, D, MULTI, TMA>(&map0, &map1, &map2, mesh, fa, cfg, cq, err, (int)blockIdx.x, (int)blockIdx.y, smem,
                               bar, band_tbl, ph, reinterpret_cast<unsigned long long*>(smem + G::CAND),
                               reinterpret_cast<unsigned*>(smem + G::CAND + 16 * kCandBuf), false, 0u);
+}
+
+// Stage 1 of 2D+t meshes (cull mode 0): a warp marches a strip of 31 x kStripRows
+// corners through the time steps of its chunk.  A lane holds one column: the
+// words of the previous slice stay in its registers, the next slice's values are
+// in flight meanwhile, its right neighbour's words come by a shuffle.  Values
+// are read straight from the arrays (of a double only the high word), so every
+// layout, stride and alignment takes the same path and no step waits for a
+// block.  Bound by issue: some 60 instructions a vertex, 150 with the slice
+// staged in shared memory.  1021 x 765 x 12 float in two arrays: 62.5 -> 36 us
+// (8 rows a strip, fewer vertices computed twice but half the warps: 39.5); 64 x
+// 64 x 10 double: 11.6 -> 4.  Chunks are long where strips alone give
+// kStripsWanted warps (a chunk's first slice is read twice) and short where they
+// do not (fewer steps in sequence); 32 to 128 warps an SM measure alike.
+constexpr int kStripRows = 4;
+constexpr int kStripWarps = 8;             // warps a block
+constexpr int kStripsWanted = 64 * 148;    // warps of the launch, at least where the mesh has them
+
+template <typename T>
+__global__ void __launch_bounds__(kStripWarps * 32, 3) strip_cull_kernel(RegularMesh mesh, FieldAccess fa,
+                                                                      ExtractConfig cfg, CandidateQueue cq,
+                                                                      int strips_x, int strips_y, int tchunk,
+                                                                      unsigned n_warps) {
+  constexpr int M = 2, R = kStripRows;
+  __shared__ unsigned band_tbl[kBandTable];
+  __shared__ unsigned long long cbuf[2 * kCandBuf];
+  __shared__ unsigned ccount[2];
+  fill_band_table<T>(band_tbl, threadIdx.x, kStripWarps * 32);
+  if (threadIdx.x == 0) ccount[0] = 0;
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  const unsigned w = blockIdx.x * kStripWarps + (threadIdx.x >> 5);
+  if (w < n_warps) {
+    const int sx = (int)(w % (unsigned)strips_x);
+    const unsigned wr = w / (unsigned)strips_x;
+    const int sy = (int)(wr % (unsigned)strips_y), chunk = (int)(wr / (unsigned)strips_y);
+    const int x = sx * 31 + lane, y0 = sy * R;
+    const int ldx = (int)mesh.ld[0], ldy = (int)mesh.ld[1], lt = (int)mesh.ld[2];
+    const int t0 = chunk * tchunk, t1 = min(t0 + tchunk, lt);
+    const int s_end = min(t1, lt - 1);  // last vertex slice this warp reads
+    // element strides and the array coordinates of local (0, 0, 0); per-vertex
+    // arrays are indexed by global vertex id
+    long long es[3], off[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+      es[k] = (fa.per_vertex ? (long long)mesh.gstride[k] : fa.estride[k]) * (long long)sizeof(T);
+      off[k] = fa.per_vertex ? mesh.off[k] : mesh.off[k] - fa.shift[k];
+    }
+    const int flip = fa.per_vertex ? 0 : fa.tflip;
+    const bool xin = x < ldx;
+    // a lane outside the mesh reads its row's last vertex and has absent words
+    const long long o0 = (min(x, ldx - 1) + off[0]) * es[0] + (y0 + off[1]) * es[1] + (long long)sizeof(T) - 4;
+    const char* base[M] = {static_cast<const char*>(fa.comp[0]) + o0, static_cast<const char*>(fa.comp[1]) + o0};
+    unsigned h[R + 1][M];
+    auto load = [&](int s) {
+      const long long ot = ((long long)((int)(s + off[2]) ^ flip)) * es[2];
+#pragma unroll
+      for (int r = 0; r <= R; ++r) {
+        const long long o = ot + min(r, ldy - 1 - y0) * es[1];
+#pragma unroll
+        for (int j = 0; j < M; ++j) h[r][j] = __ldg(reinterpret_cast<const unsigned*>(base[j] + o));
+      }
+    };
+    auto words = [&](unsigned (&v)[R + 1]) {
+#pragma unroll
+      for (int r = 0; r <= R; ++r)
+        v[r] = vertex_word_hi<T, M>(h[r], band_tbl) | (xin && y0 + r < ldy ? 0u : kAbsent);
+    };
+    unsigned prev[R + 1], cur[R + 1];
+    load(t0);
+    words(prev);
+    if (t0 + 1 <= s_end) load(t0 + 1);
+    for (int ct = t0; ct < t1; ++ct) {
+      const int s = ct + 1;
+      if (s <= s_end) {
+        words(cur);
+        if (s + 1 <= s_end) load(s + 1);
+      } else {  // no slice after the last one: the step's words are slice ct's
+#pragma unroll
+        for (int r = 0; r <= R; ++r) cur[r] = prev[r];
+      }
+      unsigned pair[R + 1];  // AND over the column's and its right neighbour's vertices of both slices
+#pragma unroll
+      for (int r = 0; r <= R; ++r) {
+        const unsigned v = prev[r] & cur[r];
+        pair[r] = v & __shfl_down_sync(0xFFFFFFFFu, v, 1);
+        prev[r] = cur[r];
+      }
+      unsigned kept = 0;
+#pragma unroll
+      for (int r = 0; r < R; ++r) kept |= (word_culled(pair[r] & pair[r + 1]) ? 0u : 1u) << r;
+      if (lane == 31 || !xin) kept = 0;
+      if (ldy - y0 < R) kept &= (1u << (ldy - y0)) - 1u;
+      if (__any_sync(0xFFFFFFFFu, kept != 0)) {
+#pragma unroll 1
+        for (int r = 0; r < R; ++r) {
+          const unsigned ball = __ballot_sync(0xFFFFFFFFu, (kept >> r) & 1u);
+          if (!ball) continue;
+          unsigned at = 0;
+          if (lane == 0) at = atomicAdd(ccount, (unsigned)__popc(ball));
+          at = __shfl_sync(0xFFFFFFFFu, at, 0) + __popc(ball & ((1u << lane) - 1));
+          if ((kept >> r) & 1u) keep_corner<3>(mesh, cfg, cq, cbuf, at, x, y0 + r, 0, ct);
+        }
+      }
+    }
+  }
+  __syncthreads();
+  flush_candidates(cbuf, ccount, cq, cq.field_id);
 }
 
 // ---------------------------------------------------------------------------
@@ -2581,6 +2695,18 @@ static cudaError_t launch_t(const RegularMesh& mesh, const FieldAccess& fa, cons
     return cudaGetLastError();
   }
   if (launches) *launches = 1;
+  if (D == 3 && cfg.stall_polls == 0) {  // the failure-path check lives in the staged form
+    if (used_tma) *used_tma = 0;
+    const long long sx = (mesh.ld[0] + 30) / 31, sy = (mesh.ld[1] + kStripRows - 1) / kStripRows;
+    long long nch = std::min<long long>(lt, (kStripsWanted + sx * sy - 1) / (sx * sy));
+    if (cfg.tchunk < lt) nch = std::max<long long>(nch, nchunks);  // the caller's chunk length
+    const long long tchunk = (lt + nch - 1) / nch;
+    nch = (lt + tchunk - 1) / tchunk;
+    const unsigned warps = (unsigned)(sx * sy * nch);
+    strip_cull_kernel<T><<<(warps + kStripWarps - 1) / kStripWarps, kStripWarps * 32, 0, st>>>(
+        mesh, fa, cfg, cq, (int)sx, (int)sy, (int)tchunk, warps);
+    return cudaGetLastError();
+  }
   if (tma) {
     auto k = extract_regular_kernel<T, D, MULTI, true>;
     e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
