@@ -679,7 +679,7 @@ __device__ __forceinline__ void star_edges_warp(const RegularMesh& mesh, int nch
                                                 unsigned* __restrict__ cnt, unsigned* __restrict__ slots,
                                                 unsigned* parent, unsigned* err,
                                                 const unsigned long long* sample = nullptr, unsigned ns = 0,
-                                                int slog = 0) {
+                                                int slog = 0, const WindowStars* win = nullptr) {
   const int d = mesh.d, m = d - 1, full = (1 << d) - 1;
   unsigned long long rem;
   unsigned long long vid = divmod_u64(local_key, (unsigned long long)nch, rem);
@@ -779,6 +779,21 @@ __device__ __forceinline__ void star_edges_warp(const RegularMesh& mesh, int nch
   // cells share only the feature), so each lane's slot is its rank among them
   const bool valid = idx >= 0 && (q ? qual[1] : qual[0]) && (unsigned)idx != i;
   const unsigned vm = __ballot_sync(0xFFFFFFFFu, valid);
+  if (win) {  // a stream's window: as stream ids, in any order
+    if (!vm) return;
+    unsigned at = 0;
+    if (lane == 0) at = atomicAdd(win->n_edges, (unsigned)__popc(vm));
+    at = __shfl_sync(0xFFFFFFFFu, at, 0) + __popc(vm & ((1u << lane) - 1));
+    if (valid) {
+      const unsigned a = win->ids[i], b = win->ids[idx];
+      if (at < win->cap - win->base) {
+        win->pairs[2 * (size_t)(win->base + at)] = a;
+        win->pairs[2 * (size_t)(win->base + at) + 1] = b;
+      }
+      uf_unite(win->parent, a, b, err);
+    }
+    return;
+  }
   unsigned rk = 0;
   for (unsigned b = vm; b; b &= b - 1) {
     const unsigned o = __shfl_sync(0xFFFFFFFFu, (unsigned)idx, __ffs(b) - 1);
@@ -789,6 +804,28 @@ __device__ __forceinline__ void star_edges_warp(const RegularMesh& mesh, int nch
     if (parent) uf_unite(parent, i, (unsigned)idx, err);
   }
   if (lane == 0) cnt[i] = __popc(vm);
+}
+
+// A stream's window: one warp per feature; its star edges go straight to the
+// store and the union-find.  Finding them, scanning their counts and appending
+// them were three launches (16 us of a push's 92 for some 300 features, now
+// 10).  Windows of up to kWindowKeys features are searched in shared memory.
+constexpr unsigned kWindowKeys = 2048;
+__global__ void __launch_bounds__(256) window_stars_kernel(RegularMesh mesh, int nch,
+                                                           const unsigned long long* __restrict__ keys,
+                                                           const unsigned* n_ptr, unsigned cap, WindowStars win) {
+  __shared__ StarTables T;
+  __shared__ unsigned long long s_key[kWindowKeys];
+  const unsigned n = min(*n_ptr, cap), warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  if (blockIdx.x * nw >= n) return;  // no feature of this block's
+  fill_star_tables(T, mesh.d);
+  if (n <= kWindowKeys)
+    for (unsigned k = threadIdx.x; k < n; k += blockDim.x) s_key[k] = keys[k];
+  __syncthreads();
+  const unsigned long long* const in = n <= kWindowKeys ? s_key : keys;
+  for (unsigned i = blockIdx.x * nw + warp; i < n; i += gridDim.x * nw)
+    star_edges_warp(mesh, nch, in, n, i, in[i], 0ull, T, threadIdx.x & 31, nullptr, nullptr, nullptr, win.err, nullptr,
+                    0, 0, &win);
 }
 
 // Batches: one warp per feature (the short chain's star_edges_warp with the
@@ -1134,24 +1171,9 @@ cudaError_t launch_uf_label(unsigned* parent, const unsigned* n_ptr, unsigned ca
   return cudaGetLastError();
 }
 
-cudaError_t launch_window_star_slots(const RegularMesh& mesh, int nch, const unsigned long long* skeys,
-                                     const unsigned* n_ptr, unsigned cap, unsigned* edge_cnt, unsigned* edge_slots,
-                                     unsigned* n_edges, cudaStream_t st) {
-  edges_regular_warp_kernel<<<grid_for(cap, 8, 8192), 256, 0, st>>>(mesh, nch, skeys, n_ptr, cap, edge_cnt,
-                                                                   edge_slots);
-  scan_inplace_kernel<<<1, 1024, 0, st>>>(edge_cnt, cap, n_edges, n_ptr, nullptr);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_window_edges_regular(const RegularMesh& mesh, int nch, const unsigned long long* skeys,
-                                        const unsigned* n_ptr, unsigned cap, unsigned* edge_cnt,
-                                        unsigned* edge_slots, unsigned* edges, unsigned* n_edges,
-                                        unsigned edge_cap, cudaStream_t st) {
-  const int g = grid_for(cap, 256, 4096);
-  const cudaError_t e =
-      launch_window_star_slots(mesh, nch, skeys, n_ptr, cap, edge_cnt, edge_slots, n_edges, st);
-  if (e) return e;
-  edges_compact_kernel<<<g, 256, 0, st>>>(n_ptr, cap, edge_cnt, n_edges, edge_slots, edges, edge_cap);
+cudaError_t launch_window_stars(const RegularMesh& mesh, int nch, const unsigned long long* skeys,
+                                const unsigned* n_ptr, unsigned cap, const WindowStars& win, cudaStream_t st) {
+  window_stars_kernel<<<grid_for(cap, 8, 8192), 256, 0, st>>>(mesh, nch, skeys, n_ptr, cap, win);
   return cudaGetLastError();
 }
 

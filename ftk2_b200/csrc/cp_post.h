@@ -66,17 +66,20 @@ cudaError_t launch_uf(unsigned* parent, const unsigned* n_ptr, unsigned cap, con
 // track[i] = root of i (the component's smallest index), roots counted
 cudaError_t launch_uf_label(unsigned* parent, const unsigned* n_ptr, unsigned cap,
                             unsigned long long* track, unsigned* n_roots, cudaStream_t st);
-// star edges as launch_window_edges_regular finds them, left in 8 padded slots
-// per feature with the scanned counts in edge_cnt and their sum in *n_edges
-cudaError_t launch_window_star_slots(const RegularMesh& mesh, int nch, const unsigned long long* skeys,
-                                     const unsigned* n_ptr, unsigned cap, unsigned* edge_cnt, unsigned* edge_slots,
-                                     unsigned* n_edges, cudaStream_t st);
+// Where the star edges of a stream's window go: pairs of stream ids (centre,
+// other) in any order from row `base` on, counted in *n_edges and joined.
+struct WindowStars {
+  const unsigned* ids;  // stream id of each sorted window feature
+  unsigned* parent;
+  unsigned* pairs;
+  unsigned base, cap;   // rows
+  unsigned* n_edges;
+  unsigned* err;
+};
 // star edges of the top cells of `mesh` (a window of the full mesh) among the
-// sorted keys, as (centre, other) index pairs, sorted; count in *n_edges
-cudaError_t launch_window_edges_regular(const RegularMesh& mesh, int nch, const unsigned long long* skeys,
-                                        const unsigned* n_ptr, unsigned cap, unsigned* edge_cnt,
-                                        unsigned* edge_slots, unsigned* edges, unsigned* n_edges,
-                                        unsigned edge_cap, cudaStream_t st);
+// sorted keys
+cudaError_t launch_window_stars(const RegularMesh& mesh, int nch, const unsigned long long* skeys,
+                                const unsigned* n_ptr, unsigned cap, const WindowStars& win, cudaStream_t st);
 // vertex ids (and, when bary is not null, float barycentrics) of keys
 cudaError_t launch_expand_regular(const RegularMesh& mesh, int nch, const unsigned long long* keys,
                                   const unsigned* n_ptr, unsigned cap, const float* bary4,

@@ -119,40 +119,6 @@ struct StoreCanon {
   }
 };
 
-// The window's star edges, from their padded slots (off: scanned counts), as
-// stream ids: united and appended to the store's edges.
-__global__ void append_star_edges_kernel(const unsigned* n_ptr, unsigned cap, const unsigned* __restrict__ off,
-                                         const unsigned* n_edges, const unsigned* __restrict__ slots,
-                                         const unsigned* __restrict__ s_id, unsigned* parent,
-                                         unsigned* __restrict__ out, unsigned base, unsigned out_cap, unsigned* err) {
-  const unsigned n = min(*n_ptr, cap), ne = *n_edges;
-  // a thread per slot: the lanes of a feature unite side by side
-  for (unsigned t = blockIdx.x * blockDim.x + threadIdx.x; t < 8 * n; t += gridDim.x * blockDim.x) {
-    const unsigned i = t >> 3, k = t & 7, o = off[i];
-    if (k >= (i + 1 < n ? off[i + 1] : ne) - o) continue;
-    const unsigned a = s_id[i], b = s_id[slots[t]];
-    if (o + k < out_cap - base) {
-      out[2 * (size_t)(base + o + k)] = a;
-      out[2 * (size_t)(base + o + k) + 1] = b;
-    }
-    uf_unite(parent, a, b, err);
-  }
-}
-
-__global__ void append_edges_kernel(const unsigned* __restrict__ wedges, const unsigned* wn_ptr, unsigned wcap,
-                                    const unsigned* __restrict__ s_id, unsigned* parent, unsigned* __restrict__ out,
-                                    unsigned base, unsigned out_cap, unsigned* err) {
-  const unsigned wn = min(*wn_ptr, wcap);
-  for (unsigned e = blockIdx.x * blockDim.x + threadIdx.x; e < wn; e += gridDim.x * blockDim.x) {
-    const unsigned a = s_id[wedges[2 * (size_t)e]], b = s_id[wedges[2 * (size_t)e + 1]];
-    uf_unite(parent, a, b, err);
-    if (base + e < out_cap) {
-      out[2 * (size_t)(base + e)] = a;
-      out[2 * (size_t)(base + e) + 1] = b;
-    }
-  }
-}
-
 __global__ void collect_spatial_kernel(const unsigned long long* __restrict__ key, unsigned first_new,
                                        unsigned n_new, int nch, unsigned long long time_chains,
                                        unsigned* __restrict__ prev, unsigned* prev_n) {
@@ -281,24 +247,20 @@ ftk2b_status push_regular(ftk2b_stream* s) {
   auto room = [&](unsigned wcap) -> ftk2b_status {
     S_TRY(ctx, s->s_key2.ensure(8 * (size_t)wcap));
     S_TRY(ctx, s->s_id2.ensure(4 * (size_t)wcap));
-    S_TRY(ctx, ctx->edge_cnt.ensure(4 * (size_t)wcap));
-    S_TRY(ctx, ctx->edge_slots.ensure(4 * 8 * (size_t)wcap));
     return ensure_stream_edges(s, 8ull * wcap);
+  };
+  auto stars = [&](const unsigned long long* skey, const unsigned* sid, unsigned wcap) -> cudaError_t {
+    const WindowStars win{sid, (unsigned*)s->parent.p, (unsigned*)s->edges.p, s->n_edges, s->edge_cap,
+                          counters + kSWinEdges, counters + kCountErr};
+    return launch_window_stars(rm, nch, skey, counters + kSWin, wcap, win, st);
   };
   auto window = [&](const RankCount& count, unsigned wcap) -> cudaError_t {
     LoadWindow ld{(const unsigned long long*)s->key.p, (const unsigned*)s->prev_ids.p, s->n_prev, first_new};
     StoreWindow sw{ld, (unsigned long long*)s->s_key2.p, (unsigned*)s->s_id2.p, (unsigned*)s->parent.p,
                    (unsigned*)s->prev_ids2.p, counters + kSPrev, nch, time_chain_mask(d)};
     cudaError_t e = launch_rank_sort<1>(ld, sw, count, wcap, counters + kSWin, ctx->num_sms, st);
-    if (!e) e = launch_window_star_slots(rm, nch, sw.skey, counters + kSWin, wcap, (unsigned*)ctx->edge_cnt.p,
-                                         (unsigned*)ctx->edge_slots.p, counters + kSWinEdges, st);
-    if (e) return e;
-    append_star_edges_kernel<<<grid_of(8ull * wcap, 256, 4096), 256, 0, st>>>(
-        counters + kSWin, wcap, (const unsigned*)ctx->edge_cnt.p, counters + kSWinEdges,
-        (const unsigned*)ctx->edge_slots.p, sw.sid, (unsigned*)s->parent.p, (unsigned*)s->edges.p, s->n_edges,
-        s->edge_cap, counters + kCountErr);
-    ctx->launches += 4;
-    return cudaGetLastError();
+    ctx->launches += 2;
+    return e ? e : stars(sw.skey, sw.sid, wcap);
   };
   // The window goes ahead of the host's look at the counters when it is no
   // larger than four times the last one: a push of a few hundred features spends
@@ -389,7 +351,6 @@ ftk2b_status push_regular(ftk2b_stream* s) {
     if (rc) return rc;
     S_TRY(ctx, s->s_key.ensure(8 * (size_t)wcap));
     S_TRY(ctx, s->s_id.ensure(4 * (size_t)wcap));
-    S_TRY(ctx, s->wedges.ensure(8 * 8 * (size_t)wcap));
     const int sgrid = ctx->sort_grid(wcap);
     S_TRY(ctx, ctx->hist.ensure(sizeof(unsigned) * 256 * (size_t)sgrid));
     const int g = grid_of(wcap, 256, 4096);
@@ -404,18 +365,13 @@ ftk2b_status push_regular(ftk2b_stream* s) {
                                 key_bits, (unsigned*)ctx->hist.p, sgrid, st, &ctx->launches);
     const unsigned long long* skeys = (const unsigned long long*)(alt ? s->s_key2.p : s->s_key.p);
     const unsigned* sids = (const unsigned*)(alt ? s->s_id2.p : s->s_id.p);
-    S_TRY(ctx, launch_window_edges_regular(rm, nch, skeys, counters + kSWin, wcap, (unsigned*)ctx->edge_cnt.p,
-                                           (unsigned*)ctx->edge_slots.p, (unsigned*)s->wedges.p,
-                                           counters + kSWinEdges, 8 * wcap, st));
     if (n_new) uf_init_range_kernel<<<grid_of(n_new, 256, 4096), 256, 0, st>>>((unsigned*)s->parent.p, first_new, n_new);
-    append_edges_kernel<<<grid_of(8ull * wcap, 256, 4096), 256, 0, st>>>(
-        (const unsigned*)s->wedges.p, counters + kSWinEdges, 8 * wcap, sids, (unsigned*)s->parent.p,
-        (unsigned*)s->edges.p, s->n_edges, s->edge_cap, counters + kCountErr);
+    S_TRY(ctx, stars(skeys, sids, wcap));
     if (n_new)
       collect_spatial_kernel<<<grid_of(n_new, 256, 4096), 256, 0, st>>>(
           (const unsigned long long*)s->key.p, first_new, n_new, nch, time_chain_mask(d), (unsigned*)s->prev_ids2.p,
           counters + kSPrev);
-    ctx->launches += 8;
+    ctx->launches += 5;
   }
 
   // classification while the window's values are resident: the new features,
@@ -747,7 +703,7 @@ extern "C" ftk2b_status ftk2b_stream_open(ftk2b_ctx* ctx, const ftk2b_mesh_desc*
   }
   for (DevBuf* b : {&s->ring[0], &s->ring[1], &s->ring[2], &s->key, &s->hi, &s->lo, &s->phase, &s->lam,
                     &s->bary4, &s->scalar, &s->cls, &s->parent, &s->edges, &s->prev_ids, &s->prev_ids2, &s->s_key,
-                    &s->s_key2, &s->s_id, &s->s_id2, &s->s_hi, &s->s_lo, &s->s_phase, &s->wedges, &s->tmp_simp,
+                    &s->s_key2, &s->s_id, &s->s_id2, &s->s_hi, &s->s_lo, &s->s_phase, &s->tmp_simp,
                     &s->dummy})
     b->st = ctx->stream;
   const int narr = s->layout == FTK2B_LAYOUT_MULTICOMPONENT ? 1 : s->m;
@@ -846,7 +802,7 @@ extern "C" void ftk2b_stream_close(ftk2b_stream* s) {
   cudaStreamSynchronize(s->ctx->stream);
   for (DevBuf* b : {&s->ring[0], &s->ring[1], &s->ring[2], &s->key, &s->hi, &s->lo, &s->phase, &s->lam, &s->bary4,
                     &s->scalar, &s->cls, &s->parent, &s->edges, &s->prev_ids, &s->prev_ids2, &s->s_key, &s->s_key2,
-                    &s->s_id, &s->s_id2, &s->s_hi, &s->s_lo, &s->s_phase, &s->wedges, &s->tmp_simp, &s->dummy})
+                    &s->s_id, &s->s_id2, &s->s_hi, &s->s_lo, &s->s_phase, &s->tmp_simp, &s->dummy})
     b->release();
   delete s;
 }
@@ -1058,7 +1014,7 @@ extern "C" ftk2b_status ftk2b_stream_restore(ftk2b_ctx* ctx, const void* buf, ui
   if (cudaSetDevice(ctx->device) != cudaSuccess) st = FTK2B_CUDA_ERROR;
   for (DevBuf* b : {&s->ring[0], &s->ring[1], &s->ring[2], &s->key, &s->hi, &s->lo, &s->phase, &s->lam,
                     &s->bary4, &s->scalar, &s->cls, &s->parent, &s->edges, &s->prev_ids, &s->prev_ids2, &s->s_key,
-                    &s->s_key2, &s->s_id, &s->s_id2, &s->s_hi, &s->s_lo, &s->s_phase, &s->wedges, &s->tmp_simp,
+                    &s->s_key2, &s->s_id, &s->s_id2, &s->s_hi, &s->s_lo, &s->s_phase, &s->tmp_simp,
                     &s->dummy})
     b->st = ctx->stream;
   const int narr = s->layout == FTK2B_LAYOUT_MULTICOMPONENT ? 1 : s->m;

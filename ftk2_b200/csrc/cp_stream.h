@@ -35,7 +35,7 @@ struct ftk2b_stream {
   ftk2b::DevBuf prev_ids, prev_ids2;
   unsigned n_first = 0;        // features of the first push (classified at the second)
   // per-push scratch
-  ftk2b::DevBuf s_key, s_key2, s_id, s_id2, s_hi, s_lo, s_phase, wedges, tmp_simp, dummy;
+  ftk2b::DevBuf s_key, s_key2, s_id, s_id2, s_hi, s_lo, s_phase, tmp_simp, dummy;
 
   double last_ms = 0;
   unsigned last_new = 0;
