@@ -736,9 +736,13 @@ def main():
             "gpu_launches": int(launches1 - launches0)}
     del pinned, host
     if rank == 0 and world == 1 and not args.no_cpu_baseline:
-        v, sample = cpu_baseline_sample()
-        line["cpu_baseline"] = {"value": v, "unit": UNIT, "cores": os.cpu_count() or 1,
-                                "kind": "reference", "sample": sample}
+        from oracle import bridge
+        if bridge.ref_available():
+            v, sample = cpu_baseline_sample()
+            line["cpu_baseline"] = {"value": v, "unit": UNIT, "cores": os.cpu_count() or 1,
+                                    "kind": "reference", "sample": sample}
+        else:  # built from the reference's headers, which not every machine has
+            line["cpu_baseline"] = {"value": None, "unit": UNIT, "unavailable": "reference engine build missing"}
     # the extra lines are one-GPU measurements (and their CPU baselines belong
     # to rank 0 at N = 1): with several ranks only the replica line is timed
     if not args.no_extra and world == 1:
