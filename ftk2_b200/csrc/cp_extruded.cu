@@ -887,7 +887,7 @@ cudaError_t enqueue_post(ftk2b_ctx* ctx, const ExtMeshDev& X, const ExtSink& sin
   if (ranked) {
     const LoadFound ld{sink.hi, sink.lo};
     const StoreFound<M> sw{sink, out, vb};
-    if ((e = launch_rank_sort<2>(ld, sw, RankCount{n, nullptr, nullptr, 0}, n ? n : 1, nullptr, ctx->num_sms, st))) return e;
+    if ((e = launch_rank_sort<2>(ld, sw, RankCount{n}, n ? n : 1, nullptr, ctx->num_sms, st))) return e;
     *nl += 1;
   } else {
     const int sgrid = ctx->sort_grid(cap);
@@ -920,7 +920,7 @@ cudaError_t enqueue_post(ftk2b_ctx* ctx, const ExtMeshDev& X, const ExtSink& sin
   if (ranked) {
     const LoadEdgeKey ld{(const unsigned long long*)C.ekeys.p};
     const StoreEdge so{(unsigned*)ctx->edges.p};
-    if ((e = launch_rank_sort<1>(ld, so, RankCount{0, counters + kCountEdges, nullptr, 0}, std::min(edge_cap, kRankCap1), nullptr,
+    if ((e = launch_rank_sort<1>(ld, so, RankCount{0, counters + kCountEdges}, std::min(edge_cap, kRankCap1), nullptr,
                                  ctx->num_sms, st)))
       return e;
     *nl += 1;
@@ -1205,7 +1205,7 @@ ftk2b_status push_extruded_t(ftk2b_stream* s) {
     if (rc) return rc;
   }
   if (!done && ranked) {
-    EXT_TRY(window({nS, nullptr, nullptr, 0}, wcap));
+    EXT_TRY(window({nS}, wcap));
     EXT_TRY(stars(wcap));
   } else if (!done) {
     EXT_TRY(s->s_key.ensure(8 * (size_t)wcap));
@@ -1286,7 +1286,7 @@ ftk2b_status result_extruded_t(ftk2b_stream* s, ftk2b_cp_result** out) {
   if (nc <= kRankCap2) {
     const LoadTuple ld{(const unsigned long long*)s->hi.p, (const unsigned long long*)s->lo.p, nullptr, 0u, 0u};
     const StoreTupleOrder so{{(unsigned*)s->s_id.p, inv, cmin}};
-    EXT_TRY(launch_rank_sort<2>(ld, so, RankCount{n, nullptr, nullptr, 0}, nc, counters + kSWin, ctx->num_sms, st));
+    EXT_TRY(launch_rank_sort<2>(ld, so, RankCount{n}, nc, counters + kSWin, ctx->num_sms, st));
     perm = so.order.perm;
   } else {
     set_u32_kernel<<<1, 1, 0, st>>>(counters + kSWin, n);

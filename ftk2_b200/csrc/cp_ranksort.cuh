@@ -22,13 +22,15 @@ constexpr unsigned kRankCap1 = 24576;  // keys of one word: 192 KB
 constexpr unsigned kRankCap2 = 12288;  // keys of two words
 
 // How many keys there are: `add`, plus *n where n is not null; none when that is
-// more than the launch holds, or *gate (not null) is above gate_max, so that a
-// launch may precede the host's look at the counters.
+// more than the launch holds, *gate (not null) is above gate_max, or *err (not
+// null) is set, so that a launch may precede the host's look at the counters: a
+// step that failed must leave no trace in what the launches behind it update.
 struct RankCount {
   unsigned add;
-  const unsigned* n;
-  const unsigned* gate;
-  unsigned gate_max;
+  const unsigned* n = nullptr;
+  const unsigned* gate = nullptr;
+  unsigned gate_max = 0;
+  const unsigned* err = nullptr;
 };
 
 // Keys of W 64-bit words, compared word by word, equal keys by index.
@@ -42,7 +44,8 @@ __global__ void __launch_bounds__(kRankThreads, 1)
   extern __shared__ unsigned long long rank_keys[];
   pdl_enter();
   const unsigned long long all = (unsigned long long)count.add + (count.n ? *count.n : 0u);
-  const unsigned n = all > cap || (count.gate && *count.gate > count.gate_max) ? 0u : (unsigned)all;
+  const bool none = all > cap || (count.gate && *count.gate > count.gate_max) || (count.err && *count.err);
+  const unsigned n = none ? 0u : (unsigned)all;
   if (n_out && blockIdx.x == 0 && threadIdx.x == 0) *n_out = n;
   if (blockIdx.x * (kRankThreads / 8) >= n) return;  // no key of this block's
   for (unsigned i = threadIdx.x; i < n; i += kRankThreads) {

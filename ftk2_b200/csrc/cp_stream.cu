@@ -265,7 +265,8 @@ ftk2b_status push_regular(ftk2b_stream* s) {
   // The window goes ahead of the host's look at the counters when it is no
   // larger than four times the last one: a push of a few hundred features spends
   // 20 us of 105 on the wait between its two halves.  The kernels find no
-  // window when it is larger, or when lists overflowed, and it is run again.
+  // window when it is larger, or when lists overflowed, and it is run again; nor
+  // when the cull raised an error: that push fails and must join no tracks.
   const unsigned guess = window_guess(s, kRankCap1);
   if (guess) {
     rc = room(guess);
@@ -317,7 +318,7 @@ ftk2b_status push_regular(ftk2b_stream* s) {
     ctx->launches += 1 + nk;
     if (guess) {
       const unsigned fits = (unsigned)std::min<unsigned long long>(guess, (unsigned long long)s->n_prev + sink.cap);
-      S_TRY(ctx, window({s->n_prev, counters + kCountFeatures, counters + kCountCand, ccap}, fits));
+      S_TRY(ctx, window({s->n_prev, counters + kCountFeatures, counters + kCountCand, ccap, counters + kCountErr}, fits));
     }
     S_TRY(ctx, cudaMemcpyAsync(ctx->h_counters, counters, sizeof(unsigned) * kNumCounters, cudaMemcpyDeviceToHost,
                                st));
@@ -345,7 +346,7 @@ ftk2b_status push_regular(ftk2b_stream* s) {
   if (!done && wcap <= kRankCap1) {
     rc = room(wcap);
     if (rc) return rc;
-    S_TRY(ctx, window({nS, nullptr, nullptr, 0}, wcap));
+    S_TRY(ctx, window({nS}, wcap));
   } else if (!done) {
     rc = room(wcap);
     if (rc) return rc;
@@ -451,7 +452,7 @@ ftk2b_status result_regular(ftk2b_stream* s, ftk2b_cp_result** out) {
   const unsigned* perm;
   if (nc <= kRankCap1) {
     const StoreCanon sc{{(unsigned*)s->s_id.p, inv, cmin}, (unsigned long long*)s->s_key.p};
-    S_TRY(ctx, launch_rank_sort<1>(LoadKey{(const unsigned long long*)s->key.p}, sc, RankCount{n, nullptr, nullptr, 0}, nc, counters + kSWin,
+    S_TRY(ctx, launch_rank_sort<1>(LoadKey{(const unsigned long long*)s->key.p}, sc, RankCount{n}, nc, counters + kSWin,
                                    ctx->num_sms, st));
     skeys = sc.skey;
     perm = sc.order.perm;
@@ -511,7 +512,7 @@ ftk2b_status canonical_edges(ftk2b_stream* s, const unsigned* inv, unsigned long
   const unsigned ne = s->n_edges, ec = ne ? ne : 1;
   if (ec <= kRankCap1) {
     S_TRY(ctx, launch_rank_sort<1>(LoadCanonEdge{(const unsigned*)s->edges.p, inv}, StoreEdge{(unsigned*)ctx->edges.p},
-                                   RankCount{ne, nullptr, nullptr, 0}, ec, counters + kSWinEdges, ctx->num_sms, st));
+                                   RankCount{ne}, ec, counters + kSWinEdges, ctx->num_sms, st));
     ctx->launches += 1;
     return FTK2B_OK;
   }
