@@ -19,10 +19,14 @@
 //   4. the resident union-find over stream ids takes the new edges.
 // The result sorts the store (canonical ids = rank in Simplex order) and
 // labels every component with its smallest canonical id (engine.hpp:46-74).
+#include <cuda.h>
+#include <cudaTypedefs.h>
+
 #include <algorithm>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <mutex>
 
 #include "cp_post.h"
 #include "cp_stream.h"
@@ -48,9 +52,11 @@ ftk2b_status sfail(ftk2b_ctx* ctx, ftk2b_status st, const char* fmt, ...) {
 #define S_TRY(ctx, call)                                                                        \
   do {                                                                                          \
     cudaError_t e_ = (call);                                                                    \
-    if (e_ != cudaSuccess)                                                                      \
+    if (e_ != cudaSuccess) {                                                                    \
+      cudaGetLastError(); /* reported here: the next call's launches must not meet it */        \
       return sfail(ctx, e_ == cudaErrorMemoryAllocation ? FTK2B_OOM : FTK2B_CUDA_ERROR,          \
                    "%s failed: %s (%s:%d)", #call, cudaGetErrorString(e_), __FILE__, __LINE__); \
+    }                                                                                           \
   } while (0)
 
 int bits_for(unsigned long long v) {
@@ -148,6 +154,33 @@ __global__ void ring_copy_kernel(RingCopy c) {
   const unsigned long long n16 = wide ? c.bytes / 16 : 0;
   for (unsigned long long i = t; i < n16; i += nt) ((uint4*)dst)[i] = __ldcs((const uint4*)src + i);
   for (unsigned long long i = 4 * n16 + t; i < c.bytes / 4; i += nt) ((unsigned*)dst)[i] = ((const unsigned*)src)[i];
+}
+
+// In how many pieces of device memory, one behind the other, [p, p + bytes)
+// lies: 1 inside one allocation, more for memory mapped in parts, -1 when it
+// runs past the end of the last, 0 when the driver does not know p.  A copy is
+// checked by the driver; a kernel that reads the array has to be checked here.
+int device_pieces(const void* p, size_t bytes) {
+  static PFN_cuMemGetAddressRange_v3020 range = nullptr;
+  static std::once_flag once;
+  std::call_once(once, [] {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &f, cudaEnableDefault, &q) == cudaSuccess &&
+        q == cudaDriverEntryPointSuccess)
+      range = reinterpret_cast<PFN_cuMemGetAddressRange_v3020>(f);
+    cudaGetLastError();
+  });
+  if (!range) return 0;
+  const CUdeviceptr end = (CUdeviceptr)p + bytes;
+  int n = 0;
+  for (CUdeviceptr at = (CUdeviceptr)p; at < end; ++n) {
+    CUdeviceptr base = 0;
+    size_t size = 0;
+    if (range(&base, &size, at) != CUDA_SUCCESS || base + size <= at) return n ? -1 : 0;
+    at = base + size;
+  }
+  return n;
 }
 
 unsigned long long time_chain_mask(int d) {
@@ -742,7 +775,8 @@ extern "C" ftk2b_status ftk2b_stream_push(ftk2b_stream* s, const ftk2b_field_des
   const size_t slot = (size_t)(s->T & 1);
   for (int j = 0; j < narr; ++j)
     if (!step->comp[j]) return sfail(ctx, FTK2B_INVALID_ARG, "component array %d is null", j);
-  // arrays in this device's memory: one launch for all and for the counters
+  // arrays in this device's memory, each inside one allocation: one launch for
+  // all and for the counters
   s->counters_clear = false;
   bool here = step->location == FTK2B_DEVICE && ctx->counters.ensure(sizeof(unsigned) * kNumCounters) == cudaSuccess;
   RingCopy rc_args;
@@ -751,6 +785,9 @@ extern "C" ftk2b_status ftk2b_stream_push(ftk2b_stream* s, const ftk2b_field_des
     cudaPointerAttributes at;
     here = cudaPointerGetAttributes(&at, step->comp[j]) == cudaSuccess && at.type == cudaMemoryTypeDevice &&
            at.device == ctx->device && (uintptr_t)step->comp[j] % s->es == 0;
+    const int pieces = here ? device_pieces(step->comp[j], bytes) : 0;
+    if (pieces < 0) return sfail(ctx, FTK2B_CUDA_ERROR, "component array %d runs past its allocation", j);
+    here = pieces == 1;
     rc_args.src[j] = step->comp[j];
     rc_args.dst[j] = (char*)s->ring[j].p + slot * bytes;
   }
