@@ -1094,9 +1094,11 @@ static cudaError_t launch_post_small(const RegularMesh& mesh, int nch, const Pos
   const unsigned cap = B.cap;
   const size_t key_smem = sizeof(unsigned long long) * (size_t)(cap ? cap : 1);
   const int g = B.num_sms > 0 ? B.num_sms : 148;
-  cudaError_t e = cudaFuncSetAttribute(small_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)key_smem);
+  // always the most any call needs: another thread may be launching the same kernels
+  constexpr int kMost = 8 * (int)kSmallPostCap;
+  cudaError_t e = cudaFuncSetAttribute(small_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost);
   if (!e) e = launch_pdl(small_sort_kernel, 1, kSortThreads, key_smem, st, B);
-  if (!e) e = cudaFuncSetAttribute(small_edges_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)key_smem);
+  if (!e) e = cudaFuncSetAttribute(small_edges_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost);
   if (!e) e = launch_pdl(small_edges_kernel, g, kSortThreads, key_smem, st, mesh, nch, B, want_edges);
   if (e) return e;
   *launches += 2;
