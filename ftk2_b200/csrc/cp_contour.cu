@@ -435,32 +435,6 @@ __global__ void __launch_bounds__(kCtThreads) ct_emit_kernel(
   }
 }
 
-// The first crossing edge (v, v + e) of every vertex starts at an edge of a lower
-// vertex w = v - a, a an axis outside e: in the triangle (w, w + a, w + a + e)
-// exactly one of (w, a) and (w, a + e) crosses too.  Most edges then hang in
-// one long tree before the joins, which otherwise meet everywhere at once.
-__global__ void __launch_bounds__(kCtThreads) ct_hook_kernel(CtGeom g, const unsigned short* __restrict__ mask,
-                                                             const unsigned* __restrict__ voff,
-                                                             unsigned* __restrict__ parent) {
-  const unsigned long long i0 = blockIdx.x * (unsigned long long)kCtBlock + threadIdx.x;
-#pragma unroll
-  for (int j = 0; j < kCtPer; ++j) {
-    const unsigned long long i = i0 + j * kCtThreads;
-    const unsigned m = i < g.nv ? mask[i] : 0u;
-    if (!m) continue;
-    unsigned long long c[4];
-    ct_coords(g, i, c);
-    const unsigned e = __ffs(m);
-    for (int k = g.d - 1; k >= 0; --k) {
-      if (((e >> k) & 1u) || c[k] == 0) continue;
-      const unsigned long long w = i - g.lstr[k];
-      const unsigned mw = mask[w], a = 1u << k;
-      parent[voff[i]] = voff[w] + ct_below(mw, (mw >> (a - 1)) & 1u ? a : a | e);
-      break;
-    }
-  }
-}
-
 // Joins the crossing edges of every mesh triangle that has two.  The crossing
 // edges of a simplex hang together through its triangles, so this gives the
 // components of the cells; a triangle (v, v + a, v + b), a a subset of b, is met
@@ -469,19 +443,21 @@ __global__ void __launch_bounds__(kCtThreads) ct_hook_kernel(CtGeom g, const uns
 //   (v, a) and (v + a, b - a)    all edges at v + a disjoint from a
 //   (v, b) and (v + a, b - a)    v has no edge to a
 // A thread takes one vertex and corner a; of edges that started joined on both
-// sides one pair is enough.  Bound by the dependent loads of ranks and roots.
-// Joining every cell's nodes from the cells kernel took four times as many
-// unions from divergent lanes and most of that kernel's time, a thread per edge
-// here 375 us, of which 75 without any union: threads that join the same two
-// large trees queue on their roots.  So the hooked trees are flattened, one
-// vertex of kCtSample joins along its axes, the trees (few by then) are
-// flattened again, and the rest mostly finds equal parents: 250 us in all
-// (96^3 x 6, 1.3 million edges).
-constexpr unsigned kCtSample = 4;
+// sides one pair is enough.  Bound by the dependent loads of ranks and roots, so
+// what counts is how many threads are at it: while the mesh has fewer than
+// kJoinBlocks shares of vertices an SM, several blocks (grid y) list the vertices
+// of one share and take its items in turn, up to one item a thread.  White noise
+// on 16 x 16 x 4 vertices (2,800 edges): 498 us with one block a share, 33 so; a
+// whole level set of 16^3 x 3 noise 2251 -> 270 us on the device, of 96^3 x 6
+// blobs (936,000 edges) 702 -> 660 (16 an SM: 703).  Hooking the vertices' first
+// edges ahead, joining a sample and flattening the trees in between paid for four
+// more launches with one block a share, but not so.  Joining every cell's nodes
+// from the cells kernel took four times as many unions from divergent lanes.
+constexpr unsigned kJoinBlocks = 64;
 
 __global__ void __launch_bounds__(kCtThreads) ct_join_kernel(CtGeom g, const unsigned short* __restrict__ mask,
                                                              const unsigned* __restrict__ voff, unsigned* parent,
-                                                             unsigned* err, bool sample) {
+                                                             unsigned* err) {
   __shared__ unsigned short s_vert[kCtBlock], s_mask[kCtBlock];
   __shared__ unsigned long long s_off[16];
   if (threadIdx.x < 16) s_off[threadIdx.x] = ct_corner_step(g, threadIdx.x);
@@ -503,9 +479,8 @@ __global__ void __launch_bounds__(kCtThreads) ct_join_kernel(CtGeom g, const uns
     }
   __syncthreads();
   const unsigned diag = (1u << g.d) - 1u;
-  const unsigned per = sample ? (unsigned)g.d : diag, step = sample ? kCtSample : 1u;
-  for (unsigned k = threadIdx.x; k < (n + step - 1) / step * per; k += kCtThreads) {
-    const unsigned z = k / per * step, mv = s_mask[z], a = sample ? 1u << k % per : k % per + 1;
+  for (unsigned k = blockIdx.y * kCtThreads + threadIdx.x; k < n * diag; k += gridDim.y * kCtThreads) {
+    const unsigned z = k / diag, mv = s_mask[z], a = k % diag + 1;
     const bool edge = (mv >> (a - 1)) & 1u;
     unsigned with = 0;  // no edge to a: the corners b above a that have one
     if (!edge) {
@@ -1049,12 +1024,10 @@ ftk2b_status run_contour(ftk2b_ctx* ctx, const CtGeom& g, const void* field, T t
   auto* first = d == 3 ? static_cast<unsigned long long*>(B[kBufFirst].p) : nullptr;
   ct_emit_kernel<T><<<(unsigned)nblk, kCtThreads, 0, st>>>(g, a, thr, mask, blk, voff, simp, lam, bary, parent);
   if (n && g.ncube) {
-    ct_hook_kernel<<<(unsigned)nblk, kCtThreads, 0, st>>>(g, mask, voff, parent);
-    uf_flatten_kernel<<<grid_of(n, 256, 8ull * sms), 256, 0, st>>>(parent, n);
-    ct_join_kernel<<<(unsigned)nblk, kCtThreads, 0, st>>>(g, mask, voff, parent, counts + 3, true);
-    uf_flatten_kernel<<<grid_of(n, 256, 8ull * sms), 256, 0, st>>>(parent, n);
-    ct_join_kernel<<<(unsigned)nblk, kCtThreads, 0, st>>>(g, mask, voff, parent, counts + 3, false);
-    ctx->launches += 5;
+    const unsigned long long most = kCtPer * ((1ull << d) - 1);  // one item a thread
+    const dim3 grid((unsigned)nblk, (unsigned)std::min(most, (kJoinBlocks * sms + nblk - 1) / nblk));
+    ct_join_kernel<<<grid, kCtThreads, 0, st>>>(g, mask, voff, parent, counts + 3);
+    ctx->launches += 1;
   }
   ctx->launches += 1;
   const unsigned wgrid = 16u * sms;  // 8 warps per block
