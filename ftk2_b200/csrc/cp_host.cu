@@ -137,9 +137,13 @@ cudaError_t copy_to_host(ftk2b_ctx* ctx, const std::vector<HostCopy>& copies) {
     }
     return cudaSuccess;
   }
-  if (!ctx->d2h_ring.h) {
-    const cudaError_t e = ctx->d2h_ring.alloc(kRingChunk * kRingChunks);
-    if (e) return e;
+  if (!ctx->d2h_ring.h && ctx->d2h_ring.alloc(kRingChunk * kRingChunks) != cudaSuccess) {
+    // no memory to pin: the driver's own copies
+    cudaError_t e = cudaSuccess;
+    for (const HostCopy& c : copies)
+      if (c.bytes && !e) e = cudaMemcpyAsync(c.dst, c.src, c.bytes, cudaMemcpyDeviceToHost, ctx->stream);
+    const cudaError_t se = cudaStreamSynchronize(ctx->stream);
+    return e ? e : se;
   }
   for (cudaEvent_t& ev : ctx->d2h_ev)
     if (!ev) {
@@ -184,7 +188,7 @@ cudaError_t copy_to_host(ftk2b_ctx* ctx, const std::vector<HostCopy>& copies) {
     queued[i].store(i + 1);
   }
   const int device = ctx->device;
-  run_threads(std::min(host_threads(total), np), [&](size_t t) {
+  run_threads(total < kCopyThreadBytes ? 1 : std::min(host_threads(total), np), [&](size_t t) {
     if (t && cudaSetDevice(device) != cudaSuccess) {
       err.store((int)cudaErrorUnknown);
       return;

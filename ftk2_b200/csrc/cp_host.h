@@ -21,6 +21,11 @@ namespace ftk2b {
 
 constexpr size_t kHostThreads = 8;
 constexpr size_t kHostThreadBytes = size_t(2) << 20;  // per thread, at least
+// Copies from the device take several threads from here on: a thread that
+// calls the driver costs 0.1 to 0.6 ms to start and end, and which it is varies
+// from call to call.  Level sets of 4.3 and 9 MB: 485 to 800 and 530 to 1,060 us
+// a call with several threads, 577 and 774 with one; of 20 MB 1,340 against 1,545.
+constexpr size_t kCopyThreadBytes = size_t(16) << 20;
 
 // f(begin, end) over [0, n) in contiguous shares, one per thread; `bytes` is
 // the memory the whole range touches.  A thread that cannot be started leaves

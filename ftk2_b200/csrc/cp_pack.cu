@@ -10,6 +10,7 @@
 #include <cstdlib>
 #include <cstring>
 
+#include "cp_host.h"
 #include "cp_pack.h"
 #include "cp_pdl.cuh"
 
@@ -60,7 +61,7 @@ cudaError_t launch_pack(const PackArgs& a, int num_sms, cudaStream_t st) {
 
 ftk2b_cp_result* new_result(uint64_t n, uint64_t ne, int m, int classify, PackLayout* out) {
   const PackLayout L = pack_layout(n, ne, m + 1, classify);
-  unsigned char* b = static_cast<unsigned char*>(std::malloc(kResultHeader + L.total));
+  unsigned char* b = static_cast<unsigned char*>(host_alloc(kResultHeader + L.total));
   if (!b) return nullptr;
   ftk2b_cp_result* r = reinterpret_cast<ftk2b_cp_result*>(b);
   std::memset(r, 0, sizeof(*r));
