@@ -7,8 +7,8 @@
 // keys is three launches per 8 bits, and a 55-bit tuple takes two such sorts.  A
 // stream's push, whose window of some 500 features was sorted that way, went
 // from 165 to 110 us (96 x 101 x 88 float) and from 880 to 720 us (100 x 100 x 40
-// tets); its result from 270 to 102 us (2,200 features).  Sets beyond what
-// shared memory holds take the radix passes.
+// tets); its result from 270 to 102 us (2,200 features).  Larger sets take the
+// radix passes.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -18,8 +18,13 @@
 namespace ftk2b {
 
 constexpr int kRankThreads = 512;
-constexpr unsigned kRankCap1 = 24576;  // keys of one word: 192 KB
-constexpr unsigned kRankCap2 = 12288;  // keys of two words
+// Keys of one word: where a push of that many takes as long by the radix passes
+// (2D and 3D noise, by rank / by passes: 12,600 keys 160 / 169 us, 14,800 185 /
+// 187, 16,600 191 / 171, 18,600 258 / 181; 231 before there was a rank sort).
+constexpr unsigned kRankCap1 = 15360;
+// Keys of two words, whose passes are twice as many: what 192 KB hold (a push of
+// 12,000 tuples 332 / 454 us).
+constexpr unsigned kRankCap2 = 12288;
 
 // How many keys there are: `add`, plus *n where n is not null; none when that is
 // more than the launch holds, *gate (not null) is above gate_max, or *err (not
