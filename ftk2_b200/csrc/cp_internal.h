@@ -88,9 +88,10 @@ struct ExtractConfig {
   int tiles[3];                // tiles along x, y, z (z = 1 for 2D)
   int skip_first_spatial;      // 1: no purely spatial simplices at local time 0
   int cull_mode;               // 0: per-vertex cull words only; 1: tile statistics first
-  // > 0: failure-path check of the fused cull: after its first slice every
-  // block waits, at most this many polls, on an mbarrier nothing completes,
-  // and leaves through the timeout path (the call reports FTK2B_TIMEOUT)
+  // > 0: failure-path check of cull mode 0: every block waits (a staged one
+  // after its first slice), at most this many polls, on an mbarrier nothing
+  // completes, and leaves through the timeout path (the call reports
+  // FTK2B_TIMEOUT)
   int stall_polls;
   // FiberPredicate<T> (predicate.hpp:341-362): no cull words (they assume the
   // solve must succeed), values are taken minus fthr[j], and a simplex whose
@@ -119,8 +120,9 @@ void upload_chain_tables();
 // CUDA call failed.
 bool ensure_device_tables(int device);
 
-// Launches the fused extraction; uses TMA tensor-tile staging when allowed
-// and the array satisfies the 16-byte alignment rules (reported in used_tma);
+// Launches the cull; 3D+t meshes and cull mode 1 use TMA tensor-tile staging
+// when allowed and the array satisfies the 16-byte alignment rules (reported in
+// used_tma);
 // *launches (optional) receives the number of kernels it launched.
 cudaError_t launch_extract_regular(int f64, const RegularMesh& mesh, const FieldAccess& fa,
                                    const ExtractConfig& cfg, const CandidateQueue& cq, unsigned* err,

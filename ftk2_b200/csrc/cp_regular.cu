@@ -700,7 +700,9 @@ __global__ void __launch_bounds__(kThreads, 2)
 // block.  Bound by issue: some 60 instructions a vertex, 150 with the slice
 // staged in shared memory.  1021 x 765 x 12 float in two arrays: 62.5 -> 36 us
 // (8 rows a strip, fewer vertices computed twice but half the warps: 39.5); 64 x
-// 64 x 10 double: 11.6 -> 4.  Chunks are long where strips alone give
+// 64 x 10 double: 11.6 -> 4.  Arrays that TMA could stage gain less but at every
+// size, so 2D+t has no staged form: 1024 x 768 x 12 float 49.5 -> 41.5, 2048^2 x
+// 16 287 -> 240, 4096^2 x 8 617 -> 460, 128 x 96 x 1000 1064 -> 63.  Chunks are long where strips alone give
 // kStripsWanted warps (a chunk's first slice is read twice) and short where they
 // do not (fewer steps in sequence); 32 to 128 warps an SM measure alike.
 constexpr int kStripRows = 4;
@@ -710,14 +712,22 @@ constexpr int kStripsWanted = 64 * 148;    // warps of the launch, at least wher
 template <typename T>
 __global__ void __launch_bounds__(kStripWarps * 32, 3) strip_cull_kernel(RegularMesh mesh, FieldAccess fa,
                                                                       ExtractConfig cfg, CandidateQueue cq,
-                                                                      int strips_x, int strips_y, int tchunk,
-                                                                      unsigned n_warps) {
+                                                                      unsigned* err, int strips_x, int strips_y,
+                                                                      int tchunk, unsigned n_warps) {
   constexpr int M = 2, R = kStripRows;
   __shared__ unsigned band_tbl[kBandTable];
   __shared__ unsigned long long cbuf[2 * kCandBuf];
   __shared__ unsigned ccount[2];
   fill_band_table<T>(band_tbl, threadIdx.x, kStripWarps * 32);
   if (threadIdx.x == 0) ccount[0] = 0;
+  if (cfg.stall_polls > 0) {  // failure-path check (host option): a bounded wait that runs out
+    __shared__ unsigned long long never;
+    if (threadIdx.x == 0) {
+      mbar_init(&never, 1);
+      if (!mbar_wait(&never, 0u, cfg.stall_polls)) atomicOr(err, 2u);
+    }
+    return;
+  }
   __syncthreads();
   const int lane = threadIdx.x & 31;
   const unsigned w = blockIdx.x * kStripWarps + (threadIdx.x >> 5);
@@ -2639,13 +2649,12 @@ static cudaError_t launch_t(const RegularMesh& mesh, const FieldAccess& fa, cons
   constexpr int M = D - 1;
 
   CUtensorMap maps[3];
-  const bool tma = build_tma_maps<T, D, MULTI>(mesh, fa, allow_tma, maps);
+  const bool staged = D == 4 || cfg.cull_mode == 1;  // the strip cull reads the arrays itself
+  const bool tma = staged && build_tma_maps<T, D, MULTI>(mesh, fa, allow_tma, maps);
   if (used_tma) *used_tma = tma ? 1 : 0;
-  const size_t shm = G::SMEM;
   const long long lt = mesh.ld[D - 1];
   const unsigned nchunks = (unsigned)((lt + cfg.tchunk - 1) / cfg.tchunk);
   const unsigned ntiles = (unsigned)cfg.tiles[0] * cfg.tiles[1] * cfg.tiles[2];
-  dim3 grid(ntiles, nchunks);
   cudaError_t e;
   // cull mode 1: arrays the TMA kernels can stage, with the caller's scratch
   const bool vec_ok = tma && cfg.tstats && cfg.runs && cfg.n_runs && cfg.runs_cap;
@@ -2695,7 +2704,7 @@ static cudaError_t launch_t(const RegularMesh& mesh, const FieldAccess& fa, cons
     return cudaGetLastError();
   }
   if (launches) *launches = 1;
-  if (D == 3 && cfg.stall_polls == 0) {  // the failure-path check lives in the staged form
+  if constexpr (D == 3) {
     if (used_tma) *used_tma = 0;
     const long long sx = (mesh.ld[0] + 30) / 31, sy = (mesh.ld[1] + kStripRows - 1) / kStripRows;
     long long nch = std::min<long long>(lt, (kStripsWanted + sx * sy - 1) / (sx * sy));
@@ -2704,16 +2713,11 @@ static cudaError_t launch_t(const RegularMesh& mesh, const FieldAccess& fa, cons
     nch = (lt + tchunk - 1) / tchunk;
     const unsigned warps = (unsigned)(sx * sy * nch);
     strip_cull_kernel<T><<<(warps + kStripWarps - 1) / kStripWarps, kStripWarps * 32, 0, st>>>(
-        mesh, fa, cfg, cq, (int)sx, (int)sy, (int)tchunk, warps);
-    return cudaGetLastError();
-  }
-  if (tma) {
-    auto k = extract_regular_kernel<T, D, MULTI, true>;
-    e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
-    if (e) return e;
-    k<<<grid, kThreads, shm, st>>>(maps[0], maps[1], maps[2], mesh, fa, cfg, cq, err);
+        mesh, fa, cfg, cq, err, (int)sx, (int)sy, (int)tchunk, warps);
   } else {
-    auto k = extract_regular_kernel<T, D, MULTI, false>;
+    const size_t shm = G::SMEM;
+    const dim3 grid(ntiles, nchunks);
+    auto k = tma ? extract_regular_kernel<T, D, MULTI, true> : extract_regular_kernel<T, D, MULTI, false>;
     e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shm);
     if (e) return e;
     k<<<grid, kThreads, shm, st>>>(maps[0], maps[1], maps[2], mesh, fa, cfg, cq, err);

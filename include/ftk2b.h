@@ -143,7 +143,8 @@ ftk2b_cp_params ftk2b_cp_params_default(void);
 enum {
   FTK2B_OPT_FEATURE_CAPACITY = 1, /* initial feature capacity; grows on overflow */
   FTK2B_OPT_TIME_CHUNK = 2,       /* time steps per extraction block (0 = all) */
-  FTK2B_OPT_DISABLE_TMA = 3,      /* 1: stage slices with plain loads instead of TMA */
+  FTK2B_OPT_DISABLE_TMA = 3,      /* 1: stage slices with plain loads instead of TMA (2D+t meshes stage none in
+                                     cull mode 0, and take that mode then) */
   FTK2B_OPT_USE_GRAPHS = 4,       /* 1 (default): replay the device pipeline as a CUDA graph */
   FTK2B_OPT_BLOCKING_SYNC = 5,    /* 1: wait for the device by blocking, not spinning (servers set it) */
   FTK2B_OPT_CULL_MODE = 6,        /* 0: per-vertex cull words only; 1: tile statistics first; 2 (default):
@@ -156,7 +157,8 @@ enum {
 };
 ftk2b_status ftk2b_ctx_set_option(ftk2b_ctx* ctx, int option, int64_t value);
 /* Reads an option back, or FTK2B_INFO_LAST_TMA: 1 when the last regular-mesh
- * extraction staged its slices with TMA tensor copies, or
+ * extraction staged its slices with TMA tensor copies (always 0 for 2D+t
+ * meshes in cull mode 0, which read the arrays directly), or
  * FTK2B_INFO_LAST_CULL_MODE: the cull mode (0 or 1) it ran, or
  * FTK2B_INFO_LAST_BATCH_TIME_CHUNK: corner time steps per cull item of the
  * last batch (65535: each field's whole time range), or
