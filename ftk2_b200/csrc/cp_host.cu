@@ -6,8 +6,9 @@
 #include <atomic>
 #include <cstdlib>
 #include <cstring>
+#include <exception>
 #include <memory>
-#include <system_error>
+#include <new>
 #include <thread>
 
 #include "cp_api_internal.h"
@@ -29,7 +30,7 @@ void run_threads(size_t k, F body) {
   size_t started = 1;
   try {
     for (; started < k; ++started) th[started] = std::thread(body, started);
-  } catch (const std::system_error&) {
+  } catch (const std::exception&) {  // no thread, or no memory for one
   }
   body(0);
   for (size_t i = started; i < k; ++i) body(i);
@@ -38,13 +39,13 @@ void run_threads(size_t k, F body) {
 
 }  // namespace
 
-void host_parallel(size_t n, size_t bytes, const std::function<void(size_t, size_t)>& f) {
+void host_parallel(size_t n, size_t bytes, void (*f)(void*, size_t, size_t), void* arg) {
   const size_t k = std::min(host_threads(bytes), std::max<size_t>(n, 1));
   if (k <= 1) {
-    f(0, n);
+    f(arg, 0, n);
     return;
   }
-  run_threads(k, [&](size_t i) { f(n * i / k, n * (i + 1) / k); });
+  run_threads(k, [&](size_t i) { f(arg, n * i / k, n * (i + 1) / k); });
 }
 
 void* host_alloc(size_t bytes) {
@@ -62,7 +63,7 @@ HostWords::~HostWords() { std::free(p_); }
 bool HostWords::alloc(size_t n) {
   std::free(p_);
   n_ = 0;
-  p_ = static_cast<uint64_t*>(host_alloc(8 * n));
+  p_ = n <= SIZE_MAX / 16 ? static_cast<uint64_t*>(host_alloc(8 * n)) : nullptr;
   if (p_) n_ = n;
   return p_ != nullptr;
 }
@@ -91,16 +92,18 @@ uint64_t hash_block(const uint64_t* p, size_t n) {
 
 uint64_t hash_blocks(size_t n, const uint64_t* src, uint64_t* copy_to, const void* copy_from) {
   const size_t nb = (n + kHashBlock - 1) / kHashBlock;
-  std::unique_ptr<uint64_t[]> hb(new uint64_t[nb ? nb : 1]);
-  host_parallel(nb, 8 * n, [&](size_t b0, size_t b1) {
-    for (size_t b = b0; b < b1; ++b) {
-      const size_t lo = b * kHashBlock, m = std::min(kHashBlock, n - lo);
-      if (copy_to) std::memcpy(copy_to + lo, static_cast<const char*>(copy_from) + 8 * lo, 8 * m);
-      hb[b] = hash_block((copy_to ? copy_to : src) + lo, m);
-    }
-  });
+  auto block = [&](size_t b) {
+    const size_t lo = b * kHashBlock, m = std::min(kHashBlock, n - lo);
+    if (copy_to) std::memcpy(copy_to + lo, static_cast<const char*>(copy_from) + 8 * lo, 8 * m);
+    return hash_block((copy_to ? copy_to : src) + lo, m);
+  };
+  std::unique_ptr<uint64_t[]> hb(new (std::nothrow) uint64_t[nb ? nb : 1]);
+  if (hb)
+    host_parallel(nb, 8 * n, [&](size_t b0, size_t b1) {
+      for (size_t b = b0; b < b1; ++b) hb[b] = block(b);
+    });
   uint64_t h = 0x9E3779B97F4A7C15ull ^ n;
-  for (size_t b = 0; b < nb; ++b) h = mix(h, hb[b]);
+  for (size_t b = 0; b < nb; ++b) h = mix(h, hb ? hb[b] : block(b));
   return h;
 }
 
@@ -116,7 +119,7 @@ constexpr size_t kRingChunks = 16;
 static_assert(kRingChunks == sizeof(ftk2b_ctx::d2h_ev) / sizeof(cudaEvent_t), "an event per chunk of the ring");
 }  // namespace
 
-cudaError_t copy_to_host(ftk2b_ctx* ctx, const std::vector<HostCopy>& copies) {
+cudaError_t copy_to_host(ftk2b_ctx* ctx, std::initializer_list<HostCopy> copies) {
   size_t sum = 0;
   for (const HostCopy& c : copies) sum += (c.bytes + 15) & ~size_t(15);
   if (sum <= ctx->pin.bytes - 256) {  // the context's own pinned block holds everything
@@ -153,20 +156,22 @@ cudaError_t copy_to_host(ftk2b_ctx* ctx, const std::vector<HostCopy>& copies) {
         return e;
       }
     }
-  struct Piece {
-    char* dst;
-    const char* src;
-    size_t n;
-  };
-  std::vector<Piece> pieces;
-  size_t total = 0;
+  size_t total = 0, np = 0;
   for (const HostCopy& c : copies) {
     total += c.bytes;
-    for (size_t o = 0; o < c.bytes; o += kRingChunk)
-      pieces.push_back({static_cast<char*>(c.dst) + o, static_cast<const char*>(c.src) + o,
-                        std::min(kRingChunk, c.bytes - o)});
+    np += (c.bytes + kRingChunk - 1) / kRingChunk;
   }
-  const size_t np = pieces.size();
+  // piece i of the copies, each cut into chunks
+  auto piece = [&copies](size_t i) {
+    for (const HostCopy& c : copies) {
+      const size_t n = (c.bytes + kRingChunk - 1) / kRingChunk, o = i * kRingChunk;
+      if (i < n)
+        return HostCopy{static_cast<char*>(c.dst) + o, static_cast<const char*>(c.src) + o,
+                        std::min(kRingChunk, c.bytes - o)};
+      i -= n;
+    }
+    return HostCopy{nullptr, nullptr, 0};
+  };
   char* ring = static_cast<char*>(ctx->d2h_ring.h);
   // piece i uses chunk i % kRingChunks; whoever empties a chunk queues the
   // next piece into it, so no thread waits for a free chunk
@@ -174,8 +179,8 @@ cudaError_t copy_to_host(ftk2b_ctx* ctx, const std::vector<HostCopy>& copies) {
   std::atomic<int> err{0};
   auto queue = [&](size_t i) {
     const size_t s = i % kRingChunks;
-    cudaError_t e = cudaMemcpyAsync(ring + s * kRingChunk, pieces[i].src, pieces[i].n, cudaMemcpyDeviceToHost,
-                                    ctx->stream);
+    const HostCopy c = piece(i);
+    cudaError_t e = cudaMemcpyAsync(ring + s * kRingChunk, c.src, c.bytes, cudaMemcpyDeviceToHost, ctx->stream);
     if (!e) e = cudaEventRecord(ctx->d2h_ev[s], ctx->stream);
     if (e) err.store((int)e);
     return e == cudaSuccess;
@@ -207,7 +212,8 @@ cudaError_t copy_to_host(ftk2b_ctx* ctx, const std::vector<HostCopy>& copies) {
         err.store((int)e);
         return;
       }
-      std::memcpy(pieces[i].dst, ring + s * kRingChunk, pieces[i].n);
+      const HostCopy c = piece(i);
+      std::memcpy(c.dst, ring + s * kRingChunk, c.bytes);
       if (i + kRingChunks < np) {
         if (!queue(i + kRingChunks)) return;
         queued[s].store(i + kRingChunks + 1, std::memory_order_release);

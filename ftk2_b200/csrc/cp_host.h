@@ -10,8 +10,7 @@
 
 #include <cstddef>
 #include <cstdint>
-#include <functional>
-#include <vector>
+#include <initializer_list>
 
 #include <cuda_runtime.h>
 
@@ -29,8 +28,13 @@ constexpr size_t kCopyThreadBytes = size_t(16) << 20;
 
 // f(begin, end) over [0, n) in contiguous shares, one per thread; `bytes` is
 // the memory the whole range touches.  A thread that cannot be started leaves
-// its share to the caller.
-void host_parallel(size_t n, size_t bytes, const std::function<void(size_t, size_t)>& f);
+// its share to the caller.  None of this file's functions throws or needs memory
+// of its own to succeed: they are called below C entry points.
+void host_parallel(size_t n, size_t bytes, void (*f)(void* arg, size_t begin, size_t end), void* arg);
+template <typename F>
+void host_parallel(size_t n, size_t bytes, F f) {
+  host_parallel(n, bytes, [](void* arg, size_t begin, size_t end) { (*static_cast<F*>(arg))(begin, end); }, &f);
+}
 
 // Memory for a large array, released with free(); from 4 MB on aligned and
 // advised for 2 MB pages, which fault once per 2 MB instead of once per 4 KB.
@@ -69,6 +73,6 @@ struct HostCopy {
 // Device arrays to pageable host memory through a ring of pinned chunks of the
 // context: the host threads empty chunks while the next ones arrive.  Waits
 // for the copies (and all work queued on the stream before).
-cudaError_t copy_to_host(ftk2b_ctx* ctx, const std::vector<HostCopy>& copies);
+cudaError_t copy_to_host(ftk2b_ctx* ctx, std::initializer_list<HostCopy> copies);
 
 }  // namespace ftk2b
