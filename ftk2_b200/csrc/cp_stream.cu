@@ -854,7 +854,11 @@ extern "C" void ftk2b_stream_close(ftk2b_stream* s) {
 namespace {
 
 constexpr char kCkptMagic[8] = {'F', 'T', 'K', '2', 'B', 'S', 'T', 'R'};
-constexpr uint32_t kCkptVersion = 1;
+// Version 2: the content hash of an unstructured stream's base cells is formed
+// block by block (hash_words); in version 1 it was one chain over all words.
+// Everything else is the same, so blobs of both are read, and regular streams,
+// which hold no hash, are written as version 1 for earlier readers.
+constexpr uint32_t kCkptVersion = 2;
 
 struct StreamCkpt {
   char magic[8];
@@ -869,7 +873,7 @@ struct StreamCkpt {
   uint32_t n, n_edges, n_prev, n_first;
 };
 
-// the content hash that earlier blobs of this version hold: one chain over all words
+// the content hash of version 1
 uint64_t serial_hash(const uint64_t* p, uint64_t n) {
   uint64_t h = 0x9E3779B97F4A7C15ull ^ n;
   for (uint64_t i = 0; i < n; ++i) {
@@ -924,7 +928,7 @@ extern "C" ftk2b_status ftk2b_stream_checkpoint(ftk2b_stream* s, void* buf, uint
   StreamCkpt h;
   memset(&h, 0, sizeof(h));
   memcpy(h.magic, kCkptMagic, 8);
-  h.version = kCkptVersion;
+  h.version = s->kind == FTK2B_MESH_REGULAR ? 1 : kCkptVersion;
   h.header_bytes = (uint32_t)sizeof(StreamCkpt);
   h.kind = s->kind;
   h.d = s->d;
@@ -972,7 +976,8 @@ extern "C" ftk2b_status ftk2b_stream_restore(ftk2b_ctx* ctx, const void* buf, ui
   if (!buf || bytes < sizeof(StreamCkpt)) return sfail(ctx, FTK2B_INVALID_ARG, "not a stream checkpoint (too short)");
   StreamCkpt h;
   memcpy(&h, buf, sizeof(h));
-  if (memcmp(h.magic, kCkptMagic, 8) != 0 || h.version != kCkptVersion || h.header_bytes != sizeof(StreamCkpt))
+  if (memcmp(h.magic, kCkptMagic, 8) != 0 || h.version < 1 || h.version > kCkptVersion ||
+      h.header_bytes != sizeof(StreamCkpt))
     return sfail(ctx, FTK2B_INVALID_ARG, "not a stream checkpoint of this library version");
   // the configuration must be one that ftk2b_stream_open accepts
   const bool regular = h.kind == FTK2B_MESH_REGULAR;
@@ -1037,6 +1042,7 @@ extern "C" ftk2b_status ftk2b_stream_restore(ftk2b_ctx* ctx, const void* buf, ui
     }
     s->emesh.base_cells = s->ecells.data();
     s->ebase_hash = copy_hash_words(s->ecells.data(), p, s->ecells.size());  // the caller's blob need not be aligned
+    // (some blobs of version 1 hold the hash of version 2)
     if (s->ebase_hash != h.ebase_hash && serial_hash(s->ecells.data(), s->ecells.size()) != h.ebase_hash) {
       delete s;
       return sfail(ctx, FTK2B_INVALID_ARG, "stream checkpoint's base cells are damaged");
