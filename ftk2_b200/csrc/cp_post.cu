@@ -276,38 +276,6 @@ __device__ __forceinline__ long long find_key_sampled(const unsigned long long* 
   return j < 0 ? -1 : (long long)r0 + j;
 }
 
-// Indices of the active faces of a top cell, ascending.
-__device__ int active_faces(const RegularMesh& mesh, int nch, const unsigned long long* keys,
-                            unsigned n, const long long cc[4], const int cm[5], long long out[5]) {
-  const int d = mesh.d, m = d - 1;
-  int na = 0;
-  for (int r = 0; r <= d; ++r) {
-    // face without vertex r: corner = cell vertex (r == 0 ? 1 : 0)
-    const int basem = (r == 0) ? cm[1] : 0;
-    int rel[4];
-    int w = 0;
-    for (int i = 0; i <= d; ++i) {
-      if (i == r || (r == 0 && i == 1) || (r != 0 && i == 0)) continue;
-      rel[w++] = cm[i] & ~basem;
-    }
-    unsigned long long vid = 0;
-    for (int k = 0; k < d; ++k)
-      vid += (unsigned long long)(cc[k] + ((basem >> k) & 1)) * mesh.gstride[k];
-    const int rk = chain_rank(d, rel);
-    const long long idx = find_key(keys, n, vid * (unsigned long long)nch + (unsigned long long)rk);
-    if (idx >= 0) out[na++] = idx;
-    (void)m;
-  }
-  // insertion sort (at most 5)
-  for (int i = 1; i < na; ++i)
-    for (int j = i; j > 0 && out[j - 1] > out[j]; --j) {
-      long long t = out[j];
-      out[j] = out[j - 1];
-      out[j - 1] = t;
-    }
-  return na;
-}
-
 constexpr int kEdgeSlots = 8;  // a codimension-1 simplex has 2 cofaces with <= 4 other faces each
 
 // Index of the face of top cell (cc, cm) without vertex r, or -1.
@@ -412,46 +380,6 @@ __global__ void edges_compact_kernel(const unsigned* n_ptr, unsigned cap, const 
         edges[2 * (size_t)(o + k)] = i;
         edges[2 * (size_t)(o + k) + 1] = slots[(size_t)i * kEdgeSlots + k];
       }
-  }
-}
-
-// pass 0: count edges per feature (as star centre); pass 1: write them
-template <int PASS>
-__global__ void edges_regular_kernel(RegularMesh mesh, int nch, const unsigned long long* __restrict__ keys,
-                                     const unsigned* n_ptr, unsigned cap, unsigned* __restrict__ cnt,
-                                     const unsigned* __restrict__ off, unsigned* __restrict__ edges,
-                                     unsigned edge_cap) {
-  const unsigned n = min(*n_ptr, cap);
-  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    Decoded dc;
-    decode_key(mesh, nch, keys[i], dc);
-    long long cc[2][4];
-    int cm[2][5];
-    const int nc = top_cells(mesh, dc, cc, cm);
-    long long others[8];
-    int no = 0;
-    for (int q = 0; q < nc; ++q) {
-      long long act[5];
-      const int na = active_faces(mesh, nch, keys, n, cc[q], cm[q], act);
-      if (na >= 2 && act[0] == (long long)i)
-        for (int t = 1; t < na; ++t) others[no++] = act[t];
-    }
-    if (PASS == 0) {
-      cnt[i] = no;
-    } else {
-      for (int a = 1; a < no; ++a)
-        for (int b = a; b > 0 && others[b - 1] > others[b]; --b) {
-          long long t = others[b];
-          others[b] = others[b - 1];
-          others[b - 1] = t;
-        }
-      const unsigned o = off[i];
-      for (int t = 0; t < no; ++t)
-        if (o + t < edge_cap) {
-          edges[2 * (size_t)(o + t)] = i;
-          edges[2 * (size_t)(o + t) + 1] = (unsigned)others[t];
-        }
-    }
   }
 }
 
@@ -1157,13 +1085,6 @@ cudaError_t launch_iota(unsigned* v, const unsigned* n_ptr, unsigned cap, cudaSt
 cudaError_t launch_scan(unsigned* a, unsigned total, unsigned* total_out, const unsigned* n_ptr,
                         cudaStream_t st) {
   scan_inplace_kernel<<<1, 1024, 0, st>>>(a, total, total_out, n_ptr, nullptr);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_uf(unsigned* parent, const unsigned* n_ptr, unsigned cap, const unsigned* edges,
-                      const unsigned* ne_ptr, unsigned edge_cap, unsigned* err, cudaStream_t st) {
-  uf_init_kernel<<<grid_for(cap, 256, 4096), 256, 0, st>>>(parent, n_ptr, cap);
-  uf_hook_kernel<<<grid_for(edge_cap, 256, 4096), 256, 0, st>>>(parent, edges, ne_ptr, edge_cap, err);
   return cudaGetLastError();
 }
 

@@ -60,9 +60,6 @@ cudaError_t launch_iota(unsigned* v, const unsigned* n_ptr, unsigned cap, cudaSt
 // the sum lands in *total_out when it is not null
 cudaError_t launch_scan(unsigned* a, unsigned total, unsigned* total_out, const unsigned* n_ptr,
                         cudaStream_t st);
-// union-find: parent[i] = i, then the edges' endpoints united
-cudaError_t launch_uf(unsigned* parent, const unsigned* n_ptr, unsigned cap, const unsigned* edges,
-                      const unsigned* ne_ptr, unsigned edge_cap, unsigned* err, cudaStream_t st);
 // track[i] = root of i (the component's smallest index), roots counted
 cudaError_t launch_uf_label(unsigned* parent, const unsigned* n_ptr, unsigned cap,
                             unsigned long long* track, unsigned* n_roots, cudaStream_t st);

@@ -44,10 +44,6 @@ static __global__ void uf_init_range_kernel(unsigned* parent, unsigned lo, unsig
     parent[lo + i] = lo + i;
 }
 
-// window edges (indices into the sorted window) -> stream ids, united and
-// appended after the `base` edges already stored
-// new features whose chain does not step in time are the spatial ones of
-// the newest layer
 static __global__ void iota_u32_kernel(unsigned* v, unsigned n) {
   for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) v[i] = i;
 }
