@@ -11,7 +11,7 @@
 #include <cstring>
 
 #include "cp_host.h"
-#include "cp_pack.h"
+#include "cp_pack.cuh"
 #include "cp_pdl.cuh"
 
 namespace ftk2b {
@@ -19,13 +19,6 @@ namespace ftk2b {
 namespace {
 
 constexpr int kPackThreads = 256;
-
-template <typename W, typename F>
-__device__ __forceinline__ void pack_words(unsigned char* dst, unsigned long long n, unsigned long long t,
-                                           unsigned long long nt, F word) {
-  W* out = reinterpret_cast<W*>(dst);
-  for (unsigned long long i = t; i < n; i += nt) out[i] = word(i);
-}
 
 __global__ void __launch_bounds__(kPackThreads) pack_kernel(PackArgs a) {
   pdl_enter();
@@ -37,19 +30,9 @@ __global__ void __launch_bounds__(kPackThreads) pack_kernel(PackArgs a) {
   if (n > a.cap || ne > a.edge_cap) return;
   const PackLayout L = pack_layout(n, ne, a.k, a.classify);
   if (L.packed > a.dst_bytes) return;
-  const unsigned k = (unsigned)a.k;
-  // consecutive lanes store consecutive words, so a warp's stores leave as
-  // whole 128-byte lines
-  pack_words<double>(a.dst + L.lam, (unsigned long long)n * k, t, nt,
-                     [&](unsigned long long i) { return k == 4 ? a.lam4[i] : a.lam4[i / k * 4 + i % k]; });
-  pack_words<unsigned long long>(a.dst + L.simplices, (unsigned long long)n * k, t, nt,
-                                 [&](unsigned long long i) { return a.simplices[i]; });
-  pack_words<unsigned long long>(a.dst + L.track, n, t, nt,
-                                 [&](unsigned long long i) { return a.want_edges ? a.track[i] : i; });
-  pack_words<float>(a.dst + L.bary, (unsigned long long)n * k, t, nt, [&](unsigned long long i) { return a.bary[i]; });
-  pack_words<float>(a.dst + L.scalar, n, t, nt, [&](unsigned long long i) { return a.scalar[i]; });
+  pack_records(a, L, n, t, nt);
+  pack_labels(a, L, n, t, nt, [&](unsigned long long i) { return a.track[i]; });
   pack_words<unsigned>(a.dst + L.edges, 2ull * ne, t, nt, [&](unsigned long long i) { return a.edges[i]; });
-  if (a.classify) pack_words<unsigned>(a.dst + L.cls, n, t, nt, [&](unsigned long long i) { return a.cls[i]; });
 }
 
 }  // namespace

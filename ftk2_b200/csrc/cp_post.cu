@@ -16,6 +16,7 @@
 #include <algorithm>
 
 #include "cp_batch.h"
+#include "cp_pack.cuh"
 #include "cp_post.h"
 #include "cp_kuhn.cuh"
 #include "cp_pdl.cuh"
@@ -886,13 +887,6 @@ __global__ void __launch_bounds__(kSortThreads, 1)
 
 constexpr int kFinishThreads = 1024;  // what block_exclusive_scan takes
 
-template <typename W, typename F>
-__device__ __forceinline__ void finish_words(unsigned char* dst, unsigned long long n, unsigned long long t,
-                                             unsigned long long nt, F word) {
-  W* out = reinterpret_cast<W*>(dst);
-  for (unsigned long long i = t; i < n; i += nt) out[i] = word(i);
-}
-
 // a.dst null: device results only.  sh: 2 n words.  The first kFinishRoots
 // blocks find roots and offsets; the others send the arrays whose place does
 // not depend on them over PCIe meanwhile.
@@ -905,21 +899,12 @@ __global__ void __launch_bounds__(kFinishThreads) small_finish_kernel(PostBuffer
   const unsigned count = *B.count, n = min(count, B.cap), t = threadIdx.x;
   unsigned* const root = sh;
   unsigned* const off = sh + n;
-  const unsigned k = (unsigned)a.k;
-  // consecutive lanes store consecutive words, so a warp's stores leave as
-  // whole 128-byte lines
   if (blockIdx.x >= kFinishRoots) {
     const PackLayout L = pack_layout(n, 0, a.k, a.classify);
     if (!a.dst || count > a.cap || L.edges > a.dst_bytes) return;
     const unsigned w = (blockIdx.x - kFinishRoots) * kFinishThreads + t;
     const unsigned nw = (gridDim.x - kFinishRoots) * kFinishThreads;
-    finish_words<double>(a.dst + L.lam, (unsigned long long)n * k, w, nw,
-                         [&](unsigned long long i) { return k == 4 ? a.lam4[i] : a.lam4[i / k * 4 + i % k]; });
-    finish_words<unsigned long long>(a.dst + L.simplices, (unsigned long long)n * k, w, nw,
-                                     [&](unsigned long long i) { return a.simplices[i]; });
-    finish_words<float>(a.dst + L.bary, (unsigned long long)n * k, w, nw,
-                        [&](unsigned long long i) { return a.bary[i]; });
-    finish_words<float>(a.dst + L.scalar, n, w, nw, [&](unsigned long long i) { return a.scalar[i]; });
+    pack_records(a, L, n, w, nw);
     return;
   }
   const unsigned gt = blockIdx.x * kFinishThreads + t, nt = min(gridDim.x, kFinishRoots) * kFinishThreads;
@@ -999,9 +984,7 @@ __global__ void __launch_bounds__(kFinishThreads) small_finish_kernel(PostBuffer
     }
   }
   if (!pack) return;
-  finish_words<unsigned long long>(a.dst + L.track, n, gt, nt,
-                                   [&](unsigned long long i) { return a.want_edges ? root[i] : i; });
-  if (a.classify) finish_words<unsigned>(a.dst + L.cls, n, gt, nt, [&](unsigned long long i) { return a.cls[i]; });
+  pack_labels(a, L, n, gt, nt, [&](unsigned long long i) { return root[i]; });
 }
 
 bool post_small(const PostBuffers& B) { return B.cap <= kSmallPostCap && B.key_bits <= 64 - kIdxBits; }
@@ -1011,7 +994,8 @@ cudaError_t launch_post_finish(const PostBuffers& B, const PackArgs& a, cudaStre
   const size_t smem = 8 * (size_t)(B.cap ? B.cap : 1);
   cudaError_t e = cudaFuncSetAttribute(small_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        8 * (int)kSmallPostCap);
-  if (!e) e = launch_pdl(small_finish_kernel, std::max(B.num_sms > 0 ? B.num_sms : 148, (int)kFinishRoots + 1), kFinishThreads, smem, st, B, a);
+  const int grid = std::max(B.num_sms > 0 ? B.num_sms : 148, (int)kFinishRoots + 1);
+  if (!e) e = launch_pdl(small_finish_kernel, grid, kFinishThreads, smem, st, B, a);
   if (e) return e;
   *launches += 1;
   return cudaGetLastError();
