@@ -732,6 +732,7 @@ static ftk2b_status run_regular(ftk2b_ctx* ctx, const ftk2b_mesh_desc* mesh,
   memset(&cfg, 0, sizeof(cfg));
   cfg.Q = prm->sos_q;
   cfg.refined = prm->precision == FTK2B_PRECISION_REFINED;
+  cfg.num_sms = ctx->num_sms;
   cfg.cull_mode = ctx->cull_mode;  // 2 is resolved below, once the buffers exist
   if (ctx->stall_polls > 0) {  // the failure-path check runs in the fused cull
     cfg.stall_polls = ctx->stall_polls;

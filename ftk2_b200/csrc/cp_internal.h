@@ -86,6 +86,7 @@ struct ExtractConfig {
   int refined;                 // 1: report FP32 + one FP64 refinement step
   int tchunk;                  // corner time steps per block
   int tiles[3];                // tiles along x, y, z (z = 1 for 2D)
+  int num_sms;                 // of the device
   int skip_first_spatial;      // 1: no purely spatial simplices at local time 0
   int cull_mode;               // 0: per-vertex cull words only; 1: tile statistics first
   // > 0: failure-path check of cull mode 0: every block waits (a staged one

@@ -140,6 +140,7 @@ extern "C" ftk2b_status ftk2b_cp_features_noalloc(const ftk2b_mesh_desc* mesh,
   memset(&cfg, 0, sizeof(cfg));
   cfg.Q = sos_q;
   cfg.tchunk = (int)rm.ld[d - 1];
+  cudaDeviceGetAttribute(&cfg.num_sms, cudaDevAttrMultiProcessorCount, dev);
   cfg.tiles[0] = (int)((rm.ld[0] + TX - 1) / TX);
   cfg.tiles[1] = (int)((rm.ld[1] + TY - 1) / TY);
   cfg.tiles[2] = (d == 4) ? (int)((rm.ld[2] + TZ - 1) / TZ) : 1;
@@ -160,8 +161,6 @@ extern "C" ftk2b_status ftk2b_cp_features_noalloc(const ftk2b_mesh_desc* mesh,
   sink.cap = capacity;
 
   cudaStream_t cs = static_cast<cudaStream_t>(stream);
-  int num_sms = 148;
-  cudaDeviceGetAttribute(&num_sms, cudaDevAttrMultiProcessorCount, dev);
   // the shared scratch keeps the last call's contents: clear the counters
   if (cudaMemsetAsync(counters, 0, 4 * sizeof(unsigned), cs) != cudaSuccess ||
       cudaMemsetAsync(count, 0, sizeof(uint32_t), cs) != cudaSuccess) {
@@ -170,7 +169,7 @@ extern "C" ftk2b_status ftk2b_cp_features_noalloc(const ftk2b_mesh_desc* mesh,
   }
   const int f64 = field->dtype == FTK2B_F64;
   if (launch_extract_regular(f64, rm, fa, cfg, cq, counters + 1, cs, true, nullptr) != cudaSuccess ||
-      launch_refine_regular(f64, rm, fa, cfg, cq, sink, num_sms, cs) != cudaSuccess) {
+      launch_refine_regular(f64, rm, fa, cfg, cq, sink, cfg.num_sms, cs) != cudaSuccess) {
     cudaGetLastError();
     return FTK2B_CUDA_ERROR;
   }

@@ -38,7 +38,7 @@ __global__ void __launch_bounds__(kPackThreads) pack_kernel(PackArgs a) {
 }  // namespace
 
 cudaError_t launch_pack(const PackArgs& a, int num_sms, cudaStream_t st) {
-  const cudaError_t e = launch_pdl(pack_kernel, num_sms > 0 ? num_sms : 148, kPackThreads, 0, st, a);
+  const cudaError_t e = launch_pdl(pack_kernel, num_sms, kPackThreads, 0, st, a);
   return e ? e : cudaGetLastError();
 }
 

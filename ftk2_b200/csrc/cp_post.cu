@@ -994,7 +994,7 @@ cudaError_t launch_post_finish(const PostBuffers& B, const PackArgs& a, cudaStre
   const size_t smem = 8 * (size_t)(B.cap ? B.cap : 1);
   cudaError_t e = cudaFuncSetAttribute(small_finish_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        8 * (int)kSmallPostCap);
-  const int grid = std::max(B.num_sms > 0 ? B.num_sms : 148, (int)kFinishRoots + 1);
+  const int grid = std::max(B.num_sms, (int)kFinishRoots + 1);
   if (!e) e = launch_pdl(small_finish_kernel, grid, kFinishThreads, smem, st, B, a);
   if (e) return e;
   *launches += 1;
@@ -1005,7 +1005,7 @@ static cudaError_t launch_post_small(const RegularMesh& mesh, int nch, const Pos
                                      cudaStream_t st, unsigned long long* launches) {
   const unsigned cap = B.cap;
   const size_t key_smem = sizeof(unsigned long long) * (size_t)(cap ? cap : 1);
-  const int g = B.num_sms > 0 ? B.num_sms : 148;
+  const int g = B.num_sms;
   // always the most any call needs: another thread may be launching the same kernels
   constexpr int kMost = 8 * (int)kSmallPostCap;
   cudaError_t e = cudaFuncSetAttribute(small_sort_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kMost);
@@ -1113,7 +1113,7 @@ cudaError_t launch_post_batch(const BatchMesh* fm, const unsigned long long* kb,
     while (((unsigned long long)cap >> slog) + 1 > 8192ull) ++slog;
     const size_t smp = sizeof(unsigned long long) * (((size_t)cap >> slog) + 1 + (nf <= kBatchKbSmem ? nf : 0));
     cudaFuncSetAttribute(edges_batch_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smp);
-    edges_batch_warp_kernel<<<(B.num_sms > 0 ? B.num_sms : 148) * 2, 512, smp, st>>>(fm, kb, nf, skey, B.count, cap,
+    edges_batch_warp_kernel<<<B.num_sms * 2, 512, smp, st>>>(fm, kb, nf, skey, B.count, cap,
                                                                                       B.edge_cnt, B.edge_slots, slog);
   }
   scan_inplace_kernel<<<1, 1024, 0, st>>>(B.edge_cnt, cap, B.n_edges, B.count, nullptr);

@@ -702,12 +702,13 @@ __global__ void __launch_bounds__(kThreads, 2)
 // (8 rows a strip, fewer vertices computed twice but half the warps: 39.5); 64 x
 // 64 x 10 double: 11.6 -> 4.  Arrays that TMA could stage gain less but at every
 // size, so 2D+t has no staged form: 1024 x 768 x 12 float 49.5 -> 41.5, 2048^2 x
-// 16 287 -> 240, 4096^2 x 8 617 -> 460, 128 x 96 x 1000 1064 -> 63.  Chunks are long where strips alone give
-// kStripsWanted warps (a chunk's first slice is read twice) and short where they
-// do not (fewer steps in sequence); 32 to 128 warps an SM measure alike.
+// 16 287 -> 240, 4096^2 x 8 617 -> 460, 128 x 96 x 1000 1064 -> 63.  Chunks are
+// long where strips alone give kStripsWanted warps an SM (a chunk's first slice is
+// read twice) and short where they do not (fewer steps in sequence); 32 to 128
+// warps an SM measure alike.
 constexpr int kStripRows = 4;
 constexpr int kStripWarps = 8;             // warps a block
-constexpr int kStripsWanted = 64 * 148;    // warps of the launch, at least where the mesh has them
+constexpr int kStripsWanted = 64;          // warps an SM, at least where the mesh has them
 
 template <typename T>
 __global__ void __launch_bounds__(kStripWarps * 32, 3) strip_cull_kernel(RegularMesh mesh, FieldAccess fa,
@@ -2707,7 +2708,8 @@ static cudaError_t launch_t(const RegularMesh& mesh, const FieldAccess& fa, cons
   if constexpr (D == 3) {
     if (used_tma) *used_tma = 0;
     const long long sx = (mesh.ld[0] + 30) / 31, sy = (mesh.ld[1] + kStripRows - 1) / kStripRows;
-    long long nch = std::min<long long>(lt, (kStripsWanted + sx * sy - 1) / (sx * sy));
+    const long long wanted = (long long)kStripsWanted * cfg.num_sms;
+    long long nch = std::min<long long>(lt, std::max<long long>(1, (wanted + sx * sy - 1) / (sx * sy)));
     if (cfg.tchunk < lt) nch = std::max<long long>(nch, nchunks);  // the caller's chunk length
     const long long tchunk = (lt + nch - 1) / nch;
     nch = (lt + tchunk - 1) / tchunk;

@@ -258,6 +258,7 @@ ftk2b_status push_regular(ftk2b_stream* s) {
   memset(&cfg, 0, sizeof(cfg));
   cfg.Q = s->prm.sos_q;
   cfg.refined = s->prm.precision == FTK2B_PRECISION_REFINED;
+  cfg.num_sms = ctx->num_sms;
   cfg.tchunk = (int)lt;
   cfg.skip_first_spatial = T > 0;
   cfg.cull_mode = ctx->cull_mode;  // 2 is resolved below, once the buffers exist
