@@ -9,6 +9,7 @@ import this module; the product never does.
 from __future__ import annotations
 
 import ctypes as C
+import itertools
 import os
 from dataclasses import dataclass
 
@@ -402,13 +403,55 @@ class OrcTracked(C.Structure):
     ]
 
 
+def _restated_tracked(vec: np.ndarray, attrs):
+    """run_reference_tracked by the restatement: its extruded mesh over the
+    Kuhn simplices of the spatial grid, whose vertex ids step by
+    grid_index_to_id(global dims) per timestep (mesh.hpp:544-560), and the
+    attributes of engine.hpp:1143-1199 in the field's precision, operation by
+    operation."""
+    T = vec.dtype.type
+    nt, m = vec.shape[0], vec.shape[-1]
+    sp = vec.shape[1:-1][::-1]  # Fortran spatial dims
+    stride = np.cumprod([1] + list(sp[:-1])).astype(np.int64)
+    ids = np.arange(int(np.prod(sp)), dtype=np.int64).reshape(sp[::-1])
+    low = ids[tuple(slice(0, d - 1) for d in sp[::-1])].ravel()
+    cells = np.concatenate([np.stack([low + sum(stride[a] for a in p[:k]) for k in range(m + 1)], 1)
+                            for p in itertools.permutations(range(m))]).astype(np.uint64)
+    step = int(sum(d * int(k) for d, k in zip(sp, stride)))
+    arrays = np.zeros((m, nt, step), dtype=vec.dtype)
+    arrays[:, :, :ids.size] = np.moveaxis(vec.reshape(nt, ids.size, m), 2, 0)
+    keep: list = []
+    mesh = make_extruded_mesh(np.zeros((step, 3)), cells, nt - 1, keep)
+    r = run_restatement(mesh, make_field([a.ravel() for a in arrays], LAYOUT_PER_VERTEX, m, keep=keep))
+    out = np.zeros((len(r.track_id), 16), dtype=np.float32)
+    for slot, (arr, magnitude, component) in enumerate(attrs):
+        arr = np.asarray(arr, dtype=vec.dtype)
+        for i, simplex in enumerate(r.simplices):
+            acc = T(0)
+            for v, vid in enumerate(int(x) for x in simplex):
+                at = (vid // step,) + tuple(int(x) for x in np.unravel_index(vid % step, sp[::-1]))  # t, [z,] y, x
+                if magnitude:
+                    sq = T(0)
+                    for c in arr[at]:
+                        sq = T(sq + T(c * c))
+                    val = T(np.sqrt(sq))
+                else:
+                    val = T(arr[at][component] if component >= 0 else arr[at])
+                acc = T(acc + T(T(r.bary[i, v]) * val))
+            out[i, slot] = np.float32(acc)
+    return r, out
+
+
 def run_reference_tracked(vec: np.ndarray, attrs=()):
     """The reference high-level caller's critical-point flow: its engine on
     ExtrudedSimplicialMesh(RegularSimplicialMesh(spatial dims), nt - 1) with
     the multicomponent array ``vec`` (C-order shape (nt, [nz,] ny, nx, m), the
     bytes of a Fortran [m, nx, ny, (nz,) nt] array) and attributes given as
     (array, magnitude, component) with arrays in C order (reversed Fortran
-    shape).  Returns (CPResult, attributes (n, 16) float32)."""
+    shape).  Returns (CPResult, attributes (n, 16) float32).  Where the
+    reference is not built, the same flow by the exact C restatement."""
+    if not ref_available():
+        return _restated_tracked(np.ascontiguousarray(vec), attrs)
     lib = _load(REF_LIB, "ftk2ref")
     if not hasattr(lib, "_tracked_bound"):
         lib.ftk2ref_run_tracked.argtypes = [C.POINTER(OrcTracked), C.POINTER(OrcResult),
