@@ -395,8 +395,11 @@ ftk2b_status run_batch(ftk2b_ctx* ctx, uint32_t n, const ftk2b_mesh_desc* meshes
       bc.ccap_hint = ccap;
       continue;
     }
-    if (h[kCountFeatures] > cap || h[kCountEdges] > edge_cap) {
-      uint64_t want = (uint64_t)h[kCountFeatures] + h[kCountFeatures] / 4 + 1024;
+    // the inside list holds cap entries too; the features are only those of the
+    // simplices it held, so a longer list shows in its own count
+    const uint64_t most = std::max(h[kCountFeatures], h[kCountAcc]);
+    if (most > cap || h[kCountEdges] > edge_cap) {
+      uint64_t want = most + most / 4 + 1024;
       const uint64_t want_e = ((uint64_t)h[kCountEdges] + 1) / 2 + 1024;
       if (want_e > want) want = want_e;
       if (want > 0x7FFFFFF0ull) return bfail(ctx, FTK2B_OVERFLOW_RETRY, "feature count exceeds 2^31");

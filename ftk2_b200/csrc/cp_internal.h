@@ -146,7 +146,7 @@ struct RefineStage {
   unsigned* big_list;            // candidates listed for the 128-bit path
   unsigned* big_count;
   unsigned long long* acc;       // simplices inside by the fast path: candidate << 8 | chain
-  unsigned* acc_count;           // may exceed acc_cap (then the call reports overflow)
+  unsigned* acc_count;           // may exceed acc_cap (the host sees that and runs the call again)
   unsigned acc_cap;
   unsigned* count;   // simplices tested (reported after the run)
   unsigned* err;     // the call's error word (bounds checks of the checked build)

@@ -2318,7 +2318,6 @@ __global__ void __launch_bounds__(kRefineWarps * 32) batch_solve_kernel(const Ba
   __syncthreads();
   const int lane = threadIdx.x & 31;
   const unsigned na = *rs.acc_count;
-  if (blockIdx.x == 0 && threadIdx.x == 0 && na > rs.acc_cap) atomicMax(sink.count, na);
   const unsigned n = min(na, rs.acc_cap);
   const unsigned stride = gridDim.x * blockDim.x;
   for (unsigned base = blockIdx.x * blockDim.x; base < n; base += stride) {
