@@ -1107,14 +1107,21 @@ cudaError_t launch_post_batch(const BatchMesh* fm, const unsigned long long* kb,
   expand_batch_kernel<<<g, 256, 0, st>>>(fm, kb, nf, skey, B.count, cap, B.bary4_sorted, B.simplices, B.bary);
   batch_bounds_kernel<<<(nf + 256) / 256, 256, 0, st>>>(kb, nf, skey, B.count, cap, fbase);
   // a persistent grid: every block copies the face tables and a sample of
-  // the sorted keys (every 2^slog-th, at most 8192 entries) into shared memory once
+  // the sorted keys (every 2^slog-th, at most kBatchSample entries) into shared
+  // memory once
   {
+    constexpr unsigned long long kBatchSample = 8192;
     int slog = 4;
-    while (((unsigned long long)cap >> slog) + 1 > 8192ull) ++slog;
+    while (((unsigned long long)cap >> slog) + 1 > kBatchSample) ++slog;
     const size_t smp = sizeof(unsigned long long) * (((size_t)cap >> slog) + 1 + (nf <= kBatchKbSmem ? nf : 0));
-    cudaFuncSetAttribute(edges_batch_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smp);
-    edges_batch_warp_kernel<<<B.num_sms * 2, 512, smp, st>>>(fm, kb, nf, skey, B.count, cap,
-                                                                                      B.edge_cnt, B.edge_slots, slog);
+    // always the most any batch needs: another thread may be launching the same
+    // kernel; the ones behind it read its counts, so nothing follows a failure
+    cudaError_t e = cudaFuncSetAttribute(edges_batch_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         8 * ((int)kBatchSample + kBatchKbSmem));
+    if (e) return e;
+    edges_batch_warp_kernel<<<B.num_sms * 2, 512, smp, st>>>(fm, kb, nf, skey, B.count, cap, B.edge_cnt, B.edge_slots,
+                                                            slog);
+    if ((e = cudaGetLastError())) return e;
   }
   scan_inplace_kernel<<<1, 1024, 0, st>>>(B.edge_cnt, cap, B.n_edges, B.count, nullptr);
   edges_compact_kernel<<<g, 256, 0, st>>>(B.count, cap, B.edge_cnt, B.n_edges, B.edge_slots, B.edges, B.edge_cap);
