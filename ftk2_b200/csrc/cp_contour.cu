@@ -435,6 +435,32 @@ __global__ void __launch_bounds__(kCtThreads) ct_emit_kernel(
   }
 }
 
+// The first crossing edge (v, v + e) of every vertex starts at an edge of a lower
+// vertex w = v - a, a an axis outside e: in the triangle (w, w + a, w + a + e)
+// exactly one of (w, a) and (w, a + e) crosses too.  Most edges then hang in
+// one long tree before the joins, which otherwise meet everywhere at once.
+__global__ void __launch_bounds__(kCtThreads) ct_hook_kernel(CtGeom g, const unsigned short* __restrict__ mask,
+                                                             const unsigned* __restrict__ voff,
+                                                             unsigned* __restrict__ parent) {
+  const unsigned long long i0 = blockIdx.x * (unsigned long long)kCtBlock + threadIdx.x;
+#pragma unroll
+  for (int j = 0; j < kCtPer; ++j) {
+    const unsigned long long i = i0 + j * kCtThreads;
+    const unsigned m = i < g.nv ? mask[i] : 0u;
+    if (!m) continue;
+    unsigned long long c[4];
+    ct_coords(g, i, c);
+    const unsigned e = __ffs(m);
+    for (int k = g.d - 1; k >= 0; --k) {
+      if (((e >> k) & 1u) || c[k] == 0) continue;
+      const unsigned long long w = i - g.lstr[k];
+      const unsigned mw = mask[w], a = 1u << k;
+      parent[voff[i]] = voff[w] + ct_below(mw, (mw >> (a - 1)) & 1u ? a : a | e);
+      break;
+    }
+  }
+}
+
 // Joins the crossing edges of every mesh triangle that has two.  The crossing
 // edges of a simplex hang together through its triangles, so this gives the
 // components of the cells; a triangle (v, v + a, v + b), a a subset of b, is met
@@ -449,15 +475,23 @@ __global__ void __launch_bounds__(kCtThreads) ct_emit_kernel(
 // of one share and take its items in turn, up to one item a thread.  White noise
 // on 16 x 16 x 4 vertices (2,800 edges): 498 us with one block a share, 33 so; a
 // whole level set of 16^3 x 3 noise 2251 -> 270 us on the device, of 96^3 x 6
-// blobs (936,000 edges) 702 -> 660 (16 an SM: 703).  Hooking the vertices' first
-// edges ahead, joining a sample and flattening the trees in between paid for four
-// more launches with one block a share, but not so.  Joining every cell's nodes
+// blobs (936,000 edges) 702 -> 660 (16 an SM: 703).  Joining every cell's nodes
 // from the cells kernel took four times as many unions from divergent lanes.
+//
+// From kCtHooked edges on, threads that join the same two large trees queue on
+// their roots: there the first edges are hooked ahead and the trees flattened,
+// one vertex of kCtSample joins along its axes, the trees (few by then) are
+// flattened again, and the rest mostly finds equal parents.  Whole level sets with
+// and without: 128^3 x 16 (9.0 million edges) 4.68 / 5.07 ms, 128^3 x 8 (4.4)
+// 2.37 / 2.57, 24^3 x 16 noise (1.5) 1.22 / 1.22, 96^3 x 6 (0.94) 0.66 / 0.66, 48^3
+// x 4 (0.15) 0.26 / 0.23, 1000 x 700 x 12 (0.06) 0.28 / 0.24.
 constexpr unsigned kJoinBlocks = 64;
+constexpr unsigned kCtHooked = 1u << 20;
+constexpr unsigned kCtSample = 4;
 
 __global__ void __launch_bounds__(kCtThreads) ct_join_kernel(CtGeom g, const unsigned short* __restrict__ mask,
                                                              const unsigned* __restrict__ voff, unsigned* parent,
-                                                             unsigned* err) {
+                                                             unsigned* err, bool sample) {
   __shared__ unsigned short s_vert[kCtBlock], s_mask[kCtBlock];
   __shared__ unsigned long long s_off[16];
   if (threadIdx.x < 16) s_off[threadIdx.x] = ct_corner_step(g, threadIdx.x);
@@ -479,8 +513,10 @@ __global__ void __launch_bounds__(kCtThreads) ct_join_kernel(CtGeom g, const uns
     }
   __syncthreads();
   const unsigned diag = (1u << g.d) - 1u;
-  for (unsigned k = blockIdx.y * kCtThreads + threadIdx.x; k < n * diag; k += gridDim.y * kCtThreads) {
-    const unsigned z = k / diag, mv = s_mask[z], a = k % diag + 1;
+  const unsigned per = sample ? (unsigned)g.d : diag, step = sample ? kCtSample : 1u;
+  for (unsigned k = blockIdx.y * kCtThreads + threadIdx.x; k < (n + step - 1) / step * per;
+       k += gridDim.y * kCtThreads) {
+    const unsigned z = k / per * step, mv = s_mask[z], a = sample ? 1u << k % per : k % per + 1;
     const bool edge = (mv >> (a - 1)) & 1u;
     unsigned with = 0;  // no edge to a: the corners b above a that have one
     if (!edge) {
@@ -1026,7 +1062,15 @@ ftk2b_status run_contour(ftk2b_ctx* ctx, const CtGeom& g, const void* field, T t
   if (n && g.ncube) {
     const unsigned long long most = kCtPer * ((1ull << d) - 1);  // one item a thread
     const dim3 grid((unsigned)nblk, (unsigned)std::min(most, (kJoinBlocks * sms + nblk - 1) / nblk));
-    ct_join_kernel<<<grid, kCtThreads, 0, st>>>(g, mask, voff, parent, counts + 3);
+    if (n >= kCtHooked) {
+      const unsigned fgrid = grid_of(n, 256, 8ull * sms);
+      ct_hook_kernel<<<(unsigned)nblk, kCtThreads, 0, st>>>(g, mask, voff, parent);
+      uf_flatten_kernel<<<fgrid, 256, 0, st>>>(parent, n);
+      ct_join_kernel<<<grid, kCtThreads, 0, st>>>(g, mask, voff, parent, counts + 3, true);
+      uf_flatten_kernel<<<fgrid, 256, 0, st>>>(parent, n);
+      ctx->launches += 4;
+    }
+    ct_join_kernel<<<grid, kCtThreads, 0, st>>>(g, mask, voff, parent, counts + 3, false);
     ctx->launches += 1;
   }
   ctx->launches += 1;

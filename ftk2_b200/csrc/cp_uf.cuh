@@ -43,4 +43,12 @@ __device__ __forceinline__ void uf_unite_flat(unsigned* parent, unsigned a, unsi
   if (__ldcg(&parent[a]) != __ldcg(&parent[b])) uf_unite(parent, a, b, err);
 }
 
+// Every element at its root (between launches that join).
+static __global__ void uf_flatten_kernel(unsigned* parent, unsigned n) {
+  for (unsigned i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+    const unsigned r = uf_root(parent, i);
+    if (r != i) atomicMin(&parent[i], r);
+  }
+}
+
 }  // namespace ftk2b

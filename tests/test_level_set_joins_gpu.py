@@ -33,3 +33,31 @@ def test_window_of_a_large_mesh(ctx, big, window):
     part = ctx.contour(api.regular_mesh_desc(window, off, big), noise, 0.0, Q)
     assert len(part.track_id) > 1000
     assert_same(as_dict(whole), as_dict(part))
+
+
+def _labels(n, cells):
+    """Smallest member of every node's component under the cells."""
+    label = np.arange(n)
+    while True:
+        low = label[cells].min(1)
+        new = label.copy()
+        for j in range(cells.shape[1]):
+            np.minimum.at(new, cells[:, j], low)
+            np.minimum.at(new, label[cells[:, j]], low)
+        while not np.array_equal(new, new[new]):
+            new = new[new]
+        if np.array_equal(new, label):
+            return label
+        label = new
+
+
+@pytest.mark.parametrize("dims,above", [([270, 230, 5], False), ([340, 270, 6], True), ([32, 30, 28, 9], True)])
+def test_tracks_around_the_hooked_size(ctx, dims, above):
+    """Tracks of noise below and above the 2^20 edges from which the trees are
+    hooked and flattened ahead, against the components of the call's own cells
+    (compared with the restatement elsewhere)."""
+    f = np.random.default_rng(23).standard_normal(tuple(dims[::-1])).astype(np.float32)
+    r = ctx.contour(api.regular_mesh_desc(dims), f, 0.6, Q)
+    assert (len(r.track_id) >= 1 << 20) == above
+    assert np.array_equal(r.track_id, _labels(len(r.track_id), r.cells.astype(np.int64)))
+    assert r.n_tracks == len(np.unique(r.track_id)) > 1
