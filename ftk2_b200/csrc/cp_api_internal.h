@@ -90,7 +90,8 @@ struct ExtCache {
   }
 };
 
-// One cached pair of instantiated graphs of the regular-mesh pipeline.
+// A regular-mesh call seen before and, from its second time on, its instantiated
+// graph (or pair of graphs).
 struct GraphEntry {
   RegularGraphKey key;
   unsigned long long gen = 0;      // buffer generation at capture
