@@ -5,22 +5,24 @@
 // device pipeline:
 //
 //   ct_sign    one pass over the field: the simulation-of-simplicity sign of
-//              value - threshold at every vertex (sos.hpp:12-20), one byte
+//              value - threshold at every vertex (sos.hpp:12-20), one bit
 //   ct_mask    per vertex c, the directions e in {0,1}^d \ 0 whose edge to
 //              c + e crosses (the signs differ, origin_inside<1>,
-//              sos.hpp:211-220), and per-block counts
+//              sos.hpp:211-220), per-block counts, and the hypercubes whose
+//              corners differ in sign
 //   scan       block offsets.  Every Freudenthal edge joins some c to c + e,
 //              so the edges in simplex order are the (c, e) pairs in vertex
 //              order with e read as a binary number, x lowest: a feature's
 //              rank is its block offset plus a prefix count, no sort needed
 //   ct_emit    vertex ids and barycentrics of every feature at its rank
+//   ct_join    the two crossing edges of every crossed triangle united
 //   ct_first   (2D+t) the position at which the reference's sequential
 //              patching first meets each node whose edge starts on an upper
 //              boundary face (those are numbered in meeting order, after the
 //              first pass's nodes, and 2D+t quads are cut along the diagonal
 //              from their smallest-numbered node)
-//   ct_cells   marching tetrahedra / pentatopes over every Kuhn simplex of
-//              every hypercube: manifold cells, union-find hooks
+//   ct_cells   marching tetrahedra / pentatopes over every Kuhn simplex of the
+//              listed hypercubes: manifold cells
 //   buckets    cells into lexicographic order: counted and scattered by
 //              their leading node, each bucket's few rows sorted, duplicates
 //              flagged

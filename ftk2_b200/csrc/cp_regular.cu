@@ -697,7 +697,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 // in flight meanwhile, its right neighbour's words come by a shuffle.  Values
 // are read straight from the arrays (of a double only the high word), so every
 // layout, stride and alignment takes the same path and no step waits for a
-// block.  Bound by issue: some 60 instructions a vertex, 150 with the slice
+// block.  Bound by issue: 74 thread instructions a vertex, 150 with the slice
 // staged in shared memory.  1021 x 765 x 12 float in two arrays: 62.5 -> 36 us
 // (8 rows a strip, fewer vertices computed twice but half the warps: 39.5); 64 x
 // 64 x 10 double: 11.6 -> 4.  Arrays that TMA could stage gain less but at every
