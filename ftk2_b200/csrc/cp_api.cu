@@ -560,7 +560,7 @@ ftk2b_status ftk2b::ensure_feature_buffers(ftk2b_ctx* ctx, unsigned cap, unsigne
   CUDA_TRY(ctx, ctx->edges.ensure(sizeof(unsigned) * 2 * (size_t)edge_cap));
   CUDA_TRY(ctx, ctx->edge_slots.ensure(sizeof(unsigned) * 8 * (size_t)cap));
   CUDA_TRY(ctx, ctx->counters.ensure(sizeof(unsigned) * kNumCounters));
-  const int grid = ctx->sort_grid(cap);
+  const int grid = ctx->chain_sort_grid(cap);
   CUDA_TRY(ctx, ctx->hist.ensure(sizeof(unsigned) * 256 * (size_t)grid));
   return FTK2B_OK;
 }
@@ -571,7 +571,7 @@ PostBuffers ftk2b_ctx::post_buffers(unsigned cap_, unsigned edge_cap_, int key_b
   B.cap = cap_;
   B.edge_cap = edge_cap_;
   B.key_bits = key_bits;
-  B.sort_grid = sort_grid(cap_);
+  B.sort_grid = chain_sort_grid(cap_);
   B.num_sms = num_sms;
   B.key = (unsigned long long*)key.p;
   B.lam = (double*)lam.p;

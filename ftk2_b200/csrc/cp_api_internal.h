@@ -255,6 +255,16 @@ struct ftk2b_ctx {
     if (g > 2 * num_sms) g = 2 * num_sms;
     return g;
   }
+  // the same for the regular chain, whose capacity follows the feature count:
+  // up to 64 blocks at half the keys each, since a scatter pass is a block's
+  // serial walk over its keys. Whole call on 12x12x12x3 noise, 21,422
+  // features: 176 us with the line above, 164 us with this one; on 20x20x20x3
+  // (109,300) 339 and 336. Past 64 blocks the digit scan costs what the pass
+  // gains: 40x40x40x3 (939,692), no edges, 534 us with 287 blocks, 546 with 296.
+  int chain_sort_grid(unsigned cap) const {
+    const int g = sort_grid(cap), h = (int)(cap / 2048u) < 64 ? (int)(cap / 2048u) : 64;
+    return h > g ? h : g;
+  }
   void release_all();
   std::vector<ftk2b::DevBuf*> all_bufs();
   ftk2b::PostBuffers post_buffers(unsigned cap, unsigned edge_cap, int key_bits);
